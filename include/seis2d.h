@@ -116,14 +116,20 @@ typedef struct {
     int kernel_launches;     /* launches of the library's own kernels         */
     int graph_used;          /* 1 if the loop ran as a CUDA graph             */
     int grad_segment;        /* s2d_gradient: checkpoint interval used (steps) */
-    int variant, block, stages;  /* launch configuration of the time loop     */
+    int variant, block, stages;  /* launch configuration of the per-step kernels
+                                (shots in the on-chip loop use none: one
+                                launch counts in kernel_launches for a whole
+                                run of their steps)                           */
     int seg_len;             /* columns per warp task (first model group)     */
-    int autotuned;           /* 1 if this call ran the autotuner's trials     */
+    int autotuned;           /* 1 if this call settled the shape's configuration:
+                                the autotuner's trials, or none for a batch that
+                                runs on chip altogether                       */
     double alg_bytes;        /* s2d_forward: algorithmic DRAM bytes of the loop:
                                 44 B per cell and pass over the state, 36 B
                                 where both pressure dampings are 1 (the cell
                                 carries p alone); a pass is one FD step, or
-                                two with the two-step variant                 */
+                                two with the two-step variant, or a whole run
+                                in the on-chip loop                           */
     double sweep_ms;         /* s2d_gradient: CUDA-event time of the forward
                                 sweep (checkpoint saves included)              */
     double recompute_ms;     /* s2d_gradient: the recomputes that keep the
@@ -213,12 +219,22 @@ S2D_API const char *s2d_last_error(const void *ctx);
  *                 inputs copied into shared memory (cp.async) 1 / 2 columns
  *                 ahead, or 15: 3 blocks per SM with the per-shot inputs
  *                 copied 2 columns ahead; every form computes the same bits
+ *   "on_chip"     1 (default): 4th-order grids whose state fits the GPU's
+ *                 registers and shared memory (up to about 1.2 M padded cells)
+ *                 run all their steps in one cooperative launch per shot or
+ *                 wave of shots where that is the faster way (s2d_forward,
+ *                 the forward sweep of s2d_gradient, s2d_forward_static; not
+ *                 with S2D_NO_GRAPH or "autotune" 0); 0: one launch per step.
+ *                 The results are the same bits.
+ *   "on_chip_shape" block shape of that loop, warps * 100 + columns per warp
+ *                 (403, 404, 803 .. 810), 0 = the fastest for the grid (default)
  *   "grad_segment" s2d_gradient checkpoint interval in FD steps, 0 = the
  *                 longest that fits in free device memory (default)
  *   "inject_wait_fault"  test knob: >= 0 makes every warp skip the copies of
  *                 that pipeline iteration of its first task (bulk-copy and TMA
  *                 kernels), or block 0 skip its arrival at the grid barrier
- *                 after that step (persistent kernel), so a bounded wait runs
+ *                 after that step (persistent kernel), or block 0 not publish
+ *                 that step's halo (on-chip loop), so a bounded wait runs
  *                 out (no fault, no hang); -1 (default) disables
  * Options apply to the next s2d_forward call.
  */
@@ -442,7 +458,8 @@ S2D_API int s2d_run_jobcard_rank(const char *jobcard_path, int device, int nb, i
  * otherwise host pointers.  Any other bit (S2D_MODEL_FREE_SURFACE and
  * S2D_MODEL_ORDER8 included: this entry has neither option) returns
  * S2D_ERR_ARG.  stream: a cudaStream_t, NULL for the legacy default stream;
- * the call returns when the shot is done.  A failed device self-check (builds
+ * the call returns when the shot is done.  A bounded wait of the on-chip loop
+ * that runs out returns S2D_ERR_TIMEOUT.  A failed device self-check (builds
  * with S2D_DEVICE_CHECKS) returns S2D_ERR_CUDA.  errbuf (optional, errlen
  * bytes) receives a message on failure.
  *

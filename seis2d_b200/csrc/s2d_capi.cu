@@ -95,6 +95,12 @@ struct Batch {
     std::vector<int> group_nnz;      // padded rows of each group's model
     int cur = 0;                     // state buffer (parity) holding step kt_next
     std::vector<long> layout;        // launch configuration the groups are laid out for
+    std::vector<char> chip;          // groups the on-chip loop runs (they get no tasks)
+    bool all_chip() const {
+        for (char f : chip)
+            if (!f) return false;
+        return !chip.empty();
+    }
     std::vector<std::unique_ptr<DevBuf>> state;   // 8 per shot
     std::vector<std::unique_ptr<DevBuf>> aux;     // amp tables, receiver tables
     DevBuf shots_d, groups_d;
@@ -173,6 +179,10 @@ struct Ctx {
     int last_segment = 0;     // interval the last gradient call used
     DevBuf dev_err;           // device error word of the step kernels
     DevBuf bar_d;             // grid-barrier counter of the persistent step kernel
+    int opt_on_chip = 1;      // on-chip time loop for the grids that fit
+    int opt_chip_shape = 0;   // its block shape (warps * 100 + columns per warp), 0 = the fastest
+    DevBuf res_frames;        // on-chip time loop: the blocks' frames
+    DevBuf res_shots;         // and the shots of its launches
     // Launch-argument block read by every step launch, and the graphs of step
     // launches captured against it (by step count and launch configuration);
     // kept for the context's lifetime, so later runs replay them.
@@ -308,7 +318,7 @@ int launch_config(Ctx *c, long max_tasks, LaunchCfg *out, int variant, int block
 // Key of a batch's shape for the autotuner: run mode and, per model group,
 // padded grid and shot count.
 std::vector<long> tune_key(const Ctx *c, const Batch &b) {
-    std::vector<long> k = {b.plain ? 1L : 0L, (long)c->sm_count, b.order8 ? 8L : 4L};
+    std::vector<long> k = {b.plain ? 1L : 0L, (long)c->sm_count, b.order8 ? 8L : 4L, b.all_chip() ? 1L : 0L};
     for (size_t g = 0; g < b.groups.size(); ++g) {
         k.push_back(b.group_nnx[g]);
         k.push_back(b.group_nnz[g]);
@@ -341,8 +351,9 @@ int base_config(Ctx *c, const Batch &b, LaunchCfg *out, bool *tuned = nullptr) {
 // `key` differs from the layout in place.
 // With `tma` a task is a CTA's: kTmaWarps (shot, strip) pairs of a group
 // over one segment, and `resident_warps` counts resident CTAs.
-int layout_groups_for(Ctx *c, Batch &b, long resident_warps, const std::vector<long> &key, bool ts = false,
+int layout_groups_for(Ctx *c, Batch &b, long resident_warps, std::vector<long> key, bool ts = false,
                       bool tma = false) {
+    for (char f : b.chip) key.push_back(f);
     if (b.layout == key) return S2D_OK;
     for (size_t gi = 0; gi < b.groups.size(); ++gi)
         b.groups[gi].nstrips = ts ? num_strips_ts(b.group_nnz[gi]) : num_strips(b.group_nnz[gi]);
@@ -350,7 +361,8 @@ int layout_groups_for(Ctx *c, Batch &b, long resident_warps, const std::vector<l
         return tma ? (long)tma_blocks(nshots, g.nstrips) : (long)nshots * g.nstrips;
     };
     long per_seg_total = 0;
-    for (auto &g : b.groups) per_seg_total += per_seg(g, g.nshots);
+    for (size_t gi = 0; gi < b.groups.size(); ++gi)
+        if (!b.chip[gi]) per_seg_total += per_seg(b.groups[gi], b.groups[gi].nshots);
     long max_tasks = 0;
     int task = 0;
     for (size_t gi = 0; gi < b.groups.size(); ++gi) {
@@ -360,7 +372,7 @@ int layout_groups_for(Ctx *c, Batch &b, long resident_warps, const std::vector<l
         const long tasks_per_seg = b.plain ? per_seg(g, 1) : per_seg_total;
         g.seg_len = c->opt_seg_len > 0 ? std::min(c->opt_seg_len, nnx)
                                        : choose_seg_len(nnx, tasks_per_seg, resident_warps, ts ? 12 : 6);
-        g.nsegs = (nnx + g.seg_len - 1) / g.seg_len;
+        g.nsegs = b.chip[gi] ? 0 : (nnx + g.seg_len - 1) / g.seg_len;
         if (b.plain) {
             g.task_begin = 0;
             max_tasks = std::max<long>(max_tasks, per_seg(g, 1) * g.nsegs);
@@ -386,7 +398,6 @@ int layout_groups(Ctx *c, Batch &b, const LaunchCfg &lc) {
     // the two-step kernel and its one-step companion share one layout
     const int v = lc.variant == kVariantTs1 ? kVariantTs2 : lc.variant;
     const std::vector<long> key = {v, lc.block, lc.stages, c->opt_seg_len};
-    if (b.layout == key) return S2D_OK;
     // resident warps of the configuration (its grid when the work is smaller);
     // resident CTAs for the TMA kernel, whose tasks are CTA tasks
     LaunchCfg full;
@@ -423,43 +434,6 @@ int step_graph(Ctx *c, const LaunchCfg &lc, int n, cudaGraphExec_t *out) {
     }
     *out = it->second;
     return S2D_OK;
-}
-
-// Rows whose coefficients are the interior constants (see ShotDev::zfast_lo):
-// damp1a = damp1b = 1, kz*damp1a1 = kz*damp1b1 = (float)kz, rows [2, nnz-3].
-void fast_rows(const Model &m, float fd_dt, int *lo, int *hi, float *kz) {
-    const double dtdz = (double)(fd_dt * (1.0f / m.dz));  // as build_coef forms it
-    const float kzi = (float)(dtdz * 1.0f);
-    auto ok = [&](int r) {
-        return r >= 2 && r <= m.nnz - 3 && m.damp1a[r] == 1.0f && m.damp1b[r] == 1.0f &&
-               (float)(dtdz * m.damp1a1[r]) == kzi && (float)(dtdz * m.damp1b1[r]) == kzi;
-    };
-    int a = 0;
-    while (a < m.nnz && !ok(a)) ++a;
-    int b = a;
-    while (b < m.nnz && ok(b)) ++b;
-    *lo = a;
-    *hi = b;  // empty when a == b
-    *kz = kzi;
-}
-
-// Columns whose coefficients are the interior constants (ShotDev::xfast_lo):
-// damp2a = damp2b = 1, kx*damp2a1 = kx*damp2b1 = (float)kx and both operator
-// pairs (a0, a1), columns [2, nnx-3].
-void fast_cols(const Model &m, float fd_dt, int *lo, int *hi, float *kx) {
-    const double dtdx = (double)(fd_dt * (1.0f / m.dx));  // as build_coef forms it
-    const float kxi = (float)(dtdx * 1.0f);
-    auto ok = [&](int x) {
-        return x >= 2 && x <= m.nnx - 3 && m.damp2a[x] == 1.0f && m.damp2b[x] == 1.0f &&
-               (float)(dtdx * m.damp2a1[x]) == kxi && (float)(dtdx * m.damp2b1[x]) == kxi;
-    };
-    int a = 0;
-    while (a < m.nnx && !ok(a)) ++a;
-    int b = a;
-    while (b < m.nnx && ok(b)) ++b;
-    *lo = a;
-    *hi = b;  // empty when a == b
-    *kx = kxi;
 }
 
 // One pass over `nsteps` FD steps starting at kt_begin, for the launch
@@ -536,6 +510,72 @@ int run_loop(Ctx *c, Batch &b, const LaunchCfg &lc, StepArgs args, int kt_begin,
         b.cur ^= 1;
     }
     return S2D_OK;
+}
+
+// Whether the on-chip loop takes the shots of group g of the batch: its grid
+// fits the chip and the loop's estimate beats the per-step kernels', which
+// take about 7.4 us per step at least (launch and latency of one short task)
+// and run at about 100 Gcell/s (a batch) or 52 (single 1301 x 501 shots, one
+// after another).
+bool on_chip_group(const Ctx *c, const Batch &b, size_t g, ResPlan *pl) {
+    const int n = b.groups[g].nshots;
+    if (!resident_plan(c->sm_count, b.group_nnx[g], b.group_nnz[g], n, b.plain, c->opt_chip_shape, pl)) return false;
+    if (c->opt_chip_shape) return true;
+    const double cells = (double)b.group_nnx[g] * b.group_nnz[g];
+    const double us = b.plain ? n * std::max(7.4, cells / 0.6e5) : std::max(7.4, n * cells / 1.0e5);
+    return pl->step_us < 0.9 * us;
+}
+
+// Decide which groups of the batch the on-chip loop runs in this call, when
+// it has at least `nsteps` >= 8 of them to run (a launch loads and writes the
+// whole state once).  Returns how many.
+int choose_on_chip(Ctx *c, Batch &b, int nsteps, bool use_graph, std::vector<ResPlan> *plans) {
+    plans->assign(b.groups.size(), ResPlan());
+    b.chip.assign(b.groups.size(), 0);
+    if (!c->opt_on_chip || !c->opt_autotune || !use_graph || b.order8 || nsteps < 8) return 0;
+    int n = 0;
+    for (size_t g = 0; g < b.groups.size(); ++g) n += b.chip[g] = on_chip_group(c, b, g, &(*plans)[g]);
+    return n;
+}
+
+// FD steps [kt0, kt0 + nsteps) of table slots [slot0, slot0 + nshots) (one
+// grid) in the on-chip loop, from state buffer par0 to par1.
+int run_resident(Ctx *c, Batch &b, const ResPlan &pl, int slot0, int nshots, int kt0, int nsteps, int par0, int par1,
+                 int *launches) {
+    const int per = pl.ncx * pl.ncz;
+    std::vector<ResShot> rs;
+    for (int i = 0; i < nshots; ++i) rs.push_back({slot0 + i, (i % pl.conc) * per, pl.ncx, pl.ncz});
+    const size_t rbytes = sizeof(ResShot) * rs.size(), fbytes = resident_frame_bytes(pl.nw, pl.c, pl.conc * per);
+    if (c->res_shots.bytes < rbytes) CK(c->res_shots.alloc(rbytes));
+    if (c->res_frames.bytes < fbytes) CK(c->res_frames.alloc(fbytes));
+    CK(cudaMemcpyAsync(c->res_shots.p, rs.data(), rbytes, cudaMemcpyHostToDevice, c->stream));
+    ResArgs a{};
+    a.shots = b.shots_d.as<ShotDev>();
+    a.kt0 = kt0;
+    a.nsteps = nsteps;
+    a.par0 = par0;
+    a.par1 = par1;
+    a.dt_factor = b.steps.dt_factor;
+    a.frames = c->res_frames.as<unsigned long long>();
+    a.err = c->dev_err.as<int>();
+    a.spin_limit = c->opt_spin_limit;
+    a.fault_step = c->opt_fault_iter;
+    for (int i = 0; i < nshots; i += pl.conc) {
+        const int n = std::min(pl.conc, nshots - i);
+        a.rs = c->res_shots.as<ResShot>() + i;
+        a.nrs = n;
+        CK(cudaMemsetAsync(c->res_frames.p, 0, resident_frame_bytes(pl.nw, pl.c, n * per), c->stream));
+        int e = launch_resident(pl.nw, pl.c, a, n * per, c->stream);
+        if (e) return fail(c, S2D_ERR_CUDA, "on-chip loop launch: %s", cudaGetErrorString((cudaError_t)e));
+        *launches += 1;
+    }
+    return S2D_OK;
+}
+
+// The state buffer a run of `nsteps` from buffer `cur` ends in.
+int end_buffer(const LaunchCfg &lc, int cur, int nsteps) {
+    const int spl = lc.variant == kVariantPersist ? 1 : steps_per_launch(lc.variant);
+    return cur ^ ((nsteps / spl + nsteps % spl) & 1);
 }
 
 // cuTensorMapEncodeTiled through the runtime's driver entry point (no link
@@ -689,8 +729,10 @@ int setup_batch(Ctx *c, const s2d_shot *shots, int nshots, const s2d_wave &wave,
         d.nfield = m.field_elems;
         d.nrec = h.nrec;
         d.nseis = (size_t)h.nrec * rs.real_nt;
-        fast_rows(m, wave.fd_dt, &d.zfast_lo, &d.zfast_hi, &d.kz_in);
-        fast_cols(m, wave.fd_dt, &d.xfast_lo, &d.xfast_hi, &d.kx_in);
+        fast_range(m.nnz, (double)(wave.fd_dt * (1.0f / m.dz)), m.damp1a, m.damp1a1, m.damp1b, m.damp1b1, &d.zfast_lo,
+                   &d.zfast_hi, &d.kz_in);
+        fast_range(m.nnx, (double)(wave.fd_dt * (1.0f / m.dx)), m.damp2a, m.damp2a1, m.damp2b, m.damp2b1, &d.xfast_lo,
+                   &d.xfast_hi, &d.kx_in);
         if (!c->opt_fast_rows) d.zfast_lo = d.zfast_hi = d.xfast_lo = d.xfast_hi = 0;
         // source amplitude per step: fd_dt * w[kt] * kappa[src] / (dx*dz)
         // (cpumodelling.cpp:136-140), kappa = vp^2 rho in double at the source
@@ -800,13 +842,7 @@ int setup_batch(Ctx *c, const s2d_shot *shots, int nshots, const s2d_wave &wave,
         int e = build_tmaps(c, b);
         if (e) return e;
     }
-    // segment lengths for the configuration the run starts with
-    {
-        LaunchCfg lc;
-        int e = base_config(c, b, &lc);
-        if (!e) e = layout_groups(c, b, lc);
-        if (e) return e;
-    }
+    b.chip.assign(b.groups.size(), 0);
     CK(cudaStreamSynchronize(c->stream));
     c->batch = std::move(bp);
     return S2D_OK;
@@ -1050,6 +1086,15 @@ int s2d_set_option(void *ctx, const char *key, long value) {
         c->opt_adj_minb = (int)value;
     } else if (k == "fast_rows") {
         c->opt_fast_rows = value ? 1 : 0;
+    } else if (k == "on_chip") {
+        if (value != 0 && value != 1) return fail(c, S2D_ERR_ARG, "on_chip must be 0 or 1");
+        c->opt_on_chip = (int)value;
+    } else if (k == "on_chip_shape") {
+        int nw, cc, known = value == 0;
+        double us;
+        for (int i = 0; resident_shapes(i, &nw, &cc, &us); ++i) known |= value == nw * 100 + cc;
+        if (!known) return fail(c, S2D_ERR_ARG, "unknown on_chip_shape %ld", value);
+        c->opt_chip_shape = (int)value;
     } else if (k == "graph_chunk") {
         if (value < 1 || value > 100000) return fail(c, S2D_ERR_ARG, "graph_chunk must be in [1, 100000]");
         c->opt_graph_chunk = (int)value;
@@ -1230,14 +1275,35 @@ int s2d_forward(void *ctx, const s2d_shot *shots, int nshots, const s2d_wave *wa
     int launches = 0;
     bool graph_used = false;
     bool tuned = false;
+    int tuned_now = 0;
     LaunchCfg lc;
-    {
+    auto configure = [&]() -> int {
         int e = base_config(c, b, &lc, &tuned);
         const int order = lc.order;
         if (!e) e = layout_groups(c, b, lc);
         if (!e) e = launch_config(c, b.max_tasks, &lc, lc.variant, lc.block, lc.stages);
-        if (e) return e;
         lc.order = order;
+        return e;
+    };
+    // Batched runs of a shape with no tuned configuration yet tune on their
+    // first steps when the call has room for the trials and a run after them.
+    // A batch that runs on chip altogether needs no trials: the default is
+    // recorded for the few steps that a later call may leave to the per-step
+    // kernels.
+    const int tune_len = b.order8 ? kTuneStepsO8 : kTuneSteps;
+    const bool room = c->opt_autotune && !b.plain && nsteps >= 2 * tune_len;
+    std::vector<ResPlan> plans;
+    int n_chip = choose_on_chip(c, b, nsteps, use_graph, &plans);
+    if (room && b.all_chip() && !c->tuned.count(tune_key(c, b))) {
+        const LaunchCfg d;
+        c->tuned[tune_key(c, b)] = {d.variant, d.block, d.stages, c->opt_order};
+        tuned_now = 1;
+    }
+    const bool tune = room && !b.all_chip() && !c->tuned.count(tune_key(c, b));
+    if (tune) b.chip.assign(b.groups.size(), 0);  // the trials are steps of every shot
+    {
+        int e = configure();
+        if (e) return e;
     }
     CK(cudaEventRecord(c->ev0, c->stream));
     StepArgs a{};
@@ -1247,11 +1313,7 @@ int s2d_forward(void *ctx, const s2d_shot *shots, int nshots, const s2d_wave *wa
     a.tmaps = b.tmaps_d.p;
     a.tmap_mat0 = b.nshots;
     int kt_run = kt_begin;  // first step left after tuning
-    int tuned_now = 0;
-    // Batched runs of a shape with no tuned configuration yet tune on their
-    // first steps when the call has room for the trials and a run after them.
-    const int tune_len = b.order8 ? kTuneStepsO8 : kTuneSteps;
-    if (c->opt_autotune && !tuned && !b.plain && nsteps >= 2 * tune_len) {
+    if (tune) {
         a.groups = b.groups_d.as<GroupDev>();
         a.ngroups = (int)b.groups.size();
         int used = 0;
@@ -1259,25 +1321,40 @@ int s2d_forward(void *ctx, const s2d_shot *shots, int nshots, const s2d_wave *wa
         if (e) return e;
         kt_run += used;
         tuned_now = 1;
+        n_chip = choose_on_chip(c, b, kt_end - kt_run, use_graph, &plans);
+        if (n_chip) e = configure();
+        if (e) return e;
     }
+    const int run = kt_end - kt_run;  // steps left after tuning
+    const int cur0 = b.cur, cur1 = end_buffer(lc, cur0, run);
     if (b.plain) {
         // every shot advances from the same buffer through the same launches
-        const int cur0 = b.cur;
         for (int s = 0; s < nshots; ++s) {
-            a.groups = b.groups_d.as<GroupDev>() + s;
-            a.ngroups = 1;
-            a.total_tasks = plain_tasks(b, s);
-            b.cur = cur0;
-            int e = run_loop(c, b, lc, a, kt_begin, nsteps, use_graph, &launches, &graph_used);
+            int e;
+            if (b.chip[s]) {
+                e = run_resident(c, b, plans[s], s, 1, kt_run, run, cur0, cur1, &launches);
+            } else {
+                a.groups = b.groups_d.as<GroupDev>() + s;
+                a.ngroups = 1;
+                a.total_tasks = plain_tasks(b, s);
+                b.cur = cur0;
+                e = run_loop(c, b, lc, a, kt_run, run, use_graph, &launches, &graph_used);
+            }
             if (e) return e;
         }
     } else {
         a.groups = b.groups_d.as<GroupDev>();
         a.ngroups = (int)b.groups.size();
         a.total_tasks = batch_tasks(b);
-        int e = run_loop(c, b, lc, a, kt_run, kt_end - kt_run, use_graph, &launches, &graph_used);
+        int e = S2D_OK;
+        if (n_chip < (int)b.groups.size()) e = run_loop(c, b, lc, a, kt_run, run, use_graph, &launches, &graph_used);
+        for (size_t g = 0; g < b.groups.size() && !e; ++g)
+            if (b.chip[g])
+                e = run_resident(c, b, plans[g], b.groups[g].shot0, b.groups[g].nshots, kt_run, run, cur0, cur1,
+                                 &launches);
         if (e) return e;
     }
+    b.cur = cur1;
     CK(cudaEventRecord(c->ev1, c->stream));
     b.kt_next = kt_end;
     // seismogram samples recorded in [kt_begin, kt_end), widened to the whole
@@ -1312,19 +1389,21 @@ int s2d_forward(void *ctx, const s2d_shot *shots, int nshots, const s2d_wave *wa
         CK(cudaEventSynchronize(c->ev1));
         float ms = 0;
         CK(cudaEventElapsedTime(&ms, c->ev0, c->ev1));
-        double cells = 0, bytes = 0;
-        for (int s = 0; s < nshots; ++s) {
-            const Model &m = *c->models[b.shots[s].model_id];
-            cells += (double)m.nnx * m.nnz;
-            bytes += m.step_bytes();
-        }
+        double cells = 0, bytes = 0, chip_bytes = 0;  // chip_bytes: shots the on-chip loop ran
+        for (size_t g = 0; g < b.groups.size(); ++g)
+            for (int i = 0; i < b.groups[g].nshots; ++i) {
+                const Model &m = *c->models[b.shots[b.table[b.groups[g].shot0 + i]].model_id];
+                cells += (double)m.nnx * m.nnz;
+                (b.chip[g] ? chip_bytes : bytes) += m.step_bytes();
+            }
         stats->loop_ms = ms;
         stats->cell_updates = cells * nsteps;
         // one pass over the state per launch (two steps per pass for the
         // two-step kernel; the autotuner's trial steps are counted as one-step)
         const int passes = steps_per_launch(lc.variant) == 2 ? (kt_end - kt_run + 1) / 2 + (kt_run - kt_begin)
                                                              : nsteps;
-        stats->alg_bytes = bytes * passes;
+        // (one pass per call for the on-chip loop, after the trial steps)
+        stats->alg_bytes = bytes * passes + chip_bytes * (1 + kt_run - kt_begin);
         stats->gcells_per_s = ms > 0 ? stats->cell_updates / (ms * 1e6) : 0.0;
         stats->kernel_launches = launches;
         stats->graph_used = graph_used ? 1 : 0;
@@ -1618,6 +1697,10 @@ extern "C" int s2d_gradient(void *ctx, const s2d_shot *shots, int nshots, const 
         int e = phase_mark(c, g, kPhaseSweep);
         if (e) return e;
     }
+    // the sweep's segments run on chip where the forward would
+    ResPlan sweep_plan;
+    const bool sweep_on_chip = c->opt_on_chip && c->opt_autotune && use_graph && !b.order8 && C >= 8 &&
+                               on_chip_group(c, b, 0, &sweep_plan);
     // ---- forward sweep, saving the state at each segment start ----
     auto save_ckpt = [&](int j) -> int {
         const int par = (j * C) & 1;
@@ -1657,7 +1740,10 @@ extern "C" int s2d_gradient(void *ctx, const s2d_shot *shots, int nshots, const 
         if (j < nseg - 1) {
             StepArgs a = fa;
             int e = save_ckpt(j);
-            if (!e) e = run_loop(c, b, lc_fwd, a, k0, n, use_graph, &launches, &graph_used);
+            if (!e && sweep_on_chip)
+                e = run_resident(c, b, sweep_plan, 0, nshots, k0, n, b.cur, b.cur ^ (n & 1), &launches);
+            else if (!e)
+                e = run_loop(c, b, lc_fwd, a, k0, n, use_graph, &launches, &graph_used);
             if (e) return e;
         } else {
             int e = backward_layout();

@@ -220,6 +220,41 @@ inline size_t bulk_smem_bytes(int warps_per_block, int stages) {
     return (size_t)warps_per_block * stages * (kStageBytes + 8);
 }
 
+// On-chip time loop (s2d_resident.cu): a launch's shots and their blocks.
+struct ResShot {
+    int shot;      // index in the shot table
+    int cta0;      // first block of the shot
+    int ncx, ncz;  // blocks along x (column segments) and z (120-row strips)
+};
+struct ResArgs {
+    const ShotDev *shots;
+    const ResShot *rs;     // nrs entries, by cta0
+    int nrs;
+    int kt0, nsteps;       // FD steps [kt0, kt0 + nsteps)
+    int par0, par1;        // state buffers of step kt0 and of the result (the same one only for 2 steps or more)
+    int dt_factor, flags;  // S2D_STEP_* bits
+    unsigned long long *frames;  // resident_frame_bytes, zeroed before every launch
+    int *err;              // device error word
+    int spin_limit;        // polls before a wait counts as timed out
+    int fault_step;        // test knob: step after which block 0 does not publish (-1: none)
+    float one;             // 1 (set by launch_resident)
+};
+size_t resident_frame_bytes(int nw, int c, int ctas);
+// One cooperative launch of `grid` blocks of nw warps with c columns each.
+int launch_resident(int nw, int c, const ResArgs &a, int grid, void *stream);
+// The i-th block shape the kernel is built for (tiles of nw*c - 6 own columns)
+// and its time per step; 0 past the last.
+int resident_shapes(int i, int *nw, int *c, double *us);
+// How the on-chip loop takes the shots of one grid: `conc` of them per
+// launch, each on ncx x ncz blocks of nw warps with c columns per warp.
+struct ResPlan {
+    int conc = 0, ncx = 0, ncz = 0, nw = 0, c = 0;
+    double step_us = 0;  // estimated time of one FD step of all the shots
+};
+// False when the grid does not fit `sm_count` SMs.  shape: nw * 100 + c, or 0
+// for the fastest.  plain: one shot per launch.
+bool resident_plan(int sm_count, int nnx, int nnz, int nshots, bool plain, int shape, ResPlan *out);
+
 // Host-side launch helpers implemented in s2d_kernels.cu.
 int launch_step(int variant, const StepArgs *args_dev, int kt_off, int grid, int block, size_t smem,
                 void *stream);

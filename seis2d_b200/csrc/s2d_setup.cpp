@@ -73,4 +73,18 @@ void cell_of(float x, float z, float dx, float dz, int nb, int &ix, int &iz) {
     iz = (int)(z * inv_dz) + nb;
 }
 
+void fast_range(int n, double dtd, const std::vector<float> &a, const std::vector<float> &a1,
+                const std::vector<float> &b, const std::vector<float> &b1, int *lo, int *hi, float *k) {
+    const float ki = (float)(dtd * 1.0f);
+    auto ok = [&](int i) {
+        return i >= 2 && i <= n - 3 && a[i] == 1.0f && b[i] == 1.0f && (float)(dtd * a1[i]) == ki &&
+               (float)(dtd * b1[i]) == ki;
+    };
+    *lo = 0;
+    while (*lo < n && !ok(*lo)) ++*lo;
+    *hi = *lo;
+    while (*hi < n && ok(*hi)) ++*hi;
+    *k = ki;
+}
+
 }  // namespace s2d

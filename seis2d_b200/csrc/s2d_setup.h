@@ -31,4 +31,11 @@ void sponge_b(int nb, int n, std::vector<float> &damp, std::vector<float> &damp1
 // (cpumodelling.cpp:288-289, cpu_modelling_kernels.cpp:15-22).
 void cell_of(float x, float z, float dx, float dz, int nb, int &ix, int &iz);
 
+// Rows (or columns) whose coefficients are the interior constants: dampings a
+// = b = 1, dtd*a1 = dtd*b1 = (float)dtd and both operator pairs (a0, a1),
+// indices [2, n-3].  The first such run [lo, hi) (empty when lo == hi); its
+// constant in *k.  dtd as the coefficient tables form it: (double)(dt * (1 / d)).
+void fast_range(int n, double dtd, const std::vector<float> &a, const std::vector<float> &a1,
+                const std::vector<float> &b, const std::vector<float> &b1, int *lo, int *hi, float *k);
+
 }  // namespace s2d

@@ -168,6 +168,17 @@ extern "C" int s2d_forward_static(int device, int nx, int nz, float dx, float dz
                    "s2d_forward_static: this job needs %zu bytes of device scratch (padded grid %d x %d, %d receivers "
                    "x %d samples); the static scratch holds %zu bytes",
                    cv.used, nnx, nnz, nrec, rs.real_nt, kScratchBytes);
+    // the on-chip time loop where the grid fits the chip and the loop's frames
+    // fit what is left of the scratch; else one launch per step
+    int sms = 1, coop = 0;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device);
+    ResPlan plan;
+    bool on_chip = coop && rs.fd_nt >= 8 && resident_plan(sms, nnx, nnz, 1, true, 0, &plan);
+    const int blocks = plan.ncx * plan.ncz;
+    const size_t frame_bytes = on_chip ? resident_frame_bytes(plan.nw, plan.c, blocks) : 0;
+    const size_t o_rshot = cv.take<ResShot>(1), o_frames = cv.take<unsigned char>(frame_bytes);
+    if (cv.used > kScratchBytes) on_chip = false;
 
     int prev = -1;
     cudaGetDevice(&prev);
@@ -268,14 +279,16 @@ extern "C" int s2d_forward_static(int device, int nx, int nz, float dx, float dz
     sd.nfield = F;          // sizes for the kernels' self-checks (S2D_DEVICE_CHECKS builds)
     sd.nrec = nrec;
     sd.nseis = seis_n;
-    sd.zfast_lo = sd.zfast_hi = 0;  // every strip takes the general row path
-    sd.xfast_lo = sd.xfast_hi = 0;  // and every column the general column path
-    sd.rec_zlo = 0;                 // receivers anywhere
-    sd.rec_zhi = nnz - 1;
+    fast_range(nnz, rs.dtdz, d1a, d1a1, d1b, d1b1, &sd.zfast_lo, &sd.zfast_hi, &sd.kz_in);
+    fast_range(nnx, rs.dtdx, d2a, d2a1, d2b, d2b1, &sd.xfast_lo, &sd.xfast_hi, &sd.kx_in);
+    sd.rec_zlo = nnz;
+    sd.rec_zhi = -1;
+    for (int g = 0; g < nrec; ++g) {
+        sd.rec_zlo = std::min(sd.rec_zlo, rz[g]);
+        sd.rec_zhi = std::max(sd.rec_zhi, rz[g]);
+    }
     int bps = 1;
     if (rc == S2D_OK && (step_kernel_occupancy(kVariantLdg, 128, 0, &bps) || bps < 1)) bps = 1;
-    int sms = 1;
-    if (rc == S2D_OK) SCK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
     const int nstrips = num_strips(nnz);
     const long resident_warps = (long)sms * bps * 4;
     int seg_len = 16;
@@ -313,17 +326,39 @@ extern "C" int s2d_forward_static(int device, int nx, int nz, float dx, float dz
         if (k) rc = say(eb, el, S2D_ERR_CUDA, "argument launch: %s", cudaGetErrorString((cudaError_t)k));
     }
     const int grid = (int)std::max<long>(1, std::min<long>((long)sms * bps, ((long)a.total_tasks * 32 + 127) / 128));
-    for (int kt = 0; kt < rs.fd_nt && rc == S2D_OK; ++kt) {
+    if (on_chip) {
+        const ResShot r{0, 0, plan.ncx, plan.ncz};
+        SCK(cudaMemcpyAsync(at(o_rshot), &r, sizeof r, cudaMemcpyHostToDevice, st));
+        SCK(cudaMemsetAsync(at(o_frames), 0, frame_bytes, st));
+        ResArgs ra{};
+        ra.shots = a.shots;
+        ra.rs = reinterpret_cast<const ResShot *>(at(o_rshot));
+        ra.nrs = 1;
+        ra.nsteps = rs.fd_nt;
+        ra.par1 = rs.fd_nt & 1;
+        ra.dt_factor = rs.dt_factor;
+        ra.frames = reinterpret_cast<unsigned long long *>(at(o_frames));
+        ra.err = a.err;
+        ra.spin_limit = a.spin_limit;
+        ra.fault_step = -1;
+        if (rc == S2D_OK) {
+            int k = launch_resident(plan.nw, plan.c, ra, blocks, st);
+            if (k) rc = say(eb, el, S2D_ERR_CUDA, "on-chip loop launch: %s", cudaGetErrorString((cudaError_t)k));
+        }
+    }
+    for (int kt = 0; kt < rs.fd_nt && rc == S2D_OK && !on_chip; ++kt) {
         int k = launch_step(kVariantLdg, args_d, kt, grid, 128, 0, st);
         if (k) rc = say(eb, el, S2D_ERR_CUDA, "step launch: %s", cudaGetErrorString((cudaError_t)k));
     }
     if (host_seis && seis_n)
         SCK(cudaMemcpyAsync(seis_out, at(o_seis), seis_n * sizeof(float), cudaMemcpyDeviceToHost, st));
     SCK(cudaStreamSynchronize(st));
-    // the step kernel's device error word: nonzero only when a self-check of a
-    // S2D_DEVICE_CHECKS build skipped a task (the plain-load kernel has no waits)
+    // the device error word: a wait of the on-chip loop that ran out, or a
+    // self-check of a S2D_DEVICE_CHECKS build that skipped a task
     int dev_err = 0;
     SCK(cudaMemcpy(&dev_err, at(o_err), sizeof(int), cudaMemcpyDeviceToHost));
+    if (rc == S2D_OK && on_chip && (dev_err & S2D_DEV_ERR_WAIT))
+        rc = say(eb, el, S2D_ERR_TIMEOUT, "s2d_forward_static: a wait of the on-chip loop ran out of its spin limit");
     if (rc == S2D_OK && dev_err)
         rc = say(eb, el, S2D_ERR_CUDA, "s2d_forward_static: device self-check failed (error word 0x%x)", dev_err);
 #undef SCK
