@@ -158,23 +158,25 @@ S2D_API const char *s2d_last_error(const void *ctx);
 /*
  * Tuning knobs of the step kernel; no counterpart in the reference.  Keys:
  *   "autotune"    1 (default): the first s2d_forward of a batched run of a new
- *                 shape (models, grids, shot counts) with at least 112 steps
- *                 (64 for the 8th-order operator) spends up to 56 (32) of them
- *                 on trials: 9 candidate configurations (variants 4, 16, 15,
- *                 2, 5, 11, 12 in task order 1, and 16 and 15 in task order 0,
- *                 unless "task_order" was set), one untimed and three timed
- *                 launches each, in rounds, then four more timed launches each
- *                 of the two fastest, alternating (the results do not change:
- *                 every candidate computes the same bits); it keeps the fastest
- *                 per FD step for that shape in the context; runs that do not
- *                 tune (shorter calls, S2D_PLAIN) use variant 16.
+ *                 shape (models, grids, shot counts) with at least 80 steps
+ *                 (64 for the 8th-order operator) spends up to 40 (32) of them
+ *                 on trials: 5 candidate configurations (variants 5, 16, 15 in
+ *                 task order 1, and 16 and 15 in task order 0, unless
+ *                 "task_order" was set), one untimed and three timed launches
+ *                 each, in rounds, then four more timed launches each of the
+ *                 two fastest, alternating (the results do not change: every
+ *                 candidate computes the same bits); it keeps the fastest per
+ *                 FD step for that shape in the context; runs that do not tune
+ *                 (shorter calls, S2D_PLAIN) use variant 5 from 1.5 M cells on
+ *                 and 16 below.
  *                 0: use "variant", "block" and "stages".
  *                 Setting any of those three turns autotuning off.
  *   "variant"     0 bulk-copy pipeline, 1 plain loads, 2 bulk-copy pipeline
  *                 compiled for 128 registers, 4 plain loads compiled for 128
  *                 registers, 5 two FD steps per launch (the state crosses HBM
  *                 once per two steps; odd step counts end with one one-step
- *                 launch), 11 a CTA of 8 warps on adjacent strips fed by a
+ *                 launch; columns copied asynchronously 3 ahead, tasks handed
+ *                 out as the warps finish), 11 a CTA of 8 warps on adjacent strips fed by a
  *                 producer warp's 2-D TMA tensor loads through a 4-stage
  *                 shared-memory ring (one block of 288 threads per SM),
  *                 12 the plain-load loop fed by per-lane asynchronous copies
@@ -187,7 +189,8 @@ S2D_API const char *s2d_last_error(const void *ctx);
  *                 cooperative launch that advances "graph_chunk" steps with a
  *                 bounded grid barrier between steps (an option only: slower
  *                 than per-step launches on the grids measured);
- *                 s2d_gradient always runs one step per launch.
+ *                 the recomputes and adjoint steps of s2d_gradient always run
+ *                 one step per launch.
  *                 For batches of S2D_MODEL_ORDER8 models: 7 register windows
  *                 at 3 blocks per SM (default), 8 the same at 2, 9 windows in
  *                 shared memory at 4 (each setting applies to its own order)

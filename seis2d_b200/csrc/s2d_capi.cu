@@ -178,6 +178,7 @@ struct Ctx {
     int opt_prod_variant = kVariantLdgPfProducts;  // s2d_gradient's product-writing forward (4th order)
     int last_segment = 0;     // interval the last gradient call used
     DevBuf dev_err;           // device error word of the step kernels
+    DevBuf queue_d;           // task counter of the step kernels (zero between launches)
     DevBuf bar_d;             // grid-barrier counter of the persistent step kernel
     int opt_on_chip = 1;      // on-chip time loop for the grids that fit
     int opt_chip_shape = 0;   // its block shape (warps * 100 + columns per warp), 0 = the fastest
@@ -252,6 +253,64 @@ int choose_seg_len(int nnx, long tasks_per_seg, long resident_warps, int halo) {
     return best;
 }
 
+// Rim and interior tasks of a two-step group (GroupDev::split) of the grid
+// and fast ranges of shot record `d`; `shots` shots of it run at a time beside
+// `share` of `resident_warps` warps.
+// Measured cost of a column: 1 in the interior, 1.6 in strips with sponge rows,
+// 1.9 in sponge columns; a task streams 9 columns besides its own.  The
+// warps draw tasks as they finish, the dear ones first, so a launch takes
+// about its work over the warps, plus half an interior task, and at least its
+// longest task.
+void split_group(GroupDev &g, const ShotDev &d, int shots, double resident_warps, int forced) {
+    constexpr double kRows = 1.6, kCols = 1.9;
+    constexpr int kHalo = 9;
+    g.split = 1;
+    auto fast = [&](int k) {
+        const int c0 = k * S2D_TS_OUT - 8;
+        return c0 >= d.zfast_lo && c0 + S2D_STRIP_ROWS - 1 < d.zfast_hi;
+    };
+    g.rim_lo = 0;
+    while (g.rim_lo < g.nstrips && !fast(g.rim_lo)) ++g.rim_lo;
+    g.rim_hi = 0;
+    while (g.rim_lo + g.rim_hi < g.nstrips && !fast(g.nstrips - 1 - g.rim_hi)) ++g.rim_hi;
+    // interior tasks: columns xa-4 .. xb+4 fast
+    g.xl = d.xfast_lo + 4;
+    g.xr = d.xfast_hi - 5;
+    if (g.xr - g.xl < 8) g.xl = g.xr = d.nnx;
+    const int nz = g.rim_lo + g.rim_hi, ni = g.nstrips - nz;
+    auto cut = [&](int L) {
+        auto pieces = [](int n, int len) { return (n + len - 1) / len; };
+        auto even = [&](int n, int len) { return n > 0 ? (n + pieces(n, len) - 1) / pieces(n, len) : len; };
+        g.seg_len = L;
+        g.nsegs = pieces(g.xr - g.xl, L);
+        const int lz = std::max(4, (int)((L + kHalo) / kRows) - kHalo), lx = std::max(4, (int)((L + kHalo) / kCols) - kHalo);
+        g.seg_z = even(d.nnx, lz);
+        g.nseg_z = pieces(d.nnx, g.seg_z);
+        g.seg_x = even(std::max(g.xl, d.nnx - g.xr), lx);
+        g.nseg_l = pieces(g.xl, g.seg_x);
+        g.nseg_r = pieces(d.nnx - g.xr, g.seg_x);
+    };
+    if (forced > 0) {
+        cut(forced);
+        return;
+    }
+    int best = 0;
+    double best_cost = 0;
+    for (int L = 7; L <= 255; L += L < 63 ? 4 : 16) {
+        cut(L);
+        const double ti = L + kHalo, tz = (g.seg_z + kHalo) * kRows, tx = (g.seg_x + kHalo) * kCols;
+        const double work = shots * (ni * (g.nsegs * ti + (g.nseg_l + g.nseg_r) * tx) + nz * g.nseg_z * tz);
+        const double longest = std::max(ni && g.nsegs ? ti : 0.0, std::max(nz ? tz : 0.0, ni ? tx : 0.0));
+        const double tasks = (double)shots * shot_tasks(g);
+        const double cost = std::max(longest, tasks <= resident_warps ? longest : work / resident_warps + 0.5 * ti);
+        if (!best || cost < best_cost) {
+            best = L;
+            best_cost = cost;
+        }
+    }
+    cut(best);
+}
+
 int build_coef(Ctx *c, Model &m, float fd_dt) {
     if (m.coef_dt == fd_dt && m.xcoef.p) return S2D_OK;
     const float inv_dx = 1.0f / m.dx, inv_dz = 1.0f / m.dz;
@@ -297,7 +356,7 @@ int launch_config(Ctx *c, long max_tasks, LaunchCfg *out, int variant, int block
     lc.smem = ldg ? 0
               : tma ? kTmaSmemBytes
               : asy ? (size_t)(lc.block / 32) * kAsyncWarpBytes
-              : ts ? (size_t)(lc.block / 32) * (lc.variant == kVariantO8s ? kO8sWarpBytes : kTsWarpBytes)
+              : ts ? (size_t)(lc.block / 32) * (lc.variant == kVariantO8s ? kO8sWarpBytes : lc.variant == kVariantTs1 ? 0 : kTs2WarpBytes)
                    : bulk_smem_bytes(lc.block / 32, lc.stages);
     int e = step_kernel_prepare(lc.variant, lc.smem);
     if (e) return fail(c, S2D_ERR_ARG, "step kernel does not accept %zu B of shared memory: %s", lc.smem,
@@ -327,6 +386,20 @@ std::vector<long> tune_key(const Ctx *c, const Batch &b) {
     return k;
 }
 
+// The 4th-order kernel of a launch that nothing else decides: two steps per
+// launch from about 1.5 M cells on (one 3301 x 1301 shot 157 Gcell/s against 102
+// with one step, 8 of 5120 x 5120 370 against 154); below, its longer halo and
+// its 8 warps per SM cost what the second step saves (780 x 580: 64 and 64).
+int default_variant(const Batch &b) {
+    double cells = 0;
+    for (size_t g = 0; g < b.groups.size(); ++g) {
+        if (g < b.chip.size() && b.chip[g]) continue;
+        const double n = (double)b.group_nnx[g] * b.group_nnz[g];
+        cells = b.plain ? std::max(cells, n) : cells + n * b.groups[g].nshots;
+    }
+    return cells >= 1.5e6 ? kVariantTs2 : kVariantLdgPf4;
+}
+
 // The configuration a run of batch `b` uses when it does not tune: the
 // options when autotuning is off, else the tuned result for the batch's
 // shape, else the built-in default.
@@ -343,7 +416,8 @@ int base_config(Ctx *c, const Batch &b, LaunchCfg *out, bool *tuned = nullptr) {
         return e;
     }
     const LaunchCfg d;
-    return launch_config(c, b.max_tasks, out, b.order8 ? kVariantO8 : d.variant, d.block, b.order8 ? 0 : d.stages);
+    return launch_config(c, b.max_tasks, out, b.order8 ? kVariantO8 : default_variant(b), d.block,
+                         b.order8 ? 0 : d.stages);
 }
 
 // Segment lengths, segment counts and task ranges of the batch's groups for
@@ -351,8 +425,9 @@ int base_config(Ctx *c, const Batch &b, LaunchCfg *out, bool *tuned = nullptr) {
 // `key` differs from the layout in place.
 // With `tma` a task is a CTA's: kTmaWarps (shot, strip) pairs of a group
 // over one segment, and `resident_warps` counts resident CTAs.
+// With `split` the groups are cut into rim and interior tasks (two-step kernel).
 int layout_groups_for(Ctx *c, Batch &b, long resident_warps, std::vector<long> key, bool ts = false,
-                      bool tma = false) {
+                      bool tma = false, bool split = false) {
     for (char f : b.chip) key.push_back(f);
     if (b.layout == key) return S2D_OK;
     for (size_t gi = 0; gi < b.groups.size(); ++gi)
@@ -360,6 +435,10 @@ int layout_groups_for(Ctx *c, Batch &b, long resident_warps, std::vector<long> k
     auto per_seg = [&](const GroupDev &g, int nshots) {
         return tma ? (long)tma_blocks(nshots, g.nstrips) : (long)nshots * g.nstrips;
     };
+    // cells of all the groups' shots (the warps' shares of a split layout)
+    double cells = 0;
+    for (size_t gi = 0; gi < b.groups.size(); ++gi)
+        if (!b.chip[gi]) cells += (double)b.groups[gi].nshots * b.group_nnx[gi] * b.group_nnz[gi];
     long per_seg_total = 0;
     for (size_t gi = 0; gi < b.groups.size(); ++gi)
         if (!b.chip[gi]) per_seg_total += per_seg(b.groups[gi], b.groups[gi].nshots);
@@ -370,15 +449,24 @@ int layout_groups_for(Ctx *c, Batch &b, long resident_warps, std::vector<long> k
         const int nnx = b.group_nnx[gi];
         // plain mode: every shot is a group of its own and runs alone
         const long tasks_per_seg = b.plain ? per_seg(g, 1) : per_seg_total;
-        g.seg_len = c->opt_seg_len > 0 ? std::min(c->opt_seg_len, nnx)
-                                       : choose_seg_len(nnx, tasks_per_seg, resident_warps, ts ? 12 : 6);
-        g.nsegs = b.chip[gi] ? 0 : (nnx + g.seg_len - 1) / g.seg_len;
-        if (b.plain) {
-            g.task_begin = 0;
-            max_tasks = std::max<long>(max_tasks, per_seg(g, 1) * g.nsegs);
+        g.split = 0;
+        if (b.chip[gi]) {
+            g.nsegs = 0;  // no tasks
+        } else if (split) {
+            const double share = b.plain ? 1.0 : (double)g.nshots * nnx * b.group_nnz[gi] / cells;
+            split_group(g, b.shot_dev[b.table[g.shot0]], g.nshots, share * (double)resident_warps, c->opt_seg_len);
         } else {
-            g.task_begin = task;
-            task += (int)(per_seg(g, g.nshots) * g.nsegs);
+            g.seg_len = c->opt_seg_len > 0 ? std::min(c->opt_seg_len, nnx)
+                                           : choose_seg_len(nnx, tasks_per_seg, resident_warps, ts ? 12 : 6);
+            g.nsegs = (nnx + g.seg_len - 1) / g.seg_len;
+        }
+        const int per_shot = shot_tasks(g);
+        g.task_begin = b.plain ? 0 : task;
+        task += tma ? tma_blocks(g.nshots, g.nstrips) * g.nsegs : g.nshots * per_shot;
+        if (b.plain) {
+            max_tasks = std::max<long>(max_tasks, tma ? tma_blocks(1, g.nstrips) * g.nsegs : per_shot);
+            task = 0;
+        } else {
             max_tasks = task;
         }
     }
@@ -404,7 +492,7 @@ int layout_groups(Ctx *c, Batch &b, const LaunchCfg &lc) {
     int e = launch_config(c, 1L << 40, &full, v, lc.block, lc.stages);
     if (e) return e;
     if (tma_variant(v)) return layout_groups_for(c, b, (long)full.grid, key, false, true);
-    return layout_groups_for(c, b, (long)full.grid * (full.block / 32), key, ts_layout(v));
+    return layout_groups_for(c, b, (long)full.grid * (full.block / 32), key, ts_layout(v), false, v == kVariantTs2);
 }
 
 // Graph of `n` step launches (kt_off = 0..n-1) for one launch configuration,
@@ -453,6 +541,8 @@ int run_loop(Ctx *c, Batch &b, const LaunchCfg &lc, StepArgs args, int kt_begin,
     args.spin_limit = c->opt_spin_limit;
     args.fault_iter = c->opt_fault_iter;
     args.task_order = lc.order >= 0 ? lc.order : c->opt_order;
+    args.queue = c->queue_d.as<int>();
+    args.one = 1.0f;
     StepArgs *args_d = c->args_d.as<StepArgs>();
     if (lc.variant == kVariantPersist) {
         // chunks of graph_chunk steps, one cooperative launch each (not
@@ -504,7 +594,7 @@ int run_loop(Ctx *c, Batch &b, const LaunchCfg &lc, StepArgs args, int kt_begin,
         args.kt_base = kt_begin + nl * spl;
         args.par0 = b.cur;
         int e = launch_set_args(args, args_d, c->stream);
-        if (!e) e = launch_step(kVariantTs1, args_d, 0, lc.grid, lc.block, lc.smem, c->stream);
+        if (!e) e = launch_step(kVariantTs1, args_d, 0, lc.grid, lc.block, 0, c->stream);  // no delay lines
         if (e) return fail(c, S2D_ERR_CUDA, "step launch: %s", cudaGetErrorString((cudaError_t)e));
         *launches += 2;
         b.cur ^= 1;
@@ -870,10 +960,12 @@ int check_device_error(Ctx *c) {
 // of a block; order 0 gives a block's warps the same strip and segment of
 // consecutive shots, which then share the segment's kappa, bx, bz through
 // the SM's L1 (the tasks of one launch are the same either way).
+// The kernels fed through shared memory (bulk copies, TMA boxes, one-step
+// asynchronous copies) and the one without the prefetch won on no shape since
+// the two-step kernel reads its columns ahead; they stay selectable.
 constexpr int kTuneCandidates[][4] = {
-    {kVariantLdg128, 128, 0, 1}, {kVariantLdgPf4, 128, 0, 1}, {kVariantLdgPf, 128, 0, 1},
-    {kVariantBulk128, 128, 3, 1}, {kVariantTs2, 128, 0, 1},    {kVariantTma, kTmaThreads, 0, 1},
-    {kVariantAsync, 128, 0, 1},   {kVariantLdgPf4, 128, 0, 0}, {kVariantLdgPf, 128, 0, 0},
+    {kVariantTs2, 128, 0, 1},    {kVariantLdgPf4, 128, 0, 1}, {kVariantLdgPf, 128, 0, 1},
+    {kVariantLdgPf4, 128, 0, 0}, {kVariantLdgPf, 128, 0, 0},
 };
 constexpr int kNumTuneCandidates = (int)(sizeof(kTuneCandidates) / sizeof(kTuneCandidates[0]));
 // Candidates of 8th-order batches: the register-window kernel at 3 blocks per
@@ -899,13 +991,13 @@ constexpr int kTuneStepsO8 = tune_steps(kTuneCandidatesO8, kNumTuneCandidatesO8)
 int batch_tasks(const Batch &b) {
     int t = 0;
     for (auto &g : b.groups)
-        t += (b.layout_tma ? tma_blocks(g.nshots, g.nstrips) : g.nshots * g.nstrips) * g.nsegs;
+        t += b.layout_tma ? tma_blocks(g.nshots, g.nstrips) * g.nsegs : g.nshots * shot_tasks(g);
     return t;
 }
 // Tasks of shot s's own group in a plain run.
 int plain_tasks(const Batch &b, int s) {
     const GroupDev &g = b.groups[s];
-    return (b.layout_tma ? tma_blocks(1, g.nstrips) : g.nstrips) * g.nsegs;
+    return b.layout_tma ? tma_blocks(1, g.nstrips) * g.nsegs : shot_tasks(g);
 }
 
 // Autotuner: advance the batch by real FD steps from kt_begin (*steps_used
@@ -1141,6 +1233,8 @@ int s2d_create(void **ctx, int device) {
     if (e == cudaSuccess) e = cudaEventCreate(&c->ev1);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&c->sm_count, cudaDevAttrMultiProcessorCount, device);
     if (e == cudaSuccess) e = c->dev_err.alloc(sizeof(int));
+    if (e == cudaSuccess) e = c->queue_d.alloc(2 * sizeof(int));
+    if (e == cudaSuccess) e = cudaMemset(c->queue_d.p, 0, 2 * sizeof(int));
     if (e == cudaSuccess) e = c->bar_d.alloc(sizeof(unsigned));
     if (e == cudaSuccess) e = c->args_d.alloc(sizeof(StepArgs));
     if (e == cudaSuccess) e = cudaMemset(c->dev_err.p, 0, sizeof(int));
@@ -1673,15 +1767,11 @@ extern "C" int s2d_gradient(void *ctx, const s2d_shot *shots, int nshots, const 
     {
         int e = base_config(c, b, &lc_fwd);
         const int order = lc_fwd.order;
-        // the gradient keeps every step's state (checkpoints at kt parity):
-        // one step per launch
-        if (!e && steps_per_launch(lc_fwd.variant) != 1)
-            e = launch_config(c, b.max_tasks, &lc_fwd, kVariantLdgPf4, 128, 0);
         if (!e) e = layout_groups(c, b, lc_fwd);
         if (!e) e = launch_config(c, b.max_tasks, &lc_fwd, lc_fwd.variant, lc_fwd.block, lc_fwd.stages);
         if (!e) e = launch_config(c, b.max_tasks, &lc_prod, prod_variant, 128, 0);
         if (e) return e;
-        lc_fwd.order = steps_per_launch(lc_fwd.variant) == 1 ? order : -1;
+        lc_fwd.order = order;
     }
     StepArgs fa{};
     fa.shots = b.shots_d.as<ShotDev>();
@@ -1703,7 +1793,7 @@ extern "C" int s2d_gradient(void *ctx, const s2d_shot *shots, int nshots, const 
                                on_chip_group(c, b, 0, &sweep_plan);
     // ---- forward sweep, saving the state at each segment start ----
     auto save_ckpt = [&](int j) -> int {
-        const int par = (j * C) & 1;
+        const int par = b.cur;
         for (int s = 0; s < nshots; ++s)
             for (int f = 0; f < 4; ++f)
                 CK(cudaMemcpyAsync(ckpt[s] + ((size_t)j * 4 + f) * F, b.shot_dev[s].st[par][f], fb,
@@ -1736,13 +1826,13 @@ extern "C" int s2d_gradient(void *ctx, const s2d_shot *shots, int nshots, const 
     };
     for (int j = 0; j < nseg; ++j) {
         const int k0 = j * C, n = std::min(C, rs.fd_nt - k0);
-        b.cur = k0 & 1;  // one step per launch: the state of step kt is in buffer kt & 1
         if (j < nseg - 1) {
             StepArgs a = fa;
             int e = save_ckpt(j);
-            if (!e && sweep_on_chip)
+            if (!e && sweep_on_chip) {
                 e = run_resident(c, b, sweep_plan, 0, nshots, k0, n, b.cur, b.cur ^ (n & 1), &launches);
-            else if (!e)
+                b.cur ^= n & 1;
+            } else if (!e)
                 e = run_loop(c, b, lc_fwd, a, k0, n, use_graph, &launches, &graph_used);
             if (e) return e;
         } else {
@@ -1787,7 +1877,7 @@ extern "C" int s2d_gradient(void *ctx, const s2d_shot *shots, int nshots, const 
         if (j < nseg - 1) {
             int e = phase_mark(c, g, kPhaseRecompute);
             if (e) return e;
-            const int par = k0 & 1;
+            const int par = b.cur;
             for (int s = 0; s < nshots; ++s)
                 for (int f = 0; f < 4; ++f)
                     CK(cudaMemcpyAsync(b.shot_dev[s].st[par][f], ckpt[s] + ((size_t)j * 4 + f) * F, fb,
@@ -1795,7 +1885,6 @@ extern "C" int s2d_gradient(void *ctx, const s2d_shot *shots, int nshots, const 
             StepArgs a = fa;
             a.flags = S2D_STEP_PRODUCTS | S2D_STEP_NO_RECORD;
             a.prod_kt0 = k0;
-            b.cur = k0 & 1;
             e = run_loop(c, b, lc_prod, a, k0, n, use_graph, &launches, &graph_used);
             if (e) return e;
         }

@@ -166,17 +166,122 @@ static __device__ __forceinline__ const ShotDev &task_of(const StepArgs &a, int 
         s = G.shot0 + tl % G.nshots;
         tl /= G.nshots;
         strip = tl % G.nstrips;
-        xa = (tl / G.nstrips) * G.seg_len;
+        tl /= G.nstrips;
     } else {
         strip = tl % G.nstrips;
         tl /= G.nstrips;
         s = G.shot0 + tl % G.nshots;
-        xa = (tl / G.nshots) * G.seg_len;
+        tl /= G.nshots;
     }
+    xa = tl * G.seg_len;
     seg_len = G.seg_len;
     return a.shots[s];
 }
 
+
+// The same for groups cut into rim and interior tasks (GroupDev::split): the
+// rim strips first, then the x-rim of the others, then the interior, so that
+// the tasks that cost most start first.
+static __device__ __forceinline__ const ShotDev &task_of_split(const StepArgs &a, int t, int &strip, int &xa,
+                                                               int &seg_len) {
+    int g = 0;
+    while (g + 1 < a.ngroups && __ldg(&a.groups[g + 1].task_begin) <= t) ++g;
+    const GroupDev &G = a.groups[g];
+    const int nz = G.rim_lo + G.rim_hi, ni = G.nstrips - nz;
+    int q = t - G.task_begin;
+    const int n1 = G.nshots * nz * G.nseg_z, n2 = G.nshots * ni * (G.nseg_l + G.nseg_r);
+    const int part = q < n1 ? 0 : q < n1 + n2 ? 1 : 2;
+    q -= part == 0 ? 0 : part == 1 ? n1 : n1 + n2;
+    const int rows = part == 0 ? nz : ni;
+    int r, s;
+    if (a.task_order == 0) {
+        s = q % G.nshots;
+        q /= G.nshots;
+        r = q % rows;
+        q /= rows;
+    } else {
+        r = q % rows;
+        q /= rows;
+        s = q % G.nshots;
+        q /= G.nshots;
+    }
+    const ShotDev &S = a.shots[G.shot0 + s];
+    int end;
+    if (part == 0) {
+        strip = r < G.rim_lo ? r : r + ni;
+        xa = q * G.seg_z;
+        end = min(S.nnx, xa + G.seg_z);
+    } else {
+        strip = G.rim_lo + r;
+        if (part == 2) {
+            xa = G.xl + q * G.seg_len;
+            end = min(G.xr, xa + G.seg_len);
+        } else if (q < G.nseg_l) {
+            xa = q * G.seg_x;
+            end = min(G.xl, xa + G.seg_x);
+        } else {
+            xa = G.xr + (q - G.nseg_l) * G.seg_x;
+            end = min(S.nnx, xa + G.seg_x);
+        }
+    }
+    seg_len = end - xa;
+    return S;
+}
+
+// The tasks of a launch, handed out as the warps ask for them: warp w starts
+// with task w, the rest come from a counter in device memory (queue[0], drawn
+// one task ahead so that the answer is there when it is needed).  The last warp
+// to leave (queue[1]) sets both back to 0 for the next launch.
+struct TaskQueue {
+    int *q;
+    int nwarp, lane, next;
+    __device__ __forceinline__ TaskQueue(int *queue, int nw, int ln) : q(queue), nwarp(nw), lane(ln), next(0) {}
+    __device__ __forceinline__ void draw() {
+        if (lane == 0) next = atomicAdd(q, 1);
+    }
+    __device__ __forceinline__ int take() { return nwarp + __shfl_sync(kFull, next, 0); }
+    __device__ __forceinline__ void leave() {
+        if (lane == 0 && atomicAdd(q + 1, 1) == nwarp - 1) {
+            q[0] = 0;
+            q[1] = 0;
+        }
+    }
+};
+
+// Receiver samples of a task whose columns come in order: the table's next
+// column and the first receiver of it are read one column ahead, so that no
+// lookup waits for memory.
+struct RecCursor {
+    int j, je, jn, z, id;
+    __device__ __forceinline__ void fetch(const ShotDev &S) {
+        const int e = min(j, S.nrec - 1);
+        z = __ldg(S.rec_z + e);
+        id = __ldg(S.rec_id + e);
+    }
+    // before column P (0 <= P)
+    __device__ __forceinline__ void start(const ShotDev &S, int P) {
+        j = __ldg(S.rec_ptr + P);
+        je = __ldg(S.rec_ptr + min(P + 1, S.nnx));
+        jn = __ldg(S.rec_ptr + min(P + 2, S.nnx));
+        fetch(S);
+    }
+    // Samples of column P: value i of the lane's four rows from `val`.
+    template <class Val>
+    __device__ __forceinline__ void column(const ShotDev &S, int P, int z0, bool owner, int slot, Val val) {
+        if (j < je) {
+            int d = z - z0;
+            if (owner && d >= 0 && d < 4) S.seis[(size_t)id * S.real_nt + slot] = val(d);
+            for (int e = j + 1; e < je; ++e) {
+                d = __ldg(S.rec_z + e) - z0;
+                if (owner && d >= 0 && d < 4) S.seis[(size_t)__ldg(S.rec_id + e) * S.real_nt + slot] = val(d);
+            }
+        }
+        j = je;
+        je = jn;
+        jn = __ldg(S.rec_ptr + min(P + 3, S.nnx));
+        fetch(S);
+    }
+};
 
 // Debug self-check (built with -DS2D_DEVICE_CHECKS): the ranges every access
 // of one task touches, from the runtime tables.  A failed check records a

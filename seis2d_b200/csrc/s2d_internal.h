@@ -94,8 +94,21 @@ struct GroupDev {
     int nstrips;      // strips per shot
     int nsegs;        // x-segments per strip
     int seg_len;      // columns per x-segment
-    int pad_[2];
+    // Two-step kernel: the tasks at the grid's rim, whose columns cost more, are
+    // cut shorter than the interior ones.  Strips [0, rim_lo) and the last
+    // rim_hi ones hold sponge rows: nseg_z segments of seg_z columns each.  The
+    // others: nseg_l and nseg_r segments of seg_x columns over [0, xl) and [xr,
+    // nnx), nsegs of seg_len over [xl, xr).
+    int rim_lo, rim_hi, seg_z, nseg_z;
+    int xl, xr, seg_x, nseg_l, nseg_r;
+    int split;        // 1: the group is cut this way
 };
+// Tasks of one shot of the group.
+S2D_HD inline int shot_tasks(const GroupDev &g) {
+    if (!g.split) return g.nstrips * g.nsegs;
+    const int nz = g.rim_lo + g.rim_hi;
+    return nz * g.nseg_z + (g.nstrips - nz) * (g.nseg_l + g.nseg_r + g.nsegs);
+}
 
 // Arguments of one launch sequence.  They live in device memory and are
 // written by a one-thread kernel in stream order before each sequence, so a
@@ -121,6 +134,8 @@ struct StepArgs {
     // every shot's model, in the same order; null for the other kernels
     const void *tmaps;
     int tmap_mat0;        // index of table slot 0's material map in tmaps
+    float one;            // 1
+    int *queue;           // task counter of the kernels that hand tasks out (TaskQueue), zero between launches
 };
 
 #define S2D_STEP_NO_RECORD 1  // forward: do not sample receivers; adjoint: do not inject the adjoint source
@@ -202,11 +217,12 @@ inline bool plain_loads(int variant) {
            variant == kVariantO8 || variant == kVariantO8r || variant == kVariantO8Products;
 }
 
-// Per-warp shared-memory delay lines of the two-step kernel (4 columns each):
-// the first step's px, pz, vz and vx and the second step's p.
-constexpr int kTsRing = 4;
-constexpr int kTsFields = 5;
-constexpr int kTsWarpBytes = kTsRing * kTsFields * S2D_STRIP_ROWS * 4;
+// Shared memory of a warp of the two-step kernel: the input ring (kTs2Depth
+// iterations of 7 column pieces: vx; px, vz, kappa; bx, bz; pz), step A's px and
+// pz of 4 columns and the 8 row coefficients (tasks that are not interior).
+constexpr int kTs2Depth = 4;  // as the column loop is unrolled: constant ring slots
+constexpr int kTs2Slots = 7;
+constexpr int kTs2WarpBytes = (kTs2Depth * kTs2Slots + 8 + 8) * S2D_STRIP_ROWS * 4;
 // Per-warp shared-memory windows of the 8th-order ring kernel: vx and new p of
 // 8 columns each, vz of 4 (one 128-row column = 32 float4).
 constexpr int kO8sWarpBytes = (8 + 8 + 4) * S2D_STRIP_ROWS * 4;

@@ -32,9 +32,12 @@
 // (the model's interior) the cell carries p = px + pz alone and pz is neither
 // read nor written: 36 B.
 #include <cuda_runtime.h>
+
+#include <climits>
 #include <cstdint>
 
 #include "s2d_device.cuh"
+#include "s2d_pack.cuh"
 
 namespace s2d {
 
@@ -744,42 +747,26 @@ __global__ void __launch_bounds__(128, MINB) step_kernel_bulk(const StepArgs *__
 // from HBM once and written once per two steps.  The warp streams along x as
 // the one-step kernel does; step A (kt) runs at the front of the stream and
 // step B (kt+1) trails it:
-//   column L of vx (step-A input) is loaded at loop index L;
+//   column L of vx (step-A input) is consumed at loop index L;
 //   step A: p at L-1, v at L-3 (as in the one-step kernel);
 //   step B: p at L-4 (needs step-A vx at L-6 .. L-3), v at L-6 (needs step-B p
 //           at L-7 .. L-4).
-// Step-A results never reach HBM: px, pz, vz and vx of step A and the
-// step-B pressure wait in per-warp shared-memory delay lines of 4 columns
-// (each lane reads back only what it wrote), which also serve as step B's
-// x-stencil windows, so the kernel fits 128 registers (4 blocks per SM);
-// kappa, bx, bz are read again for step B (L1/L2 hits: DRAM reads them once).  Two steps of z-halo leave lanes 2..29 valid
+// Step-A results never reach HBM.  Two steps of z-halo leave lanes 2..29 valid
 // (rows c+8 .. c+119 of a strip starting at c = 112k - 8), so strips write
 // 112 rows; the segment's stream starts 6 columns early and ends 5 late.
-// TWO = false is the same kernel doing step A alone (odd remainders), in the
-// same strip layout.
 
-__device__ __forceinline__ float4 &ring_at(float4 *ring, int field, int col, int lane) {
-    return ring[(field * kTsRing + ((col + 2 * S2D_GX) & (kTsRing - 1))) * 32 + lane];
-}
-
-// XF: every column either step updates or differentiates (xa-4 .. xb+4)
-// lies in the shot's x-interior: literal column coefficients.
-template <bool FAST, bool TWO, bool XF = false>
-__device__ __forceinline__ void ts_task(const StepArgs &a, const ShotDev &S, int strip, int xa, int seg_len,
-                                        int kt, int par, int lane, float4 *ring) {
+// One step of a task in the two-step kernel's strip layout.
+template <bool FAST, bool XF>
+__device__ __forceinline__ void ts1_task(const StepArgs &a, const ShotDev &S, int strip, int xa, int seg_len, int kt,
+                                         int par, int lane) {
     const int xb = min(S.nnx, xa + seg_len);
     const size_t ld = (size_t)S.ld;
     const int c = strip * S2D_TS_OUT - 8;
     Lane<FAST> la;
     lane_setup(la, S, c, lane, kt);
     la.owner = lane >= 2 && lane <= 29;
-    Lane<FAST> lb = la;
-    if (TWO) lb.amp = __ldg(S.amp + kt + 1);
-    const bool rec = !(a.flags & S2D_STEP_NO_RECORD);
-    const bool rec_a = rec && ((kt + 1) % a.dt_factor) == 0 && (kt + 1) / a.dt_factor - 1 < S.real_nt;
-    const int slot_a = (kt + 1) / a.dt_factor - 1;
-    const bool rec_b = TWO && rec && ((kt + 2) % a.dt_factor) == 0 && (kt + 2) / a.dt_factor - 1 < S.real_nt;
-    const int slot_b = (kt + 2) / a.dt_factor - 1;
+    const int slot = (kt + 1) / a.dt_factor - 1;
+    const bool rec = !(a.flags & S2D_STEP_NO_RECORD) && ((kt + 1) % a.dt_factor) == 0 && slot < S.real_nt;
     const size_t off = (size_t)(la.z0 + S2D_GZ) + (size_t)S2D_GX * ld;
     const int fs = S.fstride;
     float *const sb = S.st[0][0] + off;
@@ -796,127 +783,420 @@ __device__ __forceinline__ void ts_task(const StepArgs &a, const ShotDev &S, int
     const float *__restrict__ bxp = kap + fs;
     const float *__restrict__ bzp = kap + 2 * fs;
     const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-    // step A windows: vx at L-3..L, new p at L-4..L-1, vz at L-3..L-1
+    // windows: vx at L-3..L, new p at L-4..L-1, vz at L-3..L-1
     float4 vq0 = zero, vq1, vq2, vq3;
     float4 pq0 = zero, pq1 = zero, pq2 = zero, pq3 = zero;
     float4 zq0 = zero, zq1 = zero, zq2 = zero;
-    // step B windows: step-A vx at L-6..L-3, step-B p at L-7..L-4
-    const int h = TWO ? 3 : 0;  // step A runs over [xa - h, xb + h)
-    const int xaa = xa - h, xba = xb + h;
-    vq1 = ld4(vxi + (ptrdiff_t)(xaa - 3) * (ptrdiff_t)ld);
-    vq2 = ld4(vxi + (ptrdiff_t)(xaa - 2) * (ptrdiff_t)ld);
-    vq3 = ld4(vxi + (ptrdiff_t)(xaa - 1) * (ptrdiff_t)ld);
-    for (int L = xaa; L <= xba + 2; ++L) {
-        // ---- step A: p at PA = L-1 ----
-        const int PA = L - 1;
-        const ptrdiff_t colA = (ptrdiff_t)PA * (ptrdiff_t)ld;
-        const ptrdiff_t colV0 = (ptrdiff_t)(L - 3) * (ptrdiff_t)ld;
-        const float4 xa4 = XF ? make_float4(1.0f, la.kx, 1.0f, la.kx) : __ldg(S.xcoef + (PA + S2D_GX));
-        const bool colm = XF || xa4.x == 1.0f;
+    vq1 = ld4(vxi + (ptrdiff_t)(xa - 3) * (ptrdiff_t)ld);
+    vq2 = ld4(vxi + (ptrdiff_t)(xa - 2) * (ptrdiff_t)ld);
+    vq3 = ld4(vxi + (ptrdiff_t)(xa - 1) * (ptrdiff_t)ld);
+    for (int L = xa; L <= xb + 2; ++L) {
+        const int P = L - 1;
+        const ptrdiff_t colP = (ptrdiff_t)P * (ptrdiff_t)ld;
+        const float4 xc = XF ? make_float4(1.0f, la.kx, 1.0f, la.kx) : __ldg(S.xcoef + (P + S2D_GX));
+        const bool colm = XF || xc.x == 1.0f;
         const bool pz_live = !(FAST && colm);
-        const float4 cvx = ld4(vxi + (ptrdiff_t)L * (ptrdiff_t)ld);
-        const float4 cvz = ld4(vzi + colA);
-        const float4 cpx = ld4(pxi + colA);
-        const float4 cpz = pz_live ? ld4(pzi + colA) : zero;
-        const float4 ckk = ld4(kap + colA);
-        const float4 cbx = ld4(bxp + colV0);
-        const float4 cbz = ld4(bzp + colV0);
         vq0 = vq1; vq1 = vq2; vq2 = vq3;
-        vq3 = cvx;
-        const float4 vz = cvz;
+        vq3 = ld4(vxi + (ptrdiff_t)L * (ptrdiff_t)ld);
+        const float4 vz = ld4(vzi + colP);
         float4 pxn, pzn, dxv, dzv;
-        const float4 kka = ckk;
-        const float4 pn =
-            p_update<FAST, XF>(la, S, PA, xa4, colm, vq0, vq1, vq2, vq3, cpx, cpz, kka, vz, pxn, pzn, dxv, dzv);
-        const bool in_a = PA >= xa && PA < xb;
-        if (TWO) {
-            ring_at(ring, 0, PA, lane) = pxn;
-            ring_at(ring, 1, PA, lane) = pzn;
-        } else if (in_a && la.owner) {
-            st4(pxo + colA, pxn);
-            if (pz_live) st4(pzo + colA, pzn);
+        const float4 pn = p_update<FAST, XF>(la, S, P, xc, colm, vq0, vq1, vq2, vq3, ld4(pxi + colP),
+                                             pz_live ? ld4(pzi + colP) : zero, ld4(kap + colP), vz, pxn, pzn, dxv,
+                                             dzv);
+        const bool in_seg = P >= xa && P < xb;
+        if (in_seg && la.owner) {
+            st4(pxo + colP, pxn);
+            if (pz_live) st4(pzo + colP, pzn);
         }
-        if (rec_a && in_a) record(la, S, PA, pn, slot_a);
+        if (rec && in_seg) record(la, S, P, pn, slot);
         pq0 = pq1; pq1 = pq2; pq2 = pq3; pq3 = pn;
         zq0 = zq1; zq1 = zq2; zq2 = vz;
-        if (L < xaa + 3) continue;
-        // ---- step A: v at VA = L-3 ----
-        const int VA = L - 3;
-        const ptrdiff_t colVA = (ptrdiff_t)VA * (ptrdiff_t)ld;
-        float4 vxn, vzn, dxp, dzp;
-        const float4 bxa = cbx, bza = cbz;
-        v_update<FAST, XF>(la, S, VA, pq0, pq1, pq2, pq3, vq0, zq0, bxa, bza, vxn, vzn, dxp, dzp);
-        if (!TWO) {
-            if (la.owner) {
-                st4(vxo + colVA, vxn);
-                st4(vzo + colVA, vzn);
-            }
-            continue;
-        }
-        ring_at(ring, 2, VA, lane) = vzn;
-        ring_at(ring, 3, VA, lane) = vxn;
         if (L < xa + 3) continue;
-        // ---- step B: p at PB = L-4 ----
-        const int PB = L - 4;
-        const ptrdiff_t colB = (ptrdiff_t)PB * (ptrdiff_t)ld;
-        const float4 vzb = ring_at(ring, 2, PB, lane);
-        const float4 xb4 = XF ? make_float4(1.0f, lb.kx, 1.0f, lb.kx) : __ldg(S.xcoef + (PB + S2D_GX));
-        const bool colmb = XF || xb4.x == 1.0f;
-        const bool pz_liveb = !(FAST && colmb);
-        float4 pxm, pzm, dxw, dzw;
-        const float4 pm = p_update<FAST, XF>(lb, S, PB, xb4, colmb, ring_at(ring, 3, PB - 2, lane),
-                                             ring_at(ring, 3, PB - 1, lane),
-                                   ring_at(ring, 3, PB, lane), ring_at(ring, 3, PB + 1, lane), ring_at(ring, 0, PB, lane),
-                                   pz_liveb ? ring_at(ring, 1, PB, lane) : zero, ld4(kap + colB), vzb,
-                                   pxm, pzm, dxw, dzw);
-        const bool in_b = PB >= xa && PB < xb;
-        if (in_b && la.owner) {
-            st4(pxo + colB, pxm);
-            if (pz_liveb) st4(pzo + colB, pzm);
-        }
-        if (rec_b && in_b) record(lb, S, PB, pm, slot_b);
-        ring_at(ring, 4, PB, lane) = pm;
-        if (L < xa + 6) continue;
-        // ---- step B: v at VB = L-6 ----
-        const int VB = L - 6;
-        const ptrdiff_t colVB = (ptrdiff_t)VB * (ptrdiff_t)ld;
-        float4 vxm, vzm, dxq, dzq;
-        v_update<FAST, XF>(lb, S, VB, ring_at(ring, 4, VB - 1, lane), ring_at(ring, 4, VB, lane),
-                           ring_at(ring, 4, VB + 1, lane),
-                 ring_at(ring, 4, VB + 2, lane), ring_at(ring, 3, VB, lane), ring_at(ring, 2, VB, lane),
-                 ld4(bxp + colVB), ld4(bzp + colVB), vxm, vzm, dxq, dzq);
+        const int V = L - 3;
+        const ptrdiff_t colV = (ptrdiff_t)V * (ptrdiff_t)ld;
+        float4 vxn, vzn, dxp, dzp;
+        v_update<FAST, XF>(la, S, V, pq0, pq1, pq2, pq3, vq0, zq0, ld4(bxp + colV), ld4(bzp + colV), vxn, vzn, dxp,
+                           dzp);
         if (la.owner) {
-            st4(vxo + colVB, vxm);
-            st4(vzo + colVB, vzm);
+            st4(vxo + colV, vxn);
+            st4(vzo + colV, vzn);
         }
     }
 }
 
-template <bool TWO>
-__global__ void __launch_bounds__(128, 4) step_kernel_ts(const StepArgs *__restrict__ A, int kt_off) {
+// The two-step task, two rows at a time (packed FP32), with the columns
+// brought in kTs2Depth - 1 ahead by per-lane asynchronous copies (16 bytes, the
+// lane's four rows) into a per-warp ring.  Iteration L consumes vx at L, px,
+// vz, kappa (and pz) at L-1 and bx, bz at L-3; each lane reads back only what
+// it copied, so the copies' own wait is the whole synchronisation.  Every
+// window (step A: vx, p, vz; step B: vx, vz, p; kappa, bx, bz for step B) is
+// four columns of registers, rotating through the names of a loop unrolled by
+// four: no moves, no delay lines (interior tasks: literal row and column
+// coefficients, every cell carrying p alone).  The others keep their row
+// coefficients in shared memory (the lane's own four rows), read a column's
+// from xcoef, and pass step A's px, pz to step B through 4-column delay lines.
+struct Ts2Win {
+    V4 vx, pa, vz, vb, zb, pb, kk, bx, bz;  // one column of each window
+};
+
+struct Ts2Task {
+    V4 *ring;         // this lane's part of the warp's shared memory
+    V4 *tab, *delay;  // row coefficients (daz, kz, dbz, lz, D- pair, D+ pair); px, pz of step A
+    int xa, xb, src_x, sdz, nnx;
+    float amp_a, amp_b;
+    bool owner;
+    V4 A0, A1, one, kx, kz;  // literal pair; 1; interior kx, kz
+};
+// Column coefficients of one iteration (tasks outside the x-interior): those
+// of the pressure columns L-1, L-4 (Dax, Kx) and the velocity columns L-3, L-6
+// (Dbx, Lx), read one iteration ahead.
+struct Ts2Xc {
+    float2 pa, va, pb, vb;
+    __device__ __forceinline__ void read(const float4 *xcoef, int nnx, int L) {
+        auto at = [&](int x) {
+            return reinterpret_cast<const float2 *>(xcoef + (min(max(x, -S2D_GX), nnx + S2D_GX - 1) + S2D_GX));
+        };
+        pa = __ldg(at(L - 1));
+        va = __ldg(at(L - 3) + 1);
+        pb = __ldg(at(L - 4));
+        vb = __ldg(at(L - 6) + 1);
+    }
+};
+
+__device__ __forceinline__ void ts2_source(V4 &p, int sdz, float amp) {
+    if (sdz == 0) p.a = pk(lo(p.a) + amp, hi(p.a));
+    else if (sdz == 1) p.a = pk(lo(p.a), hi(p.a) + amp);
+    else if (sdz == 2) p.b = pk(lo(p.b) + amp, hi(p.b));
+    else if (sdz == 3) p.b = pk(lo(p.b), hi(p.b) + amp);
+}
+
+// Kinds of tasks: interior; interior columns, other rows; anything.
+enum { kTsIn = 0, kTsRows = 1, kTsAny = 2 };
+
+// New p at column P from vx at P-2 .. P+1, vz, kappa and the old px, pz there;
+// the new px, pz in px, pz (kTsIn: px = p).  xc: Dax, Kx of the column (kTsAny).
+template <int KIND>
+__device__ __forceinline__ V4 ts2_pressure(const Ts2Task &k, int P, const float2 &xc, const V4 &v0, const V4 &v1,
+                                           const V4 &v2, const V4 &v3, const V4 &vz, const V4 &kk, V4 &px, V4 &pz,
+                                           float amp) {
+    if (KIND == kTsIn) {
+        const V4 dx = dif4(k.A0, v2 - v1, k.A1, v3 - v0);
+        const V4 dz = dminus_z(k.A0, k.A1, vz);
+        px = fma4(kk, dif4(k.kx, dx, k.kz, dz), px);
+        if (P == k.src_x) ts2_source(px, k.sdz, amp);
+        return px;
+    }
+    const V4 daz = k.tab[0], kz = k.tab[32];
+    V4 dax = k.one, kx = k.kx, c0 = k.A0, c1 = k.A1;
+    if (KIND == kTsAny) {
+        float a0, a1;
+        dm_coef(P, k.nnx, a0, a1);
+        c0 = dup4(a0);
+        c1 = dup4(a1);
+        dax = dup4(xc.x);
+        kx = dup4(xc.y);
+    }
+    const V4 dx = dif4(c0, v2 - v1, c1, v3 - v0);
+    const V4 dz = dminus_z(k.tab[4 * 32], k.tab[5 * 32], vz);
+    V4 ps = fma4(dax, px, (kx * kk) * dx);
+    V4 pn = fma4(daz, pz, (kz * kk) * dz);
+    if (KIND == kTsRows || xc.x == 1.0f) {  // cells whose row is undamped too carry p alone
+        const V4 pm = fma4(kk, dif4(kx, dx, kz, dz), px);
+        const bool r0 = lo(daz.a) == 1.0f, r1 = hi(daz.a) == 1.0f, r2 = lo(daz.b) == 1.0f, r3 = hi(daz.b) == 1.0f;
+        ps = v4(pk(r0 ? lo(pm.a) : lo(ps.a), r1 ? hi(pm.a) : hi(ps.a)),
+                pk(r2 ? lo(pm.b) : lo(ps.b), r3 ? hi(pm.b) : hi(ps.b)));
+        pn = v4(pk(r0 ? 0.0f : lo(pn.a), r1 ? 0.0f : hi(pn.a)), pk(r2 ? 0.0f : lo(pn.b), r3 ? 0.0f : hi(pn.b)));
+    }
+    if (P == k.src_x) ts2_source(ps, k.sdz, amp);
+    px = ps;
+    pz = pn;
+    return ps + pn;
+}
+
+// Velocities at column V from p at V-1 .. V+2.  bx, bz: Lx bx, Lz bz (rounded
+// as upd() rounds them); xc.x: Dbx (kTsAny).
+template <int KIND>
+__device__ __forceinline__ void ts2_velocity(const Ts2Task &k, int V, const float2 &xc, const V4 &p0, const V4 &p1,
+                                             const V4 &p2, const V4 &p3, const V4 &bx, const V4 &bz, V4 &vx, V4 &vz) {
+    V4 c0 = k.A0, c1 = k.A1;
+    if (KIND == kTsAny) {
+        float a0, a1;
+        dp_coef(V, k.nnx, a0, a1);
+        c0 = dup4(a0);
+        c1 = dup4(a1);
+    }
+    const V4 ex = dif4(c0, p2 - p1, c1, p3 - p0);
+    const V4 ez = KIND == kTsIn ? dplus_z(k.A0, k.A1, p1) : dplus_z(k.tab[6 * 32], k.tab[7 * 32], p1);
+    vx = fma4(KIND == kTsAny ? dup4(xc.x) : k.one, vx, bx * ex);
+    vz = fma4(KIND == kTsIn ? k.one : k.tab[2 * 32], vz, bz * ez);
+}
+
+// Column L.  w0 holds the oldest column of every window and receives the
+// newest (vx at L; p, vz, kappa at L-1; step A's velocities and bx, bz at L-3;
+// step B's p at L-4); w1 .. w3 the three columns before, w3 the latest.
+template <int KIND, class Rec>
+__device__ __forceinline__ void ts2_column(const Ts2Task &k, const Ts2Xc &xc, const V4 *in, int L, float *pxo,
+                                           float *pzo, float *vxo, float *vzo, Ts2Win &w0, const Ts2Win &w1,
+                                           const Ts2Win &w2, const Ts2Win &w3, Rec rec) {
+    const V4 vx = in[0], vz = in[64], kk = in[96];
+    // ---- step A: p at L-1, velocities at L-3 ----
+    V4 px = in[32], pz = KIND == kTsIn ? zero4() : in[192];
+    const V4 p = ts2_pressure<KIND>(k, L - 1, xc.pa, w1.vx, w2.vx, w3.vx, vx, vz, kk, px, pz, k.amp_a);
+    rec(0, L - 1, p);
+    const V4 bx = (KIND == kTsAny ? dup4(xc.va.y) : k.kx) * in[128];
+    const V4 bz = (KIND == kTsIn ? k.kz : k.tab[3 * 32]) * in[160];
+    V4 va = w1.vx, za = w2.vz;
+    ts2_velocity<KIND>(k, L - 3, xc.va, w1.pa, w2.pa, w3.pa, p, bx, bz, va, za);
+    // ---- step B: p at L-4, velocities at L-6 ----
+    V4 qx = w1.pa, qz = zero4();
+    if (KIND != kTsIn) {
+        // step A's px, pz of column L-4, whose place column L-1's then takes
+        V4 *d = k.delay + (L - 1 & 3) * 64, *e = k.delay + (L & 3) * 64;  // L-4 = L (mod 4)
+        qx = e[0];
+        qz = e[32];
+        d[0] = px;
+        d[32] = pz;
+    }
+    const V4 q = ts2_pressure<KIND>(k, L - 4, xc.pb, w1.vb, w2.vb, w3.vb, va, w3.zb, w1.kk, qx, qz, k.amp_b);
+    rec(1, L - 4, q);
+    if (k.owner && L - 4 >= k.xa && L - 4 < k.xb) {
+        *reinterpret_cast<V4 *>(pxo) = qx;
+        if (KIND != kTsIn) *reinterpret_cast<V4 *>(pzo) = qz;
+    }
+    V4 vn = w1.vb, zn = w1.zb;
+    ts2_velocity<KIND>(k, L - 6, xc.vb, w1.pb, w2.pb, w3.pb, q, w1.bx, w1.bz, vn, zn);
+    if (k.owner && L - 6 >= k.xa && L - 6 < k.xb) {
+        *reinterpret_cast<V4 *>(vxo) = vn;
+        *reinterpret_cast<V4 *>(vzo) = zn;
+    }
+    w0.vx = vx;
+    w0.pa = p;
+    w0.vz = vz;
+    w0.vb = va;
+    w0.zb = za;
+    w0.pb = q;
+    w0.kk = kk;
+    w0.bx = bx;
+    w0.bz = bz;
+}
+
+template <int KIND>
+__device__ __forceinline__ void ts2_task(const StepArgs &a, const ShotDev &S, int strip, int xa, int seg_len, int kt,
+                                         int par, int lane, V4 *smem) {
+    const int xb = min(S.nnx, xa + seg_len);
+    const ptrdiff_t ld = (ptrdiff_t)S.ld;
+    const int c = strip * S2D_TS_OUT - 8;
+    Lane<true> la;  // rows and source of the lane
+    lane_setup(la, S, c, lane, kt);
+    la.owner = lane >= 2 && lane <= 29;
+    Ts2Task k;
+    k.ring = smem + lane;
+    k.delay = k.ring + kTs2Depth * kTs2Slots * 32;
+    k.tab = k.delay + 8 * 32;
+    k.xa = xa;
+    k.xb = xb;
+    k.src_x = __any_sync(kFull, la.sdz >= 0 && la.sdz < 4) ? la.src_x : INT_MIN;  // none of the warp's rows: no column
+    k.nnx = S.nnx;
+    k.sdz = la.sdz;
+    k.amp_a = la.amp;
+    k.amp_b = __ldg(S.amp + kt + 1);
+    k.owner = la.owner;
+    k.A0 = dup4(kA0);
+    k.A1 = dup4(kA1);
+    k.kx = dup4(la.kx);
+    k.kz = dup4(la.kz);
+    // 1, read so that the compiler does not know it: a fused multiply-add by a
+    // literal 1 would fuse the product of its addend too
+    k.one = dup4(a.one);
+    if (KIND != kTsIn) {
+        float r[8][4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float4 q = __ldg(la.zc + i);
+            r[0][i] = q.x;
+            r[1][i] = q.y;
+            r[2][i] = q.z;
+            r[3][i] = q.w;
+            dm_coef(la.z0 + i, S.nnz, r[4][i], r[5][i]);
+            dp_coef(la.z0 + i, S.nnz, r[6][i], r[7][i]);
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) k.tab[i * 32] = v4(pk(r[i][0], r[i][1]), pk(r[i][2], r[i][3]));
+    }
+    const bool rows =
+        !(a.flags & S2D_STEP_NO_RECORD) && S.nrec > 0 && c + S2D_STRIP_ROWS > S.rec_zlo && c <= S.rec_zhi;
+    const int slot_a = (kt + 1) / a.dt_factor - 1, slot_b = (kt + 2) / a.dt_factor - 1;
+    const bool rec_a = rows && (kt + 1) % a.dt_factor == 0 && slot_a < S.real_nt;
+    const bool rec_b = rows && (kt + 2) % a.dt_factor == 0 && slot_b < S.real_nt;
+    const size_t off = (size_t)(la.z0 + S2D_GZ) + (size_t)S2D_GX * ld;
+    const int fs = S.fstride;
+    const float *const sb = S.st[0][0] + off + (size_t)par * 4 * fs;
+    float *const so = S.st[0][0] + off + (size_t)(par ^ 1) * 4 * fs;
+    const float *const mb = S.kappa + off;
+    const int nnx = S.nnx;
+    const int L0 = xa - 6, Lend = xb + 5;  // columns L0 .. L0+2 fill the vx window
+    const int n4 = (Lend - (xa - 3) + 4) / 4;  // groups of four columns (the last may pass Lend)
+    const int Llast = KIND == kTsIn ? xa - 3 + 4 * n4 - 1 : Lend;
+    // Iteration L's copies into ring slot (L - L0) mod kTs2Depth.  px at the
+    // next iteration's column L-1 and kappa there; the other pieces lie at fixed
+    // distances.  kTsAny: what lies outside the allocation (columns -8 ..
+    // nnx+7) is not needed and not copied.
+    const float *np = sb + (ptrdiff_t)(L0 - 1) * ld, *nm = mb + (ptrdiff_t)(L0 - 1) * ld;
+    const ptrdiff_t ovx = ld + 2 * (ptrdiff_t)fs, ovz = 3 * (ptrdiff_t)fs, obx = fs - 2 * ld,
+                    obz = 2 * (ptrdiff_t)fs - 2 * ld;
+    auto issue = [&](int L, int slot) {
+        V4 *st = k.ring + slot * (kTs2Slots * 32);
+        const bool in_l = KIND != kTsAny || L < nnx + S2D_GX, in_b = KIND != kTsAny || L - 3 >= -S2D_GX;
+        if (in_l) cp_async16(st, np + ovx, true);
+        cp_async16(st + 32, np, true);
+        cp_async16(st + 64, np + ovz, true);
+        cp_async16(st + 96, nm, true);
+        if (in_b) {
+            cp_async16(st + 128, nm + obx, true);
+            cp_async16(st + 160, nm + obz, true);
+        }
+        if (KIND != kTsIn) cp_async16(st + 192, np + fs, true);
+        np += ld;
+        nm += ld;
+    };
+#pragma unroll
+    for (int i = 0; i < kTs2Depth - 1; ++i) {
+        issue(L0 + i, i);
+        cp_async_commit();
+    }
+    // bring iteration L + kTs2Depth - 1, wait for iteration L (in slot i)
+    auto next = [&](int L, int i) {
+        if (L + kTs2Depth - 1 <= Llast) issue(L + kTs2Depth - 1, (i + kTs2Depth - 1) % kTs2Depth);
+        cp_async_commit();
+        cp_async_wait<kTs2Depth - 1>();
+        return k.ring + i * (kTs2Slots * 32);
+    };
+    RecCursor ca, cb;
+    if (rec_a) ca.start(S, xa);
+    if (rec_b) cb.start(S, xa);
+    auto rec = [&](int step, int P, const V4 &p) {
+        if (!(step ? rec_b : rec_a) || P < xa || P >= xb) return;
+        (step ? cb : ca).column(S, P, la.z0, la.owner, step ? slot_b : slot_a, [&](int i) {
+            return i == 0 ? lo(p.a) : i == 1 ? hi(p.a) : i == 2 ? lo(p.b) : hi(p.b);
+        });
+    };
+    Ts2Win wa, wb, wc, wd;
+    {
+        const V4 z = zero4();
+        wa.vx = wa.pa = wa.vz = wa.vb = wa.zb = wa.pb = wa.kk = wa.bx = wa.bz = z;
+        wb = wc = wd = wa;
+    }
+    wb.vx = next(L0, 0)[0];
+    wc.vx = next(L0 + 1, 1)[0];
+    wd.vx = next(L0 + 2, 2)[0];
+    float *pxo = so + (ptrdiff_t)(xa - 7) * ld, *pzo = pxo + fs;      // column L-4
+    float *vxo = so + (ptrdiff_t)(xa - 9) * ld + 2 * (ptrdiff_t)fs;   // column L-6
+    float *vzo = vxo + fs;
+    int L = xa - 3;
+    Ts2Xc xc{};
+    if (KIND == kTsIn) {
+        for (int g = 0; g < n4; ++g) {
+            ts2_column<KIND>(k, xc, next(L, 3), L, pxo, pzo, vxo, vzo, wa, wb, wc, wd, rec);
+            ts2_column<KIND>(k, xc, next(L + 1, 0), L + 1, pxo + ld, pzo + ld, vxo + ld, vzo + ld, wb, wc, wd, wa, rec);
+            ts2_column<KIND>(k, xc, next(L + 2, 1), L + 2, pxo + 2 * ld, pzo + 2 * ld, vxo + 2 * ld, vzo + 2 * ld, wc, wd,
+                             wa, wb, rec);
+            ts2_column<KIND>(k, xc, next(L + 3, 2), L + 3, pxo + 3 * ld, pzo + 3 * ld, vxo + 3 * ld, vzo + 3 * ld, wd, wa,
+                             wb, wc, rec);
+            L += 4;
+            pxo += 4 * ld;
+            pzo += 4 * ld;
+            vxo += 4 * ld;
+            vzo += 4 * ld;
+        }
+    } else {
+        // not unrolled: the windows move, but the code of the few tasks at the
+        // grid's rim stays out of the interior tasks' instruction cache
+        if (KIND == kTsAny) xc.read(S.xcoef, S.nnx, L);
+        int slot = 3;
+#pragma unroll 1
+        for (; L <= Lend; ++L) {
+            Ts2Xc xn{};
+            if (KIND == kTsAny) xn.read(S.xcoef, S.nnx, L + 1);
+            ts2_column<KIND>(k, xc, next(L, slot), L, pxo, pzo, vxo, vzo, wa, wb, wc, wd, rec);
+            slot = (slot + 1) % kTs2Depth;
+            const Ts2Win t = wa;
+            wa = wb;
+            wb = wc;
+            wc = wd;
+            wd = t;
+            xc = xn;
+            pxo += ld;
+            pzo += ld;
+            vxo += ld;
+            vzo += ld;
+        }
+    }
+    cp_async_wait<0>();
+}
+
+// Two FD steps per launch: 255 registers and 22 KB of shared memory per warp, 8
+// warps per SM, three iterations of copies (9 KB per warp) in flight.
+// What bounds it: interior tasks alone run at the rate of a copy with their
+// access pattern (5.2 TB/s of the state's and materials' bytes, 450 Gcell/s on
+// 8 shots of 5120 x 5120, 275 instructions per column of 224 cell-updates); with
+// the rim tasks, whose columns cost 1.6 to 1.9 times as much, 371 Gcell/s (160
+// for the form it replaces: plain loads where they were used, step A in
+// shared-memory delay lines, 16 warps per SM).  One 3301 x 1301 shot, about one
+// round of tasks, is bound by a column's latency: 157 Gcell/s (102 one step
+// at a time).  Rim columns unrolled like the interior ones cost more than they
+// gained (instruction cache: 276 Gcell/s against 314 before the tasks were cut
+// by kind).
+__global__ void __launch_bounds__(128, 2) step_kernel_ts2(const StepArgs *__restrict__ A, int kt_off) {
     extern __shared__ __align__(128) unsigned char smem[];
     const StepArgs a = *A;
     const int lane = threadIdx.x & 31;
     const int gwarp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     const int nwarp = (int)((gridDim.x * blockDim.x) >> 5);
-    const int kt = a.kt_base + (TWO ? 2 : 1) * kt_off;
-    if (kt + (TWO ? 1 : 0) >= a.fd_nt) return;
+    const int kt = a.kt_base + 2 * kt_off;
+    if (kt + 1 >= a.fd_nt) return;
     const int par = a.par0 ^ (kt_off & 1);
-    float4 *ring = reinterpret_cast<float4 *>(smem + (size_t)(threadIdx.x >> 5) * kTsWarpBytes);
+    V4 *const mem = reinterpret_cast<V4 *>(smem + (size_t)(threadIdx.x >> 5) * kTs2WarpBytes);
     __shared__ ShotDev shot_rec[4];  // the task's shot record, one slot per warp
     ShotDev &S = shot_rec[(threadIdx.x >> 5) & 3];
-    for (int t = gwarp; t < a.total_tasks; t += nwarp) {
+    TaskQueue queue(a.queue, nwarp, lane);
+    for (int t = gwarp; t < a.total_tasks; t = queue.take()) {
+        queue.draw();
         int strip, xa, seg_len;
-        const ShotDev &G = task_of(a, t, strip, xa, seg_len);
+        const ShotDev &G = task_of_split(a, t, strip, xa, seg_len);
         warp_copy_shot(S, G, lane);
         const int c = strip * S2D_TS_OUT - 8;
         const bool zf = rows_fast(S, c, c + S2D_STRIP_ROWS - 1);
         // columns xa-4 .. xb+4 take part (step A's p reaches xb+4, feeding its v at xb+2)
         const bool xf = xa - 4 >= S.xfast_lo && min(S.nnx, xa + seg_len) + 4 < S.xfast_hi;
-        if (zf && xf) ts_task<true, TWO, true>(a, S, strip, xa, seg_len, kt, par, lane, ring);
-        else if (zf) ts_task<true, TWO, false>(a, S, strip, xa, seg_len, kt, par, lane, ring);
-        else if (xf) ts_task<false, TWO, true>(a, S, strip, xa, seg_len, kt, par, lane, ring);
-        else ts_task<false, TWO, false>(a, S, strip, xa, seg_len, kt, par, lane, ring);
+        if (zf && xf) ts2_task<kTsIn>(a, S, strip, xa, seg_len, kt, par, lane, mem);
+        else if (xf) ts2_task<kTsRows>(a, S, strip, xa, seg_len, kt, par, lane, mem);
+        else ts2_task<kTsAny>(a, S, strip, xa, seg_len, kt, par, lane, mem);
+    }
+    queue.leave();
+}
+
+// One step in the same strip layout (the last of an odd count).
+__global__ void __launch_bounds__(128, 4) step_kernel_ts1(const StepArgs *__restrict__ A, int kt_off) {
+    const StepArgs a = *A;
+    const int lane = threadIdx.x & 31;
+    const int gwarp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+    const int nwarp = (int)((gridDim.x * blockDim.x) >> 5);
+    const int kt = a.kt_base + kt_off;
+    if (kt >= a.fd_nt) return;
+    const int par = a.par0 ^ (kt_off & 1);
+    __shared__ ShotDev shot_rec[4];  // the task's shot record, one slot per warp
+    ShotDev &S = shot_rec[(threadIdx.x >> 5) & 3];
+    for (int t = gwarp; t < a.total_tasks; t += nwarp) {
+        int strip, xa, seg_len;
+        const ShotDev &G = task_of_split(a, t, strip, xa, seg_len);
+        warp_copy_shot(S, G, lane);
+        const int c = strip * S2D_TS_OUT - 8;
+        const bool zf = rows_fast(S, c, c + S2D_STRIP_ROWS - 1);
+        const bool xf = xa - 1 >= S.xfast_lo && min(S.nnx, xa + seg_len) + 1 < S.xfast_hi;
+        if (zf && xf) ts1_task<true, true>(a, S, strip, xa, seg_len, kt, par, lane);
+        else if (zf) ts1_task<true, false>(a, S, strip, xa, seg_len, kt, par, lane);
+        else if (xf) ts1_task<false, true>(a, S, strip, xa, seg_len, kt, par, lane);
+        else ts1_task<false, false>(a, S, strip, xa, seg_len, kt, par, lane);
     }
 }
 
@@ -1791,9 +2071,9 @@ int launch_step(int variant, const StepArgs *args_dev, int kt_off, int grid, int
     else if (variant == kVariantLdg128)
         step_kernel_ldg<false, 4><<<grid, block, 0, (cudaStream_t)stream>>>(args_dev, kt_off);
     else if (variant == kVariantTs2)
-        step_kernel_ts<true><<<grid, block, smem, (cudaStream_t)stream>>>(args_dev, kt_off);
+        step_kernel_ts2<<<grid, block, smem, (cudaStream_t)stream>>>(args_dev, kt_off);
     else if (variant == kVariantTs1)
-        step_kernel_ts<false><<<grid, block, smem, (cudaStream_t)stream>>>(args_dev, kt_off);
+        step_kernel_ts1<<<grid, block, 0, (cudaStream_t)stream>>>(args_dev, kt_off);
     else if (variant == kVariantO8)
         step_kernel_o8<3, false><<<grid, block, 0, (cudaStream_t)stream>>>(args_dev, kt_off);
     else if (variant == kVariantO8r)
@@ -1855,8 +2135,8 @@ const void *kernel_of(int variant) {
     if (variant == kVariantBulk128) return (const void *)step_kernel_bulk<4>;
     if (variant == kVariantLdgProducts) return (const void *)step_kernel_ldg<true, 3>;
     if (variant == kVariantLdg128) return (const void *)step_kernel_ldg<false, 4>;
-    if (variant == kVariantTs2) return (const void *)step_kernel_ts<true>;
-    if (variant == kVariantTs1) return (const void *)step_kernel_ts<false>;
+    if (variant == kVariantTs2) return (const void *)step_kernel_ts2;
+    if (variant == kVariantTs1) return (const void *)step_kernel_ts1;
     if (variant == kVariantO8) return (const void *)step_kernel_o8<3, false>;
     if (variant == kVariantO8r) return (const void *)step_kernel_o8<2, false>;
     if (variant == kVariantO8Products) return (const void *)step_kernel_o8<3, true>;
