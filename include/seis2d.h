@@ -215,13 +215,8 @@ S2D_API const char *s2d_last_error(const void *ctx);
  *   "products_variant" s2d_gradient's forward recompute that keeps the step
  *                 derivatives: 3 plain loads, 19 plain loads with the next
  *                 column prefetched (default)
- *   "adjoint_blocks" s2d_gradient adjoint kernel built for 2, 3 or 4 blocks
- *                 of 128 threads per SM, or 12: 2 blocks per SM with the next
- *                 column's loads issued before a column is computed, or
- *                 13 (default) / 14: 3 / 2 blocks per SM with the column
- *                 inputs copied into shared memory (cp.async) 1 / 2 columns
- *                 ahead, or 15: 3 blocks per SM with the per-shot inputs
- *                 copied 2 columns ahead; every form computes the same bits
+ *   "adjoint_blocks" 2, 3, 4 or 12 to 15 (default 13): names earlier builds of
+ *                 the 4th-order adjoint step; one build now serves them all
  *   "on_chip"     1 (default): 4th-order grids whose state fits the GPU's
  *                 registers and shared memory (up to about 1.2 M padded cells)
  *                 run all their steps in one cooperative launch per shot or

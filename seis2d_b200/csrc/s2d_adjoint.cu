@@ -32,61 +32,105 @@
 #include <cuda_runtime.h>
 
 #include "s2d_device.cuh"
+#include "s2d_pack.cuh"
 
 namespace s2d {
 
 namespace {
 
-__device__ __forceinline__ float xc0m(int i, int n) { float c0, c1; dm_coef(i, n, c0, c1); return c0; }
-__device__ __forceinline__ float xc1m(int i, int n) { float c0, c1; dm_coef(i, n, c0, c1); return c1; }
-__device__ __forceinline__ float xc0p(int i, int n) { float c0, c1; dp_coef(i, n, c0, c1); return c0; }
-__device__ __forceinline__ float xc1p(int i, int n) { float c0, c1; dp_coef(i, n, c0, c1); return c1; }
+// Kinds of tasks: interior (literal row and column coefficients, every cell
+// carrying one pressure); interior columns, other rows; anything.
+enum { kAdjIn = 0, kAdjRows = 1, kAdjAny = 2 };
 
+// t0 a + t1 b + t2 c + t3 d, second product rounded, then fused in the order of
+// t0, t2, t3 (the transposes' four taps; t1 and t3 hold the negated
+// coefficients).
+__device__ __forceinline__ V4 taps4(const V4 &t0, const V4 &a, const V4 &t1, const V4 &b, const V4 &t2, const V4 &c,
+                                    const V4 &t3, const V4 &d) {
+    return fma4(t3, d, fma4(t2, c, fma4(t0, a, t1 * b)));
+}
+struct Taps {
+    V4 t0, t1, t2, t3;
+};
+// The taps of a lane's rows.  Even rows round and fuse as taps4, odd rows round
+// the first product and fuse the second (the sums that this kernel's results
+// have always had, kept bit for bit); a packed pair does both when the odd
+// halves of the first two coefficients, and of their operands, change places.
+__device__ __forceinline__ Taps row_taps(const V4 &t0, const V4 &t1, const V4 &t2, const V4 &t3) {
+    return Taps{v4(pk(lo(t0.a), hi(t1.a)), pk(lo(t0.b), hi(t1.b))), v4(pk(lo(t1.a), hi(t0.a)), pk(lo(t1.b), hi(t0.b))), t2,
+                t3};
+}
+// (H^T m) along z of the lane's rows: taps m[z-1], m[z], m[z-2], m[z+1].
+__device__ __forceinline__ V4 hzt(const Taps &t, const V4 &m) {
+    const float x = lo(m.a), y = hi(m.a), z = lo(m.b), w = hi(m.b);
+    const float up_z = __shfl_up_sync(kFull, z, 1), up_w = __shfl_up_sync(kFull, w, 1);
+    const float dn_x = __shfl_down_sync(kFull, x, 1);
+    return taps4(t.t0, v4(pk(up_w, y), pk(y, w)), t.t1, v4(dup(x), dup(z)), t.t2, v4(pk(up_z, up_w), m.a), t.t3,
+                 v4(pk(y, z), pk(w, dn_x)));
+}
+// (G^T m): taps m[z], m[z+1], m[z-1], m[z+2].
+__device__ __forceinline__ V4 gzt(const Taps &t, const V4 &m) {
+    const float x = lo(m.a), y = hi(m.a), z = lo(m.b), w = hi(m.b);
+    const float up_w = __shfl_up_sync(kFull, w, 1);
+    const float dn_x = __shfl_down_sync(kFull, x, 1), dn_y = __shfl_down_sync(kFull, y, 1);
+    return taps4(t.t0, v4(pk(x, z), pk(z, dn_x)), t.t1, v4(dup(y), dup(w)), t.t2, v4(pk(up_w, x), pk(y, z)), t.t3,
+                 v4(m.b, pk(dn_x, dn_y)));
+}
 
-// (H^T m) at the lane's 4 rows from m at those rows and the neighbours' edge
-// values (up_z = m[z0-2], up_w = m[z0-1], dn_x = m[z0+4]); pairs of rows z0-2 .. z0+4.
-template <bool FAST>
-__device__ __forceinline__ float4 hzt(const Lane<FAST> &ln, const float4 &m, float up_z, float up_w, float dn_x) {
-    float a0, a1, b0, b1, c0, c1, d0, d1, e0, e1, f0, f1, g0, g1;
-    zdp(ln, -2, a0, a1);
-    zdp(ln, -1, b0, b1);
-    zdp(ln, 0, c0, c1);
-    zdp(ln, 1, d0, d1);
-    zdp(ln, 2, e0, e1);
-    zdp(ln, 3, f0, f1);
-    zdp(ln, 4, g0, g1);
-    float4 r;
-    r.x = b0 * up_w - c0 * m.x + a1 * up_z - d1 * m.y;
-    r.y = c0 * m.x - d0 * m.y + b1 * up_w - e1 * m.z;
-    r.z = d0 * m.y - e0 * m.z + c1 * m.x - f1 * m.w;
-    r.w = e0 * m.z - f0 * m.w + d1 * m.y - g1 * dn_x;
-    return r;
-}
-// (G^T m) at the lane's 4 rows (up_w = m[z0-1], dn_x = m[z0+4], dn_y = m[z0+5]);
-// pairs of rows z0-1 .. z0+5.
-template <bool FAST>
-__device__ __forceinline__ float4 gzt(const Lane<FAST> &ln, const float4 &m, float up_w, float dn_x, float dn_y) {
-    float a0, a1, b0, b1, c0, c1, d0, d1, e0, e1, f0, f1, g0, g1;
-    zdm(ln, -1, a0, a1);
-    zdm(ln, 0, b0, b1);
-    zdm(ln, 1, c0, c1);
-    zdm(ln, 2, d0, d1);
-    zdm(ln, 3, e0, e1);
-    zdm(ln, 4, f0, f1);
-    zdm(ln, 5, g0, g1);
-    float4 r;
-    r.x = b0 * m.x - c0 * m.y + a1 * up_w - d1 * m.z;
-    r.y = c0 * m.y - d0 * m.z + b1 * m.x - e1 * m.w;
-    r.z = d0 * m.z - e0 * m.w + c1 * m.y - f1 * dn_x;
-    r.w = e0 * m.w - f0 * dn_x + d1 * m.z - g1 * dn_y;
-    return r;
-}
+// The adjoint source (transpose of the receiver sampling,
+// cpumodelling.cpp:356-360) of a task whose columns come in order.  The
+// receivers of column Q, and the first one's sample, are read ahead: the first
+// one's row and trace two columns, its sample one.
+struct AdjSource {
+    int j, je, jn, z, z1, id1;
+    float v;
+    __device__ __forceinline__ void entry(const ShotDev &S, int e, int &zz, int &id) {
+        e = min(e, S.nrec - 1);
+        zz = __ldg(S.rec_z + e);
+        id = __ldg(S.rec_id + e);
+    }
+    __device__ __forceinline__ float sample(const ShotDev &S, int id, int slot) {
+        return __ldg(S.seis + (size_t)id * S.real_nt + slot);
+    }
+    __device__ __forceinline__ void start(const ShotDev &S, int Q, int slot) {
+        j = __ldg(S.rec_ptr + Q);
+        je = __ldg(S.rec_ptr + min(Q + 1, S.nnx));
+        jn = __ldg(S.rec_ptr + min(Q + 2, S.nnx));
+        int id;
+        entry(S, j, z, id);
+        v = sample(S, id, slot);
+        entry(S, je, z1, id1);
+    }
+    __device__ __forceinline__ void add(V4 &q, int d, float r) {
+        if (d == 0) q.a = pk(lo(q.a) + r, hi(q.a));
+        else if (d == 1) q.a = pk(lo(q.a), hi(q.a) + r);
+        else if (d == 2) q.b = pk(lo(q.b) + r, hi(q.b));
+        else if (d == 3) q.b = pk(lo(q.b), hi(q.b) + r);
+    }
+    // Adds column Q's samples to the lane's rows z0 .. z0+3 of q.
+    __device__ __forceinline__ void column(const ShotDev &S, int Q, int z0, int slot, V4 &q) {
+        if (j < je) {
+            add(q, z - z0, v);
+            for (int e = j + 1; e < je; ++e) {
+                int zz, id;
+                entry(S, e, zz, id);
+                if (zz - z0 >= 0 && zz - z0 < 4) add(q, zz - z0, sample(S, id, slot));
+            }
+        }
+        j = je;
+        je = jn;
+        jn = __ldg(S.rec_ptr + min(Q + 3, S.nnx));
+        z = z1;
+        v = sample(S, id1, slot);
+        entry(S, je, z1, id1);
+    }
+};
 
 // One (shot, strip, segment) task of the adjoint step.  The warp streams
-// along x: at column L it loads mvx' (the x-gather of H^T needs it at
-// Q-2 .. Q+1); the pressure adjoint, the z-velocity adjoint and the imaging
-// terms are formed at Q = L-1, the x-velocity adjoint at W = L-3 (its G^T
-// x-gather needs Kx kappa mPX at W-1 .. W+2).
+// along x: iteration L brings mvx' and bx at L (the x-gather of H^T needs Lx bx
+// mvx' at Q-2 .. Q+1); the pressure adjoint, the z-velocity adjoint and the
+// imaging terms are formed at Q = L-1, the x-velocity adjoint at W = L-3 (its
+// G^T x-gather needs Kx kappa mPX at W-1 .. W+2).
 //
 // Cells where both pressure dampings are 1 run the forward with p alone
 // (p' = p + kappa (Kx a + Kz c)); their adjoint carries one pressure field
@@ -101,314 +145,328 @@ __device__ __forceinline__ float4 gzt(const Lane<FAST> &ln, const float4 &m, flo
 // rows there are zero), so the reference's last-row / last-column
 // replication adds nothing.  tbx(Q-1) comes from the previous column
 // (computed at Q = xa-1 too), tbz(z-1) from the lane above.
-// Per-warp shared-memory delay lines of the adjoint step (4 columns each):
-// mvx', Lx bx mvx' and Kx kappa mPX, the inputs of its x-gathers.
-constexpr int kAdjRing = 4, kAdjFields = 3;
-constexpr int kAdjWarpBytes = kAdjRing * kAdjFields * S2D_STRIP_ROWS * 4;
-__device__ __forceinline__ float4 &adj_ring(float4 *ring, int field, int col, int lane) {
-    return ring[(field * kAdjRing + ((col + 2 * S2D_GX) & (kAdjRing - 1))) * 32 + lane];
-}
+//
+// The inputs come as per-lane asynchronous copies (16 bytes, the lane's four
+// rows) into a per-warp ring, AdjDepth - 1 iterations ahead; the windows are
+// registers, rotating through the names of a loop unrolled by four (interior
+// tasks) or moved (the others, whose code then stays short).
+//
+// What bounds it: the latency of one column's chain (ring reads, three rounds
+// of shuffles), with two warps on each scheduler.  1201x401, 8 shots: 72.8
+// us/step (3.5 TB/s of DRAM traffic, 26% of the issue slots, the L1 and
+// shared-memory pipe at 53%), before with the windows in shared memory 104
+// us/step.  Three blocks per SM (168 registers, spilling) took 97 us/step; the
+// row coefficients in shared memory instead of registers 79 (the pipe again).
+// 2401x1201, 4 shots: 151 us/step.  Rim and interior tasks are cut apart
+// (kSplitAdj in the host code): without their tasks the interior alone takes
+// 40 us/step of the first case.
+constexpr int kAdjSlots = 11;  // mvx', bx; mpx, mvz, bz, kappa, three products; mpz, the fourth product
+template <int KIND>
+struct AdjDepth {
+    static constexpr int value = KIND == kAdjIn ? 4 : 3;
+};
+constexpr int kAdjRing = 36;    // 4 iterations of 9 pieces, or 3 of 11
+constexpr int kAdjWarpBytes = kAdjRing * S2D_STRIP_ROWS * 4;
+static_assert(kAdjRing >= 3 * kAdjSlots, "ring of the rim tasks");
 
-// The loads of one column L of the adjoint loop (prefetching form): mvx'
-// and bx at L; at Q = L-1 the column coefficients, mpx, mvz, mpz, bz, kappa
-// and the step's products (first two slots where the lane updates Q, last two
-// where Q is imaged).
-struct AdjIn {
-    float4 m, b, xq, mpx, mvz, mpz, bz, kk, pa, pc, pg, ph;
-    float lx;
+struct AdjWin {
+    V4 mvx, mg, mk;  // mvx', Lx bx mvx', Kx kappa mPX of one column
+};
+// Column coefficients of one iteration (kAdjAny): Lx at L; Dax, Kx, Lx at Q;
+// Dbx at W; read one iteration ahead.
+struct AdjXc {
+    float lxl, dbw;
+    float4 q;
+    __device__ __forceinline__ void read(const float4 *xcoef, int nnx, int L) {
+        auto at = [&](int x) { return xcoef + (min(max(x, -S2D_GX), nnx + S2D_GX - 1) + S2D_GX); };
+        lxl = __ldg(&at(L)->w);
+        q = __ldg(at(L - 1));
+        dbw = __ldg(&at(L - 3)->z);
+    }
 };
 
-// Asynchronous form: the eleven column inputs of AdjIn (mvx', bx at L;
-// mpx, mvz, mpz, bz, kappa and the four product slots at Q = L-1) as 16-byte
-// cp.async copies into a per-warp ring of AS columns, issued AS-1 columns
-// ahead, so the loads in flight hold no registers.  Each lane reads back only
-// what it copied; inputs a column does not use are zero-filled copies that
-// read nothing.
-// With 3 or more columns in the ring the materials (bx, bz, kappa: shared by
-// the shots, L2-resident) are loaded where they are used instead, and the ring
-// holds the eight per-shot inputs, so three columns fit three blocks per SM.
-__host__ __device__ constexpr int adj_async_slots(int as) { return as == 0 ? 0 : as < 3 ? 11 : 8; }
-__host__ __device__ constexpr int adj_async_stage_bytes(int as) { return adj_async_slots(as) * S2D_STRIP_ROWS * 4; }
+struct AdjTask {
+    const ShotDev *S;
+    V4 *ring;
+    int xa, xb, z0, kt, src_q, sdz, slot;
+    bool owner, inj, row0;
+    V4 one, kx, kz;
+    Taps xt, zt;   // literal taps along x and z
+    V4 daz, kzr, dbz, lzr;  // row coefficients and taps of the lane's rows (tasks that are not interior)
+    Taps hz, gz;
+    AdjSource src;
+    V4 tbp;        // tbx at Q-1
+};
 
-// XF: every column the task touches (xa-3 .. xb+2) lies in the shot's
-// x-interior: literal column coefficients, no coefficient loads.  PF: the
-// loads of column L+1 are issued before column L is computed (two columns
-// in flight per warp); AS > 0: asynchronous copies AS-1 columns ahead into
-// `aring`; otherwise each value is loaded where it is used.
-template <bool FAST, bool XF = false, bool PF = false, int AS = 0>
-__device__ __forceinline__ void adjoint_task(const StepArgs &a, const ShotDev &S, int strip, int xa, int seg_len,
-                                             int kt, int lane, float4 *ring, float4 *aring = nullptr) {
-    const int nnx = S.nnx;
-    const size_t ld = (size_t)S.ld;
-    const int xb = min(nnx, xa + seg_len);
-    const int c = strip * S2D_STRIP_OUT - 4;
-    Lane<FAST> ln;
-    lane_setup(ln, S, c, lane, kt);
-    const int z0 = ln.z0;
-    const int pin = (kt + 1) & 1, pout = kt & 1;
-    const size_t off = (size_t)(ln.zl + S2D_GZ) + (size_t)S2D_GX * ld;
-    const size_t F = (size_t)(nnx + 2 * S2D_GX) * ld;
-    // Every buffer below is distinct: restrict lets the compiler issue the
-    // accumulator and product loads ahead of the state stores.  (Per-field
-    // pointers here: the base-and-stride form the forward kernels use costs
-    // this kernel more address arithmetic than it saves in spills.)
-    const float *__restrict__ mpxi = S.st[pin][0] + off;
-    const float *__restrict__ mpzi = S.st[pin][1] + off;
-    const float *__restrict__ mvxi = S.st[pin][2] + off;
-    const float *__restrict__ mvzi = S.st[pin][3] + off;
-    float *__restrict__ mpxo = S.st[pout][0] + off;
-    float *__restrict__ mpzo = S.st[pout][1] + off;
-    float *__restrict__ mvxo = S.st[pout][2] + off;
-    float *__restrict__ mvzo = S.st[pout][3] + off;
-    const float *__restrict__ kap = S.kappa + off;
-    const float *__restrict__ bxp = S.bx + off;
-    const float *__restrict__ bzp = S.bz + off;
-    const float *__restrict__ pr = S.prod + (size_t)(kt - a.prod_kt0) * 4 * F + off;
-    float *__restrict__ gk = S.grad[0] + off;
-    float *__restrict__ gb = S.grad[1] + off;
-    // receiver adjoint source on recording steps, in strips whose rows hold
-    // receivers (the lookup is three dependent loads per column)
-    const bool inj = !(a.flags & S2D_STEP_NO_RECORD) && ((kt + 1) % a.dt_factor) == 0 &&
-                     (kt + 1) / a.dt_factor - 1 < S.real_nt && c + S2D_STRIP_ROWS > S.rec_zlo &&
-                     c <= S.rec_zhi;
-    const int slot = (kt + 1) / a.dt_factor - 1;
-    const bool row0 = FAST || z0 >= 1;  // the lane's first row has a row above it in the grid
-
-    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-    float4 tbp = zero;                                      // tbx at Q-1
-    const float kx = S.kx_in;
-    auto fetch = [&](int L, AdjIn &in) {
-        const ptrdiff_t colL = (ptrdiff_t)L * (ptrdiff_t)ld;
-        in.m = ld4(mvxi + colL);
-        in.b = ld4(bxp + colL);
-        in.lx = XF ? kx : __ldg(S.xcoef + (L + S2D_GX)).w;
-        if (L < xa) return;
-        const int Q = L - 1;
-        const ptrdiff_t colQ = (ptrdiff_t)Q * (ptrdiff_t)ld;
-        in.xq = XF ? make_float4(1.0f, kx, 1.0f, kx) : __ldg(S.xcoef + (Q + S2D_GX));
-        const bool pz_live = !(FAST && (XF || in.xq.x == 1.0f));
-        const bool upd = Q >= xa && Q < xb && ln.owner;
-        const bool img = Q >= 0 && Q < xb;
-        in.mpx = ld4(mpxi + colQ);
-        in.mvz = ld4(mvzi + colQ);
-        in.mpz = pz_live ? ld4(mpzi + colQ) : zero;
-        in.bz = ld4(bzp + colQ);
-        in.kk = ld4(kap + colQ);
-        in.pa = upd ? ld4(pr + colQ) : zero;
-        in.pc = upd && pz_live ? ld4(pr + F + colQ) : zero;
-        in.pg = img ? ld4(pr + 2 * F + colQ) : zero;
-        in.ph = img ? ld4(pr + 3 * F + colQ) : zero;
-    };
-    AdjIn cur, nxt;
-    if (PF) fetch(xa - 3, nxt);
-    // asynchronous form: iteration i is column L = xa-3+i; ring slots
-    // (times 32 float4) of its inputs
-    constexpr bool kMatRing = AS < 3;
-    constexpr int kSlots = adj_async_slots(AS);
-    constexpr int sM = 0, sB = 1, sPX = kMatRing ? 2 : 1, sVZ = sPX + 1, sPZ = sPX + 2, sBZ = 5, sKK = 6;
-    constexpr int sPA = kMatRing ? 7 : 4, sPC = sPA + 1, sPG = sPA + 2, sPH = sPA + 3;
-    const int n_it = xb - xa + 6;
-    auto issue = [&](int i) {
-        float4 *st = aring + (i % (AS > 0 ? AS : 1)) * kSlots * 32 + lane;
-        const int L = xa - 3 + i;
-        const ptrdiff_t colL = (ptrdiff_t)L * (ptrdiff_t)ld;
-        cp_async16(st + sM * 32, mvxi + colL, true);
-        if (kMatRing) cp_async16(st + sB * 32, bxp + colL, true);
-        if (L < xa) return;
-        const int Q = L - 1;
-        const ptrdiff_t colQ = (ptrdiff_t)Q * (ptrdiff_t)ld;
-        const bool pz_live = !(FAST && (XF || __ldg(S.xcoef + (Q + S2D_GX)).x == 1.0f));
-        const bool upd = Q >= xa && Q < xb && ln.owner;
-        const bool img = Q >= 0 && Q < xb;
-        cp_async16(st + sPX * 32, mpxi + colQ, true);
-        cp_async16(st + sVZ * 32, mvzi + colQ, true);
-        cp_async16(st + sPZ * 32, mpzi + colQ, pz_live);
-        if (kMatRing) {
-            cp_async16(st + sBZ * 32, bzp + colQ, true);
-            cp_async16(st + sKK * 32, kap + colQ, true);
-        }
-        cp_async16(st + sPA * 32, pr + colQ, upd);
-        cp_async16(st + sPC * 32, pr + F + colQ, upd && pz_live);
-        cp_async16(st + sPG * 32, pr + 2 * F + colQ, img);
-        cp_async16(st + sPH * 32, pr + 3 * F + colQ, img);
-    };
-    if constexpr (AS > 0) {
-#pragma unroll
-        for (int i = 0; i < AS - 1; ++i) {
-            if (i < n_it) issue(i);
-            cp_async_commit();
-        }
-    }
-    const float4 *as = aring;  // this column's ring slots (asynchronous form)
-
-    for (int L = xa - 3; L <= xb + 2; ++L) {
-        if (PF) {
-            cur = nxt;
-            if (L < xb + 2) fetch(L + 1, nxt);
-        }
-        if constexpr (AS > 0) {
-            const int i = L - (xa - 3);
-            if (i + AS - 1 < n_it) issue(i + AS - 1);
-            cp_async_commit();
-            cp_async_wait<AS - 1>();  // column L's copies have landed
-            as = aring + (i % AS) * kSlots * 32 + lane;
-        }
-        {
-            const ptrdiff_t colL = (ptrdiff_t)L * (ptrdiff_t)ld;
-            const float4 m = PF ? cur.m : AS ? as[sM * 32] : ld4(mvxi + colL);
-            const float4 b = PF ? cur.b : AS && kMatRing ? as[sB * 32] : ld4(bxp + colL);
-            const float lx = PF ? cur.lx : XF ? kx : __ldg(S.xcoef + (L + S2D_GX)).w;
-            adj_ring(ring, 0, L, lane) = m;
-            adj_ring(ring, 1, L, lane) = make_float4((lx * b.x) * m.x, (lx * b.y) * m.y, (lx * b.z) * m.z,
-                                                     (lx * b.w) * m.w);
-        }
-        if (L < xa) continue;
-        const int Q = L - 1;
-        const ptrdiff_t colQ = (ptrdiff_t)Q * (ptrdiff_t)ld;
-        const bool in_seg = Q >= xa && Q < xb;
-        const bool upd = in_seg && ln.owner;       // this lane writes column Q
-        const bool img = Q >= 0 && Q < xb;         // buoyancy terms at Q (xa-1 feeds column xa)
-        const float4 xq = PF ? cur.xq : XF ? make_float4(1.0f, kx, 1.0f, kx) : __ldg(S.xcoef + (Q + S2D_GX));
-        const bool colm = XF || xq.x == 1.0f;  // xq: Dax, Kx, Dbx, Lx at Q
-        const bool pz_live = !(FAST && colm);  // some cell of the column keeps mpz
-        const float4 mpx = PF ? cur.mpx : AS ? as[sPX * 32] : ld4(mpxi + colQ);
-        const float4 mvz = PF ? cur.mvz : AS ? as[sVZ * 32] : ld4(mvzi + colQ);
-        const float4 mpz = PF ? cur.mpz : AS ? as[sPZ * 32] : pz_live ? ld4(mpzi + colQ) : zero;
-        const float4 bz = PF ? cur.bz : AS && kMatRing ? as[sBZ * 32] : ld4(bzp + colQ);
-        const float4 kk = PF ? cur.kk : AS && kMatRing ? as[sKK * 32] : ld4(kap + colQ);
-        float4 pa = zero, pc = zero, pg = zero, ph = zero, tk = zero, tb = zero;
-        if (PF) {
-            pa = cur.pa;
-            pc = cur.pc;
-            pg = cur.pg;
-            ph = cur.ph;
-        } else if (AS) {
-            pa = as[sPA * 32];
-            pc = as[sPC * 32];
-            pg = as[sPG * 32];
-            ph = as[sPH * 32];
-        } else {
-            if (upd) {
-                pa = ld4(pr + colQ);
-                if (pz_live) pc = ld4(pr + F + colQ);
-            }
-            if (img) {
-                pg = ld4(pr + 2 * F + colQ);
-                ph = ld4(pr + 3 * F + colQ);
-            }
-        }
-        const float4 r0 = zrow(ln, 0), r1 = zrow(ln, 1), r2 = zrow(ln, 2), r3 = zrow(ln, 3);
-        // merged cells (both pressure dampings 1) carry one pressure adjoint
-        const bool m0 = colm && (FAST || r0.x == 1.0f), m1 = colm && (FAST || r1.x == 1.0f);
-        const bool m2 = colm && (FAST || r2.x == 1.0f), m3 = colm && (FAST || r3.x == 1.0f);
-        // ---- pressure adjoint at Q ----
-        const float4 h = make_float4((r0.w * bz.x) * mvz.x, (r1.w * bz.y) * mvz.y, (r2.w * bz.z) * mvz.z,
-                                     (r3.w * bz.w) * mvz.w);
-        float4 q = hzt(ln, h, __shfl_up_sync(kFull, h.z, 1), __shfl_up_sync(kFull, h.w, 1),
-                       __shfl_down_sync(kFull, h.x, 1));
-        {
-            const float p0a = XF ? kA0 : xc0p(Q - 1, nnx), p0b = XF ? kA0 : xc0p(Q, nnx);
-            const float p1a = XF ? kA1 : xc1p(Q - 2, nnx), p1b = XF ? kA1 : xc1p(Q + 1, nnx);
-            const float4 mg0 = adj_ring(ring, 1, L - 3, lane), mg1 = adj_ring(ring, 1, L - 2, lane);
-            const float4 mg2 = adj_ring(ring, 1, L - 1, lane), mg3 = adj_ring(ring, 1, L, lane);
-            q.x += p0a * mg1.x - p0b * mg2.x + p1a * mg0.x - p1b * mg3.x;
-            q.y += p0a * mg1.y - p0b * mg2.y + p1a * mg0.y - p1b * mg3.y;
-            q.z += p0a * mg1.z - p0b * mg2.z + p1a * mg0.z - p1b * mg3.z;
-            q.w += p0a * mg1.w - p0b * mg2.w + p1a * mg0.w - p1b * mg3.w;
-        }
-        // Transpose of the receiver sampling (cpumodelling.cpp:356-360).  Every
-        // warp computing column Q adds it (halo columns included, they feed the
-        // neighbours' velocity adjoint); the receiver table covers columns
-        // [0, nnx) only.
-        if (inj && Q >= 0 && Q < nnx) {
-            const int j1 = __ldg(S.rec_ptr + Q + 1);
-            for (int j = __ldg(S.rec_ptr + Q); j < j1; ++j) {
-                const int d = __ldg(S.rec_z + j) - z0;
-                if (d >= 0 && d < 4) {
-                    const float r = __ldg(S.seis + (size_t)__ldg(S.rec_id + j) * S.real_nt + slot);
-                    if (d == 0) q.x += r;
-                    else if (d == 1) q.y += r;
-                    else if (d == 2) q.z += r;
-                    else q.w += r;
-                }
-            }
-        }
-        const float4 mPX = make_float4(mpx.x + q.x, mpx.y + q.y, mpx.z + q.z, mpx.w + q.w);
-        const float4 mPZ = make_float4(m0 ? mPX.x : mpz.x + q.x, m1 ? mPX.y : mpz.y + q.y,
-                                       m2 ? mPX.z : mpz.z + q.z, m3 ? mPX.w : mpz.w + q.w);
-        if (upd) {
-            st4(mpxo + colQ, make_float4(xq.x * mPX.x, xq.x * mPX.y, xq.x * mPX.z, xq.x * mPX.w));
-            if (pz_live)
-                st4(mpzo + colQ, make_float4(m0 ? 0.0f : r0.x * mPZ.x, m1 ? 0.0f : r1.x * mPZ.y,
-                                             m2 ? 0.0f : r2.x * mPZ.z, m3 ? 0.0f : r3.x * mPZ.w));
-            // merged cells saved Kx a + Kz c in the first product slot
-            tk.x += m0 ? pa.x * mPX.x : (xq.y * pa.x) * mPX.x + (r0.y * pc.x) * mPZ.x;
-            tk.y += m1 ? pa.y * mPX.y : (xq.y * pa.y) * mPX.y + (r1.y * pc.y) * mPZ.y;
-            tk.z += m2 ? pa.z * mPX.z : (xq.y * pa.z) * mPX.z + (r2.y * pc.z) * mPZ.z;
-            tk.w += m3 ? pa.w * mPX.w : (xq.y * pa.w) * mPX.w + (r3.y * pc.w) * mPZ.w;
-            red_add4(gk + colQ, tk);
-            if (Q == S.src_x && ln.sdz >= 0 && ln.sdz < 4) S.srcadj[kt] = comp(mPX, ln.sdz);
-        }
-        adj_ring(ring, 2, Q, lane) = make_float4((xq.y * kk.x) * mPX.x, (xq.y * kk.y) * mPX.y, (xq.y * kk.z) * mPX.z,
-                          (xq.y * kk.w) * mPX.w);
-        // ---- z-velocity adjoint at Q ----
-        {
-            const float4 mc = make_float4((r0.y * kk.x) * mPZ.x, (r1.y * kk.y) * mPZ.y, (r2.y * kk.z) * mPZ.z,
-                                          (r3.y * kk.w) * mPZ.w);
-            const float4 g = gzt(ln, mc, __shfl_up_sync(kFull, mc.w, 1), __shfl_down_sync(kFull, mc.x, 1),
-                                 __shfl_down_sync(kFull, mc.y, 1));
-            if (upd)
-                st4(mvzo + colQ, make_float4(r0.z * mvz.x + g.x, r1.z * mvz.y + g.y, r2.z * mvz.z + g.z,
-                                             r3.z * mvz.w + g.w));
-        }
-        // ---- buoyancy imaging at Q ----
-        if (img) {
-            const float4 mv2 = adj_ring(ring, 0, Q, lane);
-            const float4 tbx = make_float4((xq.w * pg.x) * mv2.x, (xq.w * pg.y) * mv2.y, (xq.w * pg.z) * mv2.z,
-                                           (xq.w * pg.w) * mv2.w);
-            const float4 tbz = make_float4((r0.w * ph.x) * mvz.x, (r1.w * ph.y) * mvz.y, (r2.w * ph.z) * mvz.z,
-                                           (r3.w * ph.w) * mvz.w);
-            const float up = __shfl_up_sync(kFull, tbz.w, 1);
-            if (upd) {
-                const float4 px = Q >= 1 ? tbp : zero;
-                tb.x += 0.5f * ((tbx.x + px.x) + (tbz.x + (row0 ? up : 0.0f)));
-                tb.y += 0.5f * ((tbx.y + px.y) + (tbz.y + tbz.x));
-                tb.z += 0.5f * ((tbx.z + px.z) + (tbz.z + tbz.y));
-                tb.w += 0.5f * ((tbx.w + px.w) + (tbz.w + tbz.z));
-                red_add4(gb + colQ, tb);
-            }
-            tbp = tbx;
-        }
-        if (L < xa + 3) continue;
-        // ---- x-velocity adjoint at W = L - 3 ----
-        const int W = L - 3;
-        const ptrdiff_t colW = (ptrdiff_t)W * (ptrdiff_t)ld;
-        const float dbx = XF ? 1.0f : __ldg(S.xcoef + (W + S2D_GX)).z;
-        const float m0a = XF ? kA0 : xc0m(W, nnx), m0b = XF ? kA0 : xc0m(W + 1, nnx);
-        const float m1a = XF ? kA1 : xc1m(W - 1, nnx), m1b = XF ? kA1 : xc1m(W + 2, nnx);
-        const float4 mv0 = adj_ring(ring, 0, W, lane);
-        const float4 ma0 = adj_ring(ring, 2, W - 1, lane), ma1 = adj_ring(ring, 2, W, lane);
-        const float4 ma2 = adj_ring(ring, 2, W + 1, lane), ma3 = adj_ring(ring, 2, W + 2, lane);
-        float4 ovx;
-        ovx.x = dbx * mv0.x + (m0a * ma1.x - m0b * ma2.x + m1a * ma0.x - m1b * ma3.x);
-        ovx.y = dbx * mv0.y + (m0a * ma1.y - m0b * ma2.y + m1a * ma0.y - m1b * ma3.y);
-        ovx.z = dbx * mv0.z + (m0a * ma1.z - m0b * ma2.z + m1a * ma0.z - m1b * ma3.z);
-        ovx.w = dbx * mv0.w + (m0a * ma1.w - m0b * ma2.w + m1a * ma0.w - m1b * ma3.w);
-        if (ln.owner) st4(mvxo + colW, ovx);
-    }
-    if constexpr (AS > 0) cp_async_wait<0>();
+__device__ __forceinline__ void red4(float *p, const V4 &v) {
+    red_add4(p, make_float4(lo(v.a), hi(v.a), lo(v.b), hi(v.b)));
 }
 
-// MINB blocks of 4 warps per SM: 2 leaves the compiler its registers, 3 caps
-// them at 168 (12 warps per SM), 4 at 128 (16 warps per SM, some spills).
-// AS > 0: the asynchronous form with an AS-column copy ring per warp after
-// its delay lines.
-template <int MINB, bool PF = false, int AS = 0>
-__global__ void __launch_bounds__(128, MINB) adjoint_kernel(const StepArgs *__restrict__ A, int kt_off) {
+// Iteration L: w0 holds the oldest column of the windows and receives the
+// newest (mvx', mg at L; mk at L-1); w1 .. w3 the three before, w3 the latest.
+template <int KIND>
+__device__ __forceinline__ void adj_column(AdjTask &k, const AdjXc &xc, const V4 *in, int L, float *mpxo, float *mpzo,
+                                           float *mvxo, float *mvzo, float *gk, float *gb, AdjWin &w0,
+                                           const AdjWin &w1, const AdjWin &w2, const AdjWin &w3) {
+    const ShotDev &S = *k.S;
+    const V4 mvx = in[0];
+    const V4 mg = ((KIND == kAdjAny ? dup4(xc.lxl) : k.kx) * in[32]) * mvx;
+    const int Q = L - 1;
+    const bool upd = k.owner && Q >= k.xa && Q < k.xb;  // this lane writes column Q
+    const V4 mvz = in[96], kk = in[160];
+    const V4 kz = KIND == kAdjIn ? k.kz : k.kzr, lz = KIND == kAdjIn ? k.kz : k.lzr;
+    V4 dax = k.one, kx = k.kx, lx = k.kx;
+    Taps hx = k.xt, gx = k.xt;
+    if (KIND == kAdjAny) {
+        dax = dup4(xc.q.x);
+        kx = dup4(xc.q.y);
+        lx = dup4(xc.q.w);
+        float c0, c1;
+        dp_coef(Q - 1, S.nnx, c0, c1);
+        hx.t0 = dup4(c0);
+        dp_coef(Q, S.nnx, c0, c1);
+        hx.t1 = dup4(-c0);
+        dp_coef(Q - 2, S.nnx, c0, c1);
+        hx.t2 = dup4(c1);
+        dp_coef(Q + 1, S.nnx, c0, c1);
+        hx.t3 = dup4(-c1);
+        const int W = L - 3;
+        dm_coef(W, S.nnx, c0, c1);
+        gx.t0 = dup4(c0);
+        dm_coef(W + 1, S.nnx, c0, c1);
+        gx.t1 = dup4(-c0);
+        dm_coef(W - 1, S.nnx, c0, c1);
+        gx.t2 = dup4(c1);
+        dm_coef(W + 2, S.nnx, c0, c1);
+        gx.t3 = dup4(-c1);
+    }
+    const Taps &hz = KIND == kAdjIn ? k.zt : k.hz, &gz = KIND == kAdjIn ? k.zt : k.gz;
+    // ---- pressure adjoint at Q ----
+    V4 q = hzt(hz, (lz * in[128]) * mvz) + taps4(hx.t0, w2.mg, hx.t1, w3.mg, hx.t2, w1.mg, hx.t3, mg);
+    if (k.inj && Q >= 0 && Q < S.nnx && Q >= k.xa - 1) k.src.column(S, Q, k.z0, k.slot, q);
+    const V4 mPX = in[64] + q;
+    V4 mPZ = mPX, daz = k.one;
+    bool m0 = true, m1 = true, m2 = true, m3 = true;
+    V4 tk = in[192] * mPX;  // one pressure: the first product is Kx a + Kz c
+    if (KIND != kAdjIn) {
+        daz = k.daz;
+        const bool colm = KIND == kAdjRows || xc.q.x == 1.0f;
+        m0 = colm && lo(daz.a) == 1.0f;
+        m1 = colm && hi(daz.a) == 1.0f;
+        m2 = colm && lo(daz.b) == 1.0f;
+        m3 = colm && hi(daz.b) == 1.0f;
+        const V4 z = in[288] + q;
+        mPZ = v4(pk(m0 ? lo(mPX.a) : lo(z.a), m1 ? hi(mPX.a) : hi(z.a)),
+                 pk(m2 ? lo(mPX.b) : lo(z.b), m3 ? hi(mPX.b) : hi(z.b)));
+        const V4 ts = fma4(kx * in[192], mPX, (kz * in[320]) * mPZ);
+        tk = v4(pk(m0 ? lo(tk.a) : lo(ts.a), m1 ? hi(tk.a) : hi(ts.a)),
+                pk(m2 ? lo(tk.b) : lo(ts.b), m3 ? hi(tk.b) : hi(ts.b)));
+    }
+    if (upd) {
+        *reinterpret_cast<V4 *>(mpxo) = KIND == kAdjAny ? dax * mPX : mPX;
+        if (KIND != kAdjIn) {
+            const V4 o = daz * mPZ;
+            *reinterpret_cast<V4 *>(mpzo) = v4(pk(m0 ? 0.0f : lo(o.a), m1 ? 0.0f : hi(o.a)),
+                                               pk(m2 ? 0.0f : lo(o.b), m3 ? 0.0f : hi(o.b)));
+        }
+        red4(gk, tk);
+        if (Q == k.src_q && k.sdz >= 0 && k.sdz < 4)
+            S.srcadj[k.kt] = k.sdz == 0 ? lo(mPX.a) : k.sdz == 1 ? hi(mPX.a) : k.sdz == 2 ? lo(mPX.b) : hi(mPX.b);
+    }
+    const V4 mk = (kx * kk) * mPX;
+    // ---- z-velocity adjoint at Q ----
+    const V4 g = gzt(gz, (kz * kk) * mPZ);
+    if (upd) *reinterpret_cast<V4 *>(mvzo) = fma4(KIND == kAdjIn ? k.one : k.dbz, mvz, g);
+    // ---- buoyancy imaging at Q (xa-1 feeds column xa; 0 outside the grid) ----
+    {
+        const V4 tbx = (lx * in[224]) * w3.mvx, tbz = (lz * in[256]) * mvz;
+        float up = __shfl_up_sync(kFull, hi(tbz.b), 1);
+        if (KIND != kAdjIn && !k.row0) up = 0.0f;
+        const V4 zs = v4(pk(up, lo(tbz.a)), pk(hi(tbz.a), lo(tbz.b)));
+        const V4 half = dup4(0.5f);
+        if (upd) red4(gb, half * ((tbx + (KIND != kAdjAny || Q >= 1 ? k.tbp : zero4())) + (tbz + zs)));
+        k.tbp = tbx;
+    }
+    // ---- x-velocity adjoint at W = L - 3 ----
+    if (k.owner && L - 3 >= k.xa && L - 3 < k.xb) {
+        const V4 o = taps4(gx.t0, w2.mk, gx.t1, w3.mk, gx.t2, w1.mk, gx.t3, mk);
+        *reinterpret_cast<V4 *>(mvxo) = fma4(KIND == kAdjAny ? dup4(xc.dbw) : k.one, w1.mvx, o);
+    }
+    w0.mvx = mvx;
+    w0.mg = mg;
+    w0.mk = mk;
+}
+
+template <int KIND>
+__device__ __forceinline__ void adjoint_task(const StepArgs &a, const ShotDev &S, int strip, int xa, int seg_len,
+                                             int kt, int lane, V4 *smem) {
+    constexpr int D = AdjDepth<KIND>::value, NS = KIND == kAdjIn ? 9 : kAdjSlots;
+    const int nnx = S.nnx;
+    const ptrdiff_t ld = S.ld;
+    const int c = strip * S2D_STRIP_OUT - 4;
+    Lane<true> ln;
+    lane_setup(ln, S, c, lane, kt);
+    AdjTask k;
+    k.S = &S;
+    k.ring = smem + lane;
+    k.xa = xa;
+    k.xb = min(nnx, xa + seg_len);
+    k.z0 = ln.z0;
+    k.kt = kt;
+    k.src_q = S.src_x;
+    k.sdz = ln.sdz;
+    k.owner = ln.owner;
+    k.row0 = ln.z0 >= 1;
+    k.slot = (kt + 1) / a.dt_factor - 1;
+    // receiver adjoint source on recording steps, in strips whose rows hold receivers
+    k.inj = !(a.flags & S2D_STEP_NO_RECORD) && S.nrec > 0 && ((kt + 1) % a.dt_factor) == 0 && k.slot < S.real_nt &&
+            c + S2D_STRIP_ROWS > S.rec_zlo && c <= S.rec_zhi;
+    if (k.inj) k.src.start(S, max(xa - 1, 0), k.slot);
+    k.one = dup4(a.one);
+    k.kx = dup4(S.kx_in);
+    k.kz = dup4(S.kz_in);
+    k.xt = Taps{dup4(kA0), dup4(-kA0), dup4(kA1), dup4(-kA1)};
+    k.zt = row_taps(k.xt.t0, k.xt.t1, k.xt.t2, k.xt.t3);
+    k.tbp = zero4();
+    if (KIND != kAdjIn) {
+        float r[12][4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int z = ln.z0 + i, n = S.nnz;
+            const float4 q = __ldg(ln.zc + i);
+            r[0][i] = q.x;
+            r[1][i] = q.y;
+            r[2][i] = q.z;
+            r[3][i] = q.w;
+            float u;
+            dp_coef(z - 1, n, r[4][i], u);
+            dp_coef(z, n, r[5][i], u);
+            dp_coef(z - 2, n, u, r[6][i]);
+            dp_coef(z + 1, n, u, r[7][i]);
+            dm_coef(z, n, r[8][i], u);
+            dm_coef(z + 1, n, r[9][i], u);
+            dm_coef(z - 1, n, u, r[10][i]);
+            dm_coef(z + 2, n, u, r[11][i]);
+        }
+        auto tab = [&](int i, float f) { return v4(pk(f * r[i][0], f * r[i][1]), pk(f * r[i][2], f * r[i][3])); };
+        k.daz = tab(0, 1.0f);
+        k.kzr = tab(1, 1.0f);
+        k.dbz = tab(2, 1.0f);
+        k.lzr = tab(3, 1.0f);
+        k.hz = row_taps(tab(4, 1.0f), tab(5, -1.0f), tab(6, 1.0f), tab(7, -1.0f));
+        k.gz = row_taps(tab(8, 1.0f), tab(9, -1.0f), tab(10, 1.0f), tab(11, -1.0f));
+    }
+    const int pin = (kt + 1) & 1, pout = kt & 1;
+    // a ghost lane reads the column's first ghost rows (zeros) and writes nothing
+    const size_t off = (size_t)(ln.zl + S2D_GZ) + (size_t)S2D_GX * ld;
+    const ptrdiff_t fs = S.fstride;
+    const size_t F = (size_t)(nnx + 2 * S2D_GX) * ld;
+    const int L0 = xa - 3, Lend = k.xb + 2;
+    const int n4 = (Lend - xa + 4) / 4;  // groups of four iterations from L = xa on (the last may pass Lend)
+    const int Llast = KIND == kAdjIn ? xa + 4 * n4 - 1 : Lend;
+    // state, materials and products at the next iteration's column Q
+    const float *ns = S.st[pin][0] + off + (ptrdiff_t)(L0 - 1) * ld;
+    const float *nm = S.kappa + off + (ptrdiff_t)(L0 - 1) * ld;
+    const float *np = S.prod + (size_t)(kt - a.prod_kt0) * 4 * F + off + (ptrdiff_t)(L0 - 1) * ld;
+    auto issue = [&](int L, int slot) {
+        V4 *st = k.ring + slot * (NS * 32);
+        const bool in_l = KIND != kAdjAny || L < nnx + S2D_GX;
+        if (in_l) {
+            cp_async16(st, ns + ld + 2 * fs, true);
+            cp_async16(st + 32, nm + ld + fs, true);
+        }
+        cp_async16(st + 64, ns, true);
+        cp_async16(st + 96, ns + 3 * fs, true);
+        cp_async16(st + 128, nm + 2 * fs, true);
+        cp_async16(st + 160, nm, true);
+        // products: zeros outside the grid and past the columns in use
+        const bool img = KIND != kAdjAny || (L >= 1 && L <= nnx);
+        cp_async16(st + 192, np, img);
+        cp_async16(st + 224, np + 2 * F, img);
+        cp_async16(st + 256, np + 3 * F, img);
+        if (KIND != kAdjIn) {
+            cp_async16(st + 288, ns + fs, true);
+            cp_async16(st + 320, np + F, img);
+        }
+        ns += ld;
+        nm += ld;
+        np += ld;
+    };
+#pragma unroll
+    for (int i = 0; i < D - 1; ++i) {
+        issue(L0 + i, i);
+        cp_async_commit();
+    }
+    auto next = [&](int L, int i) {  // bring iteration L + D - 1, wait for iteration L (in slot i)
+        if (L + D - 1 <= Llast) issue(L + D - 1, KIND == kAdjIn ? (i + D - 1) % D : i == 0 ? D - 1 : i - 1);
+        cp_async_commit();
+        cp_async_wait<D - 1>();
+        return k.ring + i * (NS * 32);
+    };
+    AdjWin wa, wb, wc, wd;
+    wa.mvx = wa.mg = wa.mk = zero4();
+    wb = wc = wd = wa;
+    // iterations xa-3 .. xa-1 fill the windows of mvx' and Lx bx mvx'
+    auto fill = [&](AdjWin &w, int i) {
+        const V4 *in = next(L0 + i, i);
+        const float lx = KIND == kAdjAny ? __ldg(S.xcoef + (L0 + i + S2D_GX)).w : S.kx_in;
+        w.mvx = in[0];
+        w.mg = (dup4(lx) * in[32]) * w.mvx;
+    };
+    fill(wb, 0);
+    fill(wc, 1);
+    fill(wd, 2);
+    float *mpxo = S.st[pout][0] + off + (ptrdiff_t)(xa - 1) * ld, *mpzo = mpxo + fs, *mvzo = mpxo + 3 * fs;
+    float *mvxo = S.st[pout][0] + off + (ptrdiff_t)(xa - 3) * ld + 2 * fs;
+    float *gk = S.grad[0] + off + (ptrdiff_t)(xa - 1) * ld, *gb = S.grad[1] + off + (ptrdiff_t)(xa - 1) * ld;
+    AdjXc xc{};
+    int L = xa;
+    if (KIND == kAdjIn) {
+        for (int g = 0; g < n4; ++g) {
+#define S2D_ADJ_COLUMN(J, I, A, B, C_, D_)                                                                        \
+    adj_column<KIND>(k, xc, next(L + J, I), L + J, mpxo + J * ld, mpzo, mvxo + J * ld, mvzo + J * ld, gk + J * ld, \
+                     gb + J * ld, A, B, C_, D_)
+            S2D_ADJ_COLUMN(0, 3, wa, wb, wc, wd);
+            S2D_ADJ_COLUMN(1, 0, wb, wc, wd, wa);
+            S2D_ADJ_COLUMN(2, 1, wc, wd, wa, wb);
+            S2D_ADJ_COLUMN(3, 2, wd, wa, wb, wc);
+#undef S2D_ADJ_COLUMN
+            L += 4;
+            mpxo += 4 * ld;
+            mvxo += 4 * ld;
+            mvzo += 4 * ld;
+            gk += 4 * ld;
+            gb += 4 * ld;
+        }
+    } else {
+        if (KIND == kAdjAny) xc.read(S.xcoef, nnx, L);
+        int slot = 3 % D;
+#pragma unroll 1
+        for (; L <= Lend; ++L) {
+            AdjXc xn{};
+            if (KIND == kAdjAny) xn.read(S.xcoef, nnx, L + 1);
+            adj_column<KIND>(k, xc, next(L, slot), L, mpxo, mpzo, mvxo, mvzo, gk, gb, wa, wb, wc, wd);
+            slot = slot + 1 == D ? 0 : slot + 1;
+            const AdjWin t = wa;
+            wa = wb;
+            wb = wc;
+            wc = wd;
+            wd = t;
+            xc = xn;
+            mpxo += ld;
+            mpzo += ld;
+            mvxo += ld;
+            mvzo += ld;
+            gk += ld;
+            gb += ld;
+        }
+    }
+    cp_async_wait<0>();
+}
+
+__global__ void __launch_bounds__(128, 2) adjoint_kernel(const StepArgs *__restrict__ A, int kt_off) {
     extern __shared__ __align__(128) unsigned char smem[];
-    constexpr int kWarpBytes = kAdjWarpBytes + AS * adj_async_stage_bytes(AS);
-    float4 *ring = reinterpret_cast<float4 *>(smem + (size_t)(threadIdx.x >> 5) * kWarpBytes);
-    float4 *aring = reinterpret_cast<float4 *>(smem + (size_t)(threadIdx.x >> 5) * kWarpBytes + kAdjWarpBytes);
+    V4 *const mem = reinterpret_cast<V4 *>(smem + (size_t)(threadIdx.x >> 5) * kAdjWarpBytes);
     const StepArgs a = *A;
     const int lane = threadIdx.x & 31;
     const int gwarp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
@@ -418,22 +476,24 @@ __global__ void __launch_bounds__(128, MINB) adjoint_kernel(const StepArgs *__re
     // the task's shot record in this warp's shared-memory slot
     __shared__ ShotDev shot_rec[4];
     ShotDev &S = shot_rec[(threadIdx.x >> 5) & 3];
-    for (int t = gwarp; t < a.total_tasks; t += nwarp) {
+    TaskQueue queue(a.queue, nwarp, lane);
+    for (int t = gwarp; t < a.total_tasks; t = queue.take()) {
+        queue.draw();
         int strip, xa, seg_len;
-        const ShotDev &G = task_of(a, t, strip, xa, seg_len);
+        const ShotDev &G = task_of_split(a, t, strip, xa, seg_len);
         if (!task_in_bounds(a, G, strip, xa, seg_len, kt, true, 2)) continue;
         warp_copy_shot(S, G, lane);
         const int c = strip * S2D_STRIP_OUT - 4;
         const int xb = min(S.nnx, xa + seg_len);
         // the z-transposes read the coefficient pairs of rows c-2 .. c+129,
         // the x-gathers those of columns xa-3 .. xb+2
-        const bool zf = rows_fast(S, c - 2, c + S2D_STRIP_ROWS + 1);
-        const bool xf = xa - 3 >= S.xfast_lo && xb + 2 < S.xfast_hi;
-        if (zf && xf) adjoint_task<true, true, PF, AS>(a, S, strip, xa, seg_len, kt, lane, ring, aring);
-        else if (zf) adjoint_task<true, false, PF, AS>(a, S, strip, xa, seg_len, kt, lane, ring, aring);
-        else if (xf) adjoint_task<false, true, PF, AS>(a, S, strip, xa, seg_len, kt, lane, ring, aring);
-        else adjoint_task<false, false, PF, AS>(a, S, strip, xa, seg_len, kt, lane, ring, aring);
+        const bool zf = rows_fast(S, c - kAdjRowMargin, c + S2D_STRIP_ROWS - 1 + kAdjRowMargin);
+        const bool xf = xa - kAdjColLo >= S.xfast_lo && xb + kAdjColHi < S.xfast_hi;
+        if (zf && xf) adjoint_task<kAdjIn>(a, S, strip, xa, seg_len, kt, lane, mem);
+        else if (xf) adjoint_task<kAdjRows>(a, S, strip, xa, seg_len, kt, lane, mem);
+        else adjoint_task<kAdjAny>(a, S, strip, xa, seg_len, kt, lane, mem);
     }
+    queue.leave();
 }
 
 // ---- gradient finalisation ----
@@ -911,40 +971,17 @@ int launch_adjoint8(const StepArgs *args_dev, int kt_off, int nnx, int nnz, int 
     return (int)cudaGetLastError();
 }
 
-namespace {
-// minb 2, 3, 4: blocks per SM the kernel is built for; 12: 2 blocks per SM
-// with the next column's loads prefetched
-using AdjKernel = void (*)(const StepArgs *, int);
-// Kernel of an `adjoint_blocks` code: 2, 3, 4 blocks per SM; 12: 2 with the
-// register prefetch; 13: 3 with a 2-column copy ring; 14: 2 with a 3-column
-// ring; 15: 3 with a 3-column ring of the per-shot inputs.
-AdjKernel adjoint_kernel_of(int minb) {
-    if (minb == 12) return adjoint_kernel<2, true>;
-    if (minb == 13) return adjoint_kernel<3, false, 2>;
-    if (minb == 14) return adjoint_kernel<2, false, 3>;
-    if (minb == 15) return adjoint_kernel<3, false, 3>;
-    return minb >= 4 ? adjoint_kernel<4> : minb == 3 ? adjoint_kernel<3> : adjoint_kernel<2>;
-}
-size_t adjoint_warp_bytes(int minb) {
-    const int as = minb == 13 ? 2 : minb == 14 || minb == 15 ? 3 : 0;
-    return (size_t)kAdjWarpBytes + (size_t)as * adj_async_stage_bytes(as);
-}
-}  // namespace
-
-int launch_adjoint(const StepArgs *args_dev, int kt_off, int grid, int block, int minb, void *stream) {
-    const size_t smem = (size_t)(block / 32) * adjoint_warp_bytes(minb);
-    adjoint_kernel_of(minb)<<<grid, block, smem, (cudaStream_t)stream>>>(args_dev, kt_off);
+int launch_adjoint(const StepArgs *args_dev, int kt_off, int grid, void *stream) {
+    adjoint_kernel<<<grid, 128, 4 * kAdjWarpBytes, (cudaStream_t)stream>>>(args_dev, kt_off);
     return (int)cudaGetLastError();
 }
 
-// Also raises the kernel's dynamic shared-memory limit (the copy-ring forms
-// take more than 48 KB per block); called before the adjoint's launches.
-int adjoint_kernel_occupancy(int block, int minb, int *blocks_per_sm) {
-    const size_t smem = (size_t)(block / 32) * adjoint_warp_bytes(minb);
-    cudaError_t e = cudaFuncSetAttribute(adjoint_kernel_of(minb), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
+// Also raises the kernel's dynamic shared-memory limit; called before the
+// adjoint's launches.
+int adjoint_kernel_occupancy(int *blocks_per_sm) {
+    cudaError_t e = cudaFuncSetAttribute(adjoint_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * kAdjWarpBytes);
     if (e != cudaSuccess) return (int)e;
-    return (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, adjoint_kernel_of(minb), block, smem);
+    return (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, adjoint_kernel, 128, 4 * kAdjWarpBytes);
 }
 
 int launch_gradient_finalize(float *const *gk, float *const *gb, int nshots, int nacc, const int *src_cells,

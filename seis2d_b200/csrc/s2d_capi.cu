@@ -173,7 +173,6 @@ struct Ctx {
     int opt_grad_segment = 0; // gradient checkpoint interval, 0 = from free memory
     int opt_graph_chunk = 64; // FD steps per captured graph
     int opt_fast_rows = 1;    // 0: every strip takes the general row path
-    int opt_adj_minb = 13;    // adjoint kernel build ("adjoint_blocks"): 3 blocks per SM, inputs by cp.async
     int opt_adj8_form = 0;    // 8th-order adjoint: 0 streaming pass, 1 two cell-parallel passes
     int opt_prod_variant = kVariantLdgPfProducts;  // s2d_gradient's product-writing forward (4th order)
     int last_segment = 0;     // interval the last gradient call used
@@ -253,29 +252,37 @@ int choose_seg_len(int nnx, long tasks_per_seg, long resident_warps, int halo) {
     return best;
 }
 
-// Rim and interior tasks of a two-step group (GroupDev::split) of the grid
-// and fast ranges of shot record `d`; `shots` shots of it run at a time beside
-// `share` of `resident_warps` warps.
-// Measured cost of a column: 1 in the interior, 1.6 in strips with sponge rows,
-// 1.9 in sponge columns; a task streams 9 columns besides its own.  The
-// warps draw tasks as they finish, the dear ones first, so a launch takes
-// about its work over the warps, plus half an interior task, and at least its
-// longest task.
-void split_group(GroupDev &g, const ShotDev &d, int shots, double resident_warps, int forced) {
-    constexpr double kRows = 1.6, kCols = 1.9;
-    constexpr int kHalo = 9;
+// How a kernel's tasks are cut by kind: rows per strip and rows a strip reads
+// before them, rows and columns past a task's own that must be interior too,
+// columns a task streams besides its own, and what a column costs in strips
+// with sponge rows and in sponge columns (1 in the interior).
+struct SplitRule {
+    int out, before, row_margin, col_lo, col_hi, halo;
+    double rows, cols;
+};
+constexpr SplitRule kSplitTs2 = {S2D_TS_OUT, 8, 0, 4, 4, 9, 1.6, 1.9};
+constexpr SplitRule kSplitAdj = {S2D_STRIP_OUT, 4, kAdjRowMargin, kAdjColLo, kAdjColHi, 6, 1.5, 1.7};
+
+// Rim and interior tasks of a group (GroupDev::split) of the grid and fast
+// ranges of shot record `d`; `shots` shots of it run at a time on
+// `resident_warps` warps.  The warps draw tasks as they finish, the dear ones
+// first, so a launch takes about its work over the warps, plus half an
+// interior task, and at least its longest task.
+void split_group(GroupDev &g, const ShotDev &d, int shots, double resident_warps, int forced,
+                 const SplitRule &R = kSplitTs2) {
+    const double kRows = R.rows, kCols = R.cols;
+    const int kHalo = R.halo;
     g.split = 1;
     auto fast = [&](int k) {
-        const int c0 = k * S2D_TS_OUT - 8;
-        return c0 >= d.zfast_lo && c0 + S2D_STRIP_ROWS - 1 < d.zfast_hi;
+        const int c0 = k * R.out - R.before;
+        return c0 - R.row_margin >= d.zfast_lo && c0 + S2D_STRIP_ROWS - 1 + R.row_margin < d.zfast_hi;
     };
     g.rim_lo = 0;
     while (g.rim_lo < g.nstrips && !fast(g.rim_lo)) ++g.rim_lo;
     g.rim_hi = 0;
     while (g.rim_lo + g.rim_hi < g.nstrips && !fast(g.nstrips - 1 - g.rim_hi)) ++g.rim_hi;
-    // interior tasks: columns xa-4 .. xb+4 fast
-    g.xl = d.xfast_lo + 4;
-    g.xr = d.xfast_hi - 5;
+    g.xl = d.xfast_lo + R.col_lo;
+    g.xr = d.xfast_hi - 1 - R.col_hi;
     if (g.xr - g.xl < 8) g.xl = g.xr = d.nnx;
     const int nz = g.rim_lo + g.rim_hi, ni = g.nstrips - nz;
     auto cut = [&](int L) {
@@ -1172,10 +1179,8 @@ int s2d_set_option(void *ctx, const char *key, long value) {
         c->opt_prod_variant = (int)value;
     } else if (k == "adjoint_blocks") {
         if ((value < 2 || value > 4) && (value < 12 || value > 15))
-            return fail(c, S2D_ERR_ARG,
-                        "adjoint_blocks must be 2, 3, 4, 12 (2 with the next column prefetched), 13, 14 or 15 (3, 2 "
-                        "or 3 blocks with asynchronous copies 1, 2 or 2 columns ahead)");
-        c->opt_adj_minb = (int)value;
+            return fail(c, S2D_ERR_ARG, "adjoint_blocks must be 2, 3, 4 or 12 to 15");
+        // builds of an earlier adjoint kernel: one form serves them all now
     } else if (k == "fast_rows") {
         c->opt_fast_rows = value ? 1 : 0;
     } else if (k == "on_chip") {
@@ -1593,19 +1598,19 @@ int run_adjoint(Ctx *c, Batch &b, GradRun &g, StepArgs args, int kt_top, int n, 
         *launches += 1 + m;
         if (!use_graph) {
             for (int k = 0; k < m; ++k) {
-                e = launch_adjoint(args_d, k, grid, 128, c->opt_adj_minb, c->stream);
+                e = launch_adjoint(args_d, k, grid, c->stream);
                 if (e) return fail(c, S2D_ERR_CUDA, "adjoint launch: %s", cudaGetErrorString((cudaError_t)e));
             }
             continue;
         }
         (void)g;
-        const std::vector<long> key = {m, grid, c->opt_adj_minb};
+        const std::vector<long> key = {m, grid};
         auto it = c->adj_graphs.find(key);
         if (it == c->adj_graphs.end()) {
             cudaGraph_t gr;
             CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
             for (int k = 0; k < m; ++k) {
-                e = launch_adjoint(args_d, k, grid, 128, c->opt_adj_minb, c->stream);
+                e = launch_adjoint(args_d, k, grid, c->stream);
                 if (e) {
                     cudaStreamEndCapture(c->stream, &gr);
                     if (gr) cudaGraphDestroy(gr);
@@ -1801,29 +1806,30 @@ extern "C" int s2d_gradient(void *ctx, const s2d_shot *shots, int nshots, const 
         return S2D_OK;
     };
     // The steps that keep their products (the last segment of the sweep, the
-    // recomputes) and the adjoint steps run with a task layout for the
-    // resident warps of the adjoint kernel: the two kernels of the backward
-    // phase then each take whole rounds of tasks.
-    int agrid = 1;
-    auto backward_layout = [&]() -> int {
-        if (b.order8) {
-            // the 8th-order products kernel and the streaming adjoint share the
-            // 112-row layout (the cell-parallel adjoint needs none)
-            int e = layout_groups(c, b, lc_prod);
-            if (!e) e = launch_config(c, b.max_tasks, &lc_prod, prod_variant, 128, 0);
-            fa.total_tasks = batch_tasks(b);
-            return e;
-        }
-        int bps = 0;
-        if (adjoint_kernel_occupancy(128, c->opt_adj_minb, &bps) || bps < 1) bps = 1;
-        const long resident = (long)c->sm_count * bps;
-        int e = layout_groups_for(c, b, resident * 4, {-1, resident, c->opt_seg_len});
-        if (!e) e = launch_config(c, b.max_tasks, &lc_prod, c->opt_prod_variant, 128, 0);
-        if (e) return e;
-        agrid = (int)std::max<long>(1, std::min<long>(resident, (b.max_tasks * 32 + 127) / 128));
+    // recomputes) run in the products kernel's own task layout; so do the
+    // 8th-order adjoint steps.  The 4th-order adjoint has one of its own, cut by
+    // kind.
+    auto products_layout = [&]() -> int {
+        int e = layout_groups(c, b, lc_prod);
+        if (!e) e = launch_config(c, b.max_tasks, &lc_prod, prod_variant, 128, 0);
         fa.total_tasks = batch_tasks(b);
-        return S2D_OK;
+        return e;
     };
+    int agrid = 1;
+    GroupDev ag = b.groups[0];
+    void *adj_group = nullptr;
+    if (!b.order8) {
+        int bps = 0;
+        if (adjoint_kernel_occupancy(&bps) || bps < 1) bps = 1;
+        const long resident = (long)c->sm_count * bps;
+        ag.nstrips = num_strips(b.group_nnz[0]);
+        ag.task_begin = 0;
+        split_group(ag, b.shot_dev[0], nshots, (double)resident * 4, c->opt_seg_len, kSplitAdj);
+        agrid = (int)std::max<long>(1, std::min<long>(resident, ((long)nshots * shot_tasks(ag) * 32 + 127) / 128));
+        int e = grad_alloc(c, g, sizeof(GroupDev), &adj_group);
+        if (e) return e;
+        CK(cudaMemcpyAsync(adj_group, &ag, sizeof ag, cudaMemcpyHostToDevice, c->stream));
+    }
     for (int j = 0; j < nseg; ++j) {
         const int k0 = j * C, n = std::min(C, rs.fd_nt - k0);
         if (j < nseg - 1) {
@@ -1836,7 +1842,7 @@ extern "C" int s2d_gradient(void *ctx, const s2d_shot *shots, int nshots, const 
                 e = run_loop(c, b, lc_fwd, a, k0, n, use_graph, &launches, &graph_used);
             if (e) return e;
         } else {
-            int e = backward_layout();
+            int e = products_layout();
             if (e) return e;
             StepArgs a = fa;
             a.flags = S2D_STEP_PRODUCTS;
@@ -1872,6 +1878,16 @@ extern "C" int s2d_gradient(void *ctx, const s2d_shot *shots, int nshots, const 
     aa.task_order = 0;
     aa.shots = adj_table.as<ShotDev>();
     aa.err = c->dev_err.as<int>();
+    aa.queue = c->queue_d.as<int>();
+    aa.one = 1.0f;
+    aa.flags = 0;
+    if (b.order8) {
+        aa.total_tasks = batch_tasks(b);
+    } else {
+        aa.groups = static_cast<const GroupDev *>(adj_group);
+        aa.ngroups = 1;
+        aa.total_tasks = nshots * shot_tasks(ag);
+    }
     for (int j = nseg - 1; j >= 0; --j) {
         const int k0 = j * C, n = std::min(C, rs.fd_nt - k0);
         if (j < nseg - 1) {

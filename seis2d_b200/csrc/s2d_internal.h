@@ -223,6 +223,9 @@ inline bool plain_loads(int variant) {
 constexpr int kTs2Depth = 4;  // as the column loop is unrolled: constant ring slots
 constexpr int kTs2Slots = 7;
 constexpr int kTs2WarpBytes = (kTs2Depth * kTs2Slots + 8 + 8) * S2D_STRIP_ROWS * 4;
+// Interior tasks of the adjoint step: rows and columns past the task's own
+// strip and segment that must be interior too.
+constexpr int kAdjRowMargin = 2, kAdjColLo = 3, kAdjColHi = 2;
 // Per-warp shared-memory windows of the 8th-order ring kernel: vx and new p of
 // 8 columns each, vz of 4 (one 128-row column = 32 float4).
 constexpr int kO8sWarpBytes = (8 + 8 + 4) * S2D_STRIP_ROWS * 4;
@@ -281,7 +284,7 @@ int launch_set_args(const StepArgs &v, StepArgs *args_dev, void *stream);
 int launch_persist(const StepArgs *args_dev, int nsteps, unsigned *bar, int grid, void *stream);
 int persist_occupancy(int *blocks_per_sm);
 // Adjoint FD step (step kt = args.kt_base - kt_off) and the gradient finalisation.
-int launch_adjoint(const StepArgs *args_dev, int kt_off, int grid, int block, int minb, void *stream);
+int launch_adjoint(const StepArgs *args_dev, int kt_off, int grid, void *stream);
 // Adjoint FD step of the 8th-order scheme: two cell-parallel passes over
 // `nshots` shots of one nnx x nnz grid.
 int launch_adjoint8(const StepArgs *args_dev, int kt_off, int nnx, int nnz, int nshots, void *stream);
@@ -289,7 +292,7 @@ int launch_adjoint8(const StepArgs *args_dev, int kt_off, int nnx, int nnz, int 
 // the 112-row strips of the batch's current layout), 4 warps per block.
 int launch_adjoint8s(const StepArgs *args_dev, int kt_off, int grid, void *stream);
 int adjoint8s_occupancy(int *blocks_per_sm);
-int adjoint_kernel_occupancy(int block, int minb, int *blocks_per_sm);
+int adjoint_kernel_occupancy(int *blocks_per_sm);
 // Add each shot's source term to its accumulator gk[s] (the entries may all
 // be the one shared pair), sum the nacc accumulator pairs gk[0..nacc),
 // gb[0..nacc) (dJ/dkappa, dJ/db), apply the kappa = vp^2 rho, b = 1/rho chain
