@@ -159,7 +159,7 @@ S2D_API const char *s2d_last_error(const void *ctx);
  * Tuning knobs of the step kernel; no counterpart in the reference.  Keys:
  *   "autotune"    1 (default): the first s2d_forward of a batched run of a new
  *                 shape (models, grids, shot counts) with at least 80 steps
- *                 (64 for the 8th-order operator) spends up to 40 (32) of them
+ *                 (48 for the 8th-order operator) spends up to 40 (24) of them
  *                 on trials: 5 candidate configurations (variants 5, 16, 15 in
  *                 task order 1, and 16 and 15 in task order 0, unless
  *                 "task_order" was set), one untimed and three timed launches
@@ -191,9 +191,8 @@ S2D_API const char *s2d_last_error(const void *ctx);
  *                 than per-step launches on the grids measured);
  *                 the recomputes and adjoint steps of s2d_gradient always run
  *                 one step per launch.
- *                 For batches of S2D_MODEL_ORDER8 models: 7 register windows
- *                 at 3 blocks per SM (default), 8 the same at 2, 9 windows in
- *                 shared memory at 4 (each setting applies to its own order)
+ *                 For batches of S2D_MODEL_ORDER8 models: 7 (default); 8 and 9
+ *                 name the same kernel (each setting applies to its own order)
  *   "block"       threads per block: 32, 64, 96 or 128 (default 128)
  *   "task_order"  0: consecutive warps take the shots of one tile (the four
  *                 warps of a block share its kappa, bx, bz through L1);

@@ -261,15 +261,23 @@ struct SplitRule {
     double rows, cols;
 };
 constexpr SplitRule kSplitTs2 = {S2D_TS_OUT, 8, 0, 4, 4, 9, 1.6, 1.9};
+constexpr SplitRule kSplitO8 = {S2D_TS_OUT, 8, 0, 3, 3, 13, 1.6, 1.9};
 constexpr SplitRule kSplitAdj = {S2D_STRIP_OUT, 4, kAdjRowMargin, kAdjColLo, kAdjColHi, 6, 1.5, 1.7};
 
 // Rim and interior tasks of a group (GroupDev::split) of the grid and fast
 // ranges of shot record `d`; `shots` shots of it run at a time on
-// `resident_warps` warps.  The warps draw tasks as they finish, the dear ones
-// first, so a launch takes about its work over the warps, plus half an
-// interior task, and at least its longest task.
-void split_group(GroupDev &g, const ShotDev &d, int shots, double resident_warps, int forced,
-                 const SplitRule &R = kSplitTs2) {
+// `resident_warps` warps, the group `alone` in its launch or with that share of
+// the warps.  The warps draw tasks as they finish, the dear ones first, so a
+// launch takes about its work over the warps, plus one interior task, and at
+// least its longest task.  (With half a task the 8th-order step of 4 shots of
+// 5120 x 5120 ran at 170 Gcell/s, with one at 184.)  Where every warp has one
+// task at most, the longest one counts, a half more than in a launch of
+// several rounds, whose warps even out: measured about 1.0 us per column of the
+// two-step kernel against 0.61.  2101 x 1101, 3 shots: one round of 79 columns
+// 155 Gcell/s, two of 35 178; 3301 x 1301, 6 shots: 195 and 258 (63); 1301 x
+// 501, 8 shots, the other way: 119 and 105.
+void split_group(GroupDev &g, const ShotDev &d, int shots, double resident_warps, bool alone, int forced,
+                 const SplitRule &R) {
     const double kRows = R.rows, kCols = R.cols;
     const int kHalo = R.halo;
     g.split = 1;
@@ -309,7 +317,7 @@ void split_group(GroupDev &g, const ShotDev &d, int shots, double resident_warps
         const double work = shots * (ni * (g.nsegs * ti + (g.nseg_l + g.nseg_r) * tx) + nz * g.nseg_z * tz);
         const double longest = std::max(ni && g.nsegs ? ti : 0.0, std::max(nz ? tz : 0.0, ni ? tx : 0.0));
         const double tasks = (double)shots * shot_tasks(g);
-        const double cost = std::max(longest, tasks <= resident_warps ? longest : work / resident_warps + 0.5 * ti);
+        const double cost = std::max(longest, alone && tasks <= resident_warps ? 1.5 * longest : work / resident_warps + ti);
         if (!best || cost < best_cost) {
             best = L;
             best_cost = cost;
@@ -340,6 +348,11 @@ int build_coef(Ctx *c, Model &m, float fd_dt) {
     return S2D_OK;
 }
 
+// Dynamic shared memory of a warp of the variants with 112-row strips.
+int ts_warp_bytes(int variant) {
+    return variant == kVariantTs2 ? kTs2WarpBytes : variant == kVariantTs1 ? 0 : kO8WarpBytes;
+}
+
 // Launch configuration for (variant, block, stages): shared memory and a grid
 // of exactly the resident blocks (the kernels loop over tasks), capped by the
 // work available.
@@ -363,7 +376,7 @@ int launch_config(Ctx *c, long max_tasks, LaunchCfg *out, int variant, int block
     lc.smem = ldg ? 0
               : tma ? kTmaSmemBytes
               : asy ? (size_t)(lc.block / 32) * kAsyncWarpBytes
-              : ts ? (size_t)(lc.block / 32) * (lc.variant == kVariantO8s ? kO8sWarpBytes : lc.variant == kVariantTs1 ? 0 : kTs2WarpBytes)
+              : ts ? (size_t)(lc.block / 32) * ts_warp_bytes(lc.variant)
                    : bulk_smem_bytes(lc.block / 32, lc.stages);
     int e = step_kernel_prepare(lc.variant, lc.smem);
     if (e) return fail(c, S2D_ERR_ARG, "step kernel does not accept %zu B of shared memory: %s", lc.smem,
@@ -461,7 +474,8 @@ int layout_groups_for(Ctx *c, Batch &b, long resident_warps, std::vector<long> k
             g.nsegs = 0;  // no tasks
         } else if (split) {
             const double share = b.plain ? 1.0 : (double)g.nshots * nnx * b.group_nnz[gi] / cells;
-            split_group(g, b.shot_dev[b.table[g.shot0]], g.nshots, share * (double)resident_warps, c->opt_seg_len);
+            split_group(g, b.shot_dev[b.table[g.shot0]], g.nshots, share * (double)resident_warps, share > 0.99, c->opt_seg_len,
+                        b.order8 ? kSplitO8 : kSplitTs2);
         } else {
             g.seg_len = c->opt_seg_len > 0 ? std::min(c->opt_seg_len, nnx)
                                            : choose_seg_len(nnx, tasks_per_seg, resident_warps, ts ? 12 : 6);
@@ -499,7 +513,7 @@ int layout_groups(Ctx *c, Batch &b, const LaunchCfg &lc) {
     int e = launch_config(c, 1L << 40, &full, v, lc.block, lc.stages);
     if (e) return e;
     if (tma_variant(v)) return layout_groups_for(c, b, (long)full.grid, key, false, true);
-    return layout_groups_for(c, b, (long)full.grid * (full.block / 32), key, ts_layout(v), false, v == kVariantTs2);
+    return layout_groups_for(c, b, (long)full.grid * (full.block / 32), key, ts_layout(v), false, queue_variant(v));
 }
 
 // Graph of `n` step launches (kt_off = 0..n-1) for one launch configuration,
@@ -975,11 +989,8 @@ constexpr int kTuneCandidates[][4] = {
     {kVariantLdgPf4, 128, 0, 0}, {kVariantLdgPf, 128, 0, 0},
 };
 constexpr int kNumTuneCandidates = (int)(sizeof(kTuneCandidates) / sizeof(kTuneCandidates[0]));
-// Candidates of 8th-order batches: the register-window kernel at 3 blocks per
-// SM (168 registers) and at 2 (224 registers, no spills), and the
-// shared-memory-window kernel at 4 (128 registers).
-constexpr int kTuneCandidatesO8[][4] = {
-    {kVariantO8, 128, 0, 1}, {kVariantO8r, 128, 0, 1}, {kVariantO8s, 128, 0, 1}, {kVariantO8, 128, 0, 0}};
+// Candidates of 8th-order batches: one kernel, the two task orders.
+constexpr int kTuneCandidatesO8[][4] = {{kVariantO8, 128, 0, 1}, {kVariantO8, 128, 0, 0}};
 constexpr int kNumTuneCandidatesO8 = (int)(sizeof(kTuneCandidatesO8) / sizeof(kTuneCandidatesO8[0]));
 constexpr int kTuneWarm = 1, kTuneTimed = 3;  // launches per candidate
 constexpr int kTuneRunoff = 4;                 // more timed launches of each of the two best
@@ -1806,9 +1817,8 @@ extern "C" int s2d_gradient(void *ctx, const s2d_shot *shots, int nshots, const 
         return S2D_OK;
     };
     // The steps that keep their products (the last segment of the sweep, the
-    // recomputes) run in the products kernel's own task layout; so do the
-    // 8th-order adjoint steps.  The 4th-order adjoint has one of its own, cut by
-    // kind.
+    // recomputes) run in the products kernel's own task layout, the adjoint
+    // steps in one of theirs (the 4th-order one cut by kind).
     auto products_layout = [&]() -> int {
         int e = layout_groups(c, b, lc_prod);
         if (!e) e = launch_config(c, b.max_tasks, &lc_prod, prod_variant, 128, 0);
@@ -1818,13 +1828,21 @@ extern "C" int s2d_gradient(void *ctx, const s2d_shot *shots, int nshots, const 
     int agrid = 1;
     GroupDev ag = b.groups[0];
     void *adj_group = nullptr;
-    if (!b.order8) {
+    {
         int bps = 0;
-        if (adjoint_kernel_occupancy(&bps) || bps < 1) bps = 1;
+        if ((b.order8 ? adjoint8s_occupancy(&bps) : adjoint_kernel_occupancy(&bps)) || bps < 1) bps = 1;
         const long resident = (long)c->sm_count * bps;
-        ag.nstrips = num_strips(b.group_nnz[0]);
+        ag.nstrips = b.order8 ? num_strips_ts(b.group_nnz[0]) : num_strips(b.group_nnz[0]);
         ag.task_begin = 0;
-        split_group(ag, b.shot_dev[0], nshots, (double)resident * 4, c->opt_seg_len, kSplitAdj);
+        if (b.order8) {
+            const int nnx = b.group_nnx[0];
+            ag.split = 0;
+            ag.seg_len = c->opt_seg_len > 0 ? std::min(c->opt_seg_len, nnx)
+                                            : choose_seg_len(nnx, (long)nshots * ag.nstrips, resident * 4, 12);
+            ag.nsegs = (nnx + ag.seg_len - 1) / ag.seg_len;
+        } else {
+            split_group(ag, b.shot_dev[0], nshots, (double)resident * 4, true, c->opt_seg_len, kSplitAdj);
+        }
         agrid = (int)std::max<long>(1, std::min<long>(resident, ((long)nshots * shot_tasks(ag) * 32 + 127) / 128));
         int e = grad_alloc(c, g, sizeof(GroupDev), &adj_group);
         if (e) return e;
@@ -1881,13 +1899,9 @@ extern "C" int s2d_gradient(void *ctx, const s2d_shot *shots, int nshots, const 
     aa.queue = c->queue_d.as<int>();
     aa.one = 1.0f;
     aa.flags = 0;
-    if (b.order8) {
-        aa.total_tasks = batch_tasks(b);
-    } else {
-        aa.groups = static_cast<const GroupDev *>(adj_group);
-        aa.ngroups = 1;
-        aa.total_tasks = nshots * shot_tasks(ag);
-    }
+    aa.groups = static_cast<const GroupDev *>(adj_group);
+    aa.ngroups = 1;
+    aa.total_tasks = nshots * shot_tasks(ag);
     for (int j = nseg - 1; j >= 0; --j) {
         const int k0 = j * C, n = std::min(C, rs.fd_nt - k0);
         if (j < nseg - 1) {

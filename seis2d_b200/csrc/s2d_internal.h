@@ -151,10 +151,8 @@ enum StepVariant { kVariantBulk = 0, kVariantLdg = 1, kVariantBulk128 = 2,
                    kVariantLdg128 = 4 /* plain loads, compiled for 128 registers */,
                    kVariantTs2 = 5 /* two FD steps per launch (112-row strips) */,
                    kVariantTs1 = 6 /* one FD step in the two-step kernel's layout (odd remainders) */,
-                   kVariantO8 = 7 /* 8th-order operator, plain loads (112-row strips), models with
-                                     S2D_MODEL_ORDER8; 3 blocks per SM */,
-                   kVariantO8r = 8 /* the same at 2 blocks per SM (no register cap below 224) */,
-                   kVariantO8s = 9 /* the same with its windows in shared memory, 4 blocks per SM */,
+                   kVariantO8 = 7 /* 8th-order operator (112-row strips), models with S2D_MODEL_ORDER8 */,
+                   kVariantO8b = 8, kVariantO8c = 9 /* other names of kVariantO8 */,
                    kVariantO8Products = 10 /* kVariantO8 + S2D_STEP_PRODUCTS, gradient runs */,
                    kVariantTma = 11 /* CTA of kTmaWarps consumer warps fed by a TMA producer warp */,
                    kVariantAsync = 12 /* plain-load loop fed by per-lane cp.async into a per-warp ring */,
@@ -201,20 +199,16 @@ constexpr int steps_per_launch(int variant) {
 }
 // Variants whose strips are S2D_TS_OUT rows (and whose tasks stream 12 or 13 halo columns).
 inline bool ts_layout(int variant) {
-    return variant == kVariantTs2 || variant == kVariantTs1 || variant == kVariantO8 || variant == kVariantO8r ||
-           variant == kVariantO8s || variant == kVariantO8Products;
+    return variant == kVariantTs2 || variant == kVariantTs1 || (variant >= kVariantO8 && variant <= kVariantO8Products);
 }
-inline bool order8_variant(int variant) {
-    return variant == kVariantO8 || variant == kVariantO8r || variant == kVariantO8s;
-}
+inline bool order8_variant(int variant) { return variant >= kVariantO8 && variant <= kVariantO8c; }
 inline bool tma_variant(int variant) { return variant == kVariantTma; }
 inline bool async_variant(int variant) { return variant == kVariantAsync || variant == kVariantAsyncProducts; }
 // Variants that use no dynamic shared memory.
 inline bool plain_loads(int variant) {
     return variant == kVariantLdg || variant == kVariantLdgProducts || variant == kVariantLdg128 || variant == kVariantLdgU4 ||
            variant == kVariantLdgPf || variant == kVariantLdgPf4 || variant == kVariantLdgPfU4 ||
-           variant == kVariantLdgPfU3 || variant == kVariantLdgPfProducts || variant == kVariantPersist ||
-           variant == kVariantO8 || variant == kVariantO8r || variant == kVariantO8Products;
+           variant == kVariantLdgPfU3 || variant == kVariantLdgPfProducts || variant == kVariantPersist;
 }
 
 // Shared memory of a warp of the two-step kernel: the input ring (kTs2Depth
@@ -226,9 +220,14 @@ constexpr int kTs2WarpBytes = (kTs2Depth * kTs2Slots + 8 + 8) * S2D_STRIP_ROWS *
 // Interior tasks of the adjoint step: rows and columns past the task's own
 // strip and segment that must be interior too.
 constexpr int kAdjRowMargin = 2, kAdjColLo = 3, kAdjColHi = 2;
-// Per-warp shared-memory windows of the 8th-order ring kernel: vx and new p of
-// 8 columns each, vz of 4 (one 128-row column = 32 float4).
-constexpr int kO8sWarpBytes = (8 + 8 + 4) * S2D_STRIP_ROWS * 4;
+// Shared memory of a warp of the 8th-order kernel: the input ring (kO8Depth
+// iterations of vx; px, vz, kappa; bx, bz; pz) and 12 row coefficients.
+constexpr int kO8Depth = 4, kO8Slots = 7;
+constexpr int kO8WarpBytes = (kO8Depth * kO8Slots + 12) * S2D_STRIP_ROWS * 4;
+// Variants whose launches draw their tasks from the queue, cut by kind (GroupDev::split).
+inline bool queue_variant(int variant) {
+    return variant == kVariantTs2 || (variant >= kVariantO8 && variant <= kVariantO8Products);
+}
 
 // Shared memory of one pipeline stage: 7 slots of one 128-row column each
 // (vx at L; px, pz, kappa, vz at L-1; bx, bz at L-3).

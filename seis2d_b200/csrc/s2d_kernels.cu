@@ -1210,277 +1210,297 @@ __global__ void __launch_bounds__(128, 4) step_kernel_ts1(const StepArgs *__rest
 // c = (1225/1024, -245/3072, 49/5120, -5/7168), and the reference's 4th-order,
 // plain-difference and zero rows where the 8-tap stencil would leave the grid.
 //
-// One fused pass per step, streamed like the plain-load kernel: the warp keeps
-// vx at P-4 .. P+3 (8 columns), new p at V-3 .. V+4 (8 columns) and vz at
-// V .. P (5 columns) in registers, forms p at P = L-3 and the velocities at
-// V = L-7.  The z-stencils reach 4 rows, one whole neighbouring lane: p is
-// exact on lanes 1..30 and the velocities on lanes 2..29, so strips are 112
-// rows (the two-step kernel's layout, read from 112k-8) and lanes 2..29 write.
+// One fused pass per step: the warp keeps vx at P-4 .. P+3 (8 columns), new p at
+// V-3 .. V+4 (8 columns) and vz at V .. P (5 columns) in registers, forms p at P
+// = L-3 and the velocities at V = L-7.  The z-stencils reach 4 rows, one whole
+// neighbouring lane: p is exact on lanes 1..30 and the velocities on lanes
+// 2..29, so strips are 112 rows (the two-step kernel's layout, read from 112k-8)
+// and lanes 2..29 write.
+//
+// What bounds it: memory.  4 shots of 5120 x 5120: 184 Gcell/s, the state and
+// the materials read once and written once 27 bytes per cell-step, 5.0 TB/s, the
+// rate of a copy with this access pattern; before (plain loads where they were
+// used, the windows moved every column, every strip one length) 88.6.  One
+// 3301 x 1301 shot: 105 (57), 4 of 1301 x 501: 96 (57), one 701 x 401, about one
+// task per warp and bound by its latency: 25.5 (19).  2 blocks per SM and 222
+// registers; at 3 blocks (168 registers, spills) 140, 81, 69 and 22; the windows
+// in shared memory at 4 blocks 69, 50, 56 and 18.
 
-// c1 d1 + c2 d2 + c3 d3 + c4 d4 with the rounding fixed (innermost product
-// rounded, then three fused steps).
-__device__ __forceinline__ float dif8(const float4 &c, float d1, float d2, float d3, float d4) {
-    return __fmaf_rn(c.x, d1, __fmaf_rn(c.y, d2, __fmaf_rn(c.z, d3, __fmul_rn(c.w, d4))));
+// c1 d1 + c2 d2 + c3 d3 + c4 d4 of packed columns with the rounding fixed
+// (innermost product rounded, then three fused steps).
+struct Pair8 {
+    V4 c1, c2, c3, c4;
+};
+__device__ __forceinline__ f2 dif8_2(f2 c1, f2 d1, f2 c2, f2 d2, f2 c3, f2 d3, f2 c4, f2 d4) {
+    return fma2(c1, d1, fma2(c2, d2, fma2(c3, d3, mul2(c4, d4))));
 }
-template <bool FAST>
-__device__ __forceinline__ float4 zdm8(const Lane<FAST> &ln, int i) {
-    if (FAST) return make_float4(kC81, kC82, kC83, kC84);
-    return dm8(ln.z0 + i, ln.nnz);
+__device__ __forceinline__ V4 dif8_4(const Pair8 &c, const V4 &d1, const V4 &d2, const V4 &d3, const V4 &d4) {
+    return v4(dif8_2(c.c1.a, d1.a, c.c2.a, d2.a, c.c3.a, d3.a, c.c4.a, d4.a),
+              dif8_2(c.c1.b, d1.b, c.c2.b, d2.b, c.c3.b, d3.b, c.c4.b, d4.b));
 }
-template <bool FAST>
-__device__ __forceinline__ float4 zdp8(const Lane<FAST> &ln, int i) {
-    if (FAST) return make_float4(kC81, kC82, kC83, kC84);
-    return dp8(ln.z0 + i, ln.nnz);
+__device__ __forceinline__ f2 sub_pk(float x0, float y0, float x1, float y1) {
+    return pk(__fsub_rn(x0, y0), __fsub_rn(x1, y1));
+}
+// D- along z: rows z0-4 .. z0+6 by shuffles (u: the lane above's four rows, d:
+// the lane below's first three).
+__device__ __forceinline__ V4 dminus_z8(const Pair8 &c, const V4 &f) {
+    const float x = lo(f.a), y = hi(f.a), z = lo(f.b), w = hi(f.b);
+    const float u0 = __shfl_up_sync(kFull, x, 1), u1 = __shfl_up_sync(kFull, y, 1);
+    const float u2 = __shfl_up_sync(kFull, z, 1), u3 = __shfl_up_sync(kFull, w, 1);
+    const float d0 = __shfl_down_sync(kFull, x, 1), d1 = __shfl_down_sync(kFull, y, 1);
+    const float d2 = __shfl_down_sync(kFull, z, 1);
+    return dif8_4(c, v4(sub_pk(x, u3, y, x), sub_pk(z, y, w, z)), v4(sub_pk(y, u2, z, u3), sub_pk(w, x, d0, y)),
+                  v4(sub_pk(z, u1, w, u2), sub_pk(d0, u3, d1, x)), v4(sub_pk(w, u0, d0, u1), sub_pk(d1, u2, d2, u3)));
+}
+// D+ along z: rows z0-3 .. z0+7.
+__device__ __forceinline__ V4 dplus_z8(const Pair8 &c, const V4 &f) {
+    const float x = lo(f.a), y = hi(f.a), z = lo(f.b), w = hi(f.b);
+    const float u1 = __shfl_up_sync(kFull, y, 1), u2 = __shfl_up_sync(kFull, z, 1);
+    const float u3 = __shfl_up_sync(kFull, w, 1);
+    const float d0 = __shfl_down_sync(kFull, x, 1), d1 = __shfl_down_sync(kFull, y, 1);
+    const float d2 = __shfl_down_sync(kFull, z, 1), d3 = __shfl_down_sync(kFull, w, 1);
+    return dif8_4(c, v4(sub_pk(y, x, z, y), sub_pk(w, z, d0, w)), v4(sub_pk(z, u3, w, x), sub_pk(d0, y, d1, z)),
+                  v4(sub_pk(w, u2, d0, u3), sub_pk(d1, x, d2, y)), v4(sub_pk(d0, u1, d1, u2), sub_pk(d2, u3, d3, x)));
 }
 
-// New p at column P from vx at P-4 .. P+3 (w), old px, pz, kappa and vz at P;
-// the step's first two products (as p_cell forms them) in dxv, dzv.
-// XF: column P lies in the 8th-order x-interior (8-tap pair, dampings 1).
-template <bool FAST, bool XF = false>
-__device__ __forceinline__ float4 p_update8(const Lane<FAST> &ln, const ShotDev &S, int P, const float4 &xc,
-                                            bool colm, const float4 (&w)[8], const float4 &px, const float4 &pz,
-                                            const float4 &kk, const float4 &vz, float4 &pxn, float4 &pzn,
-                                            float4 &dxv, float4 &dzv) {
-    // vz rows z0-4 .. z0+6: the lane above's four (u), this lane's, the lane below's first three (d)
-    const float u0 = __shfl_up_sync(kFull, vz.x, 1), u1 = __shfl_up_sync(kFull, vz.y, 1);
-    const float u2 = __shfl_up_sync(kFull, vz.z, 1), u3 = __shfl_up_sync(kFull, vz.w, 1);
-    const float d0 = __shfl_down_sync(kFull, vz.x, 1), d1 = __shfl_down_sync(kFull, vz.y, 1);
-    const float d2 = __shfl_down_sync(kFull, vz.z, 1);
-    const float dz0 = dif8(zdm8(ln, 0), vz.x - u3, vz.y - u2, vz.z - u1, vz.w - u0);
-    const float dz1 = dif8(zdm8(ln, 1), vz.y - vz.x, vz.z - u3, vz.w - u2, d0 - u1);
-    const float dz2 = dif8(zdm8(ln, 2), vz.z - vz.y, vz.w - vz.x, d0 - u3, d1 - u2);
-    const float dz3 = dif8(zdm8(ln, 3), vz.w - vz.z, d0 - vz.y, d1 - vz.x, d2 - u3);
-    const float4 cx = XF ? make_float4(kC81, kC82, kC83, kC84) : dm8(P, S.nnx);
-    const float dx0 = dif8(cx, w[4].x - w[3].x, w[5].x - w[2].x, w[6].x - w[1].x, w[7].x - w[0].x);
-    const float dx1 = dif8(cx, w[4].y - w[3].y, w[5].y - w[2].y, w[6].y - w[1].y, w[7].y - w[0].y);
-    const float dx2 = dif8(cx, w[4].z - w[3].z, w[5].z - w[2].z, w[6].z - w[1].z, w[7].z - w[0].z);
-    const float dx3 = dif8(cx, w[4].w - w[3].w, w[5].w - w[2].w, w[6].w - w[1].w, w[7].w - w[0].w);
-    const float4 r0 = zrow(ln, 0), r1 = zrow(ln, 1), r2 = zrow(ln, 2), r3 = zrow(ln, 3);
-    p_cell(colm && (FAST || r0.x == 1.0f), xc.x, xc.y, r0.x, r0.y, px.x, pz.x, kk.x, dx0, dz0, pxn.x, pzn.x, dxv.x,
-           dzv.x);
-    p_cell(colm && (FAST || r1.x == 1.0f), xc.x, xc.y, r1.x, r1.y, px.y, pz.y, kk.y, dx1, dz1, pxn.y, pzn.y, dxv.y,
-           dzv.y);
-    p_cell(colm && (FAST || r2.x == 1.0f), xc.x, xc.y, r2.x, r2.y, px.z, pz.z, kk.z, dx2, dz2, pxn.z, pzn.z, dxv.z,
-           dzv.z);
-    p_cell(colm && (FAST || r3.x == 1.0f), xc.x, xc.y, r3.x, r3.y, px.w, pz.w, kk.w, dx3, dz3, pxn.w, pzn.w, dxv.w,
-           dzv.w);
-    if (P == ln.src_x && ln.sdz >= 0 && ln.sdz < 4) {
-        if (ln.sdz == 0) pxn.x += ln.amp;
-        else if (ln.sdz == 1) pxn.y += ln.amp;
-        else if (ln.sdz == 2) pxn.z += ln.amp;
-        else pxn.w += ln.amp;
+// One (shot, strip, segment) task of the 8th-order step, two rows at a time
+// (packed FP32), its columns brought in kO8Depth - 1 iterations ahead by
+// per-lane asynchronous copies into a per-warp ring, as the two-step kernel's.
+// Iteration L brings vx at L, px, vz, kappa (and pz) at P = L-3 and bx, bz at V
+// = L-7.  The windows are registers: vx at L-7 .. L (8 columns), new p at L-10 ..
+// L-3 (8), vz at L-7 .. L-3 (5); a loop unrolled by four names them by
+// position and moves them once per four columns (interior tasks), or moves
+// them each column (the others, whose code then stays short).
+struct O8Task {
+    V4 *ring, *tab;  // this lane's part of the warp's shared memory: copies; row coefficients (daz, kz, dbz, lz, D- , D+)
+    int xa, xb, src_x, sdz, nnx;
+    float amp;
+    bool owner;
+    Pair8 c;  // literal coefficients
+    V4 one, kx, kz;
+};
+// Column coefficients of an iteration (kTsAny): Dax, Kx at P and Dbx, Lx at V,
+// read one iteration ahead.
+struct O8Xc {
+    float2 p, v;
+    __device__ __forceinline__ void read(const float4 *xcoef, int nnx, int L) {
+        auto at = [&](int x) {
+            return reinterpret_cast<const float2 *>(xcoef + (min(max(x, -S2D_GX), nnx + S2D_GX - 1) + S2D_GX));
+        };
+        p = __ldg(at(L - 3));
+        v = __ldg(at(L - 7) + 1);
     }
-    return make_float4(pxn.x + pzn.x, pxn.y + pzn.y, pxn.z + pzn.z, pxn.w + pzn.w);
-}
+};
+__device__ __forceinline__ Pair8 pair8(const float4 &c) { return Pair8{dup4(c.x), dup4(c.y), dup4(c.z), dup4(c.w)}; }
 
-// Velocities at column V from new p at V-3 .. V+4 (pw), old vx, vz and bx, bz
-// at V; D+x p and D+z p in dxp, dzp.
-// XF: column V lies in the 8th-order x-interior: no coefficient load.
-template <bool FAST, bool XF = false>
-__device__ __forceinline__ void v_update8(const Lane<FAST> &ln, const ShotDev &S, int V, const float4 (&pw)[8],
-                                          const float4 &vx, const float4 &vz, const float4 &bx, const float4 &bz,
-                                          float4 &vxn, float4 &vzn, float4 &dxp, float4 &dzp) {
-    const float4 xc = XF ? make_float4(1.0f, ln.kx, 1.0f, ln.kx) : __ldg(S.xcoef + (V + S2D_GX));
-    const float4 cx = XF ? make_float4(kC81, kC82, kC83, kC84) : dp8(V, S.nnx);
-    const float ex0 = dif8(cx, pw[4].x - pw[3].x, pw[5].x - pw[2].x, pw[6].x - pw[1].x, pw[7].x - pw[0].x);
-    const float ex1 = dif8(cx, pw[4].y - pw[3].y, pw[5].y - pw[2].y, pw[6].y - pw[1].y, pw[7].y - pw[0].y);
-    const float ex2 = dif8(cx, pw[4].z - pw[3].z, pw[5].z - pw[2].z, pw[6].z - pw[1].z, pw[7].z - pw[0].z);
-    const float ex3 = dif8(cx, pw[4].w - pw[3].w, pw[5].w - pw[2].w, pw[6].w - pw[1].w, pw[7].w - pw[0].w);
-    // p rows z0-3 .. z0+7 at V: the lane above's last three (u), this lane's (q), the lane below's four (d)
-    const float4 q = pw[3];
-    const float u1 = __shfl_up_sync(kFull, q.y, 1), u2 = __shfl_up_sync(kFull, q.z, 1);
-    const float u3 = __shfl_up_sync(kFull, q.w, 1);
-    const float d0 = __shfl_down_sync(kFull, q.x, 1), d1 = __shfl_down_sync(kFull, q.y, 1);
-    const float d2 = __shfl_down_sync(kFull, q.z, 1), d3 = __shfl_down_sync(kFull, q.w, 1);
-    const float ez0 = dif8(zdp8(ln, 0), q.y - q.x, q.z - u3, q.w - u2, d0 - u1);
-    const float ez1 = dif8(zdp8(ln, 1), q.z - q.y, q.w - q.x, d0 - u3, d1 - u2);
-    const float ez2 = dif8(zdp8(ln, 2), q.w - q.z, d0 - q.y, d1 - q.x, d2 - u3);
-    const float ez3 = dif8(zdp8(ln, 3), d0 - q.w, d1 - q.z, d2 - q.y, d3 - q.x);
-    dxp = make_float4(ex0, ex1, ex2, ex3);
-    dzp = make_float4(ez0, ez1, ez2, ez3);
-    vxn.x = upd(xc.z, vx.x, xc.w, bx.x, ex0);
-    vxn.y = upd(xc.z, vx.y, xc.w, bx.y, ex1);
-    vxn.z = upd(xc.z, vx.z, xc.w, bx.z, ex2);
-    vxn.w = upd(xc.z, vx.w, xc.w, bx.w, ex3);
-    float4 r = zrow(ln, 0);
-    vzn.x = upd(r.z, vz.x, r.w, bz.x, ez0);
-    r = zrow(ln, 1);
-    vzn.y = upd(r.z, vz.y, r.w, bz.y, ez1);
-    r = zrow(ln, 2);
-    vzn.z = upd(r.z, vz.z, r.w, bz.z, ez2);
-    r = zrow(ln, 3);
-    vzn.w = upd(r.z, vz.w, r.w, bz.w, ez3);
-}
+// Outputs of one iteration: px, pz (and the products at P) at column P, vx, vz
+// (and the products there) at column V.
+struct O8Out {
+    float *p, *v;   // px at P, vx at V; pz and vz one field on
+    float *tp, *tv; // products: first slot at P, third slot at V
+};
 
-// One (shot, strip, segment) task of the 8th-order step.  Columns read:
-// vx at xa-7 .. xb+6, px, pz, kappa, vz at xa-3 .. xb+3, bx, bz at xa .. xb-1
-// (inside the 8 ghost columns on each side).
-// XF: every column the task updates or differentiates lies in the 8th-order
-// x-interior (literal coefficients, no coefficient loads).
-template <bool FAST, bool PROD, bool XF = false>
-__device__ __forceinline__ void o8_task(const StepArgs &a, const ShotDev &S, int strip, int xa, int seg_len, int kt,
-                                        int par, bool rec_step, int slot, int lane) {
-    const int xb = min(S.nnx, xa + seg_len);
-    const size_t ld = (size_t)S.ld;
-    const int c = strip * S2D_TS_OUT - 8;
-    Lane<FAST> ln;
-    lane_setup(ln, S, c, lane, kt);
-    ln.owner = lane >= 2 && lane <= 29 && ln.z0 >= 0 && ln.z0 < S.nnz;
-    // receivers only where the strip's rows hold some
-    const bool rec = rec_step && slot < S.real_nt && !(a.flags & S2D_STEP_NO_RECORD) &&
-                     c + S2D_STRIP_ROWS > S.rec_zlo && c <= S.rec_zhi;
-    const size_t off = (size_t)(ln.z0 + S2D_GZ) + (size_t)S2D_GX * ld;
-    const int fs = S.fstride;
-    float *const sb = S.st[0][0] + off;
-    const int ib = par * 4 * fs, ob = (par ^ 1) * 4 * fs;
-    const float *__restrict__ pxi = sb + ib;
-    const float *__restrict__ pzi = sb + ib + fs;
-    const float *__restrict__ vxi = sb + ib + 2 * fs;
-    const float *__restrict__ vzi = sb + ib + 3 * fs;
-    float *__restrict__ pxo = sb + ob;
-    float *__restrict__ pzo = sb + ob + fs;
-    float *__restrict__ vxo = sb + ob + 2 * fs;
-    float *__restrict__ vzo = sb + ob + 3 * fs;
-    const float *__restrict__ kap = S.kappa + off;
-    const float *__restrict__ bxp = kap + fs;
-    const float *__restrict__ bzp = kap + 2 * fs;
-    const size_t F = (size_t)(S.nnx + 2 * S2D_GX) * ld;
-    float *__restrict__ pr = PROD ? S.prod + (size_t)(kt - a.prod_kt0) * 4 * F + off : nullptr;
-    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-    float4 w[8], pw[8], zq[5];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) pw[i] = zero;
-#pragma unroll
-    for (int i = 0; i < 5; ++i) zq[i] = zero;
-    w[0] = zero;
-#pragma unroll
-    for (int i = 1; i < 8; ++i) w[i] = ld4(vxi + (ptrdiff_t)(xa - 8 + i) * (ptrdiff_t)ld);
-    for (int L = xa; L <= xb + 6; ++L) {
-        const int P = L - 3;
-        const ptrdiff_t colP = (ptrdiff_t)P * (ptrdiff_t)ld;
-#pragma unroll
-        for (int i = 0; i < 7; ++i) w[i] = w[i + 1];
-        w[7] = ld4(vxi + (ptrdiff_t)L * (ptrdiff_t)ld);
-        const float4 vz = ld4(vzi + colP);
-        const float4 xc = XF ? make_float4(1.0f, ln.kx, 1.0f, ln.kx) : __ldg(S.xcoef + (P + S2D_GX));
-        const bool colm = XF || xc.x == 1.0f;
-        const bool pz_live = !(FAST && colm);
-        float4 pxn, pzn, dxv, dzv;
-        const float4 pn = p_update8<FAST, XF>(ln, S, P, xc, colm, w, ld4(pxi + colP),
-                                              pz_live ? ld4(pzi + colP) : zero, ld4(kap + colP), vz, pxn, pzn,
-                                              dxv, dzv);
-        const bool in_seg = P >= xa && P < xb;
-        if (in_seg && ln.owner) {
-            st4(pxo + colP, pxn);
-            if (pz_live) st4(pzo + colP, pzn);
+// Iteration L: w[0..7] vx at L-7 .. L (w[7] is set here), q[0..7] new p at
+// L-10 .. L-3 (q[7] set here), z[0..4] vz at L-7 .. L-3 (z[4] set here).
+template <int KIND, bool PROD, class Rec>
+__device__ __forceinline__ void o8_column(const O8Task &k, const O8Xc &xc, const V4 *in, int L, const O8Out &o,
+                                          size_t fs, size_t F, V4 *w, V4 *q, V4 *z, Rec rec) {
+    w[7] = in[0];
+    const V4 vz = in[64], kk = in[96];
+    z[4] = vz;
+    const int P = L - 3, V = L - 7;
+    // ---- pressure at P ----
+    const bool upd_p = k.owner && P >= k.xa && P < k.xb, upd_v = k.owner && V >= k.xa && V < k.xb;
+    const Pair8 cm = KIND == kTsAny ? pair8(dm8(P, k.nnx)) : k.c;
+    const V4 dx = dif8_4(cm, w[4] - w[3], w[5] - w[2], w[6] - w[1], w[7] - w[0]);
+    V4 px = in[32], pn;
+    if (KIND == kTsIn) {
+        const V4 t = dif4(k.kx, dx, k.kz, dminus_z8(k.c, vz));
+        px = fma4(kk, t, px);
+        if (P == k.src_x) ts2_source(px, k.sdz, k.amp);
+        pn = px;
+        if (upd_p) {
+            *reinterpret_cast<V4 *>(o.p) = px;
+            if (PROD) *reinterpret_cast<V4 *>(o.tp) = t;
+        }
+    } else {
+        const V4 daz = k.tab[0], kz = k.tab[32];
+        const V4 dax = KIND == kTsAny ? dup4(xc.p.x) : k.one, kx = KIND == kTsAny ? dup4(xc.p.y) : k.kx;
+        const V4 dz = dminus_z8(Pair8{k.tab[4 * 32], k.tab[5 * 32], k.tab[6 * 32], k.tab[7 * 32]}, vz);
+        V4 ps = fma4(dax, px, (kx * kk) * dx);
+        V4 pz = fma4(daz, in[192], (kz * kk) * dz);
+        V4 t0 = dx, t1 = dz;
+        if (KIND == kTsRows || xc.p.x == 1.0f) {  // cells whose row is undamped too carry p alone
+            const V4 t = dif4(kx, dx, kz, dz);
+            const V4 pm = fma4(kk, t, px);
+            const bool r0 = lo(daz.a) == 1.0f, r1 = hi(daz.a) == 1.0f, r2 = lo(daz.b) == 1.0f, r3 = hi(daz.b) == 1.0f;
+            auto pick = [&](const V4 &m, const V4 &s) {
+                return v4(pk(r0 ? lo(m.a) : lo(s.a), r1 ? hi(m.a) : hi(s.a)),
+                          pk(r2 ? lo(m.b) : lo(s.b), r3 ? hi(m.b) : hi(s.b)));
+            };
+            ps = pick(pm, ps);
+            pz = pick(zero4(), pz);
             if (PROD) {
-                st4(pr + colP, dxv);
-                if (pz_live) st4(pr + F + colP, dzv);
+                t0 = pick(t, t0);
+                t1 = pick(zero4(), t1);
             }
         }
-        if (rec && in_seg) record(ln, S, P, pn, slot);
-#pragma unroll
-        for (int i = 0; i < 7; ++i) pw[i] = pw[i + 1];
-        pw[7] = pn;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) zq[i] = zq[i + 1];
-        zq[4] = vz;
-        if (L >= xa + 7) {
-            const int V = L - 7;
-            const ptrdiff_t colV = (ptrdiff_t)V * (ptrdiff_t)ld;
-            float4 vxn, vzn, dxp, dzp;
-            v_update8<FAST, XF>(ln, S, V, pw, w[0], zq[0], ld4(bxp + colV), ld4(bzp + colV), vxn, vzn, dxp, dzp);
-            if (ln.owner) {
-                st4(vxo + colV, vxn);
-                st4(vzo + colV, vzn);
-                if (PROD) {
-                    st4(pr + 2 * F + colV, dxp);
-                    st4(pr + 3 * F + colV, dzp);
-                }
+        if (P == k.src_x) ts2_source(ps, k.sdz, k.amp);
+        pn = ps + pz;
+        if (upd_p) {
+            *reinterpret_cast<V4 *>(o.p) = ps;
+            *reinterpret_cast<V4 *>(o.p + fs) = pz;
+            if (PROD) {
+                *reinterpret_cast<V4 *>(o.tp) = t0;
+                *reinterpret_cast<V4 *>(o.tp + F) = t1;
             }
+        }
+    }
+    q[7] = pn;
+    rec(P, pn);
+    // ---- velocities at V ----
+    const Pair8 cp = KIND == kTsAny ? pair8(dp8(V, k.nnx)) : k.c;
+    const V4 ex = dif8_4(cp, q[4] - q[3], q[5] - q[2], q[6] - q[1], q[7] - q[0]);
+    const V4 ez = KIND == kTsIn ? dplus_z8(k.c, q[3])
+                                : dplus_z8(Pair8{k.tab[8 * 32], k.tab[9 * 32], k.tab[10 * 32], k.tab[11 * 32]}, q[3]);
+    const V4 bx = (KIND == kTsAny ? dup4(xc.v.y) : k.kx) * in[128], bz = (KIND == kTsIn ? k.kz : k.tab[3 * 32]) * in[160];
+    const V4 vxn = fma4(KIND == kTsAny ? dup4(xc.v.x) : k.one, w[0], bx * ex);
+    const V4 vzn = fma4(KIND == kTsIn ? k.one : k.tab[2 * 32], z[0], bz * ez);
+    if (upd_v) {
+        *reinterpret_cast<V4 *>(o.v) = vxn;
+        *reinterpret_cast<V4 *>(o.v + fs) = vzn;
+        if (PROD) {
+            *reinterpret_cast<V4 *>(o.tv) = ex;
+            *reinterpret_cast<V4 *>(o.tv + F) = ez;
         }
     }
 }
 
-// The same task with its windows in a per-warp shared-memory ring instead of
-// registers (kVariantO8s, 128 registers, 16 warps per SM): vx of the last 8
-// columns, new p of the last 8, vz of the last 4.  Each lane reads back only
-// the entries it wrote, so the ring needs no synchronisation.
-__device__ __forceinline__ float4 &o8_ring(float4 *ring, int field, int col, int lane) {
-    // field 0: vx (8 slots), 1: new p (8 slots), 2: vz (4 slots)
-    return field == 2 ? ring[(16 + (col & 3)) * 32 + lane] : ring[(field * 8 + (col & 7)) * 32 + lane];
-}
-
-// XF: as for o8_task, literal column coefficients on x-interior tasks.
-template <bool FAST, bool XF = false>
-__device__ __forceinline__ void o8s_task(const StepArgs &a, const ShotDev &S, int strip, int xa, int seg_len, int kt,
-                                         int par, bool rec_step, int slot, int lane, float4 *ring) {
-    const int xb = min(S.nnx, xa + seg_len);
-    const size_t ld = (size_t)S.ld;
+template <int KIND, bool PROD>
+__device__ __forceinline__ void o8_task(const StepArgs &a, const ShotDev &S, int strip, int xa, int seg_len, int kt,
+                                        int par, bool rec_step, int slot, int lane, V4 *smem) {
+    constexpr int U = KIND == kTsIn ? 4 : 1;
+    const int xb = min(S.nnx, xa + seg_len), nnx = S.nnx;
+    const ptrdiff_t ld = (ptrdiff_t)S.ld;
     const int c = strip * S2D_TS_OUT - 8;
-    Lane<FAST> ln;
+    Lane<true> ln;  // rows and source of the lane
     lane_setup(ln, S, c, lane, kt);
-    ln.owner = lane >= 2 && lane <= 29;
-    // receivers only where the strip's rows hold some
-    const bool rec = rec_step && slot < S.real_nt && !(a.flags & S2D_STEP_NO_RECORD) &&
-                     c + S2D_STRIP_ROWS > S.rec_zlo && c <= S.rec_zhi;
-    const size_t off = (size_t)(ln.z0 + S2D_GZ) + (size_t)S2D_GX * ld;
-    const int fs = S.fstride;
-    float *const sb = S.st[0][0] + off;
-    const int ib = par * 4 * fs, ob = (par ^ 1) * 4 * fs;
-    const float *__restrict__ pxi = sb + ib;
-    const float *__restrict__ pzi = sb + ib + fs;
-    const float *__restrict__ vxi = sb + ib + 2 * fs;
-    const float *__restrict__ vzi = sb + ib + 3 * fs;
-    float *__restrict__ pxo = sb + ob;
-    float *__restrict__ pzo = sb + ob + fs;
-    float *__restrict__ vxo = sb + ob + 2 * fs;
-    float *__restrict__ vzo = sb + ob + 3 * fs;
-    const float *__restrict__ kap = S.kappa + off;
-    const float *__restrict__ bxp = kap + fs;
-    const float *__restrict__ bzp = kap + 2 * fs;
-    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int col = xa - 7; col < xa; ++col) o8_ring(ring, 0, col, lane) = ld4(vxi + (ptrdiff_t)col * (ptrdiff_t)ld);
-    for (int L = xa; L <= xb + 6; ++L) {
-        const int P = L - 3;
-        const ptrdiff_t colP = (ptrdiff_t)P * (ptrdiff_t)ld;
-        float4 w[8];
-        w[7] = ld4(vxi + (ptrdiff_t)L * (ptrdiff_t)ld);
+    O8Task k;
+    k.ring = smem + lane;
+    k.tab = k.ring + kO8Depth * kO8Slots * 32;
+    k.xa = xa;
+    k.xb = xb;
+    k.nnx = nnx;
+    k.src_x = __any_sync(kFull, ln.sdz >= 0 && ln.sdz < 4) ? ln.src_x : INT_MIN;  // none of the warp's rows: no column
+    k.sdz = ln.sdz;
+    k.amp = ln.amp;
+    k.owner = lane >= 2 && lane <= 29 && ln.z0 >= 0 && ln.z0 < S.nnz;
+    k.c = pair8(make_float4(kC81, kC82, kC83, kC84));
+    k.kx = dup4(ln.kx);
+    k.kz = dup4(ln.kz);
+    k.one = dup4(a.one);  // 1 that the compiler does not know (a literal one would fuse its addend's product too)
+    if (KIND != kTsIn) {
+        float r[12][4];
 #pragma unroll
-        for (int i = 0; i < 7; ++i) w[i] = o8_ring(ring, 0, L - 7 + i, lane);
-        o8_ring(ring, 0, L, lane) = w[7];  // the slot of column L-8, no longer needed
-        const float4 vz = ld4(vzi + colP);
-        const float4 xc = XF ? make_float4(1.0f, ln.kx, 1.0f, ln.kx) : __ldg(S.xcoef + (P + S2D_GX));
-        const bool colm = XF || xc.x == 1.0f;
-        const bool pz_live = !(FAST && colm);
-        float4 pxn, pzn, dxv, dzv;
-        const float4 pn = p_update8<FAST, XF>(ln, S, P, xc, colm, w, ld4(pxi + colP),
-                                              pz_live ? ld4(pzi + colP) : zero, ld4(kap + colP), vz, pxn, pzn, dxv,
-                                              dzv);
-        const bool in_seg = P >= xa && P < xb;
-        if (in_seg && ln.owner) {
-            st4(pxo + colP, pxn);
-            if (pz_live) st4(pzo + colP, pzn);
+        for (int i = 0; i < 4; ++i) {
+            const float4 f = __ldg(ln.zc + i), m = dm8(ln.z0 + i, S.nnz), p = dp8(ln.z0 + i, S.nnz);
+            r[0][i] = f.x, r[1][i] = f.y, r[2][i] = f.z, r[3][i] = f.w;
+            r[4][i] = m.x, r[5][i] = m.y, r[6][i] = m.z, r[7][i] = m.w;
+            r[8][i] = p.x, r[9][i] = p.y, r[10][i] = p.z, r[11][i] = p.w;
         }
-        if (rec && in_seg) record(ln, S, P, pn, slot);
-        const float4 vzV = o8_ring(ring, 2, P - 4, lane);  // read before vz at P takes its slot
-        o8_ring(ring, 2, P, lane) = vz;
-        o8_ring(ring, 1, P, lane) = pn;                    // the slot of column P-8
-        if (L >= xa + 7) {
-            const int V = L - 7;
-            const ptrdiff_t colV = (ptrdiff_t)V * (ptrdiff_t)ld;
-            float4 pw[8];
 #pragma unroll
-            for (int i = 0; i < 7; ++i) pw[i] = o8_ring(ring, 1, V - 3 + i, lane);
-            pw[7] = pn;
-            float4 vxn, vzn, dxp, dzp;
-            v_update8<FAST, XF>(ln, S, V, pw, w[0], vzV, ld4(bxp + colV), ld4(bzp + colV), vxn, vzn, dxp, dzp);
-            if (ln.owner) {
-                st4(vxo + colV, vxn);
-                st4(vzo + colV, vzn);
+        for (int i = 0; i < 12; ++i) k.tab[i * 32] = v4(pk(r[i][0], r[i][1]), pk(r[i][2], r[i][3]));
+    }
+    const bool rows = rec_step && slot < S.real_nt && !(a.flags & S2D_STEP_NO_RECORD) && S.nrec > 0 &&
+                      c + S2D_STRIP_ROWS > S.rec_zlo && c <= S.rec_zhi;
+    RecCursor cur;
+    if (rows) cur.start(S, xa);
+    auto rec = [&](int P, const V4 &p) {
+        if (!rows || P < xa || P >= xb) return;
+        cur.column(S, P, ln.z0, k.owner, slot,
+                   [&](int i) { return i == 0 ? lo(p.a) : i == 1 ? hi(p.a) : i == 2 ? lo(p.b) : hi(p.b); });
+    };
+    const size_t off = (size_t)(ln.z0 + S2D_GZ) + (size_t)S2D_GX * ld;
+    const ptrdiff_t fs = S.fstride;
+    const size_t F = (size_t)(nnx + 2 * S2D_GX) * ld;
+    const int L0 = xa - 7, Lend = xb + 6;  // columns L0 .. xa-1 fill the vx window
+    const int n4 = (Lend - xa + U) / U;    // groups of U iterations from L = xa on (the last may pass Lend)
+    const int Llast = xa + U * n4 - 1;
+    // px and kappa at the next iteration's column P; the other pieces lie at
+    // fixed distances
+    const float *np = S.st[0][0] + (size_t)par * 4 * fs + off + (ptrdiff_t)(L0 - 3) * ld;
+    const float *nm = S.kappa + off + (ptrdiff_t)(L0 - 3) * ld;
+    const ptrdiff_t ovx = 3 * ld + 2 * fs, ovz = 3 * fs, obx = fs - 4 * ld, obz = 2 * fs - 4 * ld;
+    auto issue = [&](int L, int sl) {
+        V4 *st = k.ring + sl * (kO8Slots * 32);
+        cp_async16(st, np + ovx, true);
+        if (L >= xa) {
+            cp_async16(st + 32, np, true);
+            cp_async16(st + 64, np + ovz, true);
+            cp_async16(st + 96, nm, true);
+            cp_async16(st + 128, nm + obx, true);
+            cp_async16(st + 160, nm + obz, true);
+            if (KIND != kTsIn) cp_async16(st + 192, np + fs, true);
+        }
+        np += ld;
+        nm += ld;
+    };
+#pragma unroll
+    for (int i = 0; i < kO8Depth - 1; ++i) {
+        issue(L0 + i, i);
+        cp_async_commit();
+    }
+    auto next = [&](int L, int sl) {  // bring iteration L + kO8Depth - 1, wait for iteration L (in slot sl)
+        if (L + kO8Depth - 1 <= Llast) issue(L + kO8Depth - 1, (sl + kO8Depth - 1) % kO8Depth);
+        cp_async_commit();
+        cp_async_wait<kO8Depth - 1>();
+        return k.ring + sl * (kO8Slots * 32);
+    };
+    V4 w[7 + U], q[7 + U], z[4 + U];
+#pragma unroll
+    for (int i = 0; i < 7; ++i) {
+        w[i] = next(L0 + i, i % kO8Depth)[0];
+        q[i] = zero4();
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) z[i] = zero4();
+    float *const so = S.st[0][0] + (size_t)(par ^ 1) * 4 * fs + off;
+    float *const pr = PROD ? S.prod + (size_t)(kt - a.prod_kt0) * 4 * F + off : nullptr;
+    O8Out o;
+    o.p = so + (ptrdiff_t)(xa - 3) * ld;
+    o.v = so + (ptrdiff_t)(xa - 7) * ld + 2 * fs;
+    o.tp = PROD ? pr + (ptrdiff_t)(xa - 3) * ld : nullptr;
+    o.tv = PROD ? pr + (ptrdiff_t)(xa - 7) * ld + 2 * F : nullptr;
+    O8Xc xc{};
+    if (KIND == kTsAny) xc.read(S.xcoef, nnx, xa);
+    int L = xa, sl = 7 % kO8Depth;
+#pragma unroll 1
+    for (int g = 0; g < n4; ++g) {
+#pragma unroll
+        for (int j = 0; j < U; ++j) {
+            O8Xc xn{};
+            if (KIND == kTsAny) xn.read(S.xcoef, nnx, L + 1);
+            const int s = U == 4 ? (7 + j) % kO8Depth : sl;
+            o8_column<KIND, PROD>(k, xc, next(L, s), L, o, (size_t)fs, F, w + j, q + j, z + j, rec);
+            xc = xn;
+            ++L;
+            if (U == 1) sl = (sl + 1) % kO8Depth;
+            o.p += ld;
+            o.v += ld;
+            if (PROD) {
+                o.tp += ld;
+                o.tv += ld;
             }
         }
+#pragma unroll
+        for (int i = 0; i < 7; ++i) {
+            w[i] = w[i + U];
+            q[i] = q[i + U];
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) z[i] = z[i + U];
     }
+    cp_async_wait<0>();
 }
 
 // Debug self-check (S2D_DEVICE_CHECKS) of the 8th-order task's reach.
@@ -1501,10 +1521,9 @@ __device__ __forceinline__ bool o8_in_bounds(const StepArgs &a, const ShotDev &S
     return true;
 }
 
-// MINB blocks of 4 warps per SM: 3 caps registers at 168 (some spill), 2
-// leaves the 224 the windows (84 registers) and stencils need.
-template <int MINB, bool PROD>
-__global__ void __launch_bounds__(128, MINB) step_kernel_o8(const StepArgs *__restrict__ A, int kt_off) {
+template <bool PROD>
+__global__ void __launch_bounds__(128, 2) step_kernel_o8(const StepArgs *__restrict__ A, int kt_off) {
+    extern __shared__ __align__(128) unsigned char smem[];
     const StepArgs a = *A;
     const int lane = threadIdx.x & 31;
     const int gwarp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
@@ -1514,11 +1533,14 @@ __global__ void __launch_bounds__(128, MINB) step_kernel_o8(const StepArgs *__re
     const int par = a.par0 ^ (kt_off & 1);
     const bool rec_step = ((kt + 1) % a.dt_factor) == 0;
     const int slot = (kt + 1) / a.dt_factor - 1;
+    V4 *const mem = reinterpret_cast<V4 *>(smem + (size_t)(threadIdx.x >> 5) * kO8WarpBytes);
     __shared__ ShotDev shot_rec[4];  // the task's shot record, one slot per warp
     ShotDev &S = shot_rec[(threadIdx.x >> 5) & 3];
-    for (int t = gwarp; t < a.total_tasks; t += nwarp) {
+    TaskQueue queue(a.queue, nwarp, lane);
+    for (int t = gwarp; t < a.total_tasks; t = queue.take()) {
+        queue.draw();
         int strip, xa, seg_len;
-        const ShotDev &G = task_of(a, t, strip, xa, seg_len);
+        const ShotDev &G = task_of_split(a, t, strip, xa, seg_len);
         warp_copy_shot(S, G, lane);
         if (!o8_in_bounds(a, S, strip, xa, seg_len)) continue;
         const int c = strip * S2D_TS_OUT - 8;
@@ -1528,44 +1550,11 @@ __global__ void __launch_bounds__(128, MINB) step_kernel_o8(const StepArgs *__re
         // velocities on xa .. xb-1 (D+: [3, nnx-5]), all undamped in x
         const int xb = min(S.nnx, xa + seg_len);
         const bool xf = xa - 3 >= max(S.xfast_lo, 4) && xb + 3 < min(S.xfast_hi, S.nnx - 3);
-        if (zf && xf) o8_task<true, PROD, true>(a, S, strip, xa, seg_len, kt, par, rec_step, slot, lane);
-        else if (zf) o8_task<true, PROD, false>(a, S, strip, xa, seg_len, kt, par, rec_step, slot, lane);
-        else if (xf) o8_task<false, PROD, true>(a, S, strip, xa, seg_len, kt, par, rec_step, slot, lane);
-        else o8_task<false, PROD, false>(a, S, strip, xa, seg_len, kt, par, rec_step, slot, lane);
+        if (zf && xf) o8_task<kTsIn, PROD>(a, S, strip, xa, seg_len, kt, par, rec_step, slot, lane, mem);
+        else if (xf) o8_task<kTsRows, PROD>(a, S, strip, xa, seg_len, kt, par, rec_step, slot, lane, mem);
+        else o8_task<kTsAny, PROD>(a, S, strip, xa, seg_len, kt, par, rec_step, slot, lane, mem);
     }
-}
-
-// The shared-memory-ring form: 128 registers, 4 blocks of 4 warps per SM,
-// kO8sWarpBytes of dynamic shared memory per warp.
-__global__ void __launch_bounds__(128, 4) step_kernel_o8s(const StepArgs *__restrict__ A, int kt_off) {
-    extern __shared__ __align__(128) unsigned char smem[];
-    float4 *ring = reinterpret_cast<float4 *>(smem + (size_t)(threadIdx.x >> 5) * kO8sWarpBytes);
-    const StepArgs a = *A;
-    const int lane = threadIdx.x & 31;
-    const int gwarp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-    const int nwarp = (int)((gridDim.x * blockDim.x) >> 5);
-    const int kt = a.kt_base + kt_off;
-    if (kt >= a.fd_nt) return;
-    const int par = a.par0 ^ (kt_off & 1);
-    const bool rec_step = ((kt + 1) % a.dt_factor) == 0;
-    const int slot = (kt + 1) / a.dt_factor - 1;
-    __shared__ ShotDev shot_rec[4];  // the task's shot record, one slot per warp
-    ShotDev &S = shot_rec[(threadIdx.x >> 5) & 3];
-    for (int t = gwarp; t < a.total_tasks; t += nwarp) {
-        int strip, xa, seg_len;
-        const ShotDev &G = task_of(a, t, strip, xa, seg_len);
-        warp_copy_shot(S, G, lane);
-        if (!o8_in_bounds(a, S, strip, xa, seg_len)) continue;
-        const int c = strip * S2D_TS_OUT - 8;
-        const bool zf = rows_fast(S, c, c + S2D_STRIP_ROWS - 1) && c >= 4 && c + S2D_STRIP_ROWS - 1 <= S.nnz - 5;
-        // the columns of o8_task's x-interior condition
-        const int xb = min(S.nnx, xa + seg_len);
-        const bool xf = xa - 3 >= max(S.xfast_lo, 4) && xb + 3 < min(S.xfast_hi, S.nnx - 3);
-        if (zf && xf) o8s_task<true, true>(a, S, strip, xa, seg_len, kt, par, rec_step, slot, lane, ring);
-        else if (zf) o8s_task<true, false>(a, S, strip, xa, seg_len, kt, par, rec_step, slot, lane, ring);
-        else if (xf) o8s_task<false, true>(a, S, strip, xa, seg_len, kt, par, rec_step, slot, lane, ring);
-        else o8s_task<false, false>(a, S, strip, xa, seg_len, kt, par, rec_step, slot, lane, ring);
-    }
+    queue.leave();
 }
 
 // ---- model preparation (cpumodelling.cpp:207-230, cpu_modelling_kernels.cpp:64-121) ----
@@ -2074,14 +2063,10 @@ int launch_step(int variant, const StepArgs *args_dev, int kt_off, int grid, int
         step_kernel_ts2<<<grid, block, smem, (cudaStream_t)stream>>>(args_dev, kt_off);
     else if (variant == kVariantTs1)
         step_kernel_ts1<<<grid, block, 0, (cudaStream_t)stream>>>(args_dev, kt_off);
-    else if (variant == kVariantO8)
-        step_kernel_o8<3, false><<<grid, block, 0, (cudaStream_t)stream>>>(args_dev, kt_off);
-    else if (variant == kVariantO8r)
-        step_kernel_o8<2, false><<<grid, block, 0, (cudaStream_t)stream>>>(args_dev, kt_off);
+    else if (order8_variant(variant))
+        step_kernel_o8<false><<<grid, block, smem, (cudaStream_t)stream>>>(args_dev, kt_off);
     else if (variant == kVariantO8Products)
-        step_kernel_o8<3, true><<<grid, block, 0, (cudaStream_t)stream>>>(args_dev, kt_off);
-    else if (variant == kVariantO8s)
-        step_kernel_o8s<<<grid, block, smem, (cudaStream_t)stream>>>(args_dev, kt_off);
+        step_kernel_o8<true><<<grid, block, smem, (cudaStream_t)stream>>>(args_dev, kt_off);
     else if (variant == kVariantTma)
         step_kernel_tma<false><<<grid, block, smem, (cudaStream_t)stream>>>(args_dev, kt_off);
     else if (variant == kVariantAsync)
@@ -2137,10 +2122,8 @@ const void *kernel_of(int variant) {
     if (variant == kVariantLdg128) return (const void *)step_kernel_ldg<false, 4>;
     if (variant == kVariantTs2) return (const void *)step_kernel_ts2;
     if (variant == kVariantTs1) return (const void *)step_kernel_ts1;
-    if (variant == kVariantO8) return (const void *)step_kernel_o8<3, false>;
-    if (variant == kVariantO8r) return (const void *)step_kernel_o8<2, false>;
-    if (variant == kVariantO8Products) return (const void *)step_kernel_o8<3, true>;
-    if (variant == kVariantO8s) return (const void *)step_kernel_o8s;
+    if (order8_variant(variant)) return (const void *)step_kernel_o8<false>;
+    if (variant == kVariantO8Products) return (const void *)step_kernel_o8<true>;
     if (variant == kVariantTma) return (const void *)step_kernel_tma<false>;
     if (variant == kVariantAsync) return (const void *)step_kernel_async<false, 4>;
     if (variant == kVariantLdgU4) return (const void *)step_kernel_ldg<false, 4, true>;
