@@ -220,7 +220,7 @@ S2D_API const char *s2d_last_error(const void *ctx);
  *                 registers and shared memory (up to about 1.2 M padded cells)
  *                 run all their steps in one cooperative launch per shot or
  *                 wave of shots where that is the faster way (s2d_forward,
- *                 the forward sweep of s2d_gradient, s2d_forward_static; not
+ *                 the forward steps of s2d_gradient, s2d_forward_static; not
  *                 with S2D_NO_GRAPH or "autotune" 0); 0: one launch per step.
  *                 The results are the same bits.
  *   "on_chip_shape" block shape of that loop, warps * 100 + columns per warp

@@ -251,6 +251,7 @@ struct ResArgs {
     int kt0, nsteps;       // FD steps [kt0, kt0 + nsteps)
     int par0, par1;        // state buffers of step kt0 and of the result (the same one only for 2 steps or more)
     int dt_factor, flags;  // S2D_STEP_* bits
+    int prod_kt0;          // S2D_STEP_PRODUCTS: step of the first products in ShotDev::prod
     unsigned long long *frames;  // resident_frame_bytes, zeroed before every launch
     int *err;              // device error word
     int spin_limit;        // polls before a wait counts as timed out

@@ -31,7 +31,9 @@
 // at the same time), pz in shared memory and smaller frames measured no
 // better.  Against one launch per step, us per FD step: 265 x 165 cells 2.2
 // (7.5), 1080 x 1080 5.0 (12.2, 231 Gcell/s against 96), one 1301 x 501 shot
-// 3.5 (12.5).
+// 3.5 (12.5).  With the gradient's products (16 bytes per cell and step, stored
+// past the caches' reuse): 8 shots of 1301 x 501 39 us per step (65 with one
+// launch of the per-step kernel for all eight), 4 of 701 x 401 9.3 (18).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -117,9 +119,12 @@ enum { kIn = 0, kDamped = 1, kAny = 2 };
 // (undamped, literal operator pairs), bit 1 every column of the tile in its
 // fast columns; kAnyTile: decided at run time (zf_rt), for the widest tiles,
 // whose registers leave the compiler no room for the specialised copies
-// (10 columns per warp: 5.0 us per step against 6.8).
+// (10 columns per warp: 5.0 us per step against 6.8), and for products from 5
+// columns on (7 columns, 8 shots of 1301 x 501: 39 us per step against 43).
 constexpr int kAnyTile = 4;
-template <int NW, int C, int TILE>
+// PROD: every step also leaves its products (S2D_STEP_PRODUCTS, the slots that
+// the adjoint step reads) of the tile's own cells.
+template <int NW, int C, int TILE, bool PROD>
 __device__ __forceinline__ void resident_tile(const ResArgs &a, const ResShot &rs, const ShotDev &S, int cx, int cz,
                                               bool zf_rt, V4 *sm, int *s_rec, int *s_fail) {
     constexpr bool XI = TILE != kAnyTile && (TILE & 2);
@@ -314,6 +319,22 @@ __device__ __forceinline__ void resident_tile(const ResArgs &a, const ResShot &r
     int slot = (a.kt0 + 1 + a.dt_factor - 1) / a.dt_factor - 1;
     int wait = (slot + 1) * a.dt_factor - 1 - a.kt0;
     const bool merged = zf && (XI || cls == kIn);  // every cell of the warp carries p in px alone
+    // products: the lane's rows of the warp's own columns (bit j of own)
+    const size_t F = (size_t)(S.nnx + 2 * S2D_GX) * ld;
+    float *prod = nullptr;
+    unsigned own = 0;
+    if (PROD) {
+        prod = S.prod + (size_t)(a.kt0 - a.prod_kt0) * 4 * F + (z0 + S2D_GZ) + (ptrdiff_t)(xt + lc0 + S2D_GX) * ld;
+        if (lane >= 1 && lane <= 30 && z0 < S.nnz) {
+#pragma unroll
+            for (int j = 0; j < C; ++j)
+                if (lc0 + j >= 3 && lc0 + j < NC - 3 && xt + lc0 + j < S.nnx) own |= 1u << j;
+        }
+    }
+    auto keep = [&](int slot, int j, const V4 &v) {
+        if (own >> j & 1) __stcs(reinterpret_cast<float4 *>(prod + slot * F + (ptrdiff_t)j * ld),
+                                 make_float4(lo(v.a), hi(v.a), lo(v.b), hi(v.b)));
+    };
 
     for (int s = 0; s < nstep; ++s) {
         V4 q0 = vxe[-64], q1 = vxe[-32], qr = vxe[96];
@@ -383,9 +404,11 @@ __device__ __forceinline__ void resident_tile(const ResArgs &a, const ResShot &r
                 const V4 dx = dif4(cm0, q2 - q1, cm1, q3 - q0);
                 const V4 dz = dminus_z(m0, m1, vz[j]);
                 // a cell whose column and row are undamped carries p alone
-                const V4 pm = fma4(k, dif4(kx, dx, kz, dz), px[j]);
+                const V4 t = dif4(kx, dx, kz, dz);
+                const V4 pm = fma4(k, t, px[j]);
                 if (CLS == kIn && ZF) {
                     px[j] = pm;
+                    if (PROD) keep(0, j, t);
                 } else {
                     const V4 ps = fma4(dax, px[j], (kx * k) * dx);
                     // for kIn the z tables hold 0 on undamped rows: pz stays 0 there
@@ -393,6 +416,10 @@ __device__ __forceinline__ void resident_tile(const ResArgs &a, const ResShot &r
                     if (CLS == kDamped) {
                         px[j] = ps;
                         pz[j] = pn;
+                        if (PROD) {
+                            keep(0, j, dx);
+                            keep(1, j, dz);
+                        }
                     } else {
                         const bool und = CLS == kIn || lo(dax.a) == 1.0f;
                         const bool u0 = und && r0, u1 = und && r1, u2 = und && r2, u3 = und && r3;
@@ -400,6 +427,12 @@ __device__ __forceinline__ void resident_tile(const ResArgs &a, const ResShot &r
                                    pk(u2 ? lo(pm.b) : lo(ps.b), u3 ? hi(pm.b) : hi(ps.b)));
                         pz[j] = CLS == kIn ? pn : v4(pk(u0 ? 0.0f : lo(pn.a), u1 ? 0.0f : hi(pn.a)),
                                                      pk(u2 ? 0.0f : lo(pn.b), u3 ? 0.0f : hi(pn.b)));
+                        if (PROD) {
+                            keep(0, j, v4(pk(u0 ? lo(t.a) : lo(dx.a), u1 ? hi(t.a) : hi(dx.a)),
+                                          pk(u2 ? lo(t.b) : lo(dx.b), u3 ? hi(t.b) : hi(dx.b))));
+                            keep(1, j, v4(pk(u0 ? 0.0f : lo(dz.a), u1 ? 0.0f : hi(dz.a)),
+                                          pk(u2 ? 0.0f : lo(dz.b), u3 ? 0.0f : hi(dz.b))));
+                        }
                     }
                 }
                 q0 = q1;
@@ -464,6 +497,10 @@ __device__ __forceinline__ void resident_tile(const ResArgs &a, const ResShot &r
                 const V4 bx = mat[(NC + j) * 32], bz = mat[(2 * NC + j) * 32];
                 const V4 ex = dif4(cp0, g2 - g1, cp1, g3 - g0);
                 const V4 ez = dplus_z(p0, p1, g1);
+                if (PROD) {
+                    keep(2, j, ex);
+                    keep(3, j, ez);
+                }
                 vx[j] = fma4(dbx, vx[j], bx * ex);
                 vz[j] = fma4(dbz, vz[j], bz * ez);
                 g0 = g1;
@@ -548,6 +585,7 @@ __device__ __forceinline__ void resident_tile(const ResArgs &a, const ResShot &r
                 }
             }
         }
+        if (PROD) prod += 4 * F;
         if (wait == 0) {
             wait = a.dt_factor;
             ++slot;
@@ -611,7 +649,7 @@ __device__ __forceinline__ void resident_tile(const ResArgs &a, const ResShot &r
     }
 }
 
-template <int NW, int C>
+template <int NW, int C, bool PROD>
 __global__ void __launch_bounds__(NW * 32, 1) resident_kernel(const ResArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ int s_rec, s_fail;
@@ -632,27 +670,26 @@ __global__ void __launch_bounds__(NW * 32, 1) resident_kernel(const ResArgs a) {
     V4 *const sm = reinterpret_cast<V4 *>(smem);
     const bool zf = rows_fast(S, zc, zc + S2D_STRIP_ROWS - 1);
     const bool xi = xt >= S.xfast_lo && xt + NW * C <= S.xfast_hi;
-    if constexpr (C >= 8) {
-        resident_tile<NW, C, kAnyTile>(a, rs, S, cx, cz, zf, sm, &s_rec, &s_fail);
+    if constexpr (C >= 8 || (PROD && C >= 5)) {
+        resident_tile<NW, C, kAnyTile, PROD>(a, rs, S, cx, cz, zf, sm, &s_rec, &s_fail);
     } else {
-        if (zf && xi) resident_tile<NW, C, 3>(a, rs, S, cx, cz, zf, sm, &s_rec, &s_fail);
-        else if (zf) resident_tile<NW, C, 1>(a, rs, S, cx, cz, zf, sm, &s_rec, &s_fail);
-        else if (xi) resident_tile<NW, C, 2>(a, rs, S, cx, cz, zf, sm, &s_rec, &s_fail);
-        else resident_tile<NW, C, 0>(a, rs, S, cx, cz, zf, sm, &s_rec, &s_fail);
+        if (zf && xi) resident_tile<NW, C, 3, PROD>(a, rs, S, cx, cz, zf, sm, &s_rec, &s_fail);
+        else if (zf) resident_tile<NW, C, 1, PROD>(a, rs, S, cx, cz, zf, sm, &s_rec, &s_fail);
+        else if (xi) resident_tile<NW, C, 2, PROD>(a, rs, S, cx, cz, zf, sm, &s_rec, &s_fail);
+        else resident_tile<NW, C, 0, PROD>(a, rs, S, cx, cz, zf, sm, &s_rec, &s_fail);
     }
 }
 
-template <int NW, int C>
+template <int NW, int C, bool PROD>
 int launch_c(const ResArgs &a, int grid, cudaStream_t st) {
     static_assert(ResSmem<NW, C>::bytes <= 226 * 1024, "shared memory of a block");
-    cudaError_t e = cudaFuncSetAttribute(resident_kernel<NW, C>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)ResSmem<NW, C>::bytes);
+    const void *k = (const void *)resident_kernel<NW, C, PROD>;
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ResSmem<NW, C>::bytes);
     if (e != cudaSuccess) return (int)e;
     ResArgs v = a;
     v.one = 1.0f;
     void *args[] = {&v};
-    return (int)cudaLaunchCooperativeKernel((const void *)resident_kernel<NW, C>, dim3(grid), dim3(NW * 32), args,
-                                            ResSmem<NW, C>::bytes, st);
+    return (int)cudaLaunchCooperativeKernel(k, dim3(grid), dim3(NW * 32), args, ResSmem<NW, C>::bytes, st);
 }
 
 }  // namespace
@@ -670,7 +707,7 @@ size_t resident_frame_bytes(int nw, int c, int ctas) {
 int launch_resident(int nw, int c, const ResArgs &a, int grid, void *stream) {
     cudaStream_t st = (cudaStream_t)stream;
 #define X(W, N, US) \
-    if (nw == W && c == N) return launch_c<W, N>(a, grid, st);
+    if (nw == W && c == N) return a.flags & S2D_STEP_PRODUCTS ? launch_c<W, N, true>(a, grid, st) : launch_c<W, N, false>(a, grid, st);
     S2D_RES_SHAPES(X)
 #undef X
     return (int)cudaErrorInvalidValue;
