@@ -697,229 +697,368 @@ __global__ void __launch_bounds__(128) adjoint8_velocity(const StepArgs *__restr
 // algebra of adjoint8_pressure / adjoint8_velocity, the same products in the
 // same order per cell): a warp owns a 128-row strip read from 112k - 8 and
 // writes its middle 112 rows (lanes 2..29, the 8th-order forward's layout),
-// streaming along x.  At loop column L it loads mvx' and bx; at Q = L-3 it
-// forms the pressure adjoint (x-gather of Lx bx mvx' over Q-4 .. Q+3, z-gather
-// of Lz bz mvz' over the rows z-4 .. z+3 by shuffles from the neighbouring
-// lanes), the z-velocity adjoint (z-gather of Kz kappa mPZ) and the imaging
-// terms; at W = L-7 the x-velocity adjoint (x-gather of Kx kappa mPX over
-// W-3 .. W+4).  The x-gathers read 8-column per-warp shared-memory rings of
-// mvx', Lx bx mvx' and Kx kappa mPX; each lane reads back only what it wrote.
-constexpr int kAdj8Ring = 8, kAdj8Fields = 3;
-constexpr int kAdj8WarpBytes = kAdj8Ring * kAdj8Fields * S2D_STRIP_ROWS * 4;
-__device__ __forceinline__ float4 &adj8_ring(float4 *ring, int field, int col, int lane) {
-    return ring[(field * kAdj8Ring + ((col + 2 * S2D_GX) & (kAdj8Ring - 1))) * 32 + lane];
-}
-__device__ __forceinline__ float c8(const float4 &c, int k) { return comp(c, k); }
+// streaming along x.  Iteration L brings mvx' and bx at L; at Q = L-3 it forms
+// the pressure adjoint (x-gather of Lx bx mvx' over Q-4 .. Q+3, z-gather of Lz
+// bz mvz' over the rows z-4 .. z+3 by shuffles from the neighbouring lanes),
+// the z-velocity adjoint (z-gather of Kz kappa mPZ) and the imaging terms; at W
+// = L-7 the x-velocity adjoint (x-gather of Kx kappa mPX over W-3 .. W+4).
+//
+// Copies, windows, tasks and queue as the 4th-order step's: the inputs come D -
+// 1 iterations ahead by per-lane asynchronous copies, the windows (mvx', Lx bx
+// mvx', Kx kappa mPX of 8 columns each) are registers, named by position in a
+// loop unrolled by four and moved once per four columns (interior tasks), or
+// moved every column (the others).  The 20 row coefficients of tasks that are
+// not interior wait in shared memory.
+//
+// What bounds it: as the 4th-order step, the latency of one column's chain with
+// two warps on each scheduler (255 registers, no spill).  us per step, before
+// (windows in shared memory, loads where they were used, every strip one
+// length) and after: 1201x401, 4 shots 103 -> 48, 8 shots 179 -> 89; 601x301, 4
+// shots 51 -> 27; 2301x1101, 4 shots 340 -> 142 (2.8 TB/s of state, materials
+// and products).
 
-// FAST: every row the task touches is in the 8th-order z-interior (literal
-// coefficients, no z-damping); XF: likewise every column.
-template <bool FAST, bool XF>
-__device__ __forceinline__ void adjoint8s_task(const StepArgs &a, const ShotDev &S, int strip, int xa, int seg_len,
-                                               int kt, int lane, float4 *ring) {
-    const int nnx = S.nnx, nnz = S.nnz;
-    const size_t ld = (size_t)S.ld;
-    const int xb = min(nnx, xa + seg_len);
-    const int c = strip * S2D_TS_OUT - 8;
-    const int z0 = c + S2D_ZPT * lane;
-    const bool ghost = z0 < 0 || z0 >= nnz;
-    const bool owner = lane >= 2 && lane <= 29 && !ghost;
-    const int zl = ghost ? -S2D_GZ : z0;
-    const int pin = (kt + 1) & 1, pout = kt & 1;
-    const size_t off = (size_t)(zl + S2D_GZ) + (size_t)S2D_GX * ld;
-    const size_t F = (size_t)(nnx + 2 * S2D_GX) * ld;
-    const float *__restrict__ mpxi = S.st[pin][0] + off;
-    const float *__restrict__ mpzi = S.st[pin][1] + off;
-    const float *__restrict__ mvxi = S.st[pin][2] + off;
-    const float *__restrict__ mvzi = S.st[pin][3] + off;
-    float *__restrict__ mpxo = S.st[pout][0] + off;
-    float *__restrict__ mpzo = S.st[pout][1] + off;
-    float *__restrict__ mvxo = S.st[pout][2] + off;
-    float *__restrict__ mvzo = S.st[pout][3] + off;
-    const float *__restrict__ kap = S.kappa + off;
-    const float *__restrict__ bxp = S.bx + off;
-    const float *__restrict__ bzp = S.bz + off;
-    const float *__restrict__ pr = S.prod + (size_t)(kt - a.prod_kt0) * 4 * F + off;
-    float *__restrict__ gk = S.grad[0] + off;
-    float *__restrict__ gb = S.grad[1] + off;
-    // receiver adjoint source on recording steps, in strips whose rows hold
-    // receivers (the lookup is three dependent loads per column)
-    const bool inj = !(a.flags & S2D_STEP_NO_RECORD) && ((kt + 1) % a.dt_factor) == 0 &&
-                     (kt + 1) / a.dt_factor - 1 < S.real_nt && c + S2D_STRIP_ROWS > S.rec_zlo &&
-                     c <= S.rec_zhi;
-    const int slot = (kt + 1) / a.dt_factor - 1;
-    const float kx = S.kx_in, kz = S.kz_in;
-    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-    const float4 lit = make_float4(kC81, kC82, kC83, kC84);
-    // coefficient k of the forward D+ / D- row j (x: columns, z: rows)
-    auto cpx = [&](int j, int k) { return XF ? comp(lit, k) : c8(dp8(j, nnx), k); };
-    auto cmx = [&](int j, int k) { return XF ? comp(lit, k) : c8(dm8(j, nnx), k); };
-    auto cpz = [&](int j, int k) { return FAST ? comp(lit, k) : c8(dp8(j, nnz), k); };
-    auto cmz = [&](int j, int k) { return FAST ? comp(lit, k) : c8(dm8(j, nnz), k); };
-    // z-row coefficients (Daz, Kz, Dbz, Lz) of the lane's row z0 + i
-    auto zr = [&](int i) { return FAST ? make_float4(1.0f, kz, 1.0f, kz) : __ldg(S.zcoef + (z0 + i + S2D_GZ)); };
-    float4 tbp = zero;  // tbx at Q-1
-    for (int L = xa - 7; L <= xb + 6; ++L) {
-        {
-            const ptrdiff_t colL = (ptrdiff_t)L * (ptrdiff_t)ld;
-            const float4 m = ld4(mvxi + colL), b = ld4(bxp + colL);
-            const float lx = XF ? kx : __ldg(S.xcoef + (L + S2D_GX)).w;
-            adj8_ring(ring, 0, L, lane) = m;
-            adj8_ring(ring, 1, L, lane) = make_float4((lx * b.x) * m.x, (lx * b.y) * m.y, (lx * b.z) * m.z,
-                                                      (lx * b.w) * m.w);
-        }
-        const int Q = L - 3;
-        if (Q < xa - 3) continue;
-        const ptrdiff_t colQ = (ptrdiff_t)Q * (ptrdiff_t)ld;
-        const bool upd = owner && Q >= xa && Q < xb;
-        const bool img = Q >= xa - 1 && Q < xb && Q >= 0;
-        const float4 xq = XF ? make_float4(1.0f, kx, 1.0f, kx) : __ldg(S.xcoef + (Q + S2D_GX));
-        const bool colm = XF || xq.x == 1.0f;
-        const bool pz_live = !(FAST && colm);
-        const float4 mvz = ld4(mvzi + colQ), bz = ld4(bzp + colQ), kk = ld4(kap + colQ);
-        const float4 mpx = ld4(mpxi + colQ);
-        const float4 mpz = pz_live ? ld4(mpzi + colQ) : zero;
-        const float4 r0 = zr(0), r1 = zr(1), r2 = zr(2), r3 = zr(3);
-        const bool m0 = colm && r0.x == 1.0f, m1 = colm && r1.x == 1.0f;
-        const bool m2 = colm && r2.x == 1.0f, m3 = colm && r3.x == 1.0f;
-        // ---- pressure adjoint at Q ----
-        float qv[4];
-        {
-            // x-gather of g = Lx bx mvx' (columns Q-4 .. Q+3 in ring 1)
-            float4 acc = zero;
+// Kinds of tasks: interior; interior columns and taps, any damping; interior
+// columns, any row; anything.
+enum { kAdj8In = 0, kAdj8Rows = 1, kAdj8Edge = 2, kAdj8Any = 3 };
+template <int KIND>
+struct Adj8Depth {
+    static constexpr int value = KIND == kAdj8In ? 4 : 3;
+};
+constexpr int kAdj8Tab = 20;  // Daz, Kz, Dbz, Lz; taps of H^T and G^T along z, 4 + 4 each
+constexpr int kAdj8Ring = 3 * kAdjSlots + kAdj8Tab;
+constexpr int kAdj8WarpBytes = kAdj8Ring * S2D_STRIP_ROWS * 4;
+static_assert(kAdj8Ring >= 4 * 9, "ring of the interior tasks");
+
+// acc + sum_k p_k m[i-k] + n_k m[i+1+k] of packed rows, each product fused in
+// the order k = 0 (p, n), 1 (p, n) ...; without acc the first one is rounded.
+template <bool ACC, class P, class N>
+__device__ __forceinline__ f2 gather8(f2 acc, P p, N n, const f2 *a, const f2 *b) {
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const int j0 = Q - 1 - k, j1 = Q + k;
-                const float c0 = cpx(j0, k), c1 = cpx(j1, k);
-                const float4 g0 = adj8_ring(ring, 1, j0, lane), g1 = adj8_ring(ring, 1, j1, lane);
-                acc.x += c0 * g0.x; acc.x -= c1 * g1.x;
-                acc.y += c0 * g0.y; acc.y -= c1 * g1.y;
-                acc.z += c0 * g0.z; acc.z -= c1 * g1.z;
-                acc.w += c0 * g0.w; acc.w -= c1 * g1.w;
-            }
-            // z-gather of h = Lz bz mvz' over rows z-4 .. z+3: rows z0-4 .. z0+6
-            const float4 h = make_float4((r0.w * bz.x) * mvz.x, (r1.w * bz.y) * mvz.y, (r2.w * bz.z) * mvz.z,
-                                         (r3.w * bz.w) * mvz.w);
-            float hh[11];
-            hh[0] = __shfl_up_sync(kFull, h.x, 1);
-            hh[1] = __shfl_up_sync(kFull, h.y, 1);
-            hh[2] = __shfl_up_sync(kFull, h.z, 1);
-            hh[3] = __shfl_up_sync(kFull, h.w, 1);
-            hh[4] = h.x; hh[5] = h.y; hh[6] = h.z; hh[7] = h.w;
-            hh[8] = __shfl_down_sync(kFull, h.x, 1);
-            hh[9] = __shfl_down_sync(kFull, h.y, 1);
-            hh[10] = __shfl_down_sync(kFull, h.z, 1);
-            qv[0] = acc.x; qv[1] = acc.y; qv[2] = acc.z; qv[3] = acc.w;
+    for (int k = 0; k < 4; ++k) {
+        acc = !ACC && k == 0 ? mul2(p(k), a[k]) : fma2(p(k), a[k], acc);
+        acc = fma2(n(k), b[k], acc);
+    }
+    return acc;
+}
+
+// Column coefficients of one iteration (kAdj8Any): Lx at L; Dax, Kx, Lx at Q;
+// Dbx at W; read one iteration ahead.
+struct Adj8Xc {
+    float lxl, dbw;
+    float4 q;
+    __device__ __forceinline__ void read(const float4 *xcoef, int nnx, int L) {
+        auto at = [&](int x) { return xcoef + (min(max(x, -S2D_GX), nnx + S2D_GX - 1) + S2D_GX); };
+        lxl = __ldg(&at(L)->w);
+        q = __ldg(at(L - 3));
+        dbw = __ldg(&at(L - 7)->z);
+    }
+};
+
+struct Adj8Task {
+    const ShotDev *S;
+    V4 *ring, *tab;
+    int xa, xb, z0, kt, src_q, sdz, slot;
+    bool owner, inj, row0;
+    V4 one, kx, kz;
+    f2 cp[4], cn[4];  // literal taps and their negatives
+    AdjSource src;
+    V4 tbp;           // tbx at Q-1
+};
+
+// Iteration L: w[0..7] mvx' and g[0..7] Lx bx mvx' at L-7 .. L (the last set
+// here), m[0..7] Kx kappa mPX at L-10 .. L-3 (the last set here).
+template <int KIND>
+__device__ __forceinline__ void adj8_column(Adj8Task &k, const Adj8Xc &xc, const V4 *in, int L, float *po, float *vo,
+                                            float *gk, float *gb, ptrdiff_t fs, V4 *w, V4 *g, V4 *m) {
+    const ShotDev &S = *k.S;
+    const int Q = L - 3, W = L - 7, nnx = S.nnx;
+    w[7] = in[0];
+    g[7] = ((KIND == kAdj8Any ? dup4(xc.lxl) : k.kx) * in[32]) * w[7];
+    const bool upd = k.owner && Q >= k.xa && Q < k.xb;  // this lane writes column Q
+    const V4 mvz = in[96], kk = in[160];
+    const V4 kz = KIND == kAdj8In ? k.kz : k.tab[32], lz = KIND == kAdj8In ? k.kz : k.tab[96];
+    const V4 kx = KIND == kAdj8Any ? dup4(xc.q.y) : k.kx, lx = KIND == kAdj8Any ? dup4(xc.q.w) : k.kx;
+    f2 hp[4], hn[4], vp[4], vn[4];  // taps of the x-gathers at Q and W
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const int z = z0 + i;
+    for (int i = 0; i < 4; ++i) {
+        hp[i] = vp[i] = k.cp[i];
+        hn[i] = vn[i] = k.cn[i];
+    }
+    if (KIND == kAdj8Any && (Q < 11 || Q > nnx - 8)) {
 #pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    qv[i] += cpz(z - 1 - k, k) * hh[4 + i - 1 - k];
-                    qv[i] -= cpz(z + k, k) * hh[4 + i + k];
-                }
-            }
+        for (int i = 0; i < 4; ++i) {
+            hp[i] = dup(comp(dp8(Q - 1 - i, nnx), i));
+            hn[i] = dup(-comp(dp8(Q + i, nnx), i));
+            vp[i] = dup(comp(dm8(W - i, nnx), i));
+            vn[i] = dup(-comp(dm8(W + 1 + i, nnx), i));
         }
-        // transpose of the receiver sampling (cpumodelling.cpp:356-360)
-        if (inj && Q >= 0 && Q < nnx) {
-            const int j1 = __ldg(S.rec_ptr + Q + 1);
-            for (int j = __ldg(S.rec_ptr + Q); j < j1; ++j) {
-                const int d = __ldg(S.rec_z + j) - z0;
-                if (d >= 0 && d < 4) qv[d] += __ldg(S.seis + (size_t)__ldg(S.rec_id + j) * S.real_nt + slot);
-            }
+    }
+    // ---- pressure adjoint at Q ----
+    V4 q;
+    {
+        const f2 a0[4] = {g[3].a, g[2].a, g[1].a, g[0].a}, b0[4] = {g[4].a, g[5].a, g[6].a, g[7].a};
+        const f2 a1[4] = {g[3].b, g[2].b, g[1].b, g[0].b}, b1[4] = {g[4].b, g[5].b, g[6].b, g[7].b};
+        auto p = [&](int i) { return hp[i]; };
+        auto n = [&](int i) { return hn[i]; };
+        q = v4(gather8<false>(0ull, p, n, a0, b0), gather8<false>(0ull, p, n, a1, b1));
+    }
+    {
+        // rows z0-4 .. z0+6 of Lz bz mvz'
+        const V4 h = (lz * in[128]) * mvz;
+        const float x = lo(h.a), y = hi(h.a), z = lo(h.b), v = hi(h.b);
+        const float u0 = __shfl_up_sync(kFull, x, 1), u1 = __shfl_up_sync(kFull, y, 1);
+        const float u2 = __shfl_up_sync(kFull, z, 1), u3 = __shfl_up_sync(kFull, v, 1);
+        const float d0 = __shfl_down_sync(kFull, x, 1), d1 = __shfl_down_sync(kFull, y, 1);
+        const float d2 = __shfl_down_sync(kFull, z, 1);
+        const f2 u3x = pk(u3, x), yz = pk(y, z), vd0 = pk(v, d0), u23 = pk(u2, u3);
+        const f2 a0[4] = {u3x, u23, pk(u1, u2), pk(u0, u1)}, b0[4] = {h.a, yz, h.b, vd0};
+        const f2 a1[4] = {yz, h.a, u3x, u23}, b1[4] = {h.b, vd0, pk(d0, d1), pk(d1, d2)};
+        constexpr bool TAB = KIND >= kAdj8Edge;
+        q.a = gather8<true>(q.a, [&](int i) { return TAB ? k.tab[(4 + i) * 32].a : k.cp[i]; },
+                            [&](int i) { return TAB ? k.tab[(8 + i) * 32].a : k.cn[i]; }, a0, b0);
+        q.b = gather8<true>(q.b, [&](int i) { return TAB ? k.tab[(4 + i) * 32].b : k.cp[i]; },
+                            [&](int i) { return TAB ? k.tab[(8 + i) * 32].b : k.cn[i]; }, a1, b1);
+    }
+    if (k.inj && Q >= 0 && Q < nnx) k.src.column(S, Q, k.z0, k.slot, q);
+    const V4 mPX = in[64] + q;
+    V4 mPZ = mPX, daz = k.one;
+    const V4 dax = KIND == kAdj8Any ? dup4(xc.q.x) : k.one;
+    bool m0 = true, m1 = true, m2 = true, m3 = true;
+    V4 tk = in[192] * mPX;  // one pressure: the first product is Kx a + Kz c
+    if (KIND != kAdj8In) {
+        daz = k.tab[0];
+        const bool colm = KIND != kAdj8Any || xc.q.x == 1.0f;
+        m0 = colm && lo(daz.a) == 1.0f;
+        m1 = colm && hi(daz.a) == 1.0f;
+        m2 = colm && lo(daz.b) == 1.0f;
+        m3 = colm && hi(daz.b) == 1.0f;
+        const V4 z = in[288] + q;
+        mPZ = v4(pk(m0 ? lo(mPX.a) : lo(z.a), m1 ? hi(mPX.a) : hi(z.a)),
+                 pk(m2 ? lo(mPX.b) : lo(z.b), m3 ? hi(mPX.b) : hi(z.b)));
+        const V4 ts = fma4(kx * in[192], mPX, (kz * in[320]) * mPZ);
+        tk = v4(pk(m0 ? lo(tk.a) : lo(ts.a), m1 ? hi(tk.a) : hi(ts.a)),
+                pk(m2 ? lo(tk.b) : lo(ts.b), m3 ? hi(tk.b) : hi(ts.b)));
+    }
+    if (upd) {
+        *reinterpret_cast<V4 *>(po) = KIND == kAdj8Any ? dax * mPX : mPX;
+        if (KIND != kAdj8In) {
+            const V4 o = daz * mPZ;
+            *reinterpret_cast<V4 *>(po + fs) = v4(pk(m0 ? 0.0f : lo(o.a), m1 ? 0.0f : hi(o.a)),
+                                                  pk(m2 ? 0.0f : lo(o.b), m3 ? 0.0f : hi(o.b)));
         }
-        const float4 mPX = make_float4(mpx.x + qv[0], mpx.y + qv[1], mpx.z + qv[2], mpx.w + qv[3]);
-        const float4 mPZ = make_float4(m0 ? mPX.x : mpz.x + qv[0], m1 ? mPX.y : mpz.y + qv[1],
-                                       m2 ? mPX.z : mpz.z + qv[2], m3 ? mPX.w : mpz.w + qv[3]);
-        if (upd) {
-            st4(mpxo + colQ, make_float4(xq.x * mPX.x, xq.x * mPX.y, xq.x * mPX.z, xq.x * mPX.w));
-            if (pz_live)
-                st4(mpzo + colQ, make_float4(m0 ? 0.0f : r0.x * mPZ.x, m1 ? 0.0f : r1.x * mPZ.y,
-                                             m2 ? 0.0f : r2.x * mPZ.z, m3 ? 0.0f : r3.x * mPZ.w));
-            const float4 pa = ld4(pr + colQ);
-            const float4 pc = pz_live ? ld4(pr + F + colQ) : zero;
-            float4 tk;
-            tk.x = m0 ? pa.x * mPX.x : (xq.y * pa.x) * mPX.x + (r0.y * pc.x) * mPZ.x;
-            tk.y = m1 ? pa.y * mPX.y : (xq.y * pa.y) * mPX.y + (r1.y * pc.y) * mPZ.y;
-            tk.z = m2 ? pa.z * mPX.z : (xq.y * pa.z) * mPX.z + (r2.y * pc.z) * mPZ.z;
-            tk.w = m3 ? pa.w * mPX.w : (xq.y * pa.w) * mPX.w + (r3.y * pc.w) * mPZ.w;
-            red_add4(gk + colQ, tk);
-            if (Q == S.src_x && S.src_z - z0 >= 0 && S.src_z - z0 < 4) S.srcadj[kt] = comp(mPX, S.src_z - z0);
-        }
-        adj8_ring(ring, 2, Q, lane) = make_float4((xq.y * kk.x) * mPX.x, (xq.y * kk.y) * mPX.y,
-                                                  (xq.y * kk.z) * mPX.z, (xq.y * kk.w) * mPX.w);
-        // ---- z-velocity adjoint at Q: z-gather of sb = Kz kappa mPZ over rows z-3 .. z+4 ----
-        {
-            const float4 sb = make_float4((r0.y * kk.x) * mPZ.x, (r1.y * kk.y) * mPZ.y, (r2.y * kk.z) * mPZ.z,
-                                          (r3.y * kk.w) * mPZ.w);
-            float ss[11];  // rows z0-3 .. z0+7
-            ss[0] = __shfl_up_sync(kFull, sb.y, 1);
-            ss[1] = __shfl_up_sync(kFull, sb.z, 1);
-            ss[2] = __shfl_up_sync(kFull, sb.w, 1);
-            ss[3] = sb.x; ss[4] = sb.y; ss[5] = sb.z; ss[6] = sb.w;
-            ss[7] = __shfl_down_sync(kFull, sb.x, 1);
-            ss[8] = __shfl_down_sync(kFull, sb.y, 1);
-            ss[9] = __shfl_down_sync(kFull, sb.z, 1);
-            ss[10] = __shfl_down_sync(kFull, sb.w, 1);
-            float gz[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const int z = z0 + i;
-                gz[i] = 0.0f;
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    gz[i] += cmz(z - k, k) * ss[3 + i - k];
-                    gz[i] -= cmz(z + 1 + k, k) * ss[3 + i + 1 + k];
-                }
-            }
-            if (upd)
-                st4(mvzo + colQ, make_float4(r0.z * mvz.x + gz[0], r1.z * mvz.y + gz[1], r2.z * mvz.z + gz[2],
-                                             r3.z * mvz.w + gz[3]));
-        }
-        // ---- buoyancy imaging at Q ----
-        if (img) {
-            const float4 pg = ld4(pr + 2 * F + colQ);
-            const float4 mv2 = adj8_ring(ring, 0, Q, lane);
-            const float4 tbx = make_float4((xq.w * pg.x) * mv2.x, (xq.w * pg.y) * mv2.y, (xq.w * pg.z) * mv2.z,
-                                           (xq.w * pg.w) * mv2.w);
-            const float4 ph = ld4(pr + 3 * F + colQ);
-            const float4 tbz = make_float4((r0.w * ph.x) * mvz.x, (r1.w * ph.y) * mvz.y, (r2.w * ph.z) * mvz.z,
-                                           (r3.w * ph.w) * mvz.w);
-            const float up = __shfl_up_sync(kFull, tbz.w, 1);  // img is the same for the whole warp
-            if (upd) {
-                const float4 px = Q >= 1 ? tbp : zero;
-                float4 tb;
-                tb.x = 0.5f * ((tbx.x + px.x) + (tbz.x + (z0 >= 1 ? up : 0.0f)));
-                tb.y = 0.5f * ((tbx.y + px.y) + (tbz.y + tbz.x));
-                tb.z = 0.5f * ((tbx.z + px.z) + (tbz.z + tbz.y));
-                tb.w = 0.5f * ((tbx.w + px.w) + (tbz.w + tbz.z));
-                red_add4(gb + colQ, tb);
-            }
-            tbp = tbx;
-        }
-        // ---- x-velocity adjoint at W = L - 7: x-gather of Kx kappa mPX over W-3 .. W+4 ----
-        const int W = L - 7;
-        if (W < xa || W >= xb || !owner) continue;
-        const ptrdiff_t colW = (ptrdiff_t)W * (ptrdiff_t)ld;
-        const float dbx = XF ? 1.0f : __ldg(S.xcoef + (W + S2D_GX)).z;
-        const float4 mv0 = adj8_ring(ring, 0, W, lane);
-        float4 gx = zero;
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const float c0 = cmx(W - k, k), c1 = cmx(W + 1 + k, k);
-            const float4 s0 = adj8_ring(ring, 2, W - k, lane), s1 = adj8_ring(ring, 2, W + 1 + k, lane);
-            gx.x += c0 * s0.x; gx.x -= c1 * s1.x;
-            gx.y += c0 * s0.y; gx.y -= c1 * s1.y;
-            gx.z += c0 * s0.z; gx.z -= c1 * s1.z;
-            gx.w += c0 * s0.w; gx.w -= c1 * s1.w;
-        }
-        st4(mvxo + colW, make_float4(dbx * mv0.x + gx.x, dbx * mv0.y + gx.y, dbx * mv0.z + gx.z, dbx * mv0.w + gx.w));
+        red4(gk, tk);
+        if (Q == k.src_q && k.sdz >= 0 && k.sdz < 4)
+            S.srcadj[k.kt] = k.sdz == 0 ? lo(mPX.a) : k.sdz == 1 ? hi(mPX.a) : k.sdz == 2 ? lo(mPX.b) : hi(mPX.b);
+    }
+    m[7] = (kx * kk) * mPX;
+    // ---- z-velocity adjoint at Q: rows z0-3 .. z0+7 of Kz kappa mPZ ----
+    {
+        const V4 s = (kz * kk) * mPZ;
+        const float x = lo(s.a), y = hi(s.a), z = lo(s.b), v = hi(s.b);
+        const float u1 = __shfl_up_sync(kFull, y, 1), u2 = __shfl_up_sync(kFull, z, 1);
+        const float u3 = __shfl_up_sync(kFull, v, 1);
+        const float d0 = __shfl_down_sync(kFull, x, 1), d1 = __shfl_down_sync(kFull, y, 1);
+        const float d2 = __shfl_down_sync(kFull, z, 1), d3 = __shfl_down_sync(kFull, v, 1);
+        const f2 u3x = pk(u3, x), yz = pk(y, z), vd0 = pk(v, d0), d12 = pk(d1, d2);
+        const f2 a0[4] = {s.a, u3x, pk(u2, u3), pk(u1, u2)}, b0[4] = {yz, s.b, vd0, pk(d0, d1)};
+        const f2 a1[4] = {s.b, yz, s.a, u3x}, b1[4] = {vd0, pk(d0, d1), d12, pk(d2, d3)};
+        constexpr bool TAB = KIND >= kAdj8Edge;
+        const f2 ga = gather8<false>(0ull, [&](int i) { return TAB ? k.tab[(12 + i) * 32].a : k.cp[i]; },
+                                     [&](int i) { return TAB ? k.tab[(16 + i) * 32].a : k.cn[i]; }, a0, b0);
+        const f2 gc = gather8<false>(0ull, [&](int i) { return TAB ? k.tab[(12 + i) * 32].b : k.cp[i]; },
+                                     [&](int i) { return TAB ? k.tab[(16 + i) * 32].b : k.cn[i]; }, a1, b1);
+        if (upd) *reinterpret_cast<V4 *>(po + 3 * fs) = fma4(KIND == kAdj8In ? k.one : k.tab[64], mvz, v4(ga, gc));
+    }
+    // ---- buoyancy imaging at Q (xa-1 feeds column xa; 0 outside the grid) ----
+    {
+        const V4 tbx = (lx * in[224]) * w[4], tbz = (lz * in[256]) * mvz;
+        float up = __shfl_up_sync(kFull, hi(tbz.b), 1);
+        if (KIND != kAdj8In && !k.row0) up = 0.0f;
+        const V4 zs = v4(pk(up, lo(tbz.a)), pk(hi(tbz.a), lo(tbz.b)));
+        if (upd) red4(gb, dup4(0.5f) * ((tbx + (KIND != kAdj8Any || Q >= 1 ? k.tbp : zero4())) + (tbz + zs)));
+        k.tbp = tbx;
+    }
+    // ---- x-velocity adjoint at W ----
+    if (k.owner && W >= k.xa && W < k.xb) {
+        const f2 a0[4] = {m[3].a, m[2].a, m[1].a, m[0].a}, b0[4] = {m[4].a, m[5].a, m[6].a, m[7].a};
+        const f2 a1[4] = {m[3].b, m[2].b, m[1].b, m[0].b}, b1[4] = {m[4].b, m[5].b, m[6].b, m[7].b};
+        auto p = [&](int i) { return vp[i]; };
+        auto n = [&](int i) { return vn[i]; };
+        const V4 o = v4(gather8<false>(0ull, p, n, a0, b0), gather8<false>(0ull, p, n, a1, b1));
+        *reinterpret_cast<V4 *>(vo) = fma4(KIND == kAdj8Any ? dup4(xc.dbw) : k.one, w[0], o);
     }
 }
 
-template <int MINB>
-__global__ void __launch_bounds__(128, MINB) adjoint8s_kernel(const StepArgs *__restrict__ A, int kt_off) {
+template <int KIND>
+__device__ __forceinline__ void adjoint8s_task(const StepArgs &a, const ShotDev &S, int strip, int xa, int seg_len,
+                                               int kt, int lane, V4 *smem) {
+    constexpr int D = Adj8Depth<KIND>::value, NS = KIND == kAdj8In ? 9 : kAdjSlots, U = KIND == kAdj8In ? 4 : 1;
+    const int nnx = S.nnx;
+    const ptrdiff_t ld = S.ld;
+    const int c = strip * S2D_TS_OUT - 8;
+    Lane<true> ln;
+    lane_setup(ln, S, c, lane, kt);
+    Adj8Task k;
+    k.S = &S;
+    k.ring = smem + lane;
+    k.tab = k.ring + 3 * kAdjSlots * 32;
+    k.xa = xa;
+    k.xb = min(nnx, xa + seg_len);
+    k.z0 = ln.z0;
+    k.kt = kt;
+    k.src_q = S.src_x;
+    k.sdz = ln.sdz;
+    k.owner = lane >= 2 && lane <= 29 && ln.z0 >= 0 && ln.z0 < S.nnz;
+    k.row0 = ln.z0 >= 1;
+    k.slot = (kt + 1) / a.dt_factor - 1;
+    // receiver adjoint source on recording steps, in strips whose rows hold receivers
+    k.inj = !(a.flags & S2D_STEP_NO_RECORD) && S.nrec > 0 && ((kt + 1) % a.dt_factor) == 0 && k.slot < S.real_nt &&
+            c + S2D_STRIP_ROWS > S.rec_zlo && c <= S.rec_zhi;
+    if (k.inj) k.src.start(S, max(xa - 3, 0), k.slot);
+    k.one = dup4(a.one);
+    k.kx = dup4(S.kx_in);
+    k.kz = dup4(S.kz_in);
+    const float4 lit = make_float4(kC81, kC82, kC83, kC84);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        k.cp[i] = dup(comp(lit, i));
+        k.cn[i] = dup(-comp(lit, i));
+    }
+    k.tbp = zero4();
+    if (KIND != kAdj8In) {
+        float r[4][4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float4 f = __ldg(ln.zc + i);
+            r[0][i] = f.x, r[1][i] = f.y, r[2][i] = f.z, r[3][i] = f.w;
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) k.tab[i * 32] = v4(pk(r[i][0], r[i][1]), pk(r[i][2], r[i][3]));
+    }
+    if (KIND >= kAdj8Edge) {
+        const int n = S.nnz;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            float t[4][4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int z = ln.z0 + i;
+                t[0][i] = comp(dp8(z - 1 - j, n), j);
+                t[1][i] = -comp(dp8(z + j, n), j);
+                t[2][i] = comp(dm8(z - j, n), j);
+                t[3][i] = -comp(dm8(z + 1 + j, n), j);
+            }
+#pragma unroll
+            for (int f = 0; f < 4; ++f)
+                k.tab[(4 + 4 * f + j) * 32] = v4(pk(t[f][0], t[f][1]), pk(t[f][2], t[f][3]));
+        }
+    }
+    const int pin = (kt + 1) & 1, pout = kt & 1;
+    // a ghost lane reads the column's first ghost rows (zeros) and writes nothing
+    const size_t off = (size_t)(ln.zl + S2D_GZ) + (size_t)S2D_GX * ld;
+    const ptrdiff_t fs = S.fstride;
+    const size_t F = (size_t)(nnx + 2 * S2D_GX) * ld;
+    const int L0 = xa - 7, Lend = k.xb + 6;
+    const int n4 = (Lend - xa + U) / U;  // groups of U iterations from L = xa on (the last may pass Lend)
+    const int Llast = xa + U * n4 - 1;
+    // state, materials and products at the next iteration's column Q
+    const float *ns = S.st[pin][0] + off + (ptrdiff_t)(L0 - 3) * ld;
+    const float *nm = S.kappa + off + (ptrdiff_t)(L0 - 3) * ld;
+    const float *np = S.prod + (size_t)(kt - a.prod_kt0) * 4 * F + off + (ptrdiff_t)(L0 - 3) * ld;
+    const ptrdiff_t ovx = 3 * ld + 2 * fs, obx = 3 * ld + fs;
+    auto issue = [&](int L, int slot) {
+        V4 *st = k.ring + slot * (NS * 32);
+        cp_async16(st, ns + ovx, true);
+        cp_async16(st + 32, nm + obx, true);
+        if (L >= xa) {
+            cp_async16(st + 64, ns, true);
+            cp_async16(st + 96, ns + 3 * fs, true);
+            cp_async16(st + 128, nm + 2 * fs, true);
+            cp_async16(st + 160, nm, true);
+            if (KIND != kAdj8In) cp_async16(st + 288, ns + fs, true);
+            if (L - 3 >= max(xa - 1, 0) && L - 3 < k.xb) {  // the columns whose imaging terms are formed
+                cp_async16(st + 192, np, true);
+                cp_async16(st + 224, np + 2 * F, true);
+                cp_async16(st + 256, np + 3 * F, true);
+                if (KIND != kAdj8In) cp_async16(st + 320, np + F, true);
+            }
+        }
+        ns += ld;
+        nm += ld;
+        np += ld;
+    };
+#pragma unroll
+    for (int i = 0; i < D - 1; ++i) {
+        issue(L0 + i, i);
+        cp_async_commit();
+    }
+    auto next = [&](int L, int sl) {  // bring iteration L + D - 1, wait for iteration L (in slot sl)
+        if (L + D - 1 <= Llast) issue(L + D - 1, KIND == kAdj8In ? (sl + D - 1) % D : sl == 0 ? D - 1 : sl - 1);
+        cp_async_commit();
+        cp_async_wait<D - 1>();
+        return k.ring + sl * (NS * 32);
+    };
+    V4 w[7 + U], g[7 + U], m[7 + U];
+    // iterations xa-7 .. xa-1 fill the windows of mvx' and Lx bx mvx'
+#pragma unroll
+    for (int i = 0; i < 7; ++i) {
+        const V4 *in = next(L0 + i, i % D);
+        const float lx = KIND == kAdj8Any ? __ldg(S.xcoef + (L0 + i + S2D_GX)).w : S.kx_in;
+        w[i] = in[0];
+        g[i] = (dup4(lx) * in[32]) * w[i];
+        m[i] = zero4();
+    }
+    float *po = S.st[pout][0] + off + (ptrdiff_t)(xa - 3) * ld;
+    float *vo = S.st[pout][0] + off + (ptrdiff_t)(xa - 7) * ld + 2 * fs;
+    float *gk = S.grad[0] + off + (ptrdiff_t)(xa - 3) * ld, *gb = S.grad[1] + off + (ptrdiff_t)(xa - 3) * ld;
+    Adj8Xc xc{};
+    if (KIND == kAdj8Any) xc.read(S.xcoef, nnx, xa);
+    int L = xa, sl = 7 % D;
+#pragma unroll 1
+    for (int n = 0; n < n4; ++n) {
+#pragma unroll
+        for (int j = 0; j < U; ++j) {
+            Adj8Xc xn{};
+            if (KIND == kAdj8Any) xn.read(S.xcoef, nnx, L + 1);
+            adj8_column<KIND>(k, xc, next(L, U == 4 ? (7 + j) % D : sl), L, po, vo, gk, gb, fs, w + j, g + j, m + j);
+            xc = xn;
+            ++L;
+            if (U == 1) sl = sl + 1 == D ? 0 : sl + 1;
+            po += ld;
+            vo += ld;
+            gk += ld;
+            gb += ld;
+        }
+#pragma unroll
+        for (int i = 0; i < 7; ++i) {
+            w[i] = w[i + U];
+            g[i] = g[i + U];
+            m[i] = m[i + U];
+        }
+    }
+    cp_async_wait<0>();
+}
+
+// Debug self-check (S2D_DEVICE_CHECKS) of the task's reach.
+__device__ __forceinline__ bool adj8_in_bounds(const StepArgs &a, const ShotDev &S, int strip, int xa, int seg_len,
+                                               int kt) {
+#ifdef S2D_DEVICE_CHECKS
+    const long ld = S.ld;
+    const int xb = min(S.nnx, xa + seg_len);
+    const long c = (long)strip * S2D_TS_OUT - 8;
+    const size_t F = (size_t)(S.nnx + 2 * S2D_GX) * ld;
+    if (xa - 7 < -S2D_GX || xb + 6 >= S.nnx + S2D_GX || c + S2D_GZ < 0 || c + 127 + S2D_GZ >= ld || F > S.nfield ||
+        kt < a.prod_kt0 || (size_t)(kt - a.prod_kt0 + 1) * 4 * F > S.nprod) {
+        if (a.err) atomicCAS(a.err, 0, (4 << 8) | 1);
+        return false;
+    }
+#endif
+    return true;
+}
+
+__global__ void __launch_bounds__(128, 2) adjoint8s_kernel(const StepArgs *__restrict__ A, int kt_off) {
     extern __shared__ __align__(128) unsigned char smem[];
-    float4 *ring = reinterpret_cast<float4 *>(smem + (size_t)(threadIdx.x >> 5) * kAdj8WarpBytes);
+    V4 *const mem = reinterpret_cast<V4 *>(smem + (size_t)(threadIdx.x >> 5) * kAdj8WarpBytes);
     const StepArgs a = *A;
     const int lane = threadIdx.x & 31;
     const int gwarp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
@@ -928,39 +1067,44 @@ __global__ void __launch_bounds__(128, MINB) adjoint8s_kernel(const StepArgs *__
     if (kt < 0 || kt >= a.fd_nt) return;
     __shared__ ShotDev shot_rec[4];  // the task's shot record, one slot per warp
     ShotDev &S = shot_rec[(threadIdx.x >> 5) & 3];
-    for (int t = gwarp; t < a.total_tasks; t += nwarp) {
+    TaskQueue queue(a.queue, nwarp, lane);
+    for (int t = gwarp; t < a.total_tasks; t = queue.take()) {
+        queue.draw();
         int strip, xa, seg_len;
-        const ShotDev &G = task_of(a, t, strip, xa, seg_len);
+        const ShotDev &G = task_of_split(a, t, strip, xa, seg_len);
+        if (!adj8_in_bounds(a, G, strip, xa, seg_len, kt)) continue;
         warp_copy_shot(S, G, lane);
         const int c = strip * S2D_TS_OUT - 8;
         const int xb = min(S.nnx, xa + seg_len);
-        // rows c-4 .. c+131 take part (gathers reach 4 rows past the strip)
-        const bool zf = rows_fast(S, c - 4, c + S2D_STRIP_ROWS + 3) && c - 4 >= 4 &&
-                        c + S2D_STRIP_ROWS + 3 <= S.nnz - 5;
+        // Lanes 1..30 form mPZ from rows c .. c+127 of Lz bz mvz' with the taps
+        // of forward D+ rows c .. c+126, lanes 2..29 mvz with those of D- rows
+        // c+5 .. c+123.
+        const bool taps = c >= 4 && c + S2D_STRIP_ROWS - 1 <= S.nnz - 5;
+        const bool zf = taps && rows_fast(S, c, c + S2D_STRIP_ROWS - 1);
         // columns xa-7 .. xb+6 take part
-        const bool xf = xa - 7 >= max(S.xfast_lo, 4) && xb + 6 < min(S.xfast_hi, S.nnx - 4);
-        if (zf && xf) adjoint8s_task<true, true>(a, S, strip, xa, seg_len, kt, lane, ring);
-        else if (zf) adjoint8s_task<true, false>(a, S, strip, xa, seg_len, kt, lane, ring);
-        else if (xf) adjoint8s_task<false, true>(a, S, strip, xa, seg_len, kt, lane, ring);
-        else adjoint8s_task<false, false>(a, S, strip, xa, seg_len, kt, lane, ring);
+        const bool xf = xa - kAdj8ColLo >= max(S.xfast_lo, 4) && xb + kAdj8ColHi < min(S.xfast_hi, S.nnx - 4);
+        if (zf && xf) adjoint8s_task<kAdj8In>(a, S, strip, xa, seg_len, kt, lane, mem);
+        else if (taps && xf) adjoint8s_task<kAdj8Rows>(a, S, strip, xa, seg_len, kt, lane, mem);
+        else if (xf) adjoint8s_task<kAdj8Edge>(a, S, strip, xa, seg_len, kt, lane, mem);
+        else adjoint8s_task<kAdj8Any>(a, S, strip, xa, seg_len, kt, lane, mem);
     }
+    queue.leave();
 }
 
 }  // namespace
 
 int launch_adjoint8s(const StepArgs *args_dev, int kt_off, int grid, void *stream) {
-    adjoint8s_kernel<3><<<grid, 128, 4 * kAdj8WarpBytes, (cudaStream_t)stream>>>(args_dev, kt_off);
+    adjoint8s_kernel<<<grid, 128, 4 * kAdj8WarpBytes, (cudaStream_t)stream>>>(args_dev, kt_off);
     return (int)cudaGetLastError();
 }
 
-// Also raises the kernel's dynamic shared-memory limit (its 48 KB of rings
-// and the static shot records exceed the default); called before the
+// Also raises the kernel's dynamic shared-memory limit; called before the
 // launches.
 int adjoint8s_occupancy(int *blocks_per_sm) {
-    cudaError_t e = cudaFuncSetAttribute(adjoint8s_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(adjoint8s_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          4 * kAdj8WarpBytes);
     if (e != cudaSuccess) return (int)e;
-    return (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, adjoint8s_kernel<3>, 128,
+    return (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, adjoint8s_kernel, 128,
                                                              4 * kAdj8WarpBytes);
 }
 

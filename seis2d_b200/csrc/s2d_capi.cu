@@ -263,6 +263,7 @@ struct SplitRule {
 constexpr SplitRule kSplitTs2 = {S2D_TS_OUT, 8, 0, 4, 4, 9, 1.6, 1.9};
 constexpr SplitRule kSplitO8 = {S2D_TS_OUT, 8, 0, 3, 3, 13, 1.6, 1.9};
 constexpr SplitRule kSplitAdj = {S2D_STRIP_OUT, 4, kAdjRowMargin, kAdjColLo, kAdjColHi, 6, 1.5, 1.7};
+constexpr SplitRule kSplitAdj8 = {S2D_TS_OUT, 8, 0, kAdj8ColLo, kAdj8ColHi, 13, 1.5, 1.7};
 
 // Rim and interior tasks of a group (GroupDev::split) of the grid and fast
 // ranges of shot record `d`; `shots` shots of it run at a time on
@@ -1566,9 +1567,7 @@ int grad_alloc(Ctx *c, GradRun &g, size_t bytes, void **out) {
     return S2D_OK;
 }
 
-// Adjoint launches for steps kt_top, kt_top-1, ..., kt_top-n+1, as replays of
-// a graph of `graph_chunk` launches.
-// The 8th-order adjoint over steps kt_top, kt_top-1, ..., kt_top-n+1: two
+// The 8th-order adjoint over steps kt_top, kt_top-1, ... in its first form: two
 // cell-parallel launches per step, direct (no graph).
 int run_adjoint8(Ctx *c, StepArgs args, int kt_top, int n, int nnx, int nnz, int nshots, int *launches) {
     if (n <= 0) return S2D_OK;
@@ -1576,20 +1575,6 @@ int run_adjoint8(Ctx *c, StepArgs args, int kt_top, int n, int nnx, int nnz, int
     args.kt_base = kt_top;
     int e = launch_set_args(args, args_d, c->stream);
     if (e) return fail(c, S2D_ERR_CUDA, "set_args launch: %s", cudaGetErrorString((cudaError_t)e));
-    if (c->opt_adj8_form == 0) {
-        // one streaming pass per step over the warp tasks of the current
-        // (112-row) layout, the grid exactly its resident blocks
-        int bps = 0;
-        if (adjoint8s_occupancy(&bps) || bps < 1) bps = 1;
-        const int grid = (int)std::max<long>(
-            1, std::min<long>((long)c->sm_count * bps, ((long)args.total_tasks * 32 + 127) / 128));
-        *launches += 1 + n;
-        for (int k = 0; k < n; ++k) {
-            e = launch_adjoint8s(args_d, k, grid, c->stream);
-            if (e) return fail(c, S2D_ERR_CUDA, "adjoint launch: %s", cudaGetErrorString((cudaError_t)e));
-        }
-        return S2D_OK;
-    }
     *launches += 1 + 2 * n;
     for (int k = 0; k < n; ++k) {
         e = launch_adjoint8(args_d, k, nnx, nnz, nshots, c->stream);
@@ -1598,10 +1583,12 @@ int run_adjoint8(Ctx *c, StepArgs args, int kt_top, int n, int nnx, int nnz, int
     return S2D_OK;
 }
 
-int run_adjoint(Ctx *c, Batch &b, GradRun &g, StepArgs args, int kt_top, int n, int grid, bool use_graph,
-                int *launches) {
+// Adjoint launches for steps kt_top, kt_top-1, ..., kt_top-n+1, as replays of
+// a graph of `graph_chunk` launches.
+int run_adjoint(Ctx *c, Batch &b, StepArgs args, int kt_top, int n, int grid, bool use_graph, int *launches) {
     if (n <= 0) return S2D_OK;
     StepArgs *args_d = c->args_d.as<StepArgs>();
+    const auto launch = b.order8 ? launch_adjoint8s : launch_adjoint;
     const int chunk = use_graph ? std::max(1, c->opt_graph_chunk) : n;
     for (int done = 0; done < n; done += chunk) {
         const int m = std::min(chunk, n - done);
@@ -1611,19 +1598,18 @@ int run_adjoint(Ctx *c, Batch &b, GradRun &g, StepArgs args, int kt_top, int n, 
         *launches += 1 + m;
         if (!use_graph) {
             for (int k = 0; k < m; ++k) {
-                e = launch_adjoint(args_d, k, grid, c->stream);
+                e = launch(args_d, k, grid, c->stream);
                 if (e) return fail(c, S2D_ERR_CUDA, "adjoint launch: %s", cudaGetErrorString((cudaError_t)e));
             }
             continue;
         }
-        (void)g;
-        const std::vector<long> key = {m, grid};
+        const std::vector<long> key = {m, grid, b.order8 ? 1 : 0};
         auto it = c->adj_graphs.find(key);
         if (it == c->adj_graphs.end()) {
             cudaGraph_t gr;
             CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
             for (int k = 0; k < m; ++k) {
-                e = launch_adjoint(args_d, k, grid, c->stream);
+                e = launch(args_d, k, grid, c->stream);
                 if (e) {
                     cudaStreamEndCapture(c->stream, &gr);
                     if (gr) cudaGraphDestroy(gr);
@@ -1821,7 +1807,7 @@ extern "C" int s2d_gradient(void *ctx, const s2d_shot *shots, int nshots, const 
     };
     // The steps that keep their products (the last segment of the sweep, the
     // recomputes) run in the products kernel's own task layout, the adjoint
-    // steps in one of theirs (the 4th-order one cut by kind).
+    // steps in one of theirs.
     auto products_layout = [&]() -> int {
         int e = layout_groups(c, b, lc_prod);
         if (!e) e = launch_config(c, b.max_tasks, &lc_prod, prod_variant, 128, 0);
@@ -1850,15 +1836,8 @@ extern "C" int s2d_gradient(void *ctx, const s2d_shot *shots, int nshots, const 
         const long resident = (long)c->sm_count * bps;
         ag.nstrips = b.order8 ? num_strips_ts(b.group_nnz[0]) : num_strips(b.group_nnz[0]);
         ag.task_begin = 0;
-        if (b.order8) {
-            const int nnx = b.group_nnx[0];
-            ag.split = 0;
-            ag.seg_len = c->opt_seg_len > 0 ? std::min(c->opt_seg_len, nnx)
-                                            : choose_seg_len(nnx, (long)nshots * ag.nstrips, resident * 4, 12);
-            ag.nsegs = (nnx + ag.seg_len - 1) / ag.seg_len;
-        } else {
-            split_group(ag, b.shot_dev[0], nshots, (double)resident * 4, true, c->opt_seg_len, kSplitAdj);
-        }
+        split_group(ag, b.shot_dev[0], nshots, (double)resident * 4, true, c->opt_seg_len,
+                    b.order8 ? kSplitAdj8 : kSplitAdj);
         agrid = (int)std::max<long>(1, std::min<long>(resident, ((long)nshots * shot_tasks(ag) * 32 + 127) / 128));
         int e = grad_alloc(c, g, sizeof(GroupDev), &adj_group);
         if (e) return e;
@@ -1930,8 +1909,9 @@ extern "C" int s2d_gradient(void *ctx, const s2d_shot *shots, int nshots, const 
         a.prod_kt0 = k0;
         int e = phase_mark(c, g, kPhaseAdjoint);
         if (e) return e;
-        e = b.order8 ? run_adjoint8(c, a, k0 + n - 1, n, m.nnx, m.nnz, nshots, &launches)
-                         : run_adjoint(c, b, g, a, k0 + n - 1, n, agrid, use_graph, &launches);
+        e = b.order8 && c->opt_adj8_form == 1
+                ? run_adjoint8(c, a, k0 + n - 1, n, m.nnx, m.nnz, nshots, &launches)
+                : run_adjoint(c, b, a, k0 + n - 1, n, agrid, use_graph, &launches);
         if (e) return e;
     }
     // ---- source term, chain rule, fold ----

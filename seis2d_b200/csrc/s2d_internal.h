@@ -220,6 +220,7 @@ constexpr int kTs2WarpBytes = (kTs2Depth * kTs2Slots + 8 + 8) * S2D_STRIP_ROWS *
 // Interior tasks of the adjoint step: rows and columns past the task's own
 // strip and segment that must be interior too.
 constexpr int kAdjRowMargin = 2, kAdjColLo = 3, kAdjColHi = 2;
+constexpr int kAdj8ColLo = 7, kAdj8ColHi = 6;  // of the 8th-order one (no rows)
 // Shared memory of a warp of the 8th-order kernel: the input ring (kO8Depth
 // iterations of vx; px, vz, kappa; bx, bz; pz) and 12 row coefficients.
 constexpr int kO8Depth = 4, kO8Slots = 7;
@@ -289,7 +290,7 @@ int launch_adjoint(const StepArgs *args_dev, int kt_off, int grid, void *stream)
 // `nshots` shots of one nnx x nnz grid.
 int launch_adjoint8(const StepArgs *args_dev, int kt_off, int nnx, int nnz, int nshots, void *stream);
 // Adjoint FD step of the 8th-order scheme as one streaming pass (warp tasks on
-// the 112-row strips of the batch's current layout), 4 warps per block.
+// 112-row strips, drawn from the queue), 4 warps per block.
 int launch_adjoint8s(const StepArgs *args_dev, int kt_off, int grid, void *stream);
 int adjoint8s_occupancy(int *blocks_per_sm);
 int adjoint_kernel_occupancy(int *blocks_per_sm);
