@@ -14,6 +14,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <list>
 #include <map>
 #include <memory>
 #include <string>
@@ -27,6 +28,114 @@ using namespace s2d;
 
 namespace {
 
+// The device memory of one context.  Requests up to kMaxPiece are cut from
+// chunks, the others are cudaMalloc's own: a cudaMalloc and its cudaFree of 1 MB
+// or more take 0.9 ms whatever their size (so do the first and the last smaller
+// one, 10 us between them), and a call on a small grid made a dozen.  Three
+// shots of 487 x 263 in a context of their own, 300 steps: 5.6 -> 2.4 ms (with
+// the tables of a batch in one upload, below).  A piece that comes back is
+// reused at once, so releasing one waits for the context's stream, as cudaFree
+// waits for the device.  Chunks in no use go back above kMaxIdle bytes of them,
+// when an allocation fails, and with the context.
+struct Arena {
+    static constexpr size_t kAlign = 512, kMaxPiece = (size_t)64 << 20, kMinChunk = (size_t)32 << 20,
+                            kMaxChunk = (size_t)256 << 20, kMaxIdle = (size_t)256 << 20;
+    struct Chunk {
+        char *p;
+        size_t size;
+        std::map<size_t, size_t> free;  // offset -> bytes
+    };
+    std::list<Chunk> chunks;
+    cudaStream_t stream = nullptr;
+    static size_t rounded(size_t n) { return (std::max<size_t>(n, 1) + kAlign - 1) / kAlign * kAlign; }
+    Arena() = default;
+    Arena(const Arena &) = delete;
+    Arena &operator=(const Arena &) = delete;
+    ~Arena() {
+        for (auto &c : chunks) cudaFree(c.p);
+    }
+    // Gives back the chunks that no piece uses, but for `keep` bytes of them.
+    void trim(size_t keep) {
+        for (auto c = chunks.begin(); c != chunks.end();) {
+            const bool idle = c->free.size() == 1 && c->free.begin()->second == c->size;
+            if (idle && c->size <= keep) {
+                keep -= c->size;
+                ++c;
+            } else if (idle) {
+                cudaFree(c->p);
+                c = chunks.erase(c);
+            } else {
+                ++c;
+            }
+        }
+    }
+    cudaError_t grow(size_t n) {
+        Chunk c;
+        c.size = n > kMinChunk / 4 ? n : kMinChunk;
+        cudaError_t e = cudaMalloc((void **)&c.p, c.size);
+        if (e == cudaErrorMemoryAllocation && c.size > n) {  // memory is short: no more than asked for
+            cudaGetLastError();
+            c.size = n;
+            e = cudaMalloc((void **)&c.p, c.size);
+        }
+        if (e != cudaSuccess) return e;
+        c.free.emplace(0, c.size);
+        chunks.push_back(std::move(c));
+        return cudaSuccess;
+    }
+    bool fits(size_t n) const {
+        for (auto &c : chunks)
+            for (auto &f : c.free)
+                if (f.second >= n) return true;
+        return false;
+    }
+    // About to take pieces of these sizes: one chunk for those that come from
+    // chunks (a failure shows when they are taken).
+    void expect(const std::vector<size_t> &pieces) {
+        size_t n = 0;
+        for (size_t b : pieces)
+            if (b <= kMaxPiece) n += rounded(b);
+        if (n == 0 || n > kMaxChunk || fits(n)) return;
+        if (grow(n) != cudaSuccess) cudaGetLastError();
+    }
+    cudaError_t take(size_t n, void **p, Chunk **from) {
+        for (int pass = 0; pass < 2; ++pass) {
+            for (auto &c : chunks)
+                for (auto f = c.free.begin(); f != c.free.end(); ++f)
+                    if (f->second >= n) {
+                        *p = c.p + f->first;
+                        *from = &c;
+                        const size_t at = f->first, left = f->second - n;
+                        c.free.erase(f);
+                        if (left) c.free.emplace(at + n, left);
+                        return cudaSuccess;
+                    }
+            if (pass == 0) {
+                cudaError_t e = grow(n);
+                if (e != cudaSuccess) return e;
+            }
+        }
+        return cudaErrorMemoryAllocation;
+    }
+    void release(Chunk *c, void *p, size_t n) {
+        if (stream) cudaStreamSynchronize(stream);
+        auto f = c->free.emplace((size_t)((char *)p - c->p), n).first;
+        auto next = std::next(f);
+        if (next != c->free.end() && f->first + f->second == next->first) {
+            f->second += next->second;
+            c->free.erase(next);
+        }
+        if (f != c->free.begin()) {
+            auto prev = std::prev(f);
+            if (prev->first + prev->second == f->first) {
+                prev->second += f->second;
+                c->free.erase(f);
+            }
+        }
+        trim(kMaxIdle);
+    }
+};
+
 struct DevBuf {
     void *p = nullptr;
     size_t bytes = 0;
@@ -35,17 +144,32 @@ struct DevBuf {
     DevBuf &operator=(const DevBuf &) = delete;
     ~DevBuf() { reset(); }
     void reset() {
-        if (p) cudaFree(p);
+        if (p && arena) arena->release(chunk, p, Arena::rounded(bytes));
+        else if (p) cudaFree(p);
         p = nullptr;
         bytes = 0;
+        arena = nullptr;
     }
-    cudaError_t alloc(size_t n) {
+    cudaError_t alloc(Arena &a, size_t n) {
         reset();
-        cudaError_t e = cudaMalloc(&p, n);
-        if (e == cudaSuccess) bytes = n;
-        else p = nullptr;
+        cudaError_t e = cudaSuccess;
+        const bool piece = n <= Arena::kMaxPiece;
+        for (int pass = 0; pass < 2; ++pass) {
+            e = piece ? a.take(Arena::rounded(n), &p, &chunk) : cudaMalloc(&p, n);
+            if (e != cudaErrorMemoryAllocation || pass) break;
+            cudaGetLastError();
+            a.trim(0);
+        }
+        if (e != cudaSuccess) {
+            p = nullptr;
+            return e;
+        }
+        bytes = n;
+        arena = piece ? &a : nullptr;
         return e;
     }
+    Arena *arena = nullptr;  // where it came from (null: cudaMalloc)
+    Arena::Chunk *chunk = nullptr;
     template <class T> T *as() const { return reinterpret_cast<T *>(p); }
 };
 
@@ -102,7 +226,8 @@ struct Batch {
         return !chip.empty();
     }
     std::vector<std::unique_ptr<DevBuf>> state;   // 8 per shot
-    std::vector<std::unique_ptr<DevBuf>> aux;     // amp tables, receiver tables
+    DevBuf tables;                   // wavelet, source terms, receiver tables of every shot
+    const double *ksrc_d = nullptr;  // in it: kappa at every shot's source
     DevBuf shots_d, groups_d;
     DevBuf seis_int;                 // internal seismogram buffer (host output)
     float *seis_d = nullptr;         // where the kernels record
@@ -118,7 +243,7 @@ struct Batch {
 // then needs no cudaMalloc).  Flushed when an allocation fails.
 struct Pool {
     std::multimap<size_t, std::unique_ptr<DevBuf>> free;
-    std::unique_ptr<DevBuf> take(size_t bytes, cudaError_t *err) {
+    std::unique_ptr<DevBuf> take(Arena &arena, size_t bytes, cudaError_t *err) {
         auto it = free.find(bytes);
         if (it != free.end()) {
             auto b = std::move(it->second);
@@ -127,11 +252,11 @@ struct Pool {
             return b;
         }
         auto b = std::make_unique<DevBuf>();
-        *err = b->alloc(bytes);
+        *err = b->alloc(arena, bytes);
         if (*err == cudaErrorMemoryAllocation) {
             cudaGetLastError();
             free.clear();
-            *err = b->alloc(bytes);
+            *err = b->alloc(arena, bytes);
         }
         return b;
     }
@@ -156,6 +281,7 @@ struct LaunchCfg {
 };
 
 struct Ctx {
+    Arena arena;  // outlives every buffer below
     int device = 0;
     int sm_count = 0;
     // tuning options (s2d_set_option)
@@ -340,8 +466,8 @@ int build_coef(Ctx *c, Model &m, float fd_dt) {
         xc[x + S2D_GX] = make_float4(m.damp2a[x], (float)(dtdx * m.damp2a1[x]), m.damp2b[x], (float)(dtdx * m.damp2b1[x]));
     for (int z = 0; z < m.nnz; ++z)
         zc[z + S2D_GZ] = make_float4(m.damp1a[z], (float)(dtdz * m.damp1a1[z]), m.damp1b[z], (float)(dtdz * m.damp1b1[z]));
-    if (!m.xcoef.p) CK(m.xcoef.alloc(sizeof(float4) * m.nxa));
-    if (!m.zcoef.p) CK(m.zcoef.alloc(sizeof(float4) * m.ld));
+    if (!m.xcoef.p) CK(m.xcoef.alloc(c->arena, sizeof(float4) * m.nxa));
+    if (!m.zcoef.p) CK(m.zcoef.alloc(c->arena, sizeof(float4) * m.ld));
     CK(cudaMemcpyAsync(m.xcoef.p, xc.data(), sizeof(float4) * m.nxa, cudaMemcpyHostToDevice, c->stream));
     CK(cudaMemcpyAsync(m.zcoef.p, zc.data(), sizeof(float4) * m.ld, cudaMemcpyHostToDevice, c->stream));
     CK(cudaStreamSynchronize(c->stream));
@@ -492,7 +618,7 @@ int layout_groups_for(Ctx *c, Batch &b, long resident_warps, std::vector<long> k
             max_tasks = task;
         }
     }
-    if (!b.groups_d.p) CK(b.groups_d.alloc(sizeof(GroupDev) * b.groups.size()));
+    if (!b.groups_d.p) CK(b.groups_d.alloc(c->arena, sizeof(GroupDev) * b.groups.size()));
     CK(cudaMemcpyAsync(b.groups_d.p, b.groups.data(), sizeof(GroupDev) * b.groups.size(), cudaMemcpyHostToDevice,
                        c->stream));
     // the copy reads host memory that a later layout rewrites
@@ -658,8 +784,8 @@ int run_resident(Ctx *c, Batch &b, const ResPlan &pl, int slot0, int nshots, int
     std::vector<ResShot> rs;
     for (int i = 0; i < nshots; ++i) rs.push_back({slot0 + i, (i % pl.conc) * per, pl.ncx, pl.ncz});
     const size_t rbytes = sizeof(ResShot) * rs.size(), fbytes = resident_frame_bytes(pl.nw, pl.c, pl.conc * per);
-    if (c->res_shots.bytes < rbytes) CK(c->res_shots.alloc(rbytes));
-    if (c->res_frames.bytes < fbytes) CK(c->res_frames.alloc(fbytes));
+    if (c->res_shots.bytes < rbytes) CK(c->res_shots.alloc(c->arena, rbytes));
+    if (c->res_frames.bytes < fbytes) CK(c->res_frames.alloc(c->arena, fbytes));
     CK(cudaMemcpyAsync(c->res_shots.p, rs.data(), rbytes, cudaMemcpyHostToDevice, c->stream));
     ResArgs a{};
     a.shots = b.shots_d.as<ShotDev>();
@@ -732,6 +858,7 @@ int encode_fields(Ctx *c, CUtensorMap *out, const float *base, int planes, const
 // 8 state planes of every shot, then the 3 material planes of every shot's
 // model.
 int build_tmaps(Ctx *c, Batch &b) {
+    if (b.tmaps_d.p) return S2D_OK;
     const int n = (int)b.table.size();
     static_assert(sizeof(CUtensorMap) == kTmaMapBytes, "tensor map size");
     std::vector<CUtensorMap> maps(2 * (size_t)n);
@@ -742,7 +869,7 @@ int build_tmaps(Ctx *c, Batch &b) {
         if (!e) e = encode_fields(c, &maps[n + i], m.kappa(), 3, m, m.field_elems);
         if (e) return e;
     }
-    CK(b.tmaps_d.alloc(sizeof(CUtensorMap) * maps.size()));
+    CK(b.tmaps_d.alloc(c->arena, sizeof(CUtensorMap) * maps.size()));
     CK(cudaMemcpy(b.tmaps_d.p, maps.data(), sizeof(CUtensorMap) * maps.size(), cudaMemcpyHostToDevice));
     return S2D_OK;
 }
@@ -750,6 +877,9 @@ int build_tmaps(Ctx *c, Batch &b) {
 // Build the device tables of a new batch (kt_begin == 0).
 int setup_batch(Ctx *c, const s2d_shot *shots, int nshots, const s2d_wave &wave, const double *wavelet,
                 int nwavelet, float *seis_user, unsigned flags) {
+    // the caller's device buffers (models' sources, seismograms, adjoint
+    // sources) may still be written on streams this library does not know
+    CK(cudaDeviceSynchronize());
     c->drop_batch();
     auto bp = std::make_unique<Batch>();
     Batch &b = *bp;
@@ -805,12 +935,43 @@ int setup_batch(Ctx *c, const s2d_shot *shots, int nshots, const s2d_wave &wave,
     if (flags & S2D_SEIS_DEVICE) {
         b.seis_d = seis_user;
     } else {
-        CK(b.seis_int.alloc(std::max<size_t>(seis_total, 1) * sizeof(float)));
+        CK(b.seis_int.alloc(c->arena, std::max<size_t>(seis_total, 1) * sizeof(float)));
         b.seis_d = b.seis_int.as<float>();
     }
     if (seis_total) CK(cudaMemsetAsync(b.seis_d, 0, seis_total * sizeof(float), c->stream));
 
     b.shot_dev.resize(nshots);
+    // one upload for the tables of every shot: samples to inject, where each
+    // source reads its kappa, receivers by column; the source terms behind
+    // them are computed on the device
+    const int n_inj = std::min(rs.fd_nt, inject_last + 1);
+    size_t used = 0;
+    auto place = [&](size_t n) {
+        const size_t at = used;
+        used += (n + 15) / 16 * 16;
+        return at;
+    };
+    const size_t o_w = place(sizeof(double) * std::max(n_inj, 0)), o_src = place(sizeof(SourceTerm) * nshots);
+    std::vector<size_t> o_ptr(nshots), o_rz(nshots), o_id(nshots), o_amp(nshots);
+    std::vector<size_t> pieces;
+    for (int s = 0; s < nshots; ++s) {
+        const Model &m = *c->models[shots[s].model_id];
+        const size_t n_rec = (size_t)std::max(shots[s].nrec, 1);
+        o_ptr[s] = place(sizeof(int) * ((size_t)m.nnx + 1));
+        o_rz[s] = place(sizeof(int) * n_rec);
+        o_id[s] = place(sizeof(int) * n_rec);
+        pieces.push_back(8 * m.field_elems * sizeof(float));
+    }
+    const size_t n_up = used, o_ks = place(sizeof(double) * nshots);
+    for (int s = 0; s < nshots; ++s) o_amp[s] = place(sizeof(float) * (size_t)rs.fd_nt);
+    pieces.push_back(used);
+    if (!c->pool.held()) c->arena.expect(pieces);
+    CK(b.tables.alloc(c->arena, used));
+    char *const tab_d = b.tables.as<char>();
+    std::vector<char> tab(n_up, 0);
+    for (int kt = 0; kt < n_inj; ++kt)
+        reinterpret_cast<double *>(tab.data() + o_w)[kt] = kt < (int)w.size() ? w[kt] : 0.0;
+    b.ksrc_d = reinterpret_cast<const double *>(tab_d + o_ks);
     for (int s = 0; s < nshots; ++s) {
         Model &m = *c->models[shots[s].model_id];
         ShotHost &h = b.shots[s];
@@ -820,7 +981,7 @@ int setup_batch(Ctx *c, const s2d_shot *shots, int nshots, const s2d_wave &wave,
         // the 8 state fields of the shot in one allocation (ShotDev::fstride)
         {
             cudaError_t ae;
-            b.state.push_back(c->pool.take(8 * fb, &ae));
+            b.state.push_back(c->pool.take(c->arena, 8 * fb, &ae));
             CK(ae);
             CK(cudaMemsetAsync(b.state.back()->p, 0, 8 * fb, c->stream));
             for (int par = 0; par < 2; ++par)
@@ -848,21 +1009,14 @@ int setup_batch(Ctx *c, const s2d_shot *shots, int nshots, const s2d_wave &wave,
         fast_range(m.nnx, (double)(wave.fd_dt * (1.0f / m.dx)), m.damp2a, m.damp2a1, m.damp2b, m.damp2b1, &d.xfast_lo,
                    &d.xfast_hi, &d.kx_in);
         if (!c->opt_fast_rows) d.zfast_lo = d.zfast_hi = d.xfast_lo = d.xfast_hi = 0;
-        // source amplitude per step: fd_dt * w[kt] * kappa[src] / (dx*dz)
-        // (cpumodelling.cpp:136-140), kappa = vp^2 rho in double at the source
+        // kappa at the source: of the model cell it replicates; a source on the
+        // free surface or above it (kappa held at 0) injects nothing
         const int mx = std::min(std::max(h.src_x - m.nb, 0), m.nx - 1);
         const int mz = std::min(std::max(h.src_z - m.nb, 0), m.nz - 1);
-        float vr[2];
-        CK(cudaMemcpy(&vr[0], m.vp.as<float>() + (size_t)mx * m.nz + mz, sizeof(float), cudaMemcpyDeviceToHost));
-        CK(cudaMemcpy(&vr[1], m.rho.as<float>() + (size_t)mx * m.nz + mz, sizeof(float), cudaMemcpyDeviceToHost));
-        // a source on the free surface or above it (kappa held at 0) injects nothing
-        const double ksrc = m.free_surface && h.src_z <= m.nb ? 0.0 : ((double)vr[0] * (double)vr[0]) * (double)vr[1];
-        const float dxdz = m.dx * m.dz;
-        std::vector<float> amp(rs.fd_nt, 0.0f);
-        for (int kt = 0; kt < rs.fd_nt && kt <= inject_last; ++kt) {
-            const double wk = kt < (int)w.size() ? w[kt] : 0.0;
-            amp[kt] = (float)(wave.fd_dt * wk * ksrc / dxdz);
-        }
+        const bool held = m.free_surface && h.src_z <= m.nb;
+        reinterpret_cast<SourceTerm *>(tab.data() + o_src)[s] = {
+            held ? nullptr : m.vp.as<float>() + (size_t)mx * m.nz + mz, m.rho.as<float>() + (size_t)mx * m.nz + mz,
+            reinterpret_cast<float *>(tab_d + o_amp[s]), reinterpret_cast<double *>(tab_d + o_ks) + s, m.dx * m.dz};
         // receivers grouped by column
         std::vector<int> rx(h.nrec), rz(h.nrec);
         for (int g = 0; g < h.nrec; ++g) {
@@ -877,38 +1031,30 @@ int setup_batch(Ctx *c, const s2d_shot *shots, int nshots, const s2d_wave &wave,
             d.rec_zlo = std::min(d.rec_zlo, rz[g]);
             d.rec_zhi = std::max(d.rec_zhi, rz[g]);
         }
-        std::vector<int> ptr(m.nnx + 1, 0), ez(h.nrec), eid(h.nrec);
+        int *const ptr = reinterpret_cast<int *>(tab.data() + o_ptr[s]);
+        int *const ez = reinterpret_cast<int *>(tab.data() + o_rz[s]);
+        int *const eid = reinterpret_cast<int *>(tab.data() + o_id[s]);
         for (int g = 0; g < h.nrec; ++g) ptr[rx[g] + 1]++;
         for (int x = 0; x < m.nnx; ++x) ptr[x + 1] += ptr[x];
-        std::vector<int> fill(ptr.begin(), ptr.end() - 1);
+        std::vector<int> fill(ptr, ptr + m.nnx);
         for (int g = 0; g < h.nrec; ++g) {
             const int k = fill[rx[g]]++;
             ez[k] = rz[g];
             eid[k] = g;
         }
-        b.aux.emplace_back(new DevBuf());
-        DevBuf &ab = *b.aux.back();
-        const size_t n_amp = (size_t)rs.fd_nt, n_ptr = (size_t)m.nnx + 1, n_rec = (size_t)std::max(h.nrec, 1);
-        const size_t bytes = sizeof(float) * n_amp + sizeof(int) * (n_ptr + 2 * n_rec) + 64;
-        CK(ab.alloc(bytes));
-        char *base = ab.as<char>();
-        float *amp_d = reinterpret_cast<float *>(base);
-        int *ptr_d = reinterpret_cast<int *>(base + sizeof(float) * n_amp);
-        int *ez_d = ptr_d + n_ptr;
-        int *eid_d = ez_d + n_rec;
-        CK(cudaMemcpy(amp_d, amp.data(), sizeof(float) * n_amp, cudaMemcpyHostToDevice));
-        CK(cudaMemcpy(ptr_d, ptr.data(), sizeof(int) * n_ptr, cudaMemcpyHostToDevice));
-        if (h.nrec) {
-            CK(cudaMemcpy(ez_d, ez.data(), sizeof(int) * h.nrec, cudaMemcpyHostToDevice));
-            CK(cudaMemcpy(eid_d, eid.data(), sizeof(int) * h.nrec, cudaMemcpyHostToDevice));
-        }
-        d.amp = amp_d;
-        d.rec_ptr = ptr_d;
-        d.rec_z = ez_d;
-        d.rec_id = eid_d;
+        d.amp = reinterpret_cast<const float *>(tab_d + o_amp[s]);
+        d.rec_ptr = reinterpret_cast<const int *>(tab_d + o_ptr[s]);
+        d.rec_z = reinterpret_cast<const int *>(tab_d + o_rz[s]);
+        d.rec_id = reinterpret_cast<const int *>(tab_d + o_id[s]);
     }
-    CK(b.shots_d.alloc(sizeof(ShotDev) * nshots));
-    CK(cudaMemcpy(b.shots_d.p, b.shot_dev.data(), sizeof(ShotDev) * nshots, cudaMemcpyHostToDevice));
+    CK(cudaMemcpyAsync(tab_d, tab.data(), n_up, cudaMemcpyHostToDevice, c->stream));
+    {
+        int e = launch_source_terms(reinterpret_cast<const SourceTerm *>(tab_d + o_src), nshots,
+                                    reinterpret_cast<const double *>(tab_d + o_w), std::max(n_inj, 0), rs.fd_nt,
+                                    wave.fd_dt, c->stream);
+        if (e) return fail(c, S2D_ERR_CUDA, "source terms launch: %s", cudaGetErrorString((cudaError_t)e));
+    }
+    CK(b.shots_d.alloc(c->arena, sizeof(ShotDev) * nshots));
 
     // groups: shots sharing a model, tasks interleaved over the group's shots.
     // In plain mode every shot is a group of its own and runs alone.
@@ -918,7 +1064,9 @@ int setup_batch(Ctx *c, const s2d_shot *shots, int nshots, const s2d_wave &wave,
         if (!by_model.count(shots[s].model_id)) model_order.push_back(shots[s].model_id);
         by_model[shots[s].model_id].push_back(s);
     }
+    std::vector<ShotDev> reordered;
     if (b.plain) {
+        reordered = b.shot_dev;
         for (int s = 0; s < nshots; ++s) b.table.push_back(s);
         for (int s = 0; s < nshots; ++s) {
             const Model &m = *c->models[shots[s].model_id];
@@ -934,7 +1082,6 @@ int setup_batch(Ctx *c, const s2d_shot *shots, int nshots, const s2d_wave &wave,
         // shots of one model must be contiguous in the shot table for shot0
         // indexing; keep the caller's order inside each model and reorder the
         // device table only (seis offsets stay the caller's).
-        std::vector<ShotDev> reordered;
         for (int mid : model_order) {
             const Model &m = *c->models[mid];
             const std::vector<int> &ss = by_model[mid];
@@ -950,12 +1097,8 @@ int setup_batch(Ctx *c, const s2d_shot *shots, int nshots, const s2d_wave &wave,
                 b.table.push_back(s);
             }
         }
-        CK(cudaMemcpy(b.shots_d.p, reordered.data(), sizeof(ShotDev) * nshots, cudaMemcpyHostToDevice));
     }
-    {
-        int e = build_tmaps(c, b);
-        if (e) return e;
-    }
+    CK(cudaMemcpyAsync(b.shots_d.p, reordered.data(), sizeof(ShotDev) * nshots, cudaMemcpyHostToDevice, c->stream));
     b.chip.assign(b.groups.size(), 0);
     CK(cudaStreamSynchronize(c->stream));
     c->batch = std::move(bp);
@@ -1248,14 +1391,15 @@ int s2d_create(void **ctx, int device) {
     c->device = device;
     cudaError_t e = cudaSetDevice(device);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
+    c->arena.stream = c->stream;
     if (e == cudaSuccess) e = cudaEventCreate(&c->ev0);
     if (e == cudaSuccess) e = cudaEventCreate(&c->ev1);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&c->sm_count, cudaDevAttrMultiProcessorCount, device);
-    if (e == cudaSuccess) e = c->dev_err.alloc(sizeof(int));
-    if (e == cudaSuccess) e = c->queue_d.alloc(2 * sizeof(int));
+    if (e == cudaSuccess) e = c->dev_err.alloc(c->arena, sizeof(int));
+    if (e == cudaSuccess) e = c->queue_d.alloc(c->arena, 2 * sizeof(int));
     if (e == cudaSuccess) e = cudaMemset(c->queue_d.p, 0, 2 * sizeof(int));
-    if (e == cudaSuccess) e = c->bar_d.alloc(sizeof(unsigned));
-    if (e == cudaSuccess) e = c->args_d.alloc(sizeof(StepArgs));
+    if (e == cudaSuccess) e = c->bar_d.alloc(c->arena, sizeof(unsigned));
+    if (e == cudaSuccess) e = c->args_d.alloc(c->arena, sizeof(StepArgs));
     if (e == cudaSuccess) e = cudaMemset(c->dev_err.p, 0, sizeof(int));
     if (e != cudaSuccess) {
         delete c;
@@ -1277,6 +1421,7 @@ void s2d_destroy(void *ctx) {
     if (c->ev0) cudaEventDestroy(c->ev0);
     if (c->ev1) cudaEventDestroy(c->ev1);
     for (cudaEvent_t e : c->phase_ev) cudaEventDestroy(e);
+    c->arena.stream = nullptr;
     if (c->stream) cudaStreamDestroy(c->stream);
     delete c;
 }
@@ -1310,15 +1455,17 @@ int s2d_model_create(void *ctx, int nx, int nz, float dx, float dz, int nb, cons
     if (m->nnx > 65535)
         return fail(c, S2D_ERR_ARG, "padded grid has %d columns; at most 65535 are supported", m->nnx);
     const size_t raw = (size_t)nx * nz * sizeof(float);
-    CK(m->vp.alloc(raw));
-    CK(m->rho.alloc(raw));
+    c->arena.expect({raw, raw, 3 * m->field_elems * sizeof(float), m->field_elems * sizeof(float)});
+    CK(m->vp.alloc(c->arena, raw));
+    CK(m->rho.alloc(c->arena, raw));
+    const size_t fb = m->field_elems * sizeof(float);
+    CK(m->mat.alloc(c->arena, 3 * fb));
+    DevBuf bue;
+    CK(bue.alloc(c->arena, fb));
+    CK(cudaDeviceSynchronize());  // vp and rho may still be written on a stream of the caller's
     const cudaMemcpyKind kind = (flags & S2D_MODEL_DEVICE) ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
     CK(cudaMemcpyAsync(m->vp.p, vp, raw, kind, c->stream));
     CK(cudaMemcpyAsync(m->rho.p, rho, raw, kind, c->stream));
-    const size_t fb = m->field_elems * sizeof(float);
-    CK(m->mat.alloc(3 * fb));
-    DevBuf bue;
-    CK(bue.alloc(fb));
     CK(cudaMemsetAsync(m->mat.p, 0, 3 * fb, c->stream));
     CK(cudaMemsetAsync(bue.p, 0, fb, c->stream));
     int e = launch_prepare_model(m->vp.as<float>(), m->rho.as<float>(), nx, nz, nb, m->ld, m->kappa(), bue.as<float>(),
@@ -1395,6 +1542,7 @@ int s2d_forward(void *ctx, const s2d_shot *shots, int nshots, const s2d_wave *wa
         const int order = lc.order;
         if (!e) e = layout_groups(c, b, lc);
         if (!e) e = launch_config(c, b.max_tasks, &lc, lc.variant, lc.block, lc.stages);
+        if (!e && tma_variant(lc.variant)) e = build_tmaps(c, b);
         lc.order = order;
         return e;
     };
@@ -1561,7 +1709,7 @@ int phase_mark(Ctx *c, GradRun &g, int phase) {
 
 int grad_alloc(Ctx *c, GradRun &g, size_t bytes, void **out) {
     cudaError_t e;
-    g.bufs.push_back(c->pool.take(bytes, &e));
+    g.bufs.push_back(c->pool.take(c->arena, bytes, &e));
     CK(e);
     *out = g.bufs.back()->p;
     return S2D_OK;
@@ -1668,7 +1816,15 @@ extern "C" int s2d_gradient(void *ctx, const s2d_shot *shots, int nshots, const 
     // dJ/dkappa, dJ/db shared by every shot (they share the model): the
     // adjoint kernels add into it atomically
     std::vector<ShotDev> adj = b.shot_dev;
-    std::vector<float *> gk(nshots), gb(nshots), sadj(nshots);
+    std::vector<float *> gk(nshots), gb(nshots);
+    float *sadj = nullptr;  // [nshots][fd_nt]
+    {
+        void *p;
+        int e = grad_alloc(c, g, sizeof(float) * nshots * rs.fd_nt, &p);
+        if (e) return e;
+        CK(cudaMemsetAsync(p, 0, sizeof(float) * nshots * rs.fd_nt, c->stream));
+        sadj = static_cast<float *>(p);
+    }
     float *acc_pair = nullptr;
     {
         void *p;
@@ -1699,11 +1855,7 @@ extern "C" int s2d_gradient(void *ctx, const s2d_shot *shots, int nshots, const 
             CK(cudaMemsetAsync(p, 0, 2 * fb, c->stream));
             adj[s].scr = static_cast<float *>(p);
         }
-        int e = grad_alloc(c, g, sizeof(float) * rs.fd_nt, &p);
-        if (e) return e;
-        CK(cudaMemsetAsync(p, 0, sizeof(float) * rs.fd_nt, c->stream));
-        sadj[s] = static_cast<float *>(p);
-        adj[s].srcadj = sadj[s];
+        adj[s].srcadj = sadj + (size_t)s * rs.fd_nt;
     }
     // adjoint source: the caller's, or the residual d - d_obs after the forward
     const size_t nseis = b.seis_elems;
@@ -1761,7 +1913,7 @@ extern "C" int s2d_gradient(void *ctx, const s2d_shot *shots, int nshots, const 
         b.shot_dev[s].nprod = (size_t)C * 4 * F;
     }
     DevBuf adj_table;
-    CK(adj_table.alloc(sizeof(ShotDev) * nshots));
+    CK(adj_table.alloc(c->arena, sizeof(ShotDev) * nshots));
     CK(cudaMemcpyAsync(adj_table.p, adj.data(), sizeof(ShotDev) * nshots, cudaMemcpyHostToDevice, c->stream));
     CK(cudaMemcpyAsync(b.shots_d.p, b.shot_dev.data(), sizeof(ShotDev) * nshots, cudaMemcpyHostToDevice,
                        c->stream));
@@ -1773,6 +1925,7 @@ extern "C" int s2d_gradient(void *ctx, const s2d_shot *shots, int nshots, const 
         const int order = lc_fwd.order;
         if (!e) e = layout_groups(c, b, lc_fwd);
         if (!e) e = launch_config(c, b.max_tasks, &lc_fwd, lc_fwd.variant, lc_fwd.block, lc_fwd.stages);
+        if (!e && tma_variant(lc_fwd.variant)) e = build_tmaps(c, b);
         if (!e) e = launch_config(c, b.max_tasks, &lc_prod, prod_variant, 128, 0);
         if (e) return e;
         lc_fwd.order = order;
@@ -1865,7 +2018,7 @@ extern "C" int s2d_gradient(void *ctx, const s2d_shot *shots, int nshots, const 
         if (e) return e;
     }
     DevBuf sumsq;
-    CK(sumsq.alloc(sizeof(double)));
+    CK(sumsq.alloc(c->arena, sizeof(double)));
     CK(cudaMemsetAsync(sumsq.p, 0, sizeof(double), c->stream));
     const cudaMemcpyKind dk = dev_seis ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
     if (flags & S2D_GRAD_MISFIT) {
@@ -1928,22 +2081,17 @@ extern "C" int s2d_gradient(void *ctx, const s2d_shot *shots, int nshots, const 
         wv = ricker(*wave, rs.nts);
         inject_last = rs.nts;
     }
-    std::vector<float> sa(rs.fd_nt);
+    std::vector<float> all_sa((size_t)nshots * rs.fd_nt);
+    std::vector<double> all_ksrc(nshots);  // kappa at the source (cpumodelling.cpp:136-140)
     std::vector<int> cells(nshots);
     std::vector<double> vals(nshots);
     const double sfac = (double)wave->fd_dt / (double)(m.dx * m.dz);
+    CK(cudaMemcpyAsync(all_sa.data(), sadj, sizeof(float) * all_sa.size(), cudaMemcpyDeviceToHost, c->stream));
+    CK(cudaMemcpyAsync(all_ksrc.data(), b.ksrc_d, sizeof(double) * nshots, cudaMemcpyDeviceToHost, c->stream));
+    CK(cudaStreamSynchronize(c->stream));
     for (int s = 0; s < nshots; ++s) {
-        CK(cudaMemcpyAsync(sa.data(), sadj[s], sizeof(float) * rs.fd_nt, cudaMemcpyDeviceToHost, c->stream));
-        CK(cudaStreamSynchronize(c->stream));
-        // kappa at the source, in double as the amplitude uses it (cpumodelling.cpp:136-140)
-        const int mx = std::min(std::max(b.shots[s].src_x - m.nb, 0), m.nx - 1);
-        const int mz = std::min(std::max(b.shots[s].src_z - m.nb, 0), m.nz - 1);
-        float vr[2];
-        CK(cudaMemcpy(&vr[0], m.vp.as<float>() + (size_t)mx * m.nz + mz, sizeof(float), cudaMemcpyDeviceToHost));
-        CK(cudaMemcpy(&vr[1], m.rho.as<float>() + (size_t)mx * m.nz + mz, sizeof(float), cudaMemcpyDeviceToHost));
-        const double ksrc = m.free_surface && b.shots[s].src_z <= m.nb
-                                ? 0.0
-                                : ((double)vr[0] * (double)vr[0]) * (double)vr[1];
+        const float *const sa = all_sa.data() + (size_t)s * rs.fd_nt;
+        const double ksrc = all_ksrc[s];
         double v = 0;
         for (int kt = 0; kt < rs.fd_nt; ++kt) {
             const bool injected = kt <= inject_last;

@@ -306,6 +306,17 @@ int launch_gradient_finalize(float *const *gk, float *const *gb, int nshots, int
                              void *stream);
 // Residual d - d_obs in place of d_obs... : res[i] = seis[i] - obs[i]; partial sums of res^2.
 int launch_residual(const float *seis, const float *obs, float *res, size_t n, double *sumsq, void *stream);
+// Where a shot's source terms come from and go: amp[kt] = fd_dt w[kt] ksrc /
+// (dx dz) for kt < n_inj (0 after), ksrc = vp^2 rho at the source in double (0
+// without vp) (cpumodelling.cpp:136-140).
+struct SourceTerm {
+    const float *vp, *rho;
+    float *amp;
+    double *ksrc;
+    float dxdz;
+};
+int launch_source_terms(const SourceTerm *src, int nshots, const double *w, int n_inj, int fd_nt, float fd_dt,
+                        void *stream);
 int launch_prepare_model(const float *vp, const float *rho, int nx, int nz, int nb, int ld,
                          float *kappa, float *bue_scratch, float *bx, float *bz, void *stream);
 int step_kernel_prepare(int variant, size_t smem);

@@ -1559,6 +1559,22 @@ __global__ void __launch_bounds__(128, 2) step_kernel_o8(const StepArgs *__restr
 
 // ---- model preparation (cpumodelling.cpp:207-230, cpu_modelling_kernels.cpp:64-121) ----
 
+// Source terms of every shot (SourceTerm), rounded operation by operation as
+// the host's double arithmetic: on the device they need no read of vp and rho
+// back, which waited twice per shot.
+__global__ void source_terms(const SourceTerm *__restrict__ src, const double *__restrict__ w, int n_inj, int fd_nt,
+                             float fd_dt) {
+    const SourceTerm t = src[blockIdx.y];
+    const double v = t.vp ? (double)*t.vp : 0.0;
+    const double ksrc = t.vp ? __dmul_rn(__dmul_rn(v, v), (double)*t.rho) : 0.0;
+    const int kt = blockIdx.x * blockDim.x + threadIdx.x;
+    if (kt == 0) *t.ksrc = ksrc;
+    if (kt >= fd_nt) return;
+    t.amp[kt] = kt < n_inj
+                    ? (float)__ddiv_rn(__dmul_rn(__dmul_rn((double)fd_dt, w[kt]), ksrc), (double)t.dxdz)
+                    : 0.0f;
+}
+
 // kappa = vp^2 rho in double rounded to float, buoyancy 1/rho (1e10 where
 // rho <= 0) of the model expanded into the sponge by edge replication.
 __global__ void prepare_cells(const float *__restrict__ vp, const float *__restrict__ rho, int nx, int nz,
@@ -2102,6 +2118,12 @@ int persist_occupancy(int *blocks_per_sm) {
 
 int launch_set_args(const StepArgs &v, StepArgs *args_dev, void *stream) {
     set_args_kernel<<<1, 1, 0, (cudaStream_t)stream>>>(v, args_dev);
+    return (int)cudaGetLastError();
+}
+
+int launch_source_terms(const SourceTerm *src, int nshots, const double *w, int n_inj, int fd_nt, float fd_dt,
+                        void *stream) {
+    source_terms<<<dim3((fd_nt + 255) / 256, nshots), 256, 0, (cudaStream_t)stream>>>(src, w, n_inj, fd_nt, fd_dt);
     return (int)cudaGetLastError();
 }
 
