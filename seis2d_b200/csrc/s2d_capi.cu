@@ -1896,9 +1896,10 @@ extern "C" int s2d_gradient(void *ctx, const s2d_shot *shots, int nshots, const 
         void *p;
         int e = grad_alloc(c, g, (size_t)C * 4 * fb, &p);
         if (e) return e;
-        // ghost rows and the second product slot of merged cells are never
-        // written; the adjoint reads them (times zero): they must hold zeros
-        CK(cudaMemsetAsync(p, 0, (size_t)C * 4 * fb, c->stream));
+        // Not cleared: what the forward never writes (ghost cells, the second
+        // slot of cells that carry one pressure) reaches no cell of the adjoint,
+        // whose kernels select and do not multiply by zero there.  Clearing the
+        // products of 8 shots of 1201 x 401, 100 steps, took 0.7 of 86.4 ms.
         prod[s] = static_cast<float *>(p);
         ckpt[s] = nullptr;
         if (nseg > 1) {
