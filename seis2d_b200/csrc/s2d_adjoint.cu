@@ -152,14 +152,14 @@ struct AdjSource {
 // tasks) or moved (the others, whose code then stays short).
 //
 // What bounds it: the latency of one column's chain (ring reads, three rounds
-// of shuffles), with two warps on each scheduler.  1201x401, 8 shots: 72.8
-// us/step (3.5 TB/s of DRAM traffic, 26% of the issue slots, the L1 and
-// shared-memory pipe at 53%), before with the windows in shared memory 104
-// us/step.  Three blocks per SM (168 registers, spilling) took 97 us/step; the
-// row coefficients in shared memory instead of registers 79 (the pipe again).
-// 2401x1201, 4 shots: 151 us/step.  Rim and interior tasks are cut apart
-// (kSplitAdj in the host code): without their tasks the interior alone takes
-// 40 us/step of the first case.
+// of shuffles), with two warps on each scheduler.  1201x401, 8 shots: 69.6
+// us/step (75.5 when every iteration brought all its pieces), before with the
+// windows in shared memory 104 us/step.  Three blocks per SM (168 registers,
+// spilling) took 97 us/step; the row coefficients in shared memory instead of
+// registers 79 (the shared-memory pipe).  2301x1101, 4 shots, 147 us/step with
+// all pieces: 56% of the DRAM rate, 24% of the issue slots.  Rim and interior
+// tasks are cut apart (kSplitAdj in the host code): without their tasks the
+// interior alone took 40 us/step of the first case.
 constexpr int kAdjSlots = 11;  // mvx', bx; mpx, mvz, bz, kappa, three products; mpz, the fourth product
 template <int KIND>
 struct AdjDepth {
@@ -370,23 +370,28 @@ __device__ __forceinline__ void adjoint_task(const StepArgs &a, const ShotDev &S
     const float *np = S.prod + (size_t)(kt - a.prod_kt0) * 4 * F + off + (ptrdiff_t)(L0 - 1) * ld;
     auto issue = [&](int L, int slot) {
         V4 *st = k.ring + slot * (NS * 32);
-        const bool in_l = KIND != kAdjAny || L < nnx + S2D_GX;
-        if (in_l) {
+        // Only what the iteration uses (what it computes from the rest of its
+        // slot is not written): the windows' inputs first, the products and mpz
+        // of the task's own columns and the one before them.  Of a segment's
+        // 6 columns besides its own, three bring 2 pieces and two 6 instead of 9.
+        if (L <= Lend) {
             cp_async16(st, ns + ld + 2 * fs, true);
             cp_async16(st + 32, nm + ld + fs, true);
-        }
-        cp_async16(st + 64, ns, true);
-        cp_async16(st + 96, ns + 3 * fs, true);
-        cp_async16(st + 128, nm + 2 * fs, true);
-        cp_async16(st + 160, nm, true);
-        // products: zeros outside the grid and past the columns in use
-        const bool img = KIND != kAdjAny || (L >= 1 && L <= nnx);
-        cp_async16(st + 192, np, img);
-        cp_async16(st + 224, np + 2 * F, img);
-        cp_async16(st + 256, np + 3 * F, img);
-        if (KIND != kAdjIn) {
-            cp_async16(st + 288, ns + fs, true);
-            cp_async16(st + 320, np + F, img);
+            if (L >= xa) {
+                cp_async16(st + 64, ns, true);
+                cp_async16(st + 96, ns + 3 * fs, true);
+                cp_async16(st + 128, nm + 2 * fs, true);
+                cp_async16(st + 160, nm, true);
+                if (L >= 1 && L <= k.xb) {
+                    cp_async16(st + 192, np, true);
+                    cp_async16(st + 224, np + 2 * F, true);
+                    cp_async16(st + 256, np + 3 * F, true);
+                    if (KIND != kAdjIn) {
+                        cp_async16(st + 288, ns + fs, true);
+                        cp_async16(st + 320, np + F, true);
+                    }
+                }
+            }
         }
         ns += ld;
         nm += ld;
