@@ -217,6 +217,7 @@ struct Batch {
     std::vector<GroupDev> groups;    // batched mode
     std::vector<int> group_nnx;      // padded columns of each group's model
     std::vector<int> group_nnz;      // padded rows of each group's model
+    std::vector<GroupDev> rest;      // the groups as the last step of an odd count takes them (behind them in groups_d)
     int cur = 0;                     // state buffer (parity) holding step kt_next
     std::vector<long> layout;        // launch configuration the groups are laid out for
     std::vector<char> chip;          // groups the on-chip loop runs (they get no tasks)
@@ -477,7 +478,7 @@ int build_coef(Ctx *c, Model &m, float fd_dt) {
 
 // Dynamic shared memory of a warp of the variants with 112-row strips.
 int ts_warp_bytes(int variant) {
-    return variant == kVariantTs2 ? kTs2WarpBytes : variant == kVariantTs1 ? 0 : kO8WarpBytes;
+    return variant == kVariantTs2 ? kTs2WarpBytes : kO8WarpBytes;
 }
 
 // Launch configuration for (variant, block, stages): shared memory and a grid
@@ -537,7 +538,10 @@ std::vector<long> tune_key(const Ctx *c, const Batch &b) {
 // launch from about 1.5 M cells on (one 3301 x 1301 shot 157 Gcell/s against 102
 // with one step, 8 of 5120 x 5120 370 against 154); below, its longer halo and
 // its 8 warps per SM cost what the second step saves (780 x 580: 64 and 64).
-int default_variant(const Batch &b) {
+// A single step has no second one to save for: 8 shots of 5120 x 5120 1.38 ms
+// with variant 16.
+int default_variant(const Batch &b, int nsteps) {
+    if (nsteps < 2) return kVariantLdgPf4;
     double cells = 0;
     for (size_t g = 0; g < b.groups.size(); ++g) {
         if (g < b.chip.size() && b.chip[g]) continue;
@@ -547,52 +551,52 @@ int default_variant(const Batch &b) {
     return cells >= 1.5e6 ? kVariantTs2 : kVariantLdgPf4;
 }
 
-// The configuration a run of batch `b` uses when it does not tune: the
-// options when autotuning is off, else the tuned result for the batch's
-// shape, else the built-in default.
-int base_config(Ctx *c, const Batch &b, LaunchCfg *out, bool *tuned = nullptr) {
+// The configuration a run of `nsteps` steps of batch `b` uses when it does not
+// tune: the options when autotuning is off, else the tuned result for the
+// batch's shape (it holds for runs that its kernel can make whole launches of),
+// else the built-in default.
+int base_config(Ctx *c, const Batch &b, int nsteps, LaunchCfg *out, bool *tuned = nullptr) {
     if (tuned) *tuned = false;
     // 8th-order batches run the 8th-order kernel whatever the options say
     if (b.order8 && !c->opt_autotune) return launch_config(c, b.max_tasks, out, c->opt_variant8, 128, 0);
     if (!c->opt_autotune) return launch_config(c, b.max_tasks, out, c->opt_variant, c->opt_block, c->opt_stages);
     auto it = c->tuned.find(tune_key(c, b));
-    if (it != c->tuned.end()) {
+    if (it != c->tuned.end() && nsteps >= steps_per_launch(it->second[0])) {
         if (tuned) *tuned = true;
         int e = launch_config(c, b.max_tasks, out, it->second[0], it->second[1], it->second[2]);
         out->order = c->order_fixed ? -1 : it->second[3];
         return e;
     }
     const LaunchCfg d;
-    return launch_config(c, b.max_tasks, out, b.order8 ? kVariantO8 : default_variant(b), d.block,
+    return launch_config(c, b.max_tasks, out, b.order8 ? kVariantO8 : default_variant(b, nsteps), d.block,
                          b.order8 ? 0 : d.stages);
 }
 
-// Segment lengths, segment counts and task ranges of the batch's groups for
-// `resident_warps` warps looping over the tasks of a launch; uploaded when
-// `key` differs from the layout in place.
+// Cut `groups` (the batch's) into tasks for `resident_warps` warps looping over
+// the tasks of a launch: segment lengths, segment counts and task ranges.
 // With `tma` a task is a CTA's: kTmaWarps (shot, strip) pairs of a group
 // over one segment, and `resident_warps` counts resident CTAs.
-// With `split` the groups are cut into rim and interior tasks (two-step kernel).
-int layout_groups_for(Ctx *c, Batch &b, long resident_warps, std::vector<long> key, bool ts = false,
-                      bool tma = false, bool split = false) {
-    for (char f : b.chip) key.push_back(f);
-    if (b.layout == key) return S2D_OK;
-    for (size_t gi = 0; gi < b.groups.size(); ++gi)
-        b.groups[gi].nstrips = ts ? num_strips_ts(b.group_nnz[gi]) : num_strips(b.group_nnz[gi]);
+// With `split` the strips are 112 rows and cut into rim and interior tasks
+// (two-step and 8th-order kernels).  Returns the largest task count of one
+// launch sequence.
+long cut_groups(const Ctx *c, const Batch &b, std::vector<GroupDev> &groups, long resident_warps, bool tma, bool split) {
+    for (size_t gi = 0; gi < groups.size(); ++gi)
+        groups[gi].nstrips = split ? num_strips_ts(b.group_nnz[gi]) : num_strips(b.group_nnz[gi]);
     auto per_seg = [&](const GroupDev &g, int nshots) {
         return tma ? (long)tma_blocks(nshots, g.nstrips) : (long)nshots * g.nstrips;
     };
     // cells of all the groups' shots (the warps' shares of a split layout)
     double cells = 0;
-    for (size_t gi = 0; gi < b.groups.size(); ++gi)
-        if (!b.chip[gi]) cells += (double)b.groups[gi].nshots * b.group_nnx[gi] * b.group_nnz[gi];
     long per_seg_total = 0;
-    for (size_t gi = 0; gi < b.groups.size(); ++gi)
-        if (!b.chip[gi]) per_seg_total += per_seg(b.groups[gi], b.groups[gi].nshots);
+    for (size_t gi = 0; gi < groups.size(); ++gi)
+        if (!b.chip[gi]) {
+            cells += (double)groups[gi].nshots * b.group_nnx[gi] * b.group_nnz[gi];
+            per_seg_total += per_seg(groups[gi], groups[gi].nshots);
+        }
     long max_tasks = 0;
     int task = 0;
-    for (size_t gi = 0; gi < b.groups.size(); ++gi) {
-        GroupDev &g = b.groups[gi];
+    for (size_t gi = 0; gi < groups.size(); ++gi) {
+        GroupDev &g = groups[gi];
         const int nnx = b.group_nnx[gi];
         // plain mode: every shot is a group of its own and runs alone
         const long tasks_per_seg = b.plain ? per_seg(g, 1) : per_seg_total;
@@ -605,7 +609,7 @@ int layout_groups_for(Ctx *c, Batch &b, long resident_warps, std::vector<long> k
                         b.order8 ? kSplitO8 : kSplitTs2);
         } else {
             g.seg_len = c->opt_seg_len > 0 ? std::min(c->opt_seg_len, nnx)
-                                           : choose_seg_len(nnx, tasks_per_seg, resident_warps, ts ? 12 : 6);
+                                           : choose_seg_len(nnx, tasks_per_seg, resident_warps, 6);
             g.nsegs = (nnx + g.seg_len - 1) / g.seg_len;
         }
         const int per_shot = shot_tasks(g);
@@ -618,29 +622,46 @@ int layout_groups_for(Ctx *c, Batch &b, long resident_warps, std::vector<long> k
             max_tasks = task;
         }
     }
-    if (!b.groups_d.p) CK(b.groups_d.alloc(c->arena, sizeof(GroupDev) * b.groups.size()));
-    CK(cudaMemcpyAsync(b.groups_d.p, b.groups.data(), sizeof(GroupDev) * b.groups.size(), cudaMemcpyHostToDevice,
-                       c->stream));
-    // the copy reads host memory that a later layout rewrites
-    CK(cudaStreamSynchronize(c->stream));
-    b.max_tasks = max_tasks;
-    b.layout = key;
-    b.layout_tma = tma;
-    return S2D_OK;
+    return max_tasks;
 }
 
-// The layout for the resident warps of launch configuration `lc`.
+// The one-step kernel that ends an odd count of the two-step kernel's steps, in
+// a layout of its own: 3 steps of 8 shots of 5120 x 5120 2.5 ms, of one 3301 x
+// 1301 shot 122 us (3 of this kernel 4.1 ms and 152 us; a one-step kernel in the
+// two-step layout, with too few tasks for its warps, 3.0 ms and 168 us).
+constexpr int kRestVariant = kVariantLdgPf4;
+
+// The layout for the resident warps of launch configuration `lc`, uploaded when
+// it differs from the one in place.  The two-step kernel's comes with a second
+// one behind it, for the one-step kernel that ends an odd count.
 int layout_groups(Ctx *c, Batch &b, const LaunchCfg &lc) {
-    // the two-step kernel and its one-step companion share one layout
-    const int v = lc.variant == kVariantTs1 ? kVariantTs2 : lc.variant;
-    const std::vector<long> key = {v, lc.block, lc.stages, c->opt_seg_len};
+    std::vector<long> key = {lc.variant, lc.block, lc.stages, c->opt_seg_len};
+    for (char f : b.chip) key.push_back(f);
+    if (b.layout == key) return S2D_OK;
     // resident warps of the configuration (its grid when the work is smaller);
     // resident CTAs for the TMA kernel, whose tasks are CTA tasks
     LaunchCfg full;
-    int e = launch_config(c, 1L << 40, &full, v, lc.block, lc.stages);
+    int e = launch_config(c, 1L << 40, &full, lc.variant, lc.block, lc.stages);
     if (e) return e;
-    if (tma_variant(v)) return layout_groups_for(c, b, (long)full.grid, key, false, true);
-    return layout_groups_for(c, b, (long)full.grid * (full.block / 32), key, ts_layout(v), false, queue_variant(v));
+    const bool tma = tma_variant(lc.variant);
+    b.layout.clear();
+    b.max_tasks = cut_groups(c, b, b.groups, (long)full.grid * (tma ? 1 : full.block / 32), tma, ts_layout(lc.variant));
+    const size_t bytes = sizeof(GroupDev) * b.groups.size();
+    if (!b.groups_d.p) CK(b.groups_d.alloc(c->arena, 2 * bytes));
+    CK(cudaMemcpyAsync(b.groups_d.p, b.groups.data(), bytes, cudaMemcpyHostToDevice, c->stream));
+    if (steps_per_launch(lc.variant) == 2) {
+        b.rest = b.groups;
+        e = launch_config(c, 1L << 40, &full, kRestVariant, 128, 0);
+        if (e) return e;
+        cut_groups(c, b, b.rest, (long)full.grid * (full.block / 32), false, false);
+        CK(cudaMemcpyAsync(b.groups_d.as<GroupDev>() + b.rest.size(), b.rest.data(), bytes, cudaMemcpyHostToDevice,
+                           c->stream));
+    }
+    // the copies read host memory that a later layout rewrites
+    CK(cudaStreamSynchronize(c->stream));
+    b.layout = key;
+    b.layout_tma = tma;
+    return S2D_OK;
 }
 
 // Graph of `n` step launches (kt_off = 0..n-1) for one launch configuration,
@@ -676,8 +697,8 @@ int step_graph(Ctx *c, const LaunchCfg &lc, int n, cudaGraphExec_t *out) {
 // arguments `args` (a whole batch, or one shot of a plain run), as replays of
 // a graph of `graph_chunk` launches.  The state at kt_begin is in buffer
 // b.cur; each launch reads one buffer and writes the other, and b.cur follows.
-// A two-step configuration finishes an odd count with one launch of its
-// one-step companion (same strip layout).
+// A two-step configuration finishes an odd count with one launch of a one-step
+// kernel (args.groups then points into b.groups_d).
 // start_ev (direct launches only): recorded after the launch-argument update,
 // just before the first step launch, so an interval timed from it holds the
 // step kernels alone (the autotuner's trials).
@@ -741,8 +762,16 @@ int run_loop(Ctx *c, Batch &b, const LaunchCfg &lc, StepArgs args, int kt_begin,
     if (rem) {
         args.kt_base = kt_begin + nl * spl;
         args.par0 = b.cur;
-        int e = launch_set_args(args, args_d, c->stream);
-        if (!e) e = launch_step(kVariantTs1, args_d, 0, lc.grid, lc.block, 0, c->stream);  // no delay lines
+        // the same groups in the one-step kernel's layout
+        const size_t g0 = args.groups - b.groups_d.as<GroupDev>();
+        args.groups += b.rest.size();
+        args.total_tasks = 0;
+        for (int g = 0; g < args.ngroups; ++g) args.total_tasks += b.rest[g0 + g].nshots * shot_tasks(b.rest[g0 + g]);
+        LaunchCfg one;
+        int e = launch_config(c, args.total_tasks, &one, kRestVariant, 128, 0);
+        if (e) return e;
+        e = launch_set_args(args, args_d, c->stream);
+        if (!e) e = launch_step(kRestVariant, args_d, 0, one.grid, one.block, one.smem, c->stream);
         if (e) return fail(c, S2D_ERR_CUDA, "step launch: %s", cudaGetErrorString((cudaError_t)e));
         *launches += 2;
         b.cur ^= 1;
@@ -1538,7 +1567,7 @@ int s2d_forward(void *ctx, const s2d_shot *shots, int nshots, const s2d_wave *wa
     int tuned_now = 0;
     LaunchCfg lc;
     auto configure = [&]() -> int {
-        int e = base_config(c, b, &lc, &tuned);
+        int e = base_config(c, b, nsteps, &lc, &tuned);
         const int order = lc.order;
         if (!e) e = layout_groups(c, b, lc);
         if (!e) e = launch_config(c, b.max_tasks, &lc, lc.variant, lc.block, lc.stages);
@@ -1922,7 +1951,7 @@ extern "C" int s2d_gradient(void *ctx, const s2d_shot *shots, int nshots, const 
     LaunchCfg lc_fwd, lc_prod;
     const int prod_variant = b.order8 ? kVariantO8Products : c->opt_prod_variant;
     {
-        int e = base_config(c, b, &lc_fwd);
+        int e = base_config(c, b, C, &lc_fwd);
         const int order = lc_fwd.order;
         if (!e) e = layout_groups(c, b, lc_fwd);
         if (!e) e = launch_config(c, b.max_tasks, &lc_fwd, lc_fwd.variant, lc_fwd.block, lc_fwd.stages);

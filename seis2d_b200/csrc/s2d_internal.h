@@ -150,7 +150,6 @@ enum StepVariant { kVariantBulk = 0, kVariantLdg = 1, kVariantBulk128 = 2,
                    kVariantLdgProducts = 3 /* plain loads + S2D_STEP_PRODUCTS, gradient runs */,
                    kVariantLdg128 = 4 /* plain loads, compiled for 128 registers */,
                    kVariantTs2 = 5 /* two FD steps per launch (112-row strips) */,
-                   kVariantTs1 = 6 /* one FD step in the two-step kernel's layout (odd remainders) */,
                    kVariantO8 = 7 /* 8th-order operator (112-row strips), models with S2D_MODEL_ORDER8 */,
                    kVariantO8b = 8, kVariantO8c = 9 /* other names of kVariantO8 */,
                    kVariantO8Products = 10 /* kVariantO8 + S2D_STEP_PRODUCTS, gradient runs */,
@@ -197,9 +196,9 @@ constexpr int kPersistTrialSteps = 4;
 constexpr int steps_per_launch(int variant) {
     return variant == kVariantTs2 ? 2 : variant == kVariantPersist ? kPersistTrialSteps : 1;
 }
-// Variants whose strips are S2D_TS_OUT rows (and whose tasks stream 12 or 13 halo columns).
+// Variants whose strips are S2D_TS_OUT rows, cut into tasks by kind (GroupDev::split) that the launches draw from the queue.
 inline bool ts_layout(int variant) {
-    return variant == kVariantTs2 || variant == kVariantTs1 || (variant >= kVariantO8 && variant <= kVariantO8Products);
+    return variant == kVariantTs2 || (variant >= kVariantO8 && variant <= kVariantO8Products);
 }
 inline bool order8_variant(int variant) { return variant >= kVariantO8 && variant <= kVariantO8c; }
 inline bool tma_variant(int variant) { return variant == kVariantTma; }
@@ -225,10 +224,6 @@ constexpr int kAdj8ColLo = 7, kAdj8ColHi = 6;  // of the 8th-order one (no rows)
 // iterations of vx; px, vz, kappa; bx, bz; pz) and 12 row coefficients.
 constexpr int kO8Depth = 4, kO8Slots = 7;
 constexpr int kO8WarpBytes = (kO8Depth * kO8Slots + 12) * S2D_STRIP_ROWS * 4;
-// Variants whose launches draw their tasks from the queue, cut by kind (GroupDev::split).
-inline bool queue_variant(int variant) {
-    return variant == kVariantTs2 || (variant >= kVariantO8 && variant <= kVariantO8Products);
-}
 
 // Shared memory of one pipeline stage: 7 slots of one 128-row column each
 // (vx at L; px, pz, kappa, vz at L-1; bx, bz at L-3).

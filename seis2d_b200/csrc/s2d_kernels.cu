@@ -755,75 +755,6 @@ __global__ void __launch_bounds__(128, MINB) step_kernel_bulk(const StepArgs *__
 // (rows c+8 .. c+119 of a strip starting at c = 112k - 8), so strips write
 // 112 rows; the segment's stream starts 6 columns early and ends 5 late.
 
-// One step of a task in the two-step kernel's strip layout.
-template <bool FAST, bool XF>
-__device__ __forceinline__ void ts1_task(const StepArgs &a, const ShotDev &S, int strip, int xa, int seg_len, int kt,
-                                         int par, int lane) {
-    const int xb = min(S.nnx, xa + seg_len);
-    const size_t ld = (size_t)S.ld;
-    const int c = strip * S2D_TS_OUT - 8;
-    Lane<FAST> la;
-    lane_setup(la, S, c, lane, kt);
-    la.owner = lane >= 2 && lane <= 29;
-    const int slot = (kt + 1) / a.dt_factor - 1;
-    const bool rec = !(a.flags & S2D_STEP_NO_RECORD) && ((kt + 1) % a.dt_factor) == 0 && slot < S.real_nt;
-    const size_t off = (size_t)(la.z0 + S2D_GZ) + (size_t)S2D_GX * ld;
-    const int fs = S.fstride;
-    float *const sb = S.st[0][0] + off;
-    const int ib = par * 4 * fs, ob = (par ^ 1) * 4 * fs;
-    const float *__restrict__ pxi = sb + ib;
-    const float *__restrict__ pzi = sb + ib + fs;
-    const float *__restrict__ vxi = sb + ib + 2 * fs;
-    const float *__restrict__ vzi = sb + ib + 3 * fs;
-    float *__restrict__ pxo = sb + ob;
-    float *__restrict__ pzo = sb + ob + fs;
-    float *__restrict__ vxo = sb + ob + 2 * fs;
-    float *__restrict__ vzo = sb + ob + 3 * fs;
-    const float *__restrict__ kap = S.kappa + off;
-    const float *__restrict__ bxp = kap + fs;
-    const float *__restrict__ bzp = kap + 2 * fs;
-    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-    // windows: vx at L-3..L, new p at L-4..L-1, vz at L-3..L-1
-    float4 vq0 = zero, vq1, vq2, vq3;
-    float4 pq0 = zero, pq1 = zero, pq2 = zero, pq3 = zero;
-    float4 zq0 = zero, zq1 = zero, zq2 = zero;
-    vq1 = ld4(vxi + (ptrdiff_t)(xa - 3) * (ptrdiff_t)ld);
-    vq2 = ld4(vxi + (ptrdiff_t)(xa - 2) * (ptrdiff_t)ld);
-    vq3 = ld4(vxi + (ptrdiff_t)(xa - 1) * (ptrdiff_t)ld);
-    for (int L = xa; L <= xb + 2; ++L) {
-        const int P = L - 1;
-        const ptrdiff_t colP = (ptrdiff_t)P * (ptrdiff_t)ld;
-        const float4 xc = XF ? make_float4(1.0f, la.kx, 1.0f, la.kx) : __ldg(S.xcoef + (P + S2D_GX));
-        const bool colm = XF || xc.x == 1.0f;
-        const bool pz_live = !(FAST && colm);
-        vq0 = vq1; vq1 = vq2; vq2 = vq3;
-        vq3 = ld4(vxi + (ptrdiff_t)L * (ptrdiff_t)ld);
-        const float4 vz = ld4(vzi + colP);
-        float4 pxn, pzn, dxv, dzv;
-        const float4 pn = p_update<FAST, XF>(la, S, P, xc, colm, vq0, vq1, vq2, vq3, ld4(pxi + colP),
-                                             pz_live ? ld4(pzi + colP) : zero, ld4(kap + colP), vz, pxn, pzn, dxv,
-                                             dzv);
-        const bool in_seg = P >= xa && P < xb;
-        if (in_seg && la.owner) {
-            st4(pxo + colP, pxn);
-            if (pz_live) st4(pzo + colP, pzn);
-        }
-        if (rec && in_seg) record(la, S, P, pn, slot);
-        pq0 = pq1; pq1 = pq2; pq2 = pq3; pq3 = pn;
-        zq0 = zq1; zq1 = zq2; zq2 = vz;
-        if (L < xa + 3) continue;
-        const int V = L - 3;
-        const ptrdiff_t colV = (ptrdiff_t)V * (ptrdiff_t)ld;
-        float4 vxn, vzn, dxp, dzp;
-        v_update<FAST, XF>(la, S, V, pq0, pq1, pq2, pq3, vq0, zq0, ld4(bxp + colV), ld4(bzp + colV), vxn, vzn, dxp,
-                           dzp);
-        if (la.owner) {
-            st4(vxo + colV, vxn);
-            st4(vzo + colV, vzn);
-        }
-    }
-}
-
 // The two-step task, two rows at a time (packed FP32), with the columns
 // brought in kTs2Depth - 1 ahead by per-lane asynchronous copies (16 bytes, the
 // lane's four rows) into a per-warp ring.  Iteration L consumes vx at L, px,
@@ -1173,31 +1104,6 @@ __global__ void __launch_bounds__(128, 2) step_kernel_ts2(const StepArgs *__rest
         else ts2_task<kTsAny>(a, S, strip, xa, seg_len, kt, par, lane, mem);
     }
     queue.leave();
-}
-
-// One step in the same strip layout (the last of an odd count).
-__global__ void __launch_bounds__(128, 4) step_kernel_ts1(const StepArgs *__restrict__ A, int kt_off) {
-    const StepArgs a = *A;
-    const int lane = threadIdx.x & 31;
-    const int gwarp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-    const int nwarp = (int)((gridDim.x * blockDim.x) >> 5);
-    const int kt = a.kt_base + kt_off;
-    if (kt >= a.fd_nt) return;
-    const int par = a.par0 ^ (kt_off & 1);
-    __shared__ ShotDev shot_rec[4];  // the task's shot record, one slot per warp
-    ShotDev &S = shot_rec[(threadIdx.x >> 5) & 3];
-    for (int t = gwarp; t < a.total_tasks; t += nwarp) {
-        int strip, xa, seg_len;
-        const ShotDev &G = task_of_split(a, t, strip, xa, seg_len);
-        warp_copy_shot(S, G, lane);
-        const int c = strip * S2D_TS_OUT - 8;
-        const bool zf = rows_fast(S, c, c + S2D_STRIP_ROWS - 1);
-        const bool xf = xa - 1 >= S.xfast_lo && min(S.nnx, xa + seg_len) + 1 < S.xfast_hi;
-        if (zf && xf) ts1_task<true, true>(a, S, strip, xa, seg_len, kt, par, lane);
-        else if (zf) ts1_task<true, false>(a, S, strip, xa, seg_len, kt, par, lane);
-        else if (xf) ts1_task<false, true>(a, S, strip, xa, seg_len, kt, par, lane);
-        else ts1_task<false, false>(a, S, strip, xa, seg_len, kt, par, lane);
-    }
 }
 
 // ------------------------------------------ 8th-order operator (kVariantO8)
@@ -2077,8 +1983,6 @@ int launch_step(int variant, const StepArgs *args_dev, int kt_off, int grid, int
         step_kernel_ldg<false, 4><<<grid, block, 0, (cudaStream_t)stream>>>(args_dev, kt_off);
     else if (variant == kVariantTs2)
         step_kernel_ts2<<<grid, block, smem, (cudaStream_t)stream>>>(args_dev, kt_off);
-    else if (variant == kVariantTs1)
-        step_kernel_ts1<<<grid, block, 0, (cudaStream_t)stream>>>(args_dev, kt_off);
     else if (order8_variant(variant))
         step_kernel_o8<false><<<grid, block, smem, (cudaStream_t)stream>>>(args_dev, kt_off);
     else if (variant == kVariantO8Products)
@@ -2143,7 +2047,6 @@ const void *kernel_of(int variant) {
     if (variant == kVariantLdgProducts) return (const void *)step_kernel_ldg<true, 3>;
     if (variant == kVariantLdg128) return (const void *)step_kernel_ldg<false, 4>;
     if (variant == kVariantTs2) return (const void *)step_kernel_ts2;
-    if (variant == kVariantTs1) return (const void *)step_kernel_ts1;
     if (order8_variant(variant)) return (const void *)step_kernel_o8<false>;
     if (variant == kVariantO8Products) return (const void *)step_kernel_o8<true>;
     if (variant == kVariantTma) return (const void *)step_kernel_tma<false>;
