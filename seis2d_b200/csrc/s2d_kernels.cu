@@ -1470,10 +1470,12 @@ __global__ void __launch_bounds__(128, 2) step_kernel_o8(const StepArgs *__restr
 // back, which waited twice per shot.
 __global__ void source_terms(const SourceTerm *__restrict__ src, const double *__restrict__ w, int n_inj, int fd_nt,
                              float fd_dt) {
-    const SourceTerm t = src[blockIdx.y];
+    // the shots and their pieces of 256 steps share gridDim.x, whose limit no batch reaches
+    const int per = (fd_nt + blockDim.x - 1) / blockDim.x;
+    const SourceTerm t = src[blockIdx.x / per];
     const double v = t.vp ? (double)*t.vp : 0.0;
     const double ksrc = t.vp ? __dmul_rn(__dmul_rn(v, v), (double)*t.rho) : 0.0;
-    const int kt = blockIdx.x * blockDim.x + threadIdx.x;
+    const int kt = (blockIdx.x % per) * blockDim.x + threadIdx.x;
     if (kt == 0) *t.ksrc = ksrc;
     if (kt >= fd_nt) return;
     t.amp[kt] = kt < n_inj
@@ -2027,7 +2029,7 @@ int launch_set_args(const StepArgs &v, StepArgs *args_dev, void *stream) {
 
 int launch_source_terms(const SourceTerm *src, int nshots, const double *w, int n_inj, int fd_nt, float fd_dt,
                         void *stream) {
-    source_terms<<<dim3((fd_nt + 255) / 256, nshots), 256, 0, (cudaStream_t)stream>>>(src, w, n_inj, fd_nt, fd_dt);
+    source_terms<<<(unsigned)nshots * ((fd_nt + 255) / 256), 256, 0, (cudaStream_t)stream>>>(src, w, n_inj, fd_nt, fd_dt);
     return (int)cudaGetLastError();
 }
 
