@@ -99,8 +99,8 @@ struct ResSmem {
     static constexpr int vxe = mat + 3 * NC * 32;             // [NW + 2][3][32]: vx at the warps' edges
     static constexpr int pe = vxe + (NW + 2) * 96;            // [NW + 2][3][32]: p at the warps' edges
     static constexpr int ct = pe + (NW + 2) * 96;             // [NC][4]
-    static constexpr int rt = ct + NC * 4;                    // [9][32]
-    static constexpr int rowo = rt + 9 * 32;                  // [NW][2][C][2]: rows to publish
+    static constexpr int rt = ct + NC * 4;                    // [8][32]
+    static constexpr int rowo = rt + 8 * 32;                  // [NW][2][C][2]: rows to publish
     static constexpr int rowi = rowo + NW * 4 * C + 8;        // the same: halo rows received (+8: a piece may overhang)
     static constexpr int colh = rowi + NW * 4 * C + 8;        // [kColItems][32]: halo columns received
     static constexpr int rid = colh + kColItems * 32;         // [NC] int
@@ -184,7 +184,7 @@ __device__ __forceinline__ void resident_tile(const ResArgs &a, const ResShot &r
     for (int i = L::vxe + threadIdx.x; i < L::total; i += NT) sm[i] = zero4();
     __syncthreads();
     if (w == 0) {
-        float r[9][4];
+        float r[8][4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const float4 q = __ldg(S.zcoef + (z0 + i + S2D_GZ));
@@ -193,12 +193,12 @@ __device__ __forceinline__ void resident_tile(const ResArgs &a, const ResShot &r
             r[4][i] = q.z;
             dm_coef(z0 + i, S.nnz, r[2][i], r[3][i]);
             dp_coef(z0 + i, S.nnz, r[5][i], r[6][i]);
-            // rows undamped in z: 0 for cells that carry p in px alone
-            r[7][i] = q.x == 1.0f ? 0.0f : q.x;
-            r[8][i] = q.x == 1.0f ? 0.0f : q.y;
+            // bits of pz that rows keep (none of undamped ones: the cell carries p in px alone).  A mask, not a
+            // factor 0: an overflowed derivative times 0 would leave NaN there
+            r[7][i] = q.x == 1.0f ? 0.0f : __int_as_float(-1);
         }
 #pragma unroll
-        for (int k = 0; k < 9; ++k) sm[L::rt + k * 32 + lane] = v4(pk(r[k][0], r[k][1]), pk(r[k][2], r[k][3]));
+        for (int k = 0; k < 8; ++k) sm[L::rt + k * 32 + lane] = v4(pk(r[k][0], r[k][1]), pk(r[k][2], r[k][3]));
     }
     // column coefficients, doubled for the packed operations:
     // (Dax, Kx), (Dbx, D+ c0), (D- pair), (D+ c1)
@@ -384,7 +384,7 @@ __device__ __forceinline__ void resident_tile(const ResArgs &a, const ResShot &r
             constexpr bool ZF = decltype(zf_)::value;
             const V4 kz = ZF ? kz_in : rt[1 * 32], daz = ZF ? one : rt[0];
             const V4 m0 = ZF ? A0 : rt[2 * 32], m1 = ZF ? A1 : rt[3 * 32];
-            const V4 dazm = ZF ? one : rt[7 * 32], kzm = ZF ? one : rt[8 * 32];
+            const V4 keep_pz = ZF ? one : rt[7 * 32];
             const bool r0 = lo(daz.a) == 1.0f, r1 = hi(daz.a) == 1.0f, r2 = lo(daz.b) == 1.0f, r3 = hi(daz.b) == 1.0f;
 #pragma unroll
             for (int j = 0; j < C; ++j) {
@@ -411,8 +411,7 @@ __device__ __forceinline__ void resident_tile(const ResArgs &a, const ResShot &r
                     if (PROD) keep(0, j, t);
                 } else {
                     const V4 ps = fma4(dax, px[j], (kx * k) * dx);
-                    // for kIn the z tables hold 0 on undamped rows: pz stays 0 there
-                    const V4 pn = fma4(CLS == kIn ? dazm : daz, pz[j], ((CLS == kIn ? kzm : kz) * k) * dz);
+                    const V4 pn = fma4(daz, pz[j], (kz * k) * dz);
                     if (CLS == kDamped) {
                         px[j] = ps;
                         pz[j] = pn;
@@ -425,8 +424,9 @@ __device__ __forceinline__ void resident_tile(const ResArgs &a, const ResShot &r
                         const bool u0 = und && r0, u1 = und && r1, u2 = und && r2, u3 = und && r3;
                         px[j] = v4(pk(u0 ? lo(pm.a) : lo(ps.a), u1 ? hi(pm.a) : hi(ps.a)),
                                    pk(u2 ? lo(pm.b) : lo(ps.b), u3 ? hi(pm.b) : hi(ps.b)));
-                        pz[j] = CLS == kIn ? pn : v4(pk(u0 ? 0.0f : lo(pn.a), u1 ? 0.0f : hi(pn.a)),
-                                                     pk(u2 ? 0.0f : lo(pn.b), u3 ? 0.0f : hi(pn.b)));
+                        pz[j] = CLS == kIn ? v4(pn.a & keep_pz.a, pn.b & keep_pz.b)
+                                           : v4(pk(u0 ? 0.0f : lo(pn.a), u1 ? 0.0f : hi(pn.a)),
+                                                pk(u2 ? 0.0f : lo(pn.b), u3 ? 0.0f : hi(pn.b)));
                         if (PROD) {
                             keep(0, j, v4(pk(u0 ? lo(t.a) : lo(dx.a), u1 ? hi(t.a) : hi(dx.a)),
                                           pk(u2 ? lo(t.b) : lo(dx.b), u3 ? hi(t.b) : hi(dx.b))));
