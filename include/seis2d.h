@@ -200,8 +200,11 @@ S2D_API const char *s2d_last_error(const void *ctx);
  *                 default); setting it keeps the autotuner off this choice
  *   "stages"      bulk-copy ring depth per warp, 2..16 (default 3)
  *   "seg_len"     columns per x-segment of a warp task, 0 = automatic
- *   "spin_limit"  polls of a pipeline barrier before the wait gives up and the
- *                 call returns S2D_ERR_TIMEOUT (default 2^20)
+ *   "spin_limit"  polls of a pipeline barrier, or of a neighbour in the on-chip
+ *                 loop, before the wait gives up and the call returns
+ *                 S2D_ERR_TIMEOUT (default 2^20).  Work of other streams that
+ *                 keeps blocks of the on-chip loop from starting does not count
+ *                 (that wait has a limit of its own, some 20 s)
  *   "fast_rows"   1 (default): strips clear of the z-sponge and the edge rows
  *                 use literal row coefficients; 0: every strip reads them
  *                 (same results, a check of the fast path)
@@ -222,7 +225,9 @@ S2D_API const char *s2d_last_error(const void *ctx);
  *                 wave of shots where that is the faster way (s2d_forward,
  *                 the forward steps of s2d_gradient, s2d_forward_static; not
  *                 with S2D_NO_GRAPH or "autotune" 0); 0: one launch per step.
- *                 The results are the same bits.
+ *                 The results are the same bits (once fields have overflowed
+ *                 at the grid's outer rows and columns, NaN may stand there for
+ *                 an infinity).
  *   "on_chip_shape" block shape of that loop, warps * 100 + columns per warp
  *                 (403, 404, 803 .. 810), 0 = the fastest for the grid (default)
  *   "grad_segment" s2d_gradient checkpoint interval in FD steps, 0 = the
@@ -456,7 +461,8 @@ S2D_API int s2d_run_jobcard_rank(const char *jobcard_path, int device, int nb, i
  * S2D_MODEL_ORDER8 included: this entry has neither option) returns
  * S2D_ERR_ARG.  stream: a cudaStream_t, NULL for the legacy default stream;
  * the call returns when the shot is done.  A bounded wait of the on-chip loop
- * that runs out returns S2D_ERR_TIMEOUT.  A failed device self-check (builds
+ * that runs out returns S2D_ERR_TIMEOUT; work of other streams only delays the
+ * call, up to some 20 s.  A failed device self-check (builds
  * with S2D_DEVICE_CHECKS) returns S2D_ERR_CUDA.  errbuf (optional, errlen
  * bytes) receives a message on failure.
  *

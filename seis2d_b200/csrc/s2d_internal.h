@@ -249,12 +249,13 @@ struct ResArgs {
     int dt_factor, flags;  // S2D_STEP_* bits
     int prod_kt0;          // S2D_STEP_PRODUCTS: step of the first products in ShotDev::prod
     unsigned long long *frames;  // resident_frame_bytes, zeroed before every launch
+    unsigned *started;     // blocks of the launch that have started (before the frames, set by launch_resident)
     int *err;              // device error word
     int spin_limit;        // polls before a wait counts as timed out
     int fault_step;        // test knob: step after which block 0 does not publish (-1: none)
     float one;             // 1 (set by launch_resident)
 };
-size_t resident_frame_bytes(int nw, int c, int ctas);
+size_t resident_frame_bytes(int nw, int c, int ctas);  // the count of blocks that have started, then their frames
 // One cooperative launch of `grid` blocks of nw warps with c columns each.
 int launch_resident(int nw, int c, const ResArgs &a, int grid, void *stream);
 // The i-th block shape the kernel is built for (tiles of nw*c - 6 own columns)

@@ -22,7 +22,10 @@
 //
 // Every poll is bounded (spin_limit); a block that gives up records
 // S2D_DEV_ERR_WAIT and leaves, and its neighbours follow when they see the
-// error word.  All blocks of a launch are co-resident (cooperative launch).
+// error word.  All blocks of a launch are co-resident (cooperative launch), but
+// work of other streams may let some of them start later than others: the
+// blocks count themselves in when they start and no neighbour is waited for
+// before all have (a wait of its own, kStartLimit).
 //
 // What bounds it: latency.  Of a step of 8 warps with 8 columns (1.9 us of
 // 4.05 at 1.965 GHz are arithmetic, the FP32 pipe busy for 1.0 of them) about
@@ -110,6 +113,30 @@ struct ResSmem {
 };
 
 constexpr unsigned kNoPiece = 0xffffffffu;
+
+// Bytes before the frames, for the count of started blocks: whole lines, so that
+// a warp's 512 bytes of pieces stay four of them (with 16 bytes, five: 5.3
+// against 5.5 us per step of 1080 x 1080).
+constexpr size_t kFramesHead = 512;
+// Polls (1 us or more each) for all blocks of a launch to start.  Whatever else
+// runs on the GPU delays them by its own length; 2^24 are some 20 s.
+constexpr int kStartLimit = 1 << 24;
+__device__ __forceinline__ unsigned ld_count(const unsigned *p) {
+    unsigned v;
+    asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ bool all_started(const ResArgs &a) {
+    for (int t = 0; ld_count(a.started) < gridDim.x; ++t) {
+        if (t >= kStartLimit) {
+            atomicOr(a.err, S2D_DEV_ERR_WAIT);
+            return false;
+        }
+        if ((t & 255) == 255 && *reinterpret_cast<volatile int *>(a.err) != 0) return false;
+        __nanosleep(500);
+    }
+    return true;
+}
 
 // What the columns of a warp are: all in the shot's fast columns (dampings 1,
 // literal operator pairs); all damped, with literal pairs; anything.
@@ -658,11 +685,16 @@ __global__ void __launch_bounds__(NW * 32, 1) resident_kernel(const ResArgs a) {
     int g = 0;
     while (g + 1 < a.nrs && __ldg(&a.rs[g + 1].cta0) <= (int)blockIdx.x) ++g;
     const ResShot rs = a.rs[g];
-    if (threadIdx.x == 0) s_rec = s_fail = 0;
+    if (threadIdx.x == 0) {
+        atomicAdd(a.started, 1u);
+        s_rec = 0;
+        s_fail = !all_started(a);
+    }
     if (threadIdx.x < sizeof(ShotDev) / 8)
         reinterpret_cast<unsigned long long *>(&S)[threadIdx.x] =
             reinterpret_cast<const unsigned long long *>(a.shots + rs.shot)[threadIdx.x];
     __syncthreads();
+    if (s_fail) return;
     const int b = (int)blockIdx.x - rs.cta0;
     const int cz = b % rs.ncz, cx = b / rs.ncz;
     const int zc = cz * S2D_STRIP_OUT - 4;
@@ -688,6 +720,8 @@ int launch_c(const ResArgs &a, int grid, cudaStream_t st) {
     if (e != cudaSuccess) return (int)e;
     ResArgs v = a;
     v.one = 1.0f;
+    v.started = reinterpret_cast<unsigned *>(v.frames);
+    v.frames += kFramesHead / sizeof(*v.frames);
     void *args[] = {&v};
     return (int)cudaLaunchCooperativeKernel(k, dim3(grid), dim3(NW * 32), args, ResSmem<NW, C>::bytes, st);
 }
@@ -701,7 +735,7 @@ int launch_c(const ResArgs &a, int grid, cudaStream_t st) {
     X(8, 9, 4.4) X(8, 10, 5.0)
 
 size_t resident_frame_bytes(int nw, int c, int ctas) {
-    return (size_t)2 * ctas * (kColPieces * 32 + nw * row_pieces(c)) * 16;
+    return kFramesHead + (size_t)2 * ctas * (kColPieces * 32 + nw * row_pieces(c)) * 16;
 }
 
 int launch_resident(int nw, int c, const ResArgs &a, int grid, void *stream) {
