@@ -285,6 +285,7 @@ struct Ctx {
     Arena arena;  // outlives every buffer below
     int device = 0;
     int sm_count = 0;
+    int cooperative = 0;  // the device takes cooperative launches
     // tuning options (s2d_set_option)
     // explicit launch configuration, used when autotuning is off
     int opt_variant = kVariantLdgPf4;
@@ -403,8 +404,9 @@ constexpr SplitRule kSplitAdj8 = {S2D_TS_OUT, 8, 0, kAdj8ColLo, kAdj8ColHi, 13, 
 // several rounds, whose warps even out: measured about 1.0 us per column of the
 // two-step kernel against 0.61.  2101 x 1101, 3 shots: one round of 79 columns
 // 155 Gcell/s, two of 35 178; 3301 x 1301, 6 shots: 195 and 258 (63); 1301 x
-// 501, 8 shots, the other way: 119 and 105.
-void split_group(GroupDev &g, const ShotDev &d, int shots, double resident_warps, bool alone, int forced,
+// 501, 8 shots, the other way: 119 and 105.  Returns that estimate, in columns
+// of an interior task (0 with a forced length).
+double split_group(GroupDev &g, const ShotDev &d, int shots, double resident_warps, bool alone, int forced,
                  const SplitRule &R) {
     const double kRows = R.rows, kCols = R.cols;
     const int kHalo = R.halo;
@@ -435,7 +437,7 @@ void split_group(GroupDev &g, const ShotDev &d, int shots, double resident_warps
     };
     if (forced > 0) {
         cut(forced);
-        return;
+        return 0;
     }
     int best = 0;
     double best_cost = 0;
@@ -452,6 +454,7 @@ void split_group(GroupDev &g, const ShotDev &d, int shots, double resident_warps
         }
     }
     cut(best);
+    return best_cost;
 }
 
 int build_coef(Ctx *c, Model &m, float fd_dt) {
@@ -779,27 +782,51 @@ int run_loop(Ctx *c, Batch &b, const LaunchCfg &lc, StepArgs args, int kt_begin,
     return S2D_OK;
 }
 
-// Whether the on-chip loop takes the shots of group g of the batch: its grid
-// fits the chip and the loop's estimate beats the per-step kernels', which
-// take about 7.4 us per step at least (launch and latency of one short task)
-// and run at about 100 Gcell/s (a batch) or 52 (single 1301 x 501 shots, one
-// after another).
-bool on_chip_group(const Ctx *c, const Batch &b, size_t g, ResPlan *pl) {
-    const int n = b.groups[g].nshots;
-    if (!resident_plan(c->sm_count, b.group_nnx[g], b.group_nnz[g], n, b.plain, c->opt_chip_shape, pl)) return false;
-    if (c->opt_chip_shape) return true;
-    const double cells = (double)b.group_nnx[g] * b.group_nnz[g];
-    const double us = b.plain ? n * std::max(7.4, cells / 0.6e5) : std::max(7.4, n * cells / 1.0e5);
-    return pl->step_us < 0.9 * us;
+// Estimated time, us, of one FD step of group g's shots by the kernels with a
+// launch per step or two.  The two-step kernel takes 0.32 us per column of
+// split_group's estimate (0.28 to 0.38 on grids of 551 x 327 to 1080 x 1080, 4
+// to 64 shots: 29 at 4 shots of 1080 x 1080 for 29 measured, 159 at 32 for 151,
+// 290 at 64 for 266; 120 at 32 of 1301 x 501 for 133), a launch 7.4 us a step at
+// least; the kernels that leave the step products 100 Gcell/s at best (64 at 8
+// shots of 701 x 401, 80 at 8 of 1301 x 501, 105 at 32 of 1080 x 1080).
+double launched_us(Ctx *c, const Batch &b, size_t g, bool products) {
+    GroupDev t = b.groups[g];
+    const int n = b.plain ? 1 : t.nshots, runs = b.plain ? t.nshots : 1;
+    if (products) return runs * std::max(7.4, n * (double)b.group_nnx[g] * b.group_nnz[g] / 1.0e5);
+    LaunchCfg full;
+    if (launch_config(c, 1L << 40, &full, kVariantTs2, 128, 0)) return 0;
+    t.nstrips = num_strips_ts(b.group_nnz[g]);
+    const double cost =
+        split_group(t, b.shot_dev[b.table[t.shot0]], n, (double)full.grid * (full.block / 32), true, 0, kSplitTs2);
+    return runs * std::max(7.4, 0.32 * cost);
 }
 
-// Decide which groups of the batch the on-chip loop runs in this call, when
-// it has at least `nsteps` >= 8 of them to run (a launch loads and writes the
-// whole state once).  Returns how many.
+// Whether the on-chip loop takes the shots of group g of the batch: its grid
+// fits the chip and the loop's estimate beats the launches'.  Large grids run
+// there one shot after another, whatever their number, while the two-step kernel
+// gains with it.  us per step, on chip and launched: 1080 x 1080, 8 shots 44 and
+// 52, 16 shots 86 and 85, 32 shots 173 and 151, 64 shots 348 and 266; 1301 x 501,
+// 32 shots 113 and 133, 64 shots 226 and 217; 701 x 401, 64 shots 108 and 115.
+// With `products` (1.2 to 1.43 times the loop's time): 1080 x 1080, 32 shots 240
+// and 355.
+bool on_chip_group(Ctx *c, const Batch &b, size_t g, ResPlan *pl, bool products = false) {
+    if (!resident_plan(c->sm_count, b.group_nnx[g], b.group_nnz[g], b.groups[g].nshots, b.plain, c->opt_chip_shape, pl))
+        return false;
+    return c->opt_chip_shape || pl->step_us * (products ? 1.35 : 1.0) < launched_us(c, b, g, products);
+}
+
+// Whether a run of `nsteps` steps may use the on-chip loop at all (a launch
+// loads and writes the whole state once: 8 steps or more).
+bool on_chip_allowed(const Ctx *c, const Batch &b, int nsteps, bool use_graph) {
+    return c->opt_on_chip && c->cooperative && c->opt_autotune && use_graph && !b.order8 && nsteps >= 8;
+}
+
+// Decide which groups of the batch the on-chip loop runs in a call of `nsteps`
+// steps.  Returns how many.
 int choose_on_chip(Ctx *c, Batch &b, int nsteps, bool use_graph, std::vector<ResPlan> *plans) {
     plans->assign(b.groups.size(), ResPlan());
     b.chip.assign(b.groups.size(), 0);
-    if (!c->opt_on_chip || !c->opt_autotune || !use_graph || b.order8 || nsteps < 8) return 0;
+    if (!on_chip_allowed(c, b, nsteps, use_graph)) return 0;
     int n = 0;
     for (size_t g = 0; g < b.groups.size(); ++g) n += b.chip[g] = on_chip_group(c, b, g, &(*plans)[g]);
     return n;
@@ -1424,6 +1451,7 @@ int s2d_create(void **ctx, int device) {
     if (e == cudaSuccess) e = cudaEventCreate(&c->ev0);
     if (e == cudaSuccess) e = cudaEventCreate(&c->ev1);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&c->sm_count, cudaDevAttrMultiProcessorCount, device);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&c->cooperative, cudaDevAttrCooperativeLaunch, device);
     if (e == cudaSuccess) e = c->dev_err.alloc(c->arena, sizeof(int));
     if (e == cudaSuccess) e = c->queue_d.alloc(c->arena, 2 * sizeof(int));
     if (e == cudaSuccess) e = cudaMemset(c->queue_d.p, 0, 2 * sizeof(int));
@@ -1974,11 +2002,13 @@ extern "C" int s2d_gradient(void *ctx, const s2d_shot *shots, int nshots, const 
         int e = phase_mark(c, g, kPhaseSweep);
         if (e) return e;
     }
-    // the forward steps run on chip where a forward would (with the products the
-    // gain is larger: 1301 x 501, 8 shots 65 -> 39 us per step, without 50 -> 28)
-    ResPlan sweep_plan;
-    const bool sweep_on_chip = c->opt_on_chip && c->opt_autotune && use_graph && !b.order8 && C >= 8 &&
-                               on_chip_group(c, b, 0, &sweep_plan);
+    // the sweep's steps run on chip where a forward's would, those that keep their
+    // products where that is faster by itself (their gain is larger: 1301 x 501, 8
+    // shots 65 -> 39 us per step, without 50 -> 28)
+    ResPlan sweep_plan, prod_plan;
+    const bool may = on_chip_allowed(c, b, C, use_graph);
+    const bool sweep_on_chip = may && on_chip_group(c, b, 0, &sweep_plan);
+    const bool prod_on_chip = may && on_chip_group(c, b, 0, &prod_plan, true);
     // ---- forward sweep, saving the state at each segment start ----
     auto save_ckpt = [&](int j) -> int {
         const int par = b.cur;
@@ -1998,8 +2028,8 @@ extern "C" int s2d_gradient(void *ctx, const s2d_shot *shots, int nshots, const 
         return e;
     };
     auto run_products = [&](int k0, int n, int flags) -> int {
-        if (sweep_on_chip && n >= 2) {
-            int e = run_resident(c, b, sweep_plan, 0, nshots, k0, n, b.cur, b.cur ^ (n & 1), &launches, flags);
+        if (prod_on_chip && n >= 2) {
+            int e = run_resident(c, b, prod_plan, 0, nshots, k0, n, b.cur, b.cur ^ (n & 1), &launches, flags);
             b.cur ^= n & 1;
             return e;
         }

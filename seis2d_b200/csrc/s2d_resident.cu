@@ -731,8 +731,8 @@ int launch_c(const ResArgs &a, int grid, cudaStream_t st) {
 // Block shapes (warps, columns per warp) and the measured time of one step of
 // such a tile, us (exchange included, all SMs busy).
 #define S2D_RES_SHAPES(X)                                                                                        \
-    X(4, 3, 2.1) X(4, 4, 2.25) X(8, 3, 2.25) X(8, 4, 2.5) X(8, 5, 2.95) X(8, 6, 3.2) X(8, 7, 3.5) X(8, 8, 4.05) \
-    X(8, 9, 4.4) X(8, 10, 5.0)
+    X(4, 3, 2.3) X(4, 4, 2.4) X(8, 3, 2.35) X(8, 4, 2.55) X(8, 5, 2.95) X(8, 6, 3.3) X(8, 7, 3.55) X(8, 8, 4.35) \
+    X(8, 9, 4.8) X(8, 10, 5.4)
 
 size_t resident_frame_bytes(int nw, int c, int ctas) {
     return kFramesHead + (size_t)2 * ctas * (kColPieces * 32 + nw * row_pieces(c)) * 16;
