@@ -286,6 +286,7 @@ struct Ctx {
     int device = 0;
     int sm_count = 0;
     int cooperative = 0;  // the device takes cooperative launches
+    int ts2_warps = 0;    // resident warps of the two-step kernel (0: not asked for yet)
     // tuning options (s2d_set_option)
     // explicit launch configuration, used when autotuning is off
     int opt_variant = kVariantLdgPf4;
@@ -526,13 +527,14 @@ int launch_config(Ctx *c, long max_tasks, LaunchCfg *out, int variant, int block
 }
 
 // Key of a batch's shape for the autotuner: run mode and, per model group,
-// padded grid and shot count.
+// padded grid, shot count and whether it runs on chip.
 std::vector<long> tune_key(const Ctx *c, const Batch &b) {
-    std::vector<long> k = {b.plain ? 1L : 0L, (long)c->sm_count, b.order8 ? 8L : 4L, b.all_chip() ? 1L : 0L};
+    std::vector<long> k = {b.plain ? 1L : 0L, (long)c->sm_count, b.order8 ? 8L : 4L};
     for (size_t g = 0; g < b.groups.size(); ++g) {
         k.push_back(b.group_nnx[g]);
         k.push_back(b.group_nnz[g]);
         k.push_back(b.groups[g].nshots);
+        k.push_back(b.chip[g]);
     }
     return k;
 }
@@ -558,14 +560,12 @@ int default_variant(const Batch &b, int nsteps) {
 // tune: the options when autotuning is off, else the tuned result for the
 // batch's shape (it holds for runs that its kernel can make whole launches of),
 // else the built-in default.
-int base_config(Ctx *c, const Batch &b, int nsteps, LaunchCfg *out, bool *tuned = nullptr) {
-    if (tuned) *tuned = false;
+int base_config(Ctx *c, const Batch &b, int nsteps, LaunchCfg *out) {
     // 8th-order batches run the 8th-order kernel whatever the options say
     if (b.order8 && !c->opt_autotune) return launch_config(c, b.max_tasks, out, c->opt_variant8, 128, 0);
     if (!c->opt_autotune) return launch_config(c, b.max_tasks, out, c->opt_variant, c->opt_block, c->opt_stages);
     auto it = c->tuned.find(tune_key(c, b));
     if (it != c->tuned.end() && nsteps >= steps_per_launch(it->second[0])) {
-        if (tuned) *tuned = true;
         int e = launch_config(c, b.max_tasks, out, it->second[0], it->second[1], it->second[2]);
         out->order = c->order_fixed ? -1 : it->second[3];
         return e;
@@ -789,16 +789,19 @@ int run_loop(Ctx *c, Batch &b, const LaunchCfg &lc, StepArgs args, int kt_begin,
 // 290 at 64 for 266; 120 at 32 of 1301 x 501 for 133), a launch 7.4 us a step at
 // least; the kernels that leave the step products 100 Gcell/s at best (64 at 8
 // shots of 701 x 401, 80 at 8 of 1301 x 501, 105 at 32 of 1080 x 1080).
+constexpr double kLaunchedStepUs = 7.4;
 double launched_us(Ctx *c, const Batch &b, size_t g, bool products) {
     GroupDev t = b.groups[g];
     const int n = b.plain ? 1 : t.nshots, runs = b.plain ? t.nshots : 1;
-    if (products) return runs * std::max(7.4, n * (double)b.group_nnx[g] * b.group_nnz[g] / 1.0e5);
-    LaunchCfg full;
-    if (launch_config(c, 1L << 40, &full, kVariantTs2, 128, 0)) return 0;
+    if (products) return runs * std::max(kLaunchedStepUs, n * (double)b.group_nnx[g] * b.group_nnz[g] / 1.0e5);
+    if (!c->ts2_warps) {  // the device's, asked for once
+        LaunchCfg full;
+        if (launch_config(c, 1L << 40, &full, kVariantTs2, 128, 0)) return 0;
+        c->ts2_warps = full.grid * (full.block / 32);
+    }
     t.nstrips = num_strips_ts(b.group_nnz[g]);
-    const double cost =
-        split_group(t, b.shot_dev[b.table[t.shot0]], n, (double)full.grid * (full.block / 32), true, 0, kSplitTs2);
-    return runs * std::max(7.4, 0.32 * cost);
+    const double cost = split_group(t, b.shot_dev[b.table[t.shot0]], n, c->ts2_warps, true, 0, kSplitTs2);
+    return runs * std::max(kLaunchedStepUs, 0.32 * cost);
 }
 
 // Whether the on-chip loop takes the shots of group g of the batch: its grid
@@ -812,7 +815,9 @@ double launched_us(Ctx *c, const Batch &b, size_t g, bool products) {
 bool on_chip_group(Ctx *c, const Batch &b, size_t g, ResPlan *pl, bool products = false) {
     if (!resident_plan(c->sm_count, b.group_nnx[g], b.group_nnz[g], b.groups[g].nshots, b.plain, c->opt_chip_shape, pl))
         return false;
-    return c->opt_chip_shape || pl->step_us * (products ? 1.35 : 1.0) < launched_us(c, b, g, products);
+    const double us = pl->step_us * (products ? 1.35 : 1.0);
+    return c->opt_chip_shape || us < (b.plain ? b.groups[g].nshots : 1) * kLaunchedStepUs ||
+           us < launched_us(c, b, g, products);
 }
 
 // Whether a run of `nsteps` steps may use the on-chip loop at all (a launch
@@ -1591,37 +1596,30 @@ int s2d_forward(void *ctx, const s2d_shot *shots, int nshots, const s2d_wave *wa
     const bool use_graph = !(flags & S2D_NO_GRAPH);
     int launches = 0;
     bool graph_used = false;
-    bool tuned = false;
     int tuned_now = 0;
     LaunchCfg lc;
-    auto configure = [&]() -> int {
-        int e = base_config(c, b, nsteps, &lc, &tuned);
-        const int order = lc.order;
-        if (!e) e = layout_groups(c, b, lc);
-        if (!e) e = launch_config(c, b.max_tasks, &lc, lc.variant, lc.block, lc.stages);
-        if (!e && tma_variant(lc.variant)) e = build_tmaps(c, b);
-        lc.order = order;
-        return e;
-    };
     // Batched runs of a shape with no tuned configuration yet tune on their
     // first steps when the call has room for the trials and a run after them.
-    // A batch that runs on chip altogether needs no trials: the default is
-    // recorded for the few steps that a later call may leave to the per-step
-    // kernels.
+    // The trials are steps of the groups that the per-step kernels run; a batch
+    // that runs on chip altogether needs none and counts as settled once.
     const int tune_len = b.order8 ? kTuneStepsO8 : kTuneSteps;
     const bool room = c->opt_autotune && !b.plain && nsteps >= 2 * tune_len;
     std::vector<ResPlan> plans;
-    int n_chip = choose_on_chip(c, b, nsteps, use_graph, &plans);
+    const int n_chip = choose_on_chip(c, b, nsteps, use_graph, &plans);
     if (room && b.all_chip() && !c->tuned.count(tune_key(c, b))) {
         const LaunchCfg d;
         c->tuned[tune_key(c, b)] = {d.variant, d.block, d.stages, c->opt_order};
         tuned_now = 1;
     }
     const bool tune = room && !b.all_chip() && !c->tuned.count(tune_key(c, b));
-    if (tune) b.chip.assign(b.groups.size(), 0);  // the trials are steps of every shot
     {
-        int e = configure();
+        int e = base_config(c, b, nsteps, &lc);
+        const int order = lc.order;
+        if (!e) e = layout_groups(c, b, lc);
+        if (!e) e = launch_config(c, b.max_tasks, &lc, lc.variant, lc.block, lc.stages);
+        if (!e && tma_variant(lc.variant)) e = build_tmaps(c, b);
         if (e) return e;
+        lc.order = order;
     }
     CK(cudaEventRecord(c->ev0, c->stream));
     StepArgs a{};
@@ -1630,7 +1628,8 @@ int s2d_forward(void *ctx, const s2d_shot *shots, int nshots, const s2d_wave *wa
     a.fd_nt = rs.fd_nt;
     a.tmaps = b.tmaps_d.p;
     a.tmap_mat0 = b.nshots;
-    int kt_run = kt_begin;  // first step left after tuning
+    const int cur0 = b.cur;
+    int kt_run = kt_begin;  // first step that the trials left to the per-step kernels
     if (tune) {
         a.groups = b.groups_d.as<GroupDev>();
         a.ngroups = (int)b.groups.size();
@@ -1639,24 +1638,20 @@ int s2d_forward(void *ctx, const s2d_shot *shots, int nshots, const s2d_wave *wa
         if (e) return e;
         kt_run += used;
         tuned_now = 1;
-        n_chip = choose_on_chip(c, b, kt_end - kt_run, use_graph, &plans);
-        if (n_chip) e = configure();
-        if (e) return e;
     }
-    const int run = kt_end - kt_run;  // steps left after tuning
-    const int cur0 = b.cur, cur1 = end_buffer(lc, cur0, run);
+    const int cur1 = end_buffer(lc, b.cur, kt_end - kt_run);
     if (b.plain) {
         // every shot advances from the same buffer through the same launches
         for (int s = 0; s < nshots; ++s) {
             int e;
             if (b.chip[s]) {
-                e = run_resident(c, b, plans[s], s, 1, kt_run, run, cur0, cur1, &launches);
+                e = run_resident(c, b, plans[s], s, 1, kt_begin, nsteps, cur0, cur1, &launches);
             } else {
                 a.groups = b.groups_d.as<GroupDev>() + s;
                 a.ngroups = 1;
                 a.total_tasks = plain_tasks(b, s);
                 b.cur = cur0;
-                e = run_loop(c, b, lc, a, kt_run, run, use_graph, &launches, &graph_used);
+                e = run_loop(c, b, lc, a, kt_begin, nsteps, use_graph, &launches, &graph_used);
             }
             if (e) return e;
         }
@@ -1665,10 +1660,11 @@ int s2d_forward(void *ctx, const s2d_shot *shots, int nshots, const s2d_wave *wa
         a.ngroups = (int)b.groups.size();
         a.total_tasks = batch_tasks(b);
         int e = S2D_OK;
-        if (n_chip < (int)b.groups.size()) e = run_loop(c, b, lc, a, kt_run, run, use_graph, &launches, &graph_used);
+        if (n_chip < (int)b.groups.size())
+            e = run_loop(c, b, lc, a, kt_run, kt_end - kt_run, use_graph, &launches, &graph_used);
         for (size_t g = 0; g < b.groups.size() && !e; ++g)
             if (b.chip[g])
-                e = run_resident(c, b, plans[g], b.groups[g].shot0, b.groups[g].nshots, kt_run, run, cur0, cur1,
+                e = run_resident(c, b, plans[g], b.groups[g].shot0, b.groups[g].nshots, kt_begin, nsteps, cur0, cur1,
                                  &launches);
         if (e) return e;
     }
@@ -1720,8 +1716,8 @@ int s2d_forward(void *ctx, const s2d_shot *shots, int nshots, const s2d_wave *wa
         // two-step kernel; the autotuner's trial steps are counted as one-step)
         const int passes = steps_per_launch(lc.variant) == 2 ? (kt_end - kt_run + 1) / 2 + (kt_run - kt_begin)
                                                              : nsteps;
-        // (one pass per call for the on-chip loop, after the trial steps)
-        stats->alg_bytes = bytes * passes + chip_bytes * (1 + kt_run - kt_begin);
+        // (one pass per call for the on-chip loop)
+        stats->alg_bytes = bytes * passes + chip_bytes;
         stats->gcells_per_s = ms > 0 ? stats->cell_updates / (ms * 1e6) : 0.0;
         stats->kernel_launches = launches;
         stats->graph_used = graph_used ? 1 : 0;

@@ -59,3 +59,27 @@ def test_a_sweep_by_launches_and_products_on_chip():
     # shots add to the gradient in any order: n * steps terms, each sum rounded to 2^-24
     for a, b in zip(got[0][1:3], got[1][1:3]):
         assert np.linalg.norm(a - b) <= n * steps * 2.0 ** -24 * np.linalg.norm(b)
+
+
+def test_trials_beside_groups_on_chip():
+    """Two grids on chip and one launched: the call that runs the trials, one
+    that finds them, and one cut into pieces record the same bits."""
+    import torch
+    from seis2d_b200 import Context, Wave
+    steps, out = 130, []
+    wave = Wave((steps - 0.5) * 0.001, 0.001, 0.001001, 25.0)
+    for on in (1, 0):
+        with Context(0) as c:
+            c.set_option("on_chip", on)
+            shots = [s for g in ((200, 180), (2304, 800), (330, 390)) for s in _setup(c, *g, 2)]
+            size = sum(s.rec.shape[0] for s in shots) * steps
+            for cuts in ((), (), (85,), (3, 90), (9, 8)):
+                buf = torch.zeros(size, device="cuda")
+                k = 0
+                for n in (*cuts, 0):
+                    c.forward(shots, wave, kt_begin=k, kt_count=n, out=buf)
+                    k += n
+                out.append(buf)
+            assert c.last_stats.autotuned == 0
+    assert out[0].abs().max() > 0
+    assert all(torch.equal(out[0], o) for o in out[1:])
