@@ -161,6 +161,7 @@ struct DevBuf {
             a.trim(0);
         }
         if (e != cudaSuccess) {
+            cudaGetLastError();  // not the next launch's
             p = nullptr;
             return e;
         }
@@ -1919,47 +1920,64 @@ extern "C" int s2d_gradient(void *ctx, const s2d_shot *shots, int nshots, const 
         if (e) return e;
         adj_src = static_cast<float *>(p);
     }
-    // checkpoint interval: the longest whose products and checkpoints fit in
-    // free memory (pooled buffers count as free: the pool releases itself when
-    // an allocation fails)
-    size_t free_b = 0, total_b = 0;
-    CK(cudaMemGetInfo(&free_b, &total_b));
-    const double budget = 0.85 * ((double)free_b + (double)c->pool.held()) - 4.0 * fb - 64e6;
+    // checkpoint interval: the longest whose products and checkpoints fit in free
+    // memory.  Pooled buffers count as free at first: they are taken again, or
+    // given back when an allocation fails.  Those in a chunk that holds a buffer
+    // in use stay with the context, so where memory runs out all the same, the
+    // pool is emptied and the free memory measured anew.
     const double per_step_all = (double)nshots * 4.0 * fb;
     auto need = [&](int C) { return per_step_all * (C + (rs.fd_nt + C - 1) / C - 1); };
-    int C = -1;
-    const int cmax = c->opt_grad_segment > 0 ? std::min(rs.fd_nt, c->opt_grad_segment) : rs.fd_nt;
-    for (int t = cmax; t >= 1; --t)
-        if (need(t) <= budget) {
-            C = t;
-            break;
+    std::vector<float *> prod(nshots), ckpt(nshots);
+    auto take_segment = [&](int C) -> int {
+        const int nseg = (rs.fd_nt + C - 1) / C;
+        for (int s = 0; s < nshots; ++s) {
+            void *p;
+            int e = grad_alloc(c, g, (size_t)C * 4 * fb, &p);
+            if (e) return e;
+            // Not cleared: what the forward never writes (ghost cells, the second
+            // slot of cells that carry one pressure) reaches no cell of the adjoint,
+            // whose kernels select and do not multiply by zero there.  Clearing the
+            // products of 8 shots of 1201 x 401, 100 steps, took 0.7 of 86.4 ms.
+            prod[s] = static_cast<float *>(p);
+            ckpt[s] = nullptr;
+            if (nseg > 1) {
+                e = grad_alloc(c, g, (size_t)(nseg - 1) * 4 * fb, &p);
+                if (e) return e;
+                ckpt[s] = static_cast<float *>(p);
+            }
         }
-    if (C < 1) {
-        int best = 1;
-        for (int t = 1; t <= rs.fd_nt; ++t)
-            if (need(t) < need(best)) best = t;
-        return fail(c, S2D_ERR_NOMEM,
-                    "gradient of %d shots needs at least %.1f GB for checkpoints and step products, %.1f GB "
-                    "available; use fewer shots per call",
-                    nshots, need(best) / 1e9, budget / 1e9);
+        return S2D_OK;
+    };
+    const size_t held_bufs = g.bufs.size();
+    int C = 0;
+    for (int pass = 0; pass < 2; ++pass) {
+        if (pass) {
+            g.bufs.resize(held_bufs);
+            c->pool.free.clear();
+            c->arena.trim(0);
+        }
+        size_t free_b = 0, total_b = 0;
+        CK(cudaMemGetInfo(&free_b, &total_b));
+        const double budget = 0.85 * ((double)free_b + (double)c->pool.held()) - 4.0 * fb - 64e6;
+        C = c->opt_grad_segment > 0 ? std::min(rs.fd_nt, c->opt_grad_segment) : rs.fd_nt;
+        while (C >= 1 && need(C) > budget) --C;
+        int e = S2D_ERR_NOMEM;
+        if (C >= 1) {
+            e = take_segment(C);
+        } else if (pass) {
+            int best = 1;
+            for (int t = 1; t <= rs.fd_nt; ++t)
+                if (need(t) < need(best)) best = t;
+            fail(c, e,
+                 "gradient of %d shots needs at least %.1f GB for checkpoints and step products, %.1f GB "
+                 "available; use fewer shots per call",
+                 nshots, need(best) / 1e9, budget / 1e9);
+        }
+        if (!e) break;
+        if (pass || e != S2D_ERR_NOMEM) return e;
     }
     const int nseg = (rs.fd_nt + C - 1) / C;
-    std::vector<float *> prod(nshots), ckpt(nshots);
     for (int s = 0; s < nshots; ++s) {
-        void *p;
-        int e = grad_alloc(c, g, (size_t)C * 4 * fb, &p);
-        if (e) return e;
-        // Not cleared: what the forward never writes (ghost cells, the second
-        // slot of cells that carry one pressure) reaches no cell of the adjoint,
-        // whose kernels select and do not multiply by zero there.  Clearing the
-        // products of 8 shots of 1201 x 401, 100 steps, took 0.7 of 86.4 ms.
-        prod[s] = static_cast<float *>(p);
-        ckpt[s] = nullptr;
-        if (nseg > 1) {
-            e = grad_alloc(c, g, (size_t)(nseg - 1) * 4 * fb, &p);
-            if (e) return e;
-            ckpt[s] = static_cast<float *>(p);
-        }
         adj[s].prod = prod[s];
         adj[s].nprod = (size_t)C * 4 * F;
         adj[s].seis = adj_src + b.shots[s].seis_off;
