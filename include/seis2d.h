@@ -146,7 +146,11 @@ typedef struct {
 S2D_API int s2d_abi_version(void);
 
 /* Create a context on CUDA device `device`.  No counterpart in the reference
- * (its backends use globals and cudaSetDevice(0), src/src_gpu/gpumodelling.cu:285). */
+ * (its backends use globals and cudaSetDevice(0), src/src_gpu/gpumodelling.cu:285).
+ * A context holds 32 MB of device memory from its creation (less where less is
+ * free) and keeps up to 256 MB that its models and batches no longer use, and
+ * the last batch's buffers, for the next; an allocation that fails gives back
+ * what it can and tries again. */
 S2D_API int s2d_create(void **ctx, int device);
 
 /* Free every device buffer and graph of the context. */

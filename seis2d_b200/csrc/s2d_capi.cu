@@ -36,13 +36,19 @@ namespace {
 // the tables of a batch in one upload, below).  A piece that comes back is
 // reused at once, so releasing one waits for the context's stream, as cudaFree
 // waits for the device.  Chunks in no use go back above kMaxIdle bytes of them,
-// when an allocation fails, and with the context.
+// when an allocation fails, and with the context.  Pieces that last (models, the
+// context's own) and those of batches lie in chunks of their own, or a model
+// would keep the chunks of a whole batch; all share the first chunk, which a
+// context of any size holds.
 struct Arena {
     static constexpr size_t kAlign = 512, kMaxPiece = (size_t)64 << 20, kMinChunk = (size_t)32 << 20,
                             kMaxChunk = (size_t)256 << 20, kMaxIdle = (size_t)256 << 20;
+    enum Kind { kShared, kLasting, kBatch };
     struct Chunk {
         char *p;
         size_t size;
+        Kind kind;
+        bool takes(Kind k) const { return kind == kShared || kind == k; }
         std::map<size_t, size_t> free;  // offset -> bytes
     };
     std::list<Chunk> chunks;
@@ -69,8 +75,9 @@ struct Arena {
             }
         }
     }
-    cudaError_t grow(size_t n) {
+    cudaError_t grow(size_t n, Kind kind) {
         Chunk c;
+        c.kind = chunks.empty() ? kShared : kind;
         c.size = n > kMinChunk / 4 ? n : kMinChunk;
         cudaError_t e = cudaMalloc((void **)&c.p, c.size);
         if (e == cudaErrorMemoryAllocation && c.size > n) {  // memory is short: no more than asked for
@@ -83,26 +90,26 @@ struct Arena {
         chunks.push_back(std::move(c));
         return cudaSuccess;
     }
-    bool fits(size_t n) const {
+    bool fits(size_t n, Kind kind) const {
         for (auto &c : chunks)
             for (auto &f : c.free)
-                if (f.second >= n) return true;
+                if (c.takes(kind) && f.second >= n) return true;
         return false;
     }
     // About to take pieces of these sizes: one chunk for those that come from
     // chunks (a failure shows when they are taken).
-    void expect(const std::vector<size_t> &pieces) {
+    void expect(const std::vector<size_t> &pieces, Kind kind) {
         size_t n = 0;
         for (size_t b : pieces)
             if (b <= kMaxPiece) n += rounded(b);
-        if (n == 0 || n > kMaxChunk || fits(n)) return;
-        if (grow(n) != cudaSuccess) cudaGetLastError();
+        if (n == 0 || n > kMaxChunk || fits(n, kind)) return;
+        if (grow(n, kind) != cudaSuccess) cudaGetLastError();
     }
-    cudaError_t take(size_t n, void **p, Chunk **from) {
+    cudaError_t take(size_t n, Kind kind, void **p, Chunk **from) {
         for (int pass = 0; pass < 2; ++pass) {
             for (auto &c : chunks)
                 for (auto f = c.free.begin(); f != c.free.end(); ++f)
-                    if (f->second >= n) {
+                    if (c.takes(kind) && f->second >= n) {
                         *p = c.p + f->first;
                         *from = &c;
                         const size_t at = f->first, left = f->second - n;
@@ -111,7 +118,7 @@ struct Arena {
                         return cudaSuccess;
                     }
             if (pass == 0) {
-                cudaError_t e = grow(n);
+                cudaError_t e = grow(n, kind);
                 if (e != cudaSuccess) return e;
             }
         }
@@ -150,12 +157,12 @@ struct DevBuf {
         bytes = 0;
         arena = nullptr;
     }
-    cudaError_t alloc(Arena &a, size_t n) {
+    cudaError_t alloc(Arena &a, size_t n, Arena::Kind kind = Arena::kBatch) {
         reset();
         cudaError_t e = cudaSuccess;
         const bool piece = n <= Arena::kMaxPiece;
         for (int pass = 0; pass < 2; ++pass) {
-            e = piece ? a.take(Arena::rounded(n), &p, &chunk) : cudaMalloc(&p, n);
+            e = piece ? a.take(Arena::rounded(n), kind, &p, &chunk) : cudaMalloc(&p, n);
             if (e != cudaErrorMemoryAllocation || pass) break;
             cudaGetLastError();
             a.trim(0);
@@ -472,8 +479,8 @@ int build_coef(Ctx *c, Model &m, float fd_dt) {
         xc[x + S2D_GX] = make_float4(m.damp2a[x], (float)(dtdx * m.damp2a1[x]), m.damp2b[x], (float)(dtdx * m.damp2b1[x]));
     for (int z = 0; z < m.nnz; ++z)
         zc[z + S2D_GZ] = make_float4(m.damp1a[z], (float)(dtdz * m.damp1a1[z]), m.damp1b[z], (float)(dtdz * m.damp1b1[z]));
-    if (!m.xcoef.p) CK(m.xcoef.alloc(c->arena, sizeof(float4) * m.nxa));
-    if (!m.zcoef.p) CK(m.zcoef.alloc(c->arena, sizeof(float4) * m.ld));
+    if (!m.xcoef.p) CK(m.xcoef.alloc(c->arena, sizeof(float4) * m.nxa, Arena::kLasting));
+    if (!m.zcoef.p) CK(m.zcoef.alloc(c->arena, sizeof(float4) * m.ld, Arena::kLasting));
     CK(cudaMemcpyAsync(m.xcoef.p, xc.data(), sizeof(float4) * m.nxa, cudaMemcpyHostToDevice, c->stream));
     CK(cudaMemcpyAsync(m.zcoef.p, zc.data(), sizeof(float4) * m.ld, cudaMemcpyHostToDevice, c->stream));
     CK(cudaStreamSynchronize(c->stream));
@@ -846,8 +853,8 @@ int run_resident(Ctx *c, Batch &b, const ResPlan &pl, int slot0, int nshots, int
     std::vector<ResShot> rs;
     for (int i = 0; i < nshots; ++i) rs.push_back({slot0 + i, (i % pl.conc) * per, pl.ncx, pl.ncz});
     const size_t rbytes = sizeof(ResShot) * rs.size(), fbytes = resident_frame_bytes(pl.nw, pl.c, pl.conc * per);
-    if (c->res_shots.bytes < rbytes) CK(c->res_shots.alloc(c->arena, rbytes));
-    if (c->res_frames.bytes < fbytes) CK(c->res_frames.alloc(c->arena, fbytes));
+    if (c->res_shots.bytes < rbytes) CK(c->res_shots.alloc(c->arena, rbytes, Arena::kLasting));
+    if (c->res_frames.bytes < fbytes) CK(c->res_frames.alloc(c->arena, fbytes, Arena::kLasting));
     CK(cudaMemcpyAsync(c->res_shots.p, rs.data(), rbytes, cudaMemcpyHostToDevice, c->stream));
     ResArgs a{};
     a.shots = b.shots_d.as<ShotDev>();
@@ -1027,7 +1034,7 @@ int setup_batch(Ctx *c, const s2d_shot *shots, int nshots, const s2d_wave &wave,
     const size_t n_up = used, o_ks = place(sizeof(double) * nshots);
     for (int s = 0; s < nshots; ++s) o_amp[s] = place(sizeof(float) * (size_t)rs.fd_nt);
     pieces.push_back(used);
-    if (!c->pool.held()) c->arena.expect(pieces);
+    if (!c->pool.held()) c->arena.expect(pieces, Arena::kBatch);
     CK(b.tables.alloc(c->arena, used));
     char *const tab_d = b.tables.as<char>();
     std::vector<char> tab(n_up, 0);
@@ -1458,11 +1465,11 @@ int s2d_create(void **ctx, int device) {
     if (e == cudaSuccess) e = cudaEventCreate(&c->ev1);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&c->sm_count, cudaDevAttrMultiProcessorCount, device);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&c->cooperative, cudaDevAttrCooperativeLaunch, device);
-    if (e == cudaSuccess) e = c->dev_err.alloc(c->arena, sizeof(int));
-    if (e == cudaSuccess) e = c->queue_d.alloc(c->arena, 2 * sizeof(int));
+    if (e == cudaSuccess) e = c->dev_err.alloc(c->arena, sizeof(int), Arena::kLasting);
+    if (e == cudaSuccess) e = c->queue_d.alloc(c->arena, 2 * sizeof(int), Arena::kLasting);
     if (e == cudaSuccess) e = cudaMemset(c->queue_d.p, 0, 2 * sizeof(int));
-    if (e == cudaSuccess) e = c->bar_d.alloc(c->arena, sizeof(unsigned));
-    if (e == cudaSuccess) e = c->args_d.alloc(c->arena, sizeof(StepArgs));
+    if (e == cudaSuccess) e = c->bar_d.alloc(c->arena, sizeof(unsigned), Arena::kLasting);
+    if (e == cudaSuccess) e = c->args_d.alloc(c->arena, sizeof(StepArgs), Arena::kLasting);
     if (e == cudaSuccess) e = cudaMemset(c->dev_err.p, 0, sizeof(int));
     if (e != cudaSuccess) {
         delete c;
@@ -1518,13 +1525,13 @@ int s2d_model_create(void *ctx, int nx, int nz, float dx, float dz, int nb, cons
     if (m->nnx > 65535)
         return fail(c, S2D_ERR_ARG, "padded grid has %d columns; at most 65535 are supported", m->nnx);
     const size_t raw = (size_t)nx * nz * sizeof(float);
-    c->arena.expect({raw, raw, 3 * m->field_elems * sizeof(float), m->field_elems * sizeof(float)});
-    CK(m->vp.alloc(c->arena, raw));
-    CK(m->rho.alloc(c->arena, raw));
+    c->arena.expect({raw, raw, 3 * m->field_elems * sizeof(float), m->field_elems * sizeof(float)}, Arena::kLasting);
+    CK(m->vp.alloc(c->arena, raw, Arena::kLasting));
+    CK(m->rho.alloc(c->arena, raw, Arena::kLasting));
     const size_t fb = m->field_elems * sizeof(float);
-    CK(m->mat.alloc(c->arena, 3 * fb));
+    CK(m->mat.alloc(c->arena, 3 * fb, Arena::kLasting));
     DevBuf bue;
-    CK(bue.alloc(c->arena, fb));
+    CK(bue.alloc(c->arena, fb, Arena::kLasting));
     CK(cudaDeviceSynchronize());  // vp and rho may still be written on a stream of the caller's
     const cudaMemcpyKind kind = (flags & S2D_MODEL_DEVICE) ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
     CK(cudaMemcpyAsync(m->vp.p, vp, raw, kind, c->stream));

@@ -65,3 +65,29 @@ def test_short_memory():
     for a, b, r in zip(got, (again.grad_vp, again.grad_rho), ref):
         for v in (a, np.asarray(b)):
             assert np.linalg.norm(v.astype(np.float64) - r) <= n * steps * 2.0 ** -24 * np.linalg.norm(r)
+
+
+def test_pooled_memory_goes_back():
+    """The states of a batch of many shots, between models that stay, make room
+    for a batch of another size."""
+    import torch
+    from seis2d_b200 import Context, Shot, Wave
+    with Context(0) as c:
+        shots, wave = _job(c, 300, 20)
+        c.forward(shots, wave, kt_count=2)
+        keep = [_job(c, 1, 20)[0] for _ in range(80)]
+        vp = np.full((2400, 2400), 2000.0, np.float32)
+        m = c.model(vp, vp, H, H, NB)
+        big = [Shot(m, ((k + 1) * 300 * H, 100 * H), np.array([[(k + 1) * 300 * H, 110 * H]], np.float32)) for k in range(7)]
+        ref = c.forward(big[:1], wave)[0]
+        c.forward(shots, wave, kt_count=2)
+        torch.cuda.synchronize()
+        torch.cuda.empty_cache()
+        hog = torch.empty(torch.cuda.mem_get_info()[0] - (256 << 20), dtype=torch.uint8, device="cuda")
+        try:
+            got = c.forward(big, wave)  # 7 states of 200 MB; 2 GB in the pool
+        finally:
+            del hog
+            torch.cuda.empty_cache()
+        assert keep and np.abs(ref).max() > 0
+    np.testing.assert_array_equal(got[0], ref)
