@@ -221,8 +221,8 @@ S2D_API const char *s2d_last_error(const void *ctx);
  *   "products_variant" s2d_gradient's forward recompute that keeps the step
  *                 derivatives: 3 plain loads, 19 plain loads with the next
  *                 column prefetched (default)
- *   "adjoint_blocks" 2, 3, 4 or 12 to 15 (default 13): names earlier builds of
- *                 the 4th-order adjoint step; one build now serves them all
+ *   "adjoint_blocks" 2, 3, 4 or 12 to 15 (default 13): names of the one build
+ *                 of the 4th-order adjoint step; no effect
  *   "on_chip"     1 (default): 4th-order grids whose state fits the GPU's
  *                 registers and shared memory (up to about 1.2 M padded cells)
  *                 run all their steps in one cooperative launch per shot or

@@ -1406,7 +1406,7 @@ int s2d_set_option(void *ctx, const char *key, long value) {
     } else if (k == "adjoint_blocks") {
         if ((value < 2 || value > 4) && (value < 12 || value > 15))
             return fail(c, S2D_ERR_ARG, "adjoint_blocks must be 2, 3, 4 or 12 to 15");
-        // builds of an earlier adjoint kernel: one form serves them all now
+        // one build of the kernel serves every name
     } else if (k == "fast_rows") {
         c->opt_fast_rows = value ? 1 : 0;
     } else if (k == "on_chip") {

@@ -155,7 +155,6 @@ enum StepVariant { kVariantBulk = 0, kVariantLdg = 1, kVariantBulk128 = 2,
                    kVariantO8Products = 10 /* kVariantO8 + S2D_STEP_PRODUCTS, gradient runs */,
                    kVariantTma = 11 /* CTA of kTmaWarps consumer warps fed by a TMA producer warp */,
                    kVariantAsync = 12 /* plain-load loop fed by per-lane cp.async into a per-warp ring */,
-                   kVariantAsyncProducts = 13 /* kVariantAsync + S2D_STEP_PRODUCTS, gradient runs */,
                    kVariantLdgU4 = 14 /* kVariantLdg128 with its column loop unrolled by 4 */,
                    kVariantLdgPf = 15 /* plain loads, next column prefetched, 3 blocks per SM */,
                    kVariantLdgPf4 = 16 /* the same compiled for 4 blocks per SM */,
@@ -202,7 +201,7 @@ inline bool ts_layout(int variant) {
 }
 inline bool order8_variant(int variant) { return variant >= kVariantO8 && variant <= kVariantO8c; }
 inline bool tma_variant(int variant) { return variant == kVariantTma; }
-inline bool async_variant(int variant) { return variant == kVariantAsync || variant == kVariantAsyncProducts; }
+inline bool async_variant(int variant) { return variant == kVariantAsync; }
 // Variants that use no dynamic shared memory.
 inline bool plain_loads(int variant) {
     return variant == kVariantLdg || variant == kVariantLdgProducts || variant == kVariantLdg128 || variant == kVariantLdgU4 ||

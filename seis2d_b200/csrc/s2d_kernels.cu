@@ -1071,8 +1071,8 @@ __device__ __forceinline__ void ts2_task(const StepArgs &a, const ShotDev &S, in
 // access pattern (5.2 TB/s of the state's and materials' bytes, 450 Gcell/s on
 // 8 shots of 5120 x 5120, 275 instructions per column of 224 cell-updates); with
 // the rim tasks, whose columns cost 1.6 to 1.9 times as much, 371 Gcell/s (160
-// for the form it replaces: plain loads where they were used, step A in
-// shared-memory delay lines, 16 warps per SM).  One 3301 x 1301 shot, about one
+// with plain loads where they are used, step A in shared-memory delay lines and
+// 16 warps per SM).  One 3301 x 1301 shot, about one
 // round of tasks, is bound by a column's latency: 157 Gcell/s (102 one step
 // at a time).  Rim columns unrolled like the interior ones cost more than they
 // gained (instruction cache: 276 Gcell/s against 314 before the tasks were cut
@@ -1125,10 +1125,10 @@ __global__ void __launch_bounds__(128, 2) step_kernel_ts2(const StepArgs *__rest
 //
 // What bounds it: memory.  4 shots of 5120 x 5120: 184 Gcell/s, the state and
 // the materials read once and written once 27 bytes per cell-step, 5.0 TB/s, the
-// rate of a copy with this access pattern; before (plain loads where they were
-// used, the windows moved every column, every strip one length) 88.6.  One
-// 3301 x 1301 shot: 105 (57), 4 of 1301 x 501: 96 (57), one 701 x 401, about one
-// task per warp and bound by its latency: 25.5 (19).  2 blocks per SM and 222
+// rate of a copy with this access pattern; with plain loads where they are used,
+// windows moved every column and one length for every strip 88.6.  One 3301 x
+// 1301 shot: 105 (57 that way), 4 of 1301 x 501: 96 (57), one 701 x 401, about
+// one task per warp and bound by its latency: 25.5 (19).  2 blocks per SM and 222
 // registers; at 3 blocks (168 registers, spills) 140, 81, 69 and 22; the windows
 // in shared memory at 4 blocks 69, 50, 56 and 18.
 
@@ -1534,8 +1534,7 @@ __global__ void set_args_kernel(StepArgs v, StepArgs *dst) { *dst = v; }
 // own copy groups is the whole synchronisation.  A ghost lane's copies are
 // zero-fills that read nothing.  The arithmetic is ldg_task's: the same bits.
 
-
-template <bool PROD, bool FAST, bool XF>
+template <bool FAST, bool XF>
 __device__ __forceinline__ void async_task(const StepArgs &a, const ShotDev &S, int strip, int xa, int seg_len,
                                            int kt, int par, bool rec_step, int slot, int lane, float4 *ring) {
     const int xb = min(S.nnx, xa + seg_len);
@@ -1547,8 +1546,6 @@ __device__ __forceinline__ void async_task(const StepArgs &a, const ShotDev &S, 
     const bool rec = rec_step && slot < S.real_nt && !(a.flags & S2D_STEP_NO_RECORD) &&
                      c + S2D_STRIP_ROWS > S.rec_zlo && c <= S.rec_zhi;
     const size_t off = (size_t)(ln.z0 + S2D_GZ) + (size_t)S2D_GX * ld;
-    const size_t F = (size_t)(S.nnx + 2 * S2D_GX) * ld;
-    float *__restrict__ pr = PROD ? S.prod + (size_t)(kt - a.prod_kt0) * 4 * F + off : nullptr;
     const int fs = S.fstride;
     float *const sb = S.st[0][0] + off;
     const int ib = par * 4 * fs, ob = (par ^ 1) * 4 * fs;
@@ -1616,10 +1613,6 @@ __device__ __forceinline__ void async_task(const StepArgs &a, const ShotDev &S, 
         if (in_seg && ln.owner) {
             st4(pxo + colP, pxn);
             if (pz_live) st4(pzo + colP, pzn);
-            if (PROD) {
-                st4(pr + colP, dxv);
-                if (pz_live) st4(pr + F + colP, dzv);
-            }
         }
         if (rec && in_seg) record(ln, S, P, pn, slot);
         pq0 = pq1; pq1 = pq2; pq2 = pq3; pq3 = pn;
@@ -1632,18 +1625,13 @@ __device__ __forceinline__ void async_task(const StepArgs &a, const ShotDev &S, 
             if (ln.owner) {
                 st4(vxo + colV, vxn);
                 st4(vzo + colV, vzn);
-                if (PROD) {
-                    st4(pr + 2 * F + colV, dxp);
-                    st4(pr + 3 * F + colV, dzp);
-                }
             }
         }
     }
     cp_async_wait<0>();
 }
 
-template <bool PROD, int MINB>
-__global__ void __launch_bounds__(128, MINB) step_kernel_async(const StepArgs *__restrict__ A, int kt_off) {
+__global__ void __launch_bounds__(128, 4) step_kernel_async(const StepArgs *__restrict__ A, int kt_off) {
     extern __shared__ __align__(128) unsigned char smem[];
     float4 *ring = reinterpret_cast<float4 *>(smem + (size_t)(threadIdx.x >> 5) * kAsyncWarpBytes);
     const StepArgs a = *A;
@@ -1661,15 +1649,15 @@ __global__ void __launch_bounds__(128, MINB) step_kernel_async(const StepArgs *_
         int strip, xa, seg_len;
         const ShotDev &G = task_of(a, t, strip, xa, seg_len);
         warp_copy_shot(S, G, lane);
-        if (!task_in_bounds(a, S, strip, xa, seg_len, kt, PROD, 1)) continue;
+        if (!task_in_bounds(a, S, strip, xa, seg_len, kt, false, 1)) continue;
         const int c = strip * S2D_STRIP_OUT - 4;
         const int xb = min(S.nnx, xa + seg_len);
         const bool zf = rows_fast(S, c, c + S2D_STRIP_ROWS - 1);
         const bool xf = xa - 1 >= S.xfast_lo && xb + 1 < S.xfast_hi;
-        if (zf && xf) async_task<PROD, true, true>(a, S, strip, xa, seg_len, kt, par, rec_step, slot, lane, ring);
-        else if (zf) async_task<PROD, true, false>(a, S, strip, xa, seg_len, kt, par, rec_step, slot, lane, ring);
-        else if (xf) async_task<PROD, false, true>(a, S, strip, xa, seg_len, kt, par, rec_step, slot, lane, ring);
-        else async_task<PROD, false, false>(a, S, strip, xa, seg_len, kt, par, rec_step, slot, lane, ring);
+        if (zf && xf) async_task<true, true>(a, S, strip, xa, seg_len, kt, par, rec_step, slot, lane, ring);
+        else if (zf) async_task<true, false>(a, S, strip, xa, seg_len, kt, par, rec_step, slot, lane, ring);
+        else if (xf) async_task<false, true>(a, S, strip, xa, seg_len, kt, par, rec_step, slot, lane, ring);
+        else async_task<false, false>(a, S, strip, xa, seg_len, kt, par, rec_step, slot, lane, ring);
     }
 }
 
@@ -1992,7 +1980,7 @@ int launch_step(int variant, const StepArgs *args_dev, int kt_off, int grid, int
     else if (variant == kVariantTma)
         step_kernel_tma<false><<<grid, block, smem, (cudaStream_t)stream>>>(args_dev, kt_off);
     else if (variant == kVariantAsync)
-        step_kernel_async<false, 4><<<grid, block, smem, (cudaStream_t)stream>>>(args_dev, kt_off);
+        step_kernel_async<<<grid, block, smem, (cudaStream_t)stream>>>(args_dev, kt_off);
     else if (variant == kVariantLdgU4)
         step_kernel_ldg<false, 4, true><<<grid, block, 0, (cudaStream_t)stream>>>(args_dev, kt_off);
     else if (variant == kVariantLdgPf)
@@ -2005,8 +1993,6 @@ int launch_step(int variant, const StepArgs *args_dev, int kt_off, int grid, int
         step_kernel_ldg<false, 3, true, true><<<grid, block, 0, (cudaStream_t)stream>>>(args_dev, kt_off);
     else if (variant == kVariantLdgPfProducts)
         step_kernel_ldg<true, 3, false, true><<<grid, block, 0, (cudaStream_t)stream>>>(args_dev, kt_off);
-    else if (variant == kVariantAsyncProducts)
-        step_kernel_async<true, 3><<<grid, block, smem, (cudaStream_t)stream>>>(args_dev, kt_off);
     else
         step_kernel_ldg<false, 1><<<grid, block, 0, (cudaStream_t)stream>>>(args_dev, kt_off);
     return (int)cudaGetLastError();
@@ -2052,7 +2038,7 @@ const void *kernel_of(int variant) {
     if (order8_variant(variant)) return (const void *)step_kernel_o8<false>;
     if (variant == kVariantO8Products) return (const void *)step_kernel_o8<true>;
     if (variant == kVariantTma) return (const void *)step_kernel_tma<false>;
-    if (variant == kVariantAsync) return (const void *)step_kernel_async<false, 4>;
+    if (variant == kVariantAsync) return (const void *)step_kernel_async;
     if (variant == kVariantLdgU4) return (const void *)step_kernel_ldg<false, 4, true>;
     if (variant == kVariantLdgPf) return (const void *)step_kernel_ldg<false, 3, false, true>;
     if (variant == kVariantLdgPf4) return (const void *)step_kernel_ldg<false, 4, false, true>;
@@ -2060,7 +2046,6 @@ const void *kernel_of(int variant) {
     if (variant == kVariantLdgPfU3) return (const void *)step_kernel_ldg<false, 3, true, true>;
     if (variant == kVariantLdgPfProducts) return (const void *)step_kernel_ldg<true, 3, false, true>;
     if (variant == kVariantPersist) return (const void *)step_kernel_persist<4>;
-    if (variant == kVariantAsyncProducts) return (const void *)step_kernel_async<true, 3>;
     return (const void *)step_kernel_ldg<false, 1>;
 }
 }  // namespace

@@ -27,16 +27,18 @@
 // blocks count themselves in when they start and no neighbour is waited for
 // before all have (a wait of its own, kStartLimit).
 //
-// What bounds it: latency.  Of a step of 8 warps with 8 columns (1.9 us of
-// 4.05 at 1.965 GHz are arithmetic, the FP32 pipe busy for 1.0 of them) about
-// 0.85 us are the exchange's way from one SM to another, the rest barriers and
-// shared-memory round trips.  More warps per tile, two blocks per SM (both wait
-// at the same time), pz in shared memory and smaller frames measured no
-// better.  Against one launch per step, us per FD step: 265 x 165 cells 2.2
-// (7.5), 1080 x 1080 5.0 (12.2, 231 Gcell/s against 96), one 1301 x 501 shot
-// 3.5 (12.5).  With the gradient's products (16 bytes per cell and step, stored
-// past the caches' reuse): 8 shots of 1301 x 501 39 us per step (65 with one
-// launch of the per-step kernel for all eight), 4 of 701 x 401 9.3 (18).
+// What bounds it: latency.  Counters of 100 steps of 1080 x 1080 (8 warps with 10
+// columns on 135 SMs): 29 % of the issue slots and 20 % of the FMA pipe's cycles
+// in use, 7.1 cycles from one instruction of a warp to its next:
+// 1.6 in fixed latencies, 1.3 in the poll for the neighbours' pieces and other
+// loads, 1.0 in shared memory, 0.4 each at the barriers, in branches and for the
+// FMA pipe; L2 at 6 %, DRAM at 1 %.  More warps per tile, two blocks per SM (both
+// wait at the same time), pz in shared memory and smaller frames measured no
+// better.  us per FD step, with one launch of the two-step kernel per two steps
+// in brackets: 265 x 165 cells 2.2 (7.6), 1080 x 1080 5.3 (11.1), one 1301 x 501
+// shot 3.5 (10.6).  With the gradient's products (16 bytes per cell and step,
+// stored past the caches' reuse): 8 shots of 1301 x 501 39 us per step (65 with
+// one launch of the per-step kernel for all eight), 4 of 701 x 401 9.3 (18).
 #include <cuda_runtime.h>
 
 #include <algorithm>
