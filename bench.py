@@ -39,10 +39,11 @@ import numpy as np
 ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, ROOT)
 
-# Algorithmic bytes per padded-cell update (the library reports them per run
-# in stats.alg_bytes): 4 state fields read and written (32 B) + 3 materials
-# (12 B) = 44 B; 36 B where both pressure dampings are 1 and the cell carries
-# p = px + pz alone.
+# Algorithmic bytes per padded cell and pass over the state (the library reports
+# them per run in stats.alg_bytes): 4 state fields read and written (32 B) + 3
+# materials (12 B) = 44 B; 36 B where both pressure dampings are 1 and the cell
+# carries p = px + pz alone.  The rooflines count the materials once per launch
+# for all shots of a model (shared_bytes), as they have to cross HBM.
 
 WORKLOADS = {
     "c2": dict(nx=5000, nz=5000, d=5.0, nb=60, vp=(2000.0, 3500.0), rho=(1800.0, 2300.0), iface=2500,
@@ -227,8 +228,8 @@ def traffic_per_launch(workload, nshots, variant=None):
 
 
 def dram_minimal_bytes(w, nshots):
-    """DRAM bytes per padded-cell update if the state crosses HBM once per FD
-    step and the materials once per launch for all shots of the model:
+    """DRAM bytes per padded cell and pass over the state if the state crosses HBM once per
+    pass and the materials once per launch for all shots of the model:
     state 32 B per cell (24 B where the cell carries p alone), materials
     12 B / nshots.  Cells carry p alone where both pressure dampings are 1:
     columns and rows [nb-1, n+nb] of the padded grid."""
@@ -236,6 +237,20 @@ def dram_minimal_bytes(w, nshots):
     inner = (nnx - 2 * (nb - 1)) * (nnz - 2 * (nb - 1))
     frac = inner / (nnx * nnz)
     return 24.0 * frac + 32.0 * (1 - frac) + 12.0 / max(1, nshots)
+
+
+def shared_bytes(alg_bytes, w, nshots):
+    """The library's algorithmic bytes (materials once per shot) with the
+    materials counted once for the ``nshots`` shots that share them."""
+    return alg_bytes * dram_minimal_bytes(w, nshots) / dram_minimal_bytes(w, 1)
+
+
+def launch_record(st, steps):
+    """What ran: the per-step kernel's configuration, or the on-chip loop (far
+    fewer launches than steps; the configuration then names no kernel that ran)."""
+    if st.kernel_launches * 8 < steps:
+        return {"on_chip_loop": True, "launches": st.kernel_launches}
+    return {"variant": st.variant, "seg_len": st.seg_len, "task_order": st.task_order}
 
 
 # ---------------------------------------------------------------------------
@@ -288,7 +303,7 @@ def gradient_leg(ctx, nshots=32, T=3.0, fd_order=4):
     ms = ctx.model(start, rho, 10.0, 10.0, 50, fd_order=fd_order)
     shots = [Shot(ms, s_, rec) for s_ in src]
     fbuf = torch.zeros_like(dobs)
-    ctx.forward(shots, wave, kt_count=120, out=fbuf)  # autotunes this shape (>= 112 steps) outside the timing
+    ctx.forward(shots, wave, kt_count=120, out=fbuf)  # autotunes this shape (>= 80 steps) outside the timing
     tf, _ = _timed(lambda: ctx.forward(shots, wave, out=fbuf, sync=False))
     gvp = torch.zeros(1201, 401, dtype=torch.float32, device="cuda")
     grho = torch.zeros_like(gvp)
@@ -312,32 +327,6 @@ def gradient_leg(ctx, nshots=32, T=3.0, fd_order=4):
     return res
 
 
-def l2_copy_rate():
-    """Copy rate of an L2-resident buffer (GB/s, read + write bytes): torch's
-    copy of 48 MB into 48 MB (96 MB, inside the 126 MB L2), 20 copies
-    captured in a CUDA graph and the graph replayed 10 times, CUDA events —
-    the L2 counterpart of the measured HBM copy peak, for the grids whose
-    whole state stays in L2 (the graph keeps launch gaps out of the rate)."""
-    import torch
-    n = 12 * 1024 * 1024
-    a = torch.randn(n, device="cuda")
-    b = torch.empty_like(a)
-    s = torch.cuda.Stream()
-    s.wait_stream(torch.cuda.current_stream())
-    with torch.cuda.stream(s):
-        for _ in range(3):
-            b.copy_(a)
-    torch.cuda.current_stream().wait_stream(s)
-    g = torch.cuda.CUDAGraph()
-    with torch.cuda.graph(g):
-        for _ in range(20):
-            b.copy_(a)
-    g.replay()
-    t, _ = _timed(lambda: [g.replay() for _ in range(10)])
-    del g
-    return 2.0 * 4 * n * 200 / t / 1e9
-
-
 def extra_legs(device):
     """Rates of the other workload configurations (each a bounded part of its job)."""
     import torch
@@ -353,16 +342,16 @@ def extra_legs(device):
         st = derive_steps(wave)
         buf = torch.zeros(rec.shape[0] * st["real_nt"], dtype=torch.float32, device="cuda")
         shots = [Shot(m, src[0], rec)]
-        ctx.forward(shots, wave, kt_count=120, out=buf)  # warm-up; autotunes this shape (>= 112 steps)
+        ctx.forward(shots, wave, kt_count=120, out=buf)  # warm-up; autotunes this shape (>= 80 steps)
         t, _ = _timed(lambda: ctx.forward(shots, wave, out=buf, sync=False))
         l1 = ctx.last_stats
         cells = m.padded_cells * st["fd_nt"]
-        l2 = l2_copy_rate()
+        launch = launch_record(l1, st["fd_nt"])
         out["c1"] = {"workload": "1000x1000 two-layer, nb 40, 1 shot, full 2000 steps", "gcells_per_s": cells / t / 1e9,
-                     "shots_per_s": 1.0 / t, "job_s": t, "roofline_frac": ctx.last_stats.alg_bytes / t / 1e9 / peak,
-                     "l2_copy_gbs": l2, "roofline_frac_l2": ctx.last_stats.alg_bytes / t / 1e9 / l2,
-                     "note": "whole job ~37 MB of state: L2-resident; roofline_frac_l2 against the L2 copy rate",
-                     "launch": {"variant": l1.variant, "seg_len": l1.seg_len, "task_order": l1.task_order}}
+                     "shots_per_s": 1.0 / t, "job_s": t, "us_per_fd_step": t / st["fd_nt"] * 1e6,
+                     "roofline_frac": None if "on_chip_loop" in launch else l1.alg_bytes / t / 1e9 / peak,
+                     "note": "the on-chip loop keeps the state in registers and shared memory: no memory roofline",
+                     "launch": launch}
         m.release()
         # c3: salt 3201x1201, d 7.62, nb 50, 20 Hz, dt 0.6 ms, nt 10000, 1 shot; 1000 of the 10000 steps
         vp, rho = salt_model()
@@ -373,7 +362,7 @@ def extra_legs(device):
         rec = np.stack([np.arange(3201, dtype=np.float32) * np.float32(7.62), np.full(3201, 2 * 7.62, np.float32)], 1)
         buf = torch.zeros(3201 * st["real_nt"], dtype=torch.float32, device="cuda")
         shots = [Shot(m, src, rec)]
-        ctx.forward(shots, wave, kt_count=120, out=buf)  # warm-up; autotunes this shape (>= 112 steps)
+        ctx.forward(shots, wave, kt_count=120, out=buf)  # warm-up; autotunes this shape (>= 80 steps)
         t, _ = _timed(lambda: ctx.forward(shots, wave, kt_begin=120, kt_count=1000, out=buf, sync=False))
         cells = m.padded_cells * 1000
         rate = cells / t / 1e9
@@ -381,7 +370,7 @@ def extra_legs(device):
         l3 = ctx.last_stats
         out["c3"] = {"workload": "3201x1201 salt (seeded), d 7.62, nb 50, 1 shot, 1000 of 10000 steps",
                      "gcells_per_s": rate, "shots_per_s": rate * 1e9 / (m.padded_cells * st["fd_nt"]),
-                     "roofline_frac": frac, "launch": {"variant": l3.variant, "seg_len": l3.seg_len, "task_order": l3.task_order}}
+                     "roofline_frac": frac, "launch": launch_record(l3, 1000)}
         m.release()
         # c4: 48 shots on three layered models of uneven size, one launch sequence; 300 of 3000 steps
         wave = Wave(2.3996, 0.0008, 0.0008, 15.0)
@@ -397,11 +386,12 @@ def extra_legs(device):
             cells_step += 16 * mm.padded_cells
             total_rec += 16 * rec.shape[0]
         buf = torch.zeros(total_rec * st["real_nt"], dtype=torch.float32, device="cuda")
-        ctx.forward(shots, wave, kt_count=120, out=buf)  # warm-up; autotunes this shape (>= 112 steps)
+        ctx.forward(shots, wave, kt_count=120, out=buf)  # warm-up; autotunes this shape (>= 80 steps)
         t, _ = _timed(lambda: ctx.forward(shots, wave, kt_begin=120, kt_count=300, out=buf, sync=False))
         rate = cells_step * 300 / t / 1e9
-        frac = ctx.last_stats.alg_bytes / t / 1e9 / peak
         l4 = ctx.last_stats
+        # the large grid, nearly all of the bytes, shares its materials among 16 shots
+        frac = shared_bytes(l4.alg_bytes, {"nx": 2401, "nz": 801, "nb": 50}, 16) / t / 1e9 / peak
         ctx.forward(shots, wave, kt_count=60, out=buf, plain=True)  # warm-up of the plain launch sequence
         tp, _ = _timed(lambda: ctx.forward(shots, wave, kt_count=300, out=buf, plain=True, sync=False))
         prate = cells_step * 300 / tp / 1e9
@@ -409,7 +399,8 @@ def extra_legs(device):
                                  "one launch per step for all; 300 of 3000 steps",
                      "gcells_per_s": rate, "shots_per_s": rate * 1e9 / (cells_step / 48 * st["fd_nt"]),
                      "plain_gcells_per_s": prate, "roofline_frac": frac,
-                     "launch": {"variant": l4.variant, "seg_len": l4.seg_len, "task_order": l4.task_order}}
+                     "note": "grids that run in the on-chip loop add time and hardly any bytes to roofline_frac",
+                     "launch": launch_record(l4, 300)}
         for mm in models:
             mm.release()
         # the 8th-order operator ("Order of FD Operator" : "8") on the 5000x5000
@@ -423,14 +414,15 @@ def extra_legs(device):
             st = derive_steps(wave)
             shots = [Shot(m, s_, rec2) for s_ in src2[:16]]
             buf = torch.zeros(16 * rec2.shape[0] * st["real_nt"], dtype=torch.float32, device="cuda")
-            ctx.forward(shots, wave, kt_count=70, out=buf)  # autotunes the shape (>= 64 steps)
+            ctx.forward(shots, wave, kt_count=70, out=buf)  # autotunes the shape (>= 48 steps)
             t, _ = _timed(lambda: ctx.forward(shots, wave, kt_begin=70, kt_count=200, out=buf, sync=False))
             l8 = ctx.last_stats
             rate = 16 * m.padded_cells * 200 / t / 1e9
             out["c2_order8"] = {"workload": "5000x5000 two-layer, nb 60, 8th-order operator, 16 shots x 5000 "
                                             "receivers; 200 of 4000 steps",
-                                "gcells_per_s": rate, "roofline_frac": l8.alg_bytes / t / 1e9 / peak,
-                                "launch": {"variant": l8.variant, "seg_len": l8.seg_len, "task_order": l8.task_order}}
+                                "gcells_per_s": rate,
+                                "roofline_frac": shared_bytes(l8.alg_bytes, w2, 16) / t / 1e9 / peak,
+                                "launch": launch_record(l8, 200)}
             m.release()
             del buf
         except Exception as exc:  # a failed extra leg must not cost the main line
@@ -675,15 +667,19 @@ def main():
     ms_per_step = ms / args.steps
 
     # roofline of the step kernel over exactly the timed calls: algorithmic
-    # bytes of the launches / their device time (library events on its stream)
+    # bytes of the launches (materials once per launch) / their device time
+    # (library events on its stream)
+    alg_bytes = shared_bytes(alg_bytes, w, nshots)
     peak, peak_kind = measured_peak()
     achieved = alg_bytes / (loop_ms * 1e-3) / 1e9
-    tr = traffic_per_launch(args.workload, nshots, next(iter(variants)) if len(variants) == 1 else None)
+    # (a record per step kernel: the two-step kernel's under a name of its own)
+    tr = traffic_per_launch(args.workload + (" two steps" if variants == {5} else ""), nshots,
+                            next(iter(variants)) if len(variants) == 1 else None)
     roof = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
             "traffic": tr["bytes"] if tr else None, "traffic_source": tr["source"] if tr else None,
             "peak_source": peak_kind, "bytes_per_launch": alg_bytes / max(1, fd_launches),
             "bytes_per_cell_update": alg_bytes / (cells_step * chunk * args.steps),
-            "dram_minimal_bytes_per_cell_update": dram_minimal_bytes(w, nshots),
+            "bytes_per_cell_and_pass": dram_minimal_bytes(w, nshots),
             "launch_ms": loop_ms / max(1, fd_launches), "launches": fd_launches,
             "fd_steps_per_launch": 2 if variants == {5} else 1,
             "timed_region": f"the {args.steps} timed calls ({fd_launches} step launches)"}
