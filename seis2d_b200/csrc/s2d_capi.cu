@@ -413,7 +413,9 @@ constexpr SplitRule kSplitAdj8 = {S2D_TS_OUT, 8, 0, kAdj8ColLo, kAdj8ColHi, 13, 
 // several rounds, whose warps even out: measured about 1.0 us per column of the
 // two-step kernel against 0.61.  2101 x 1101, 3 shots: one round of 79 columns
 // 155 Gcell/s, two of 35 178; 3301 x 1301, 6 shots: 195 and 258 (63); 1301 x
-// 501, 8 shots, the other way: 119 and 105.  Returns that estimate, in columns
+// 501, 8 shots, the other way: 119 and 105.  A few tasks past one round cost some
+// warps a second one, 2.5 of the shortest at least: 8th-order step of one 2000 x
+// 300 shot, 1298 tasks of 7 columns 20.4 us, 1154 of 15 15.6.  Returns that estimate, in columns
 // of an interior task (0 with a forced length).
 double split_group(GroupDev &g, const ShotDev &d, int shots, double resident_warps, bool alone, int forced,
                  const SplitRule &R) {
@@ -455,8 +457,11 @@ double split_group(GroupDev &g, const ShotDev &d, int shots, double resident_war
         const double ti = L + kHalo, tz = (g.seg_z + kHalo) * kRows, tx = (g.seg_x + kHalo) * kCols;
         const double work = shots * (ni * (g.nsegs * ti + (g.nseg_l + g.nseg_r) * tx) + nz * g.nseg_z * tz);
         const double longest = std::max(ni && g.nsegs ? ti : 0.0, std::max(nz ? tz : 0.0, ni ? tx : 0.0));
+        const double shortest = std::min(ni && g.nsegs ? ti : longest, std::min(nz ? tz : longest, ni ? tx : longest));
         const double tasks = (double)shots * shot_tasks(g);
-        const double cost = std::max(longest, alone && tasks <= resident_warps ? 1.5 * longest : work / resident_warps + ti);
+        const double cost = alone && tasks <= resident_warps
+                                ? 1.5 * longest
+                                : std::max({longest, work / resident_warps + ti, alone ? 2.5 * shortest : 0.0});
         if (!best || cost < best_cost) {
             best = L;
             best_cost = cost;
